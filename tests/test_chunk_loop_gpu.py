@@ -93,3 +93,20 @@ def test_loop_kernel_other_shapes_against_oracle(oracle):
     w, d = _with_loop("1", lambda: run_case(oracle, 74, n_obs=1, P=30, pos_base=27, pad=(20, 29), model=1, L=4, H=192, n_q=6, n_kv=2,
                                            hd=64, inter=384, chunk=10, A=32, sd=32, T=2, self_every=2))
     assert w < 1e-2 and d < 3e-2, (w, d)
+
+
+@pytest.mark.parametrize("kw", [
+    # a CTA's share of the keys does not fit at once: several key blocks with a running maximum
+    dict(P=2100, model=0, L=2, H=256, n_q=8, n_kv=1, hd=256, inter=512, chunk=50, A=32, sd=32, T=2),
+    # 64 suffix rows, pi0's widths: the longest A tile, staged sums behind it
+    dict(P=24, model=0, L=1, H=1024, n_q=8, n_kv=1, hd=256, inter=4096, chunk=63, A=32, sd=32, T=1),
+    # widths that are no multiple of 64 columns or of the CTA groups, CTAs without keys, one action token
+    dict(P=3, pos_base=3, model=1, L=3, H=208, n_q=5, n_kv=5, hd=64, inter=336, chunk=1, A=16, sd=32, T=2, self_every=2),
+    # more attention units than CTA groups of two
+    dict(P=70, pos_base=70, model=1, L=2, H=320, n_q=32, n_kv=32, hd=64, inter=640, chunk=50, A=48, sd=32, T=1, self_every=2),
+], ids=["key_blocks", "rows64", "ragged", "many_units"])
+def test_loop_kernel_work_split_edges(oracle, kw):
+    from tests.test_engine_gpu import run_case
+
+    w, d = _with_loop("1", lambda: run_case(oracle, 81, n_obs=1, **kw))
+    assert w < 1e-2 and d < 3e-2, (w, d)

@@ -2,37 +2,40 @@
 //
 // With a single observation the suffix is 50 / 51 rows: every product of the loop streams its weights once and does
 // almost no arithmetic, and a launch per operator spends most of its time between kernels (about 1,600 launches per
-// chunk for a pi0-shaped expert).  Here one persistent cooperative kernel (one CTA of 256 threads per SM) walks a
-// table of PHASES -- the operators of one Euler step, src/models/pi0.cpp:570-588, src/models/smolvla.cpp:1393-1418 --
-// and separates them with a grid-wide barrier (one atomic arrival + a bounded acquire spin per CTA).  Per layer:
-// q|k|v, attention, key-slice merge, Wo + residual, gate/up, Wdown + residual = six phases.
+// chunk for a pi0-shaped expert).  Here one persistent cooperative kernel (clusters of eight CTAs, one CTA of 256 + 32
+// threads per SM) walks a table of PHASES -- the operators of one Euler step, src/models/pi0.cpp:570-588,
+// src/models/smolvla.cpp:1393-1418 -- and separates them with a grid-wide barrier (one atomic arrival + a bounded acquire
+// spin per CTA).  Per layer: q|k|v, attention, Wo + residual, gate/up, Wdown + residual = five phases.
 //
 // Phase kinds
-//   GEMM     C[M <= 64][N] = A[M][K] W[N][K]^T.  A unit is NG (2 or 4) groups of 8 output columns; units are dealt to
-//            the CTAs in contiguous ranges.  A unit's weights arrive as K chunks of 2048 / NG columns, one
-//            cp.async.bulk per chunk, in a 3-stage ring that is fed by one thread from a cursor that runs AHEAD of the
-//            computation, across phase boundaries and barriers (weights do not depend on anything the loop computes),
-//            so HBM streams while the CTAs wait for each other.  A is brought in K slices of at most 1024 columns (all
-//            M rows, one bulk copy); a product with a longer K (Wo, Wdown) walks its slices one after the other and
-//            keeps accumulating in registers, so its residual update needs no second pass over partial sums.  The 8
-//            warps are 2 row halves x 4 K quarters of mma.sync m16n8k16 with ldmatrix operands; the quarters are added
-//            through shared memory in a fixed order by all threads (one row, 4 adjacent columns each).  Epilogues:
-//            residual += projection with the bf16 mirror and per-unit sums of squares (the consumer's RMS factor),
-//            act(gate) * up, RMS factor + NeoX rotation + append of q|k|v, bias + activation, and the Euler update.
-//            A bulk copy costs the issuing thread 40-60 ns whatever its size (measured: 51 row copies of 2 KB took
-//            3 us, 192 of 512 B 7.8 us), so every operand tile has to be ONE contiguous range: all bf16 matrices the
-//            loop reads (weights, activations, q, K/V pages) live in PADDED images -- [K slice][row][slice columns + 8]
-//            -- whose rows are 16 bytes apart modulo 128, which is also what makes the ldmatrix reads conflict-free.
-//   ATT      (kv head, 32 stacked query rows, key slice) units: S = Q K^T and P V by mma.sync on tiles staged by three
-//            bulk copies; un-normalised O rows, maximum and row sum per unit.      COMBINE merges the key slices.
+//   GEMM     C[M <= 64][N] = A[M][K] W[N][K]^T on the tensor cores with the operands SWAPPED: 128 weight rows are tcgen05's M, the
+//            tokens its N = 64 columns, so a tile of the accumulator is [weight row = TMEM lane][token].  Groups of kd = 1, 2, 4
+//            or 8 CTAs of one cluster share a contiguous range of 8-column groups; each CTA multiplies ITS 1 / kd of K and sends
+//            every column's partial sums to the CTA of the group that owns the column (one bulk copy into its shared memory per
+//            destination, counted on an mbarrier there), which adds the kd parts in a fixed order and runs the epilogue: residual +=
+//            projection with the bf16 mirror and sums of squares (the consumer's RMS factor), act(gate) * up, RMS factor + NeoX
+//            rotation + append of q|k|v, bias + activation, the Euler update.  A CTA so reads M x K / kd of the activations
+//            instead of all of them: without the split the 148 copies of A alone were 2 us of L2 traffic per phase (4 x that
+//            for Wdown), and Wo / Wdown kept 64 of 148 SMs busy.  kd is chosen per product by choose_kd.
+//            Weights and activations lie as tcgen05 reads them (K-major, SWIZZLE_128B blocks of 64 columns), weights as
+//            [CTA group][pass][64-column block][row], so that any range of blocks is one contiguous cp.async.bulk (a bulk copy costs
+//            its issuing thread 40-60 ns whatever its size; 51 row copies of 2 KB took 3 us).  They arrive in a ring that one
+//            thread feeds from a cursor which runs AHEAD of the computation, across phase boundaries and barriers (weights do
+//            not depend on anything the loop computes), so HBM streams while the CTAs wait for each other; another thread
+//            issues the products as soon as the A tile and the next ring stage have landed.  Products of 64 columns that
+//            accumulate into ONE place follow each other at 130 clocks (each waits for the sums of the one before); dealt to
+//            four accumulators, added when they are read, they do not.
+//            (mma.sync on the same tiles ran at 410 - 460 multiply-adds per clock and SM, a ninth of tcgen05's rate: 2840
+//            clocks for Wo's 64 x 72 x 256, 5755 for Wdown's.)
+//   ATT      units of (kv head, 32 stacked query rows), a group of CTAs each, the keys split between its CTAs: S = Q K^T and P V
+//            by mma.sync on tiles staged by bulk copies, several key blocks with a running maximum where a CTA's keys do not fit
+//            at once; un-normalised O rows, maximum and row sum go to the CTA of the group that merges the row.
 //   EMBED    action-in projection (+ pi0's state token) on CUDA cores.
-// Everything one CTA writes for another goes through L2 (st / ld .cg, bulk copies), never through L1.  Phase
-// descriptors are fetched one phase ahead into shared memory (cp.async), the weight cursor's table sits there too.
+// Everything one CTA writes for another outside its cluster goes through L2 (st / ld .cg, bulk copies), never through L1.  Phase
+// descriptors are fetched one phase ahead into shared memory (cp.async), the weight feeder's table sits there too.
 // Results do not depend on the run: every sum has a fixed order.
-// The tensor-core path of the large-batch kernels (tcgen05 + TMEM) costs an allocation, a commit and a TMEM read per
-// tile, which is what a 51-row problem cannot amortise; mma.sync with register accumulators has no such fixed cost.
-// What bounds a phase here is a chain of L2 round trips (barrier arrival + poll, A tile, rms partials, residual
-// read-modify-write, store drain), about 0.7 us each, not the tensor pipe and not HBM.
+// What bounds a phase here is a chain of round trips (barrier arrival + poll, A tile, products, exchange, store drain),
+// not the tensor pipe and not HBM.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -50,57 +53,56 @@
 namespace vb {
 namespace {
 
-enum { PH_GEMM = 0, PH_ATT = 2, PH_COMBINE = 3, PH_EMBED = 4 };
+enum { PH_GEMM = 0, PH_ATT = 2, PH_EMBED = 4 };
 enum { OUT_RESID = 0, OUT_GATED = 1, OUT_QKV = 2, OUT_BIAS_ACT = 3, OUT_EULER = 4 };
-enum { RMS_NONE = 0, RMS_PARTS = 1, RMS_LOCAL = 2 };  // use_rms: row sums of squares from the producer's per-sub-unit partials, or from the A tile
 
 constexpr int CL_THREADS = 256;   // the eight computing warps
-constexpr int CL_BLOCK = 288;     // + one warp whose lane 0 feeds the weight ring
-constexpr int CL_STAGES = 3;
-constexpr int CL_MAX_KSLICE = 1024;                               // columns of one K slice
-constexpr int CL_STAGE_BYTES = 16 * (CL_MAX_KSLICE * 2 + 16);     // 16 padded weight rows of at most 1024 columns
+constexpr int CL_BLOCK = 320;     // + one warp whose lane 0 feeds the weight ring, one whose lane 0 issues the products
+constexpr int CL_CLUSTER = 8;     // CTAs per cluster (the portable maximum)
+constexpr int CL_STAGES = 4;
+constexpr int CL_STAGE_BYTES = 22528;                             // 22 tiles (8 columns x 64 K) of 1 KB
+constexpr int CL_PASS_N8 = 22;                                    // 8-column groups a CTA group works on at once: 176 weight rows, two tiles of 128
+constexpr int CL_PASSES = 2;                                      // at most two passes per group: the exchange has a buffer for each
+constexpr int CL_ACC = 4;                                         // accumulators per tile: consecutive products go to different ones
+constexpr int CL_TMEM_COLS = 2 * CL_ACC * 64;                     // [tile][accumulator] of 64 columns
 constexpr int CL_DESC_BYTES = 352;                                // one phase descriptor slot (two of them: this phase, the next)
 constexpr int CL_DESC_OFF = 1536;
-constexpr int CL_WTAB_OFF = 2304;                                 // weight cursor table: one 32-byte entry per GEMM phase of a step
+constexpr int CL_WTAB_OFF = 2304;                                 // weight feeder table: one 32-byte entry per GEMM phase of a step
 constexpr int CL_WTAB_MAX = 104;
-constexpr int CL_HEADER = 5632;                                   // barriers, abort flag, small float arrays, descriptors, cursor table
+constexpr int CL_HEADER = 6144;                                   // barriers, abort flag, small float arrays, descriptors, feeder table
 constexpr int CL_RING_OFF = CL_HEADER;
 constexpr int CL_ARENA_OFF = CL_RING_OFF + CL_STAGES * CL_STAGE_BYTES;
 constexpr int CL_SMEM = 232448;
 constexpr int CL_ARENA = CL_SMEM - CL_ARENA_OFF;
-constexpr int CL_SC_LD = 20;                                      // floats per scratch row (16 columns + 4: conflict-free float2 writes)
-constexpr int CL_SC_ROW = CL_SC_LD * 4;                           // bytes; the scratch tile holds the four K quarters of M x 16 sums
 constexpr int CL_EMBED_ROWS = 10;
 constexpr int CL_DEV_TIMEOUT = 105;
 
-// A bf16 matrix [rows][cols] as a padded image: K slices of `kslice` columns, each a block of `rows` rows of
-// kslice * 2 + 16 bytes.  Element (row, col) sits at this byte offset.
-__host__ __device__ __forceinline__ size_t pad_off(int rows, int kslice, int row, int col) {
-    const int s = col / kslice, c = col - s * kslice;
-    return ((size_t)s * rows + row) * ((size_t)kslice * 2 + 16) + (size_t)c * 2;
+// A bf16 matrix [rows][cols] as tcgen05 reads it: blocks of 64 columns, each rows8 rows (rows rounded up to 8) of 128 bytes whose
+// 16-byte chunks are permuted by the row (SWIZZLE_128B).  Element (row, col) sits at this byte offset.
+__host__ __device__ __forceinline__ uint32_t sw_off(int rows8, int row, int col) {
+    return (uint32_t)((col >> 6) * rows8 + row) * 128u + (uint32_t)((((col >> 3) & 7) ^ (row & 7)) << 4) + (uint32_t)(col & 7) * 2u;
 }
 
 struct alignas(16) LoopPhase {
     int type, out_mode, act, use_rms;
-    int M, N, K, kslices, n_sub, half;  // half > 0: q|k|v pairing distance (head_dim / 2)
-    int row_off, hd, out_rows, out_kslice;
-    int ng, kchunk;                     // GEMM: 8-column groups per unit (2 / 4 / 8; n_sub counts units), columns per weight chunk
+    int M, N8, K, kd;                   // N8: 8-column groups; kd: CTAs that share a product's K / an attention unit's keys
+    int half, ssq_n, row_off, out_rows8;  // half = head_dim / 2 (q|k|v)
     float eps, scale_log2, dt;
     int bias_step_stride;
-    const uint8_t *Ap, *Wp;             // padded images of A ([M][K]) and W ([N][K]), both cut into `kslices` slices
+    const uint8_t *Ap, *Wp;             // images of A ([M][K]) and W ([N][K])
     float *out_f32, *h, *x;
-    float *ssq_out;                     // [n_sub][64]: sum of squares of the bf16 values this phase writes, per sub-unit and row (optional)
-    const float *ssq_in;                // RMS_PARTS: the producer's partials, ssq_n of them per row
-    long long ssq_n;
+    float *ssq_out;                     // [N8][64]: sum of squares of the bf16 values this phase writes, per 8-column group and row (optional)
+    const float *ssq_in;                // use_rms: the producer's partials, ssq_n of them per row
     // pi0.5 (adaptive RMSNorm, gated residuals): per-step vectors, element stride mod_stride between steps
     const float *colscale;              // OUT_RESID: gate on the projection before it is added
     const float *scale_next;            // OUT_RESID / EMBED: the mirror is written as bf16(h * (1 + scale_next[col])) for the norm that reads it
     long long mod_stride;
-    uint8_t *outp;                      // padded image the phase writes (out_rows rows, slices of out_kslice columns)
-    uint8_t *hbp, *qp, *kpp, *vpp;      // padded: residual mirror [S][H], q [n_q S][hd], this layer's K / V pages [n_kv cap][hd]
+    uint8_t *outp;                      // image the phase writes
+    uint8_t *hbp;                       // EMBED: image of the residual mirror [S][H]
+    uint8_t *qp, *kpp, *vpp;            // padded rows of hd * 2 + 16 bytes: q [n_q S][hd], this layer's K / V pages [n_kv cap][hd]
     const float *bias, *rope;
-    int n_q, n_kvp, n_kv, g, S, R, n_rt, ns, ks, kv_len, P, mask_mode, cap, chunk, A_dim, sd, H;
-    float *ws_o, *ws_ml;
+    int n_q, n_kvp, n_kv, g, S, R, n_rt, per, ks, kv_len, P, mask_mode, cap, chunk, A_dim, sd, H;
+    int k_off, p_off, stage_off, recv_off, early_k, early_v;  // ATT: K, probabilities, staged and received rows in the arena; may K / V be copied before the barrier
     const __nv_bfloat16 *w_dense, *w2;  // EMBED: W_ain [H][A], W_sp [H][sd] (plain row-major)
     const float *b2;                    // EMBED: b_sp
 };
@@ -108,7 +110,7 @@ struct alignas(16) LoopPhase {
 struct LoopParams {
     const LoopPhase *phases;
     const void *wtab;  // WEntry per GEMM phase of a step, in phase order
-    int n_phases, steps, n_wtab;
+    int n_phases, steps, n_wtab, att_cta;  // att_cta: CTAs per attention unit
     unsigned *counter;
     int *status;
     const float *state;
@@ -120,6 +122,7 @@ struct LoopParams {
     size_t src_layer_stride;  // elements
     int L, n_kv, cap, P, hd;
 };
+
 
 // ------------------------------------------------------------------------------------------ device helpers
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
@@ -164,69 +167,99 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 
+// what other CTAs wrote with ordinary stores (seen through the grid barrier) -> the bulk copies this thread issues next
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-struct WEntry {  // what the weight cursor needs to know about one GEMM phase
-    const uint8_t *Wp;   // padded image cut into chunks of kchunk columns
-    int n_units, n_chunks, N, half;
-    uint32_t stride;     // kchunk * 2 + 16
-    int ng;
+// Distributed shared memory: the address of the same variable in another CTA of the cluster, a bulk copy into it that counts its
+// bytes on an mbarrier there, an arrival on an mbarrier there.  (Plain stores of 16 bytes a lane followed by a release arrival,
+// or st.async, took 3100 clocks for the 18 KB a CTA sends after q|k|v.)
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void bulk_s2rank(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void arrive_rank(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+struct WEntry {  // what the weight feeder and the product issuer need to know about one GEMM phase
+    const uint8_t *Wp;
+    int N8, K, kd, M, unused[2];
 };
 static_assert(sizeof(LoopPhase) <= CL_DESC_BYTES && sizeof(LoopPhase) % 16 == 0, "descriptor slot");
-static_assert(sizeof(WEntry) == 32, "cursor table entry");
+static_assert(sizeof(WEntry) == 32, "feeder table entry");
 
 // barrier of the computing warps (the feeder warp is not part of it)
 __device__ __forceinline__ void cons_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 struct Smem {
-    uint64_t *full, *a_full, *empty, *done;
+    uint64_t *full, *empty, *a_full, *acc_full, *acc_free, *k_full, *v_full, *x_full, *xa_full, *rdy, *done;
     const WEntry *wtab;
     int n_wtab;
     volatile int *abort_flag;
-    float *rms, *red_max, *red_sum;
+    volatile unsigned *issued, *consumed;
+    uint32_t *tmem_slot;
+    float *row_m, *red, *red_max, *red_sum;
     uint8_t *ring, *arena;
 };
 
 // The carve-up of the dynamic shared memory; every phase function rebuilds it from the base (a few constant offsets) instead
 // of taking it by reference, which would put it into local memory.
 __device__ __forceinline__ Smem get_smem() {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem sm;
-    sm.full = reinterpret_cast<uint64_t *>(smem_raw);          // [CL_STAGES]
-    sm.a_full = sm.full + CL_STAGES;                          // [2]
-    sm.empty = sm.a_full + 2;                                 // [CL_STAGES]
-    sm.done = sm.empty + CL_STAGES;
-    sm.abort_flag = reinterpret_cast<volatile int *>(smem_raw + 120);
-    sm.n_wtab = *reinterpret_cast<const int *>(smem_raw + 124);
-    sm.rms = reinterpret_cast<float *>(smem_raw + 128);
-    sm.red_max = reinterpret_cast<float *>(smem_raw + 512);
-    sm.red_sum = reinterpret_cast<float *>(smem_raw + 1024);
+    sm.full = reinterpret_cast<uint64_t *>(smem_raw);  // [CL_STAGES]
+    sm.empty = sm.full + CL_STAGES;                    // [CL_STAGES]
+    sm.a_full = sm.empty + CL_STAGES;                  // a product's A tile has landed
+    sm.acc_full = sm.a_full + 1;                       // its accumulators are complete
+    sm.acc_free = sm.acc_full + 1;                     // they have been read
+    sm.k_full = sm.acc_free + 1;                       // attention: Q and K, V
+    sm.v_full = sm.k_full + 1;
+    sm.x_full = sm.v_full + 1;                         // [CL_PASSES]: the group's partial sums have arrived
+    sm.xa_full = sm.x_full + CL_PASSES;                // attention: its rows have
+    sm.rdy = sm.xa_full + 1;
+    sm.done = sm.rdy + 1;
+    sm.abort_flag = reinterpret_cast<volatile int *>(smem_raw + 224);
+    sm.n_wtab = *reinterpret_cast<const int *>(smem_raw + 228);
+    sm.issued = reinterpret_cast<volatile unsigned *>(smem_raw + 232);
+    sm.consumed = reinterpret_cast<volatile unsigned *>(smem_raw + 236);
+    sm.tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + 240);
+    sm.row_m = reinterpret_cast<float *>(smem_raw + 256);     // [32]
+    sm.red = reinterpret_cast<float *>(smem_raw + 512);       // GEMM: [4][64] partial sums of squares; attention: [32][4] maxima, sums
+    sm.red_max = sm.red;
+    sm.red_sum = sm.red + 128;
     sm.wtab = reinterpret_cast<const WEntry *>(smem_raw + CL_WTAB_OFF);
     sm.ring = smem_raw + CL_RING_OFF;
     sm.arena = smem_raw + CL_ARENA_OFF;
     return sm;
 }
 
-// Sub-units of a phase dealt to this CTA: ids [b, e) with id = unit * chunks + chunk: the range is cut between units.
-__device__ __forceinline__ void sub_range(int n_chunks, int n_units, int &b, int &e) {
-    b = (int)((unsigned)n_units * blockIdx.x / gridDim.x) * n_chunks;
-    e = (int)((unsigned)n_units * (blockIdx.x + 1) / gridDim.x) * n_chunks;
+// The computing warps' barrier parities, one bit each, carried from phase to phase.
+constexpr unsigned PAR_K = 0, PAR_V = 1, PAR_RDY = 2, PAR_XA = 3, PAR_ACC = 4, PAR_X = 5 /* + pass */;
+__device__ __forceinline__ uint32_t par_bit(unsigned par, unsigned which) { return (par >> which) & 1u; }
+
+// This CTA's part of a product: its group's 8-column groups [j0, j0 + w8) and the 64-column blocks [kb0, kb1) of K it multiplies.
+struct GemmPart {
+    int kr, j0, w8, kb0, kb1;
+};
+__device__ __forceinline__ GemmPart gemm_part(int N8, int K, int kd) {
+    const int sh = 31 - __clz(kd), G = gridDim.x >> sh, grp = blockIdx.x >> sh, kb = (K + 63) >> 6;
+    GemmPart r;
+    r.kr = blockIdx.x & (kd - 1);
+    r.j0 = (int)((unsigned)(N8 * grp) / (unsigned)G);
+    r.w8 = (int)((unsigned)(N8 * (grp + 1)) / (unsigned)G) - r.j0;
+    r.kb0 = kb * r.kr >> sh;
+    r.kb1 = kb * (r.kr + 1) >> sh;
+    return r;
 }
 
-// weight rows of the 16-column block `sub16`: two groups of 8 rows
-__device__ __forceinline__ void sub_rows(int half, int sub16, int &r0, int &r1) {
-    if (half > 0) {
-        const int per = half >> 3, hh = sub16 / per, j = sub16 - hh * per;
-        r0 = hh * 2 * half + 8 * j;
-        r1 = r0 + half;
-    } else {
-        r0 = 16 * sub16;
-        r1 = r0 + 8;
-    }
-}
-
-// The feeder: one thread walks the GEMM phases of every step in order and copies each (unit, chunk) of this CTA into the
-// next ring stage as soon as the eight computing warps have released it.  It runs ahead of the computation by the depth
-// of the ring, across phase boundaries and grid barriers.
+// The feeder: one thread walks the GEMM phases of every step in order and copies each weight chunk of this CTA into the next
+// ring stage as soon as the products of its last content are done.  It runs ahead of the computation by the depth of the ring,
+// across phase boundaries and grid barriers.
 __device__ __noinline__ void feeder_loop(const LoopParams &lp) {
     const Smem sm = get_smem();
     const WaitCtx wc{sm.abort_flag, lp.status};
@@ -235,322 +268,385 @@ __device__ __noinline__ void feeder_loop(const LoopParams &lp) {
     for (int step = 0; ok && step < lp.steps; ++step)
         for (int gi = 0; ok && gi < sm.n_wtab; ++gi) {
             const WEntry w = sm.wtab[gi];
-            int id0, id1;
-            sub_range(w.n_chunks, w.n_units, id0, id1);
-            for (int id = id0; id < id1; ++id, ++issued) {
-                const int u = id / w.n_chunks, c = id - u * w.n_chunks;
-                const unsigned stage = issued % CL_STAGES;
-                if (issued >= CL_STAGES && !mbar_wait_backoff(&sm.empty[stage], ((issued / CL_STAGES) - 1u) & 1u, wc, CL_DEV_TIMEOUT, 20)) {
-                    ok = false;
-                    break;
-                }
-                uint64_t *bar = &sm.full[stage];
-                uint8_t *dst = sm.ring + (size_t)stage * CL_STAGE_BYTES;
-                const uint8_t *src = w.Wp + (size_t)c * w.N * w.stride;
-                mbar_expect_tx(bar, 16u * w.stride);
-                if (w.half > 0) {
-                    int r0, r1;
-                    sub_rows(w.half, u, r0, r1);
-                    bulk_g2s(dst, src + (size_t)r0 * w.stride, 8u * w.stride, bar);
-                    bulk_g2s(dst + 8u * w.stride, src + (size_t)r1 * w.stride, 8u * w.stride, bar);
-                } else {
-                    bulk_g2s(dst, src + (size_t)u * 16u * w.stride, 16u * w.stride, bar);
+            const GemmPart gp = gemm_part(w.N8, w.K, w.kd);
+            const int kb = (w.K + 63) >> 6;
+            for (int p0 = 0; ok && p0 < gp.w8; p0 += CL_PASS_N8) {
+                const int w8p = min(CL_PASS_N8, gp.w8 - p0), kc = CL_STAGE_BYTES / (w8p * 1024);
+                const uint8_t *src = w.Wp + (size_t)(gp.j0 + p0) * kb * 1024;
+                for (int k0 = gp.kb0; k0 < gp.kb1; k0 += kc, ++issued) {
+                    const unsigned stage = issued % CL_STAGES;
+                    if (issued >= CL_STAGES && !mbar_wait_backoff(&sm.empty[stage], ((issued / CL_STAGES) - 1u) & 1u, wc, CL_DEV_TIMEOUT, 20)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t bytes = (uint32_t)(min(kc, gp.kb1 - k0) * w8p) * 1024u;
+                    mbar_expect_tx(&sm.full[stage], bytes);
+                    bulk_g2s(sm.ring + (size_t)stage * CL_STAGE_BYTES, src + (size_t)k0 * w8p * 1024, bytes, &sm.full[stage]);
                 }
             }
         }
-    *reinterpret_cast<volatile unsigned *>(reinterpret_cast<uint8_t *>(sm.full) + 384) = issued;
+    *sm.issued = issued;
     mbar_arrive(sm.done);
 }
 
-// Grid-wide barrier: every CTA arrives once; `target` counts arrivals since the launch.
-__device__ __forceinline__ bool grid_barrier(const LoopParams &lp, unsigned target, const Smem &sm, const WaitCtx &wc) {
-    cons_sync();
-    if (threadIdx.x == 0 && !*sm.abort_flag) {
-        __threadfence();
-        atomicAdd(lp.counter, 1u);
-        const long long t0 = clock64();
-        for (uint32_t it = 0;; ++it) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(lp.counter) : "memory");
-            if (v >= target) break;
-            if ((it & 255u) == 255u) {
-                int st;
-                asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(st) : "l"(lp.status) : "memory");
-                if (st != 0 || clock64() - t0 > wc.budget) {
-                    atomicCAS(lp.status, 0, CL_DEV_TIMEOUT);
-                    *sm.abort_flag = 1;
-                    break;
+// The issuer: one thread walks the same list and issues the products of a chunk as soon as it and the phase's A tile have landed
+// (A is copied after the grid barrier before the phase, so the accumulator of the phase before has been read by then).
+__device__ __noinline__ void issuer_loop(const LoopParams &lp, uint32_t tmem) {
+    const Smem sm = get_smem();
+    const WaitCtx wc{sm.abort_flag, lp.status};
+    unsigned cons = 0, a_cnt = 0, acc_cnt = 0;
+    bool ok = true;
+    const uint64_t a_desc0 = smem_desc_sw128(smem_u32(sm.ring), 16, 1024), b_desc0 = smem_desc_sw128(smem_u32(sm.arena), 16, 1024);
+    for (int step = 0; ok && step < lp.steps; ++step)
+        for (int gi = 0; ok && gi < sm.n_wtab; ++gi) {
+            const WEntry w = sm.wtab[gi];
+            const GemmPart gp = gemm_part(w.N8, w.K, w.kd);
+            if (gp.w8 <= 0 || gp.kb0 >= gp.kb1) continue;
+            const uint32_t idesc = make_idesc(1, 1, 1, 0, 0, 128, (w.M + 15) & ~15);
+            const uint32_t b_blk = (uint32_t)((w.M + 7) & ~7) * 8u;  // one 64-column block of A, in descriptor units of 16 bytes
+            ok = mbar_wait(sm.a_full, a_cnt & 1u, wc, CL_DEV_TIMEOUT);
+            ++a_cnt;
+            tc_fence_after();
+            for (int p0 = 0; ok && p0 < gp.w8; p0 += CL_PASS_N8, ++acc_cnt) {
+                const int w8p = min(CL_PASS_N8, gp.w8 - p0), kc = CL_STAGE_BYTES / (w8p * 1024);
+                if (p0 > 0) {  // (before a phase's first pass the grid barrier has seen to it)
+                    ok = mbar_wait(sm.acc_free, (acc_cnt & 1u) ^ 1u, wc, CL_DEV_TIMEOUT);
+                    tc_fence_after();
                 }
+                for (int k0 = gp.kb0; k0 < gp.kb1; k0 += kc, ++cons) {
+                    const unsigned stage = cons % CL_STAGES;
+                    ok = mbar_wait(&sm.full[stage], (cons / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const int nk = min(kc, gp.kb1 - k0);
+                    for (int kk = 0; kk < nk; ++kk) {
+                        const uint64_t a = a_desc0 + (uint64_t)(stage * (CL_STAGE_BYTES / 16) + (unsigned)(kk * w8p) * 64u);
+                        const uint64_t b = b_desc0 + (uint64_t)((uint32_t)(k0 + kk - gp.kb0) * b_blk);
+                        const uint32_t acc = k0 + kk > gp.kb0 ? 1u : 0u;
+                        if (w8p > 16) {
+#pragma unroll
+                            for (int k = 0; k < CL_ACC; ++k) {
+                                mma_f16(tmem + k * 64u, a + 2 * k, b + 2 * k, idesc, acc);
+                                mma_f16(tmem + (CL_ACC + k) * 64u, a + 1024 + 2 * k, b + 2 * k, idesc, acc);
+                            }
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < CL_ACC; ++k) mma_f16(tmem + k * 64u, a + 2 * k, b + 2 * k, idesc, acc);
+                        }
+                    }
+                    tc_commit(&sm.empty[stage]);
+                }
+                if (ok) tc_commit(sm.acc_full);
+            }
+        }
+    *sm.consumed = cons;
+    mbar_arrive(sm.done);
+}
+
+// Grid-wide barrier in two halves, so that what a phase can prepare without the phase before is done between them.
+__device__ __forceinline__ void grid_arrive(const LoopParams &lp) {
+    cons_sync();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(lp.counter) : "memory");
+}
+// thread 0 only: `target` counts arrivals since the launch
+__device__ __forceinline__ bool grid_poll(const LoopParams &lp, unsigned target, const Smem &sm) {
+    const long long t0 = clock64();
+    for (uint32_t it = 0;; ++it) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(lp.counter) : "memory");
+        if (v >= target) return true;
+        if ((it & 255u) == 255u) {
+            int st;
+            asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(st) : "l"(lp.status) : "memory");
+            if (st != 0 || *sm.abort_flag || clock64() - t0 > kWaitCycles) {
+                atomicCAS(lp.status, 0, CL_DEV_TIMEOUT);
+                *sm.abort_flag = 1;
+                return false;
             }
         }
     }
+}
+__device__ __forceinline__ void grid_wait(const LoopParams &lp, unsigned target, const Smem &sm) {
+    if (threadIdx.x == 0) grid_poll(lp, target, sm);
     cons_sync();
-    return *sm.abort_flag == 0;
 }
 
 // ------------------------------------------------------------------------------------------------ GEMM
-// The epilogue of one 16-column block (two 8-column groups) of a unit: every thread owns one row and four adjacent columns
-// of the block; the four K quarters are added from the scratch tile in a fixed order.
-__device__ __forceinline__ void gemm_epilogue(const LoopPhase &pg, const Smem &sm, const float *sc, int sub16, int step, int M, int N,
-                                              int half, int out_mode, int use_rms, int act, int erow, int ec4) {
-    const int tid = threadIdx.x;
-    float ssq = 0.0f;
-    if (erow < M && (out_mode != OUT_QKV || ec4 < 8)) {
-        int r0, r1;
-        sub_rows(half, sub16, r0, r1);
-        const float *src = sc + (size_t)erow * CL_SC_LD + ec4;
-        float4 v = *reinterpret_cast<const float4 *>(src);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) {
-            const float4 t = *reinterpret_cast<const float4 *>(src + (size_t)k * M * CL_SC_LD);
-            v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+// One item of the epilogue: a row and the 8 columns of a group that this CTA owns (q|k|v: 4 columns and their rotation partners).
+// What it needs besides the products is fetched before the products are waited for.
+struct EpiPre {
+    float4 a0, a1, b0, b1, c0, c1;  // residual, gate, next scale; q|k|v: cos, sin (a0, b0), bias (c); others: bias, x
+};
+__device__ __forceinline__ float4 ldg4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ float4 ldcg4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
+// what does not depend on the phases before
+__device__ __forceinline__ void epi_static(const LoopPhase &pg, EpiPre &e, int step, int n8, int row) {
+    const int col = n8 * 8;
+    if (pg.out_mode == OUT_RESID) {
+        if (pg.colscale) {
+            const float *s = pg.colscale + (size_t)step * pg.mod_stride + col, *n = pg.scale_next + (size_t)step * pg.mod_stride + col;
+            e.b0 = ldg4(s); e.b1 = ldg4(s + 4);
+            e.c0 = ldg4(n); e.c1 = ldg4(n + 4);
         }
-        const float rms = use_rms ? sm.rms[erow] : 1.0f;
-        v.x *= rms; v.y *= rms; v.z *= rms; v.w *= rms;
-        const int wrow = ec4 < 8 ? r0 + ec4 : r1 + ec4 - 8;  // first of the four output columns
-        if (out_mode == OUT_RESID) {  // residual stream += projection; bf16 mirror; sums of squares of the mirror
-            float4 *hp = reinterpret_cast<float4 *>(pg.h + (size_t)erow * N + wrow);
-            float4 hv = __ldcg(hp);
-            if (pg.colscale) {
-                const float4 gt = *reinterpret_cast<const float4 *>(pg.colscale + (size_t)step * pg.mod_stride + wrow);
-                v.x *= gt.x; v.y *= gt.y; v.z *= gt.z; v.w *= gt.w;
-            }
-            hv.x += v.x; hv.y += v.y; hv.z += v.z; hv.w += v.w;
-            __stcg(hp, hv);
-            if (pg.scale_next) {  // the adaptive norm's (1 + scale) goes into the mirror, its sums of squares come from h itself
-                const float4 sn = *reinterpret_cast<const float4 *>(pg.scale_next + (size_t)step * pg.mod_stride + wrow);
-                __stcg(reinterpret_cast<uint2 *>(pg.hbp + pad_off(M, N, erow, wrow)),
-                       make_uint2(pack_bf16(hv.x + hv.x * sn.x, hv.y + hv.y * sn.y), pack_bf16(hv.z + hv.z * sn.z, hv.w + hv.w * sn.w)));
-                ssq = fmaf(hv.x, hv.x, fmaf(hv.y, hv.y, fmaf(hv.z, hv.z, hv.w * hv.w)));
-            } else {
-                const uint2 pk = make_uint2(pack_bf16(hv.x, hv.y), pack_bf16(hv.z, hv.w));
-                __stcg(reinterpret_cast<uint2 *>(pg.hbp + pad_off(M, N, erow, wrow)), pk);
-                const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&pk.x));
-                const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&pk.y));
-                ssq = fmaf(f0.x, f0.x, fmaf(f0.y, f0.y, fmaf(f1.x, f1.x, f1.y * f1.y)));
-            }
-        } else if (out_mode == OUT_GATED) {
-            // interleaved weight rows: even = gate, odd = up
-            if (pg.bias) {
-                const float4 b = *reinterpret_cast<const float4 *>(pg.bias + (size_t)step * pg.bias_step_stride + wrow);
-                v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-            }
-            const float o0 = act_rt(v.x, act) * v.y, o1 = act_rt(v.z, act) * v.w;
-            __stcg(reinterpret_cast<unsigned *>(pg.outp + pad_off(pg.out_rows, pg.out_kslice, erow, wrow >> 1)), pack_bf16(o0, o1));
-        } else if (out_mode == OUT_QKV) {
-            float4 w = *reinterpret_cast<const float4 *>(src + 8);  // the partner columns (k + half)
-#pragma unroll
-            for (int k = 1; k < 4; ++k) {
-                const float4 t = *reinterpret_cast<const float4 *>(src + 8 + (size_t)k * M * CL_SC_LD);
-                w.x += t.x; w.y += t.y; w.z += t.z; w.w += t.w;
-            }
-            w.x *= rms; w.y *= rms; w.z *= rms; w.w *= rms;
-            if (pg.bias) {
-                const float *bp = pg.bias + (size_t)step * pg.bias_step_stride;
-                const float4 b0 = *reinterpret_cast<const float4 *>(bp + r0 + ec4), b1 = *reinterpret_cast<const float4 *>(bp + r1 + ec4);
-                v.x += b0.x; v.y += b0.y; v.z += b0.z; v.w += b0.w;
-                w.x += b1.x; w.y += b1.y; w.z += b1.z; w.w += b1.w;
-            }
-            const int hd = 2 * half, head = r0 / hd, k = r0 - head * hd + ec4;
-            const int n_q = pg.n_q, n_kvp = pg.n_kvp, S = pg.S;
-            const uint32_t sq = (uint32_t)hd * 2u + 16u;
-            uint8_t *dst;
-            float4 lo = v, hi = w;
-            if (head < n_q + n_kvp) {
-                const float4 c = *reinterpret_cast<const float4 *>(pg.rope + (size_t)erow * half + k);
-                const float4 sn = *reinterpret_cast<const float4 *>(pg.rope + (size_t)(S + erow) * half + k);
-                lo = make_float4(v.x * c.x - w.x * sn.x, v.y * c.y - w.y * sn.y, v.z * c.z - w.z * sn.z, v.w * c.w - w.w * sn.w);
-                hi = make_float4(w.x * c.x + v.x * sn.x, w.y * c.y + v.y * sn.y, w.z * c.z + v.z * sn.z, w.w * c.w + v.w * sn.w);
-                dst = head < n_q ? pg.qp + ((size_t)head * S + erow) * sq : pg.kpp + ((size_t)(head - n_q) * pg.cap + pg.P + erow) * sq;
-            } else {
-                dst = pg.vpp + ((size_t)(head - n_q - n_kvp) * pg.cap + pg.P + erow) * sq;
-            }
-            __stcg(reinterpret_cast<uint2 *>(dst + k * 2), make_uint2(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w)));
-            __stcg(reinterpret_cast<uint2 *>(dst + (k + half) * 2), make_uint2(pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w)));
-        } else {
-            if (pg.bias) {
-                const float4 b = *reinterpret_cast<const float4 *>(pg.bias + (size_t)step * pg.bias_step_stride + wrow);
-                v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-            }
-            if (out_mode == OUT_EULER) {
-                const int t = erow - (pg.S - pg.chunk);
-                if (t >= 0) {
-                    float4 *xp = reinterpret_cast<float4 *>(pg.x + (size_t)t * N + wrow);
-                    float4 xv = __ldcg(xp);
-                    const float dt = pg.dt;
-                    xv.x += dt * v.x; xv.y += dt * v.y; xv.z += dt * v.z; xv.w += dt * v.w;
-                    __stcg(xp, xv);
-                }
-            } else {
-                v.x = act_rt(v.x, act); v.y = act_rt(v.y, act); v.z = act_rt(v.z, act); v.w = act_rt(v.w, act);
-                const int orow = erow + pg.row_off;
-                __stcg(reinterpret_cast<uint2 *>(pg.outp + pad_off(pg.out_rows, pg.out_kslice, orow, wrow)),
-                       make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w)));
-                if (pg.out_f32) __stcg(reinterpret_cast<float4 *>(pg.out_f32 + (size_t)orow * N + wrow), v);
-            }
+    } else if (pg.out_mode == OUT_QKV) {
+        const int per = pg.half >> 2, head = (int)((unsigned)n8 / (unsigned)per), k = (n8 - head * per) * 4;
+        if (head < pg.n_q + pg.n_kvp) {
+            e.a0 = ldg4(pg.rope + (size_t)row * pg.half + k);
+            e.b0 = ldg4(pg.rope + (size_t)(pg.S + row) * pg.half + k);
         }
+        if (pg.bias) {
+            const float *bp = pg.bias + (size_t)step * pg.bias_step_stride + head * 2 * pg.half + k;
+            e.c0 = ldg4(bp); e.c1 = ldg4(bp + pg.half);
+        }
+    } else if (pg.bias) {
+        const float *bp = pg.bias + (size_t)step * pg.bias_step_stride + col;
+        e.a0 = ldg4(bp); e.a1 = ldg4(bp + 4);
     }
-    if (pg.ssq_out) {  // the four threads of a row hold its 16 columns
-        ssq += __shfl_xor_sync(0xffffffffu, ssq, 1);
-        ssq += __shfl_xor_sync(0xffffffffu, ssq, 2);
-        if ((tid & 3) == 0 && erow < M) __stcg(pg.ssq_out + (size_t)sub16 * 64 + erow, ssq);
+}
+// what they wrote
+__device__ __forceinline__ void epi_dynamic(const LoopPhase &pg, EpiPre &e, int n8, int row) {
+    const int col = n8 * 8, N = pg.N8 * 8;
+    if (pg.out_mode == OUT_RESID) {
+        const float *h = pg.h + (size_t)row * N + col;
+        e.a0 = ldcg4(h); e.a1 = ldcg4(h + 4);
+    } else if (pg.out_mode == OUT_EULER && row >= pg.S - pg.chunk) {
+        const float *x = pg.x + (size_t)(row - (pg.S - pg.chunk)) * N + col;
+        e.b0 = ldcg4(x); e.b1 = ldcg4(x + 4);
+    }
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+__device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+__device__ __forceinline__ float sq4(float4 a) { return fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, a.w * a.w))); }
+__device__ __forceinline__ uint4 pack8(float4 a, float4 b) {
+    return make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+}
+__device__ __forceinline__ float4 act4(float4 v, int act) {
+    return make_float4(act_rt(v.x, act), act_rt(v.y, act), act_rt(v.z, act), act_rt(v.w, act));
+}
+__device__ __forceinline__ float bf2_sq(uint32_t v) {
+    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v));
+    return fmaf(f.x, f.x, f.y * f.y);
+}
+__device__ __forceinline__ float sq8(uint4 v) { return (bf2_sq(v.x) + bf2_sq(v.y)) + (bf2_sq(v.z) + bf2_sq(v.w)); }
+// v, w: the products of the group's columns 0 .. 3 and 4 .. 7, RMS factor applied.  Returns the sum of squares of what the next norm reads.
+__device__ __forceinline__ float epi_item(const LoopPhase &pg, const EpiPre &e, int n8, int row, float4 v, float4 w) {
+    const int N = pg.N8 * 8, col = n8 * 8;
+    switch (pg.out_mode) {
+    case OUT_RESID: {  // residual stream += projection; bf16 mirror; sums of squares of the mirror
+        if (pg.colscale) {
+            v = mul4(v, e.b0);
+            w = mul4(w, e.b1);
+        }
+        const float4 h0 = add4(e.a0, v), h1 = add4(e.a1, w);
+        float *hp = pg.h + (size_t)row * N + col;
+        __stcg(reinterpret_cast<float4 *>(hp), h0);
+        __stcg(reinterpret_cast<float4 *>(hp + 4), h1);
+        uint4 *mp = reinterpret_cast<uint4 *>(pg.outp + sw_off(pg.out_rows8, row, col));
+        if (pg.colscale) {  // the adaptive norm's (1 + scale) goes into the mirror, its sums of squares come from h itself
+            __stcg(mp, pack8(add4(h0, mul4(h0, e.c0)), add4(h1, mul4(h1, e.c1))));
+            return sq4(h0) + sq4(h1);
+        }
+        const uint4 pk = pack8(h0, h1);
+        __stcg(mp, pk);
+        return sq8(pk);
+    }
+    case OUT_GATED: {  // interleaved weight rows: even = gate, odd = up
+        v = add4(v, e.a0);
+        w = add4(w, e.a1);
+        const int act = pg.act;
+        __stcg(reinterpret_cast<uint2 *>(pg.outp + sw_off(pg.out_rows8, row, col >> 1)),
+               make_uint2(pack_bf16(act_rt(v.x, act) * v.y, act_rt(v.z, act) * v.w), pack_bf16(act_rt(w.x, act) * w.y, act_rt(w.z, act) * w.w)));
+        return 0.0f;
+    }
+    case OUT_QKV: {
+        const int half = pg.half, per = half >> 2, head = (int)((unsigned)n8 / (unsigned)per), k = (n8 - head * per) * 4;
+        v = add4(v, e.c0);
+        w = add4(w, e.c1);
+        const int n_q = pg.n_q, n_kvp = pg.n_kvp, S = pg.S;
+        const uint32_t sq = (uint32_t)half * 4u + 16u;
+        uint8_t *dst;
+        float4 lo = v, hi = w;
+        if (head < n_q + n_kvp) {
+            const float4 c = e.a0, sn = e.b0;
+            lo = make_float4(v.x * c.x - w.x * sn.x, v.y * c.y - w.y * sn.y, v.z * c.z - w.z * sn.z, v.w * c.w - w.w * sn.w);
+            hi = make_float4(w.x * c.x + v.x * sn.x, w.y * c.y + v.y * sn.y, w.z * c.z + v.z * sn.z, w.w * c.w + v.w * sn.w);
+            dst = head < n_q ? pg.qp + ((size_t)head * S + row) * sq : pg.kpp + ((size_t)(head - n_q) * pg.cap + pg.P + row) * sq;
+        } else {
+            dst = pg.vpp + ((size_t)(head - n_q - n_kvp) * pg.cap + pg.P + row) * sq;
+        }
+        __stcg(reinterpret_cast<uint2 *>(dst + k * 2), make_uint2(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w)));
+        __stcg(reinterpret_cast<uint2 *>(dst + (k + half) * 2), make_uint2(pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w)));
+        return 0.0f;
+    }
+    case OUT_EULER: {
+        const int t = row - (pg.S - pg.chunk);
+        if (t >= 0) {
+            const float dt = pg.dt;
+            const float4 d4 = make_float4(dt, dt, dt, dt);
+            float *xp = pg.x + (size_t)t * N + col;
+            __stcg(reinterpret_cast<float4 *>(xp), add4(e.b0, mul4(d4, add4(v, e.a0))));
+            __stcg(reinterpret_cast<float4 *>(xp + 4), add4(e.b1, mul4(d4, add4(w, e.a1))));
+        }
+        return 0.0f;
+    }
+    default: {
+        v = act4(add4(v, e.a0), pg.act);
+        w = act4(add4(w, e.a1), pg.act);
+        const int orow = row + pg.row_off;
+        const uint4 pk = pack8(v, w);
+        __stcg(reinterpret_cast<uint4 *>(pg.outp + sw_off(pg.out_rows8, orow, col)), pk);
+        if (pg.out_f32) {
+            float *fp = pg.out_f32 + (size_t)orow * N + col;
+            __stcg(reinterpret_cast<float4 *>(fp), v);
+            __stcg(reinterpret_cast<float4 *>(fp + 4), w);
+        }
+        return sq8(pk);
+    }
     }
 }
 
-// A unit = NG groups of 8 output columns; its weights arrive as K chunks of 2048 / NG columns (one ring stage each), A as
-// K slices of at most 1024 columns; the accumulators live in registers across all chunks and slices of the unit.
-template <int NG>
-__device__ __noinline__ void gemm_phase(const LoopPhase &pg, const LoopParams &lp, int step, unsigned &cons, unsigned &a_cnt_ref) {
+// Floats per column of exchanged sums: the tokens, rounded up so that columns are an odd number of 16-byte chunks apart.
+__host__ __device__ __forceinline__ int token_pitch(int M) { return ((M + 3) >> 2 | 1) * 4; }
+
+// A group of kd CTAs computes a range of 8-column groups; this CTA multiplies its 1 / kd of K and sends every owner its part.
+__device__ __noinline__ unsigned gemm_phase(const LoopPhase &pg, const LoopParams &lp, int step, unsigned par, unsigned target, uint32_t tmem) {
     const Smem sm = get_smem();
     const WaitCtx wc{sm.abort_flag, lp.status};
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int mh = warp & 1, kq = warp >> 1;
-    const int M = pg.M, N = pg.N, K = pg.K, kslices = pg.kslices, n_units = pg.n_sub, half = pg.half;
-    const int out_mode = pg.out_mode, use_rms = pg.use_rms, act = pg.act;
-    const int kchunk = pg.kchunk, n_chunks = K / kchunk;
-    int id0, id1;
-    sub_range(n_chunks, n_units, id0, id1);
-    if (id0 >= id1) return;
-    const uint8_t *Ap = pg.Ap;
-    const float eps = pg.eps;
-    const int kslice = K / kslices, cps = kslice / kchunk;  // chunks per A slice
-    const uint32_t astride = (uint32_t)kslice * 2u + 16u, wstride = (uint32_t)kchunk * 2u + 16u;
-    const uint32_t slot_bytes = kslices > 1 ? (uint32_t)M * astride : 0u;  // two A buffers when A comes in slices
-    float *sc = reinterpret_cast<float *>(sm.arena + (size_t)(kslices > 1 ? 2 : 1) * M * astride);  // [4 K quarters][M][CL_SC_LD]
-    const uint32_t as_addr = smem_u32(sm.arena);
-    unsigned a_cnt = a_cnt_ref, a_iss = a_cnt_ref;  // A tiles consumed / issued since the launch: barrier and buffer alternate with them
-    const int nk = kchunk >> 4, ks0 = kq * nk / 4, ks1 = (kq + 1) * nk / 4;
-    // ldmatrix lane addressing
-    const int mi = lane >> 3, lr = lane & 7;
-    uint32_t a_off[2];
-#pragma unroll
-    for (int mtl = 0; mtl < 2; ++mtl) {
-        int row = (2 * mh + mtl) * 16 + lr + (mi & 1) * 8;
-        row = min(row, M - 1);
-        a_off[mtl] = as_addr + (uint32_t)row * astride + (uint32_t)(mi >> 1) * 16u;
+    const int M = pg.M, K = pg.K, kd = pg.kd;
+    const GemmPart gp = gemm_part(pg.N8, K, kd);
+    if (gp.w8 <= 0) {
+        grid_wait(lp, target, sm);
+        return par;
     }
-    const uint32_t b_lane = (uint32_t)(lr + (mi >> 1) * 8) * wstride + (uint32_t)(mi & 1) * 16u;
-    const bool mt_ok[2] = {(2 * mh) * 16 < M, (2 * mh + 1) * 16 < M};
-    const int g = lane >> 2, q2 = (lane & 3) * 2;
-    const int erow = tid >> 2, ec4 = (tid & 3) * 4;
-    float acc[2][NG][4];
-    uint32_t a_slot = 0;  // byte offset of the A buffer in use
-    for (int id = id0; id < id1; ++id) {
-        const int u = id / n_chunks, c = id - u * n_chunks, slice = c / cps, cs = c - slice * cps;
-        if (cs == 0 && (kslices > 1 || id == id0)) {  // an unsliced A serves every unit of the phase
-            cons_sync();  // every warp is done with the slice before: the buffer that is filled next is free
-            if (tid == 0) {
-                if (slice == 0) {
-                    mbar_expect_tx(&sm.a_full[a_iss & 1u], (uint32_t)M * astride);
-                    bulk_g2s(sm.arena + (a_iss & 1u) * slot_bytes, Ap, (uint32_t)M * astride, &sm.a_full[a_iss & 1u]);
-                }
-                if (slice + 1 < kslices) {  // the next slice loads while this one is multiplied
-                    const unsigned nx = a_iss + (slice == 0 ? 1u : 0u);
-                    mbar_expect_tx(&sm.a_full[nx & 1u], (uint32_t)M * astride);
-                    bulk_g2s(sm.arena + (nx & 1u) * slot_bytes, Ap + (size_t)(slice + 1) * M * astride, (uint32_t)M * astride, &sm.a_full[nx & 1u]);
+    const int sh = 31 - __clz(kd), kr = gp.kr, base_rank = (int)(blockIdx.x % CL_CLUSTER) - kr;
+    const uint32_t blk_bytes = (uint32_t)((M + 7) & ~7) * 128u, a_bytes = (uint32_t)(gp.kb1 - gp.kb0) * blk_bytes;
+    // arena: A (the longest of the group) | what the group sends, per pass [source][owned column][token]; this CTA's own sums are staged
+    // over A when one pass does it all (A has been multiplied by then), else behind
+    const int tp = token_pitch(M), w8m = min(CL_PASS_N8, gp.w8), row = tid & 63, cg = tid >> 6;
+    const uint32_t recv_bytes = (uint32_t)((((w8m + kd - 1) >> sh) << sh) * 8 * tp) * 4u;  // kd parts of the most columns one CTA owns
+    const uint32_t recv_off = (uint32_t)((((K + 63) >> 6) + kd - 1) >> sh) * blk_bytes;
+    const bool one_pass = gp.w8 <= CL_PASS_N8;
+    const uint32_t stage_off = one_pass && recv_bytes <= recv_off ? 0u : recv_off + (one_pass ? 1u : (uint32_t)CL_PASSES) * recv_bytes;
+    const int hw = warp & 3, th = warp >> 2;  // this warp's quarter of the TMEM lanes and half of the tokens
+    // ---- before the barrier: everything that does not depend on the phase before
+    const int own00 = w8m * kr >> sh, oN0 = (w8m * (kr + 1) >> sh) - own00;
+    EpiPre pre;
+    pre.a0 = pre.a1 = pre.b0 = pre.b1 = pre.c0 = pre.c1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool first = row < M && cg < oN0;
+    if (first) epi_static(pg, pre, step, gp.j0 + own00 + cg, row);
+    if (tid == 0) {
+        for (int p0 = 0, pass = 0; p0 < gp.w8; p0 += CL_PASS_N8, ++pass) {
+            const int w8p = min(CL_PASS_N8, gp.w8 - p0), oN = (w8p * (kr + 1) >> sh) - (w8p * kr >> sh);
+            mbar_expect_tx(&sm.x_full[pass], (uint32_t)(kd * oN * 8 * tp) * 4u);
+        }
+        if (grid_poll(lp, target, sm) && a_bytes) {
+            fence_proxy_async_all();
+            mbar_expect_tx(sm.a_full, a_bytes);
+            bulk_g2s(sm.arena, pg.Ap + (size_t)gp.kb0 * blk_bytes, a_bytes, sm.a_full);
+        }
+    }
+    cons_sync();
+    // ---- after it
+    if (first) epi_dynamic(pg, pre, gp.j0 + own00 + cg, row);
+    const bool use_rms = pg.use_rms != 0;
+    if (use_rms) {  // row sums of squares from the producer's partial sums, fixed order
+        const int n = pg.ssq_n;
+        const float *src = pg.ssq_in + row;
+        float ss = 0.0f;
+        for (int p0 = cg; p0 < n; p0 += 128) {
+            float part[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) part[j] = (row < M && p0 + 4 * j < n) ? __ldcg(src + (size_t)(p0 + 4 * j) * 64) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) ss += part[j];
+        }
+        sm.red[cg * 64 + row] = ss;
+    }
+    for (int p0 = 0, pass = 0; p0 < gp.w8; p0 += CL_PASS_N8, ++pass) {
+        const int w8p = min(CL_PASS_N8, gp.w8 - p0);
+        const int own0 = w8p * kr >> sh, ownN = (w8p * (kr + 1) >> sh) - own0;
+        if (a_bytes) {
+            mbar_wait(sm.acc_full, par_bit(par, PAR_ACC), wc, CL_DEV_TIMEOUT);
+            par ^= 1u << PAR_ACC;
+            tc_fence_after();
+        }
+        // ---- this CTA's K part into its staging area, [column][token]: a lane holds one column, 32 tokens
+        float *stg = reinterpret_cast<float *>(sm.arena + stage_off + (uint32_t)pass * recv_bytes);
+        for (int n0 = hw * 32; n0 < w8p * 8; n0 += 128) {
+            float v[32];
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[e] = 0.0f;
+            if (a_bytes) {
+                const uint32_t ta = tmem + (uint32_t)((n0 >> 7) * CL_ACC * 64 + th * 32) + ((uint32_t)(hw * 32) << 16);
+#pragma unroll
+                for (int k = 0; k < CL_ACC; k += 2) {
+                    uint32_t r0[32], r1[32];
+                    tmem_ld32(ta + (uint32_t)k * 64u, r0);
+                    tmem_ld32(ta + (uint32_t)(k + 1) * 64u, r1);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) v[e] += __uint_as_float(r0[e]) + __uint_as_float(r1[e]);
                 }
             }
-            a_iss += (slice == 0 ? 1u : 0u) + (slice + 1 < kslices ? 1u : 0u);
-            if (use_rms == RMS_PARTS && id == id0) {  // rms factors from the producer's partial sums, fixed order
-                const int r = tid >> 2, q = tid & 3, n = (int)pg.ssq_n;
-                float part[16];
+            const int n = n0 + lane;
+            if (n < w8p * 8) {
+                float4 *dst = reinterpret_cast<float4 *>(stg + (size_t)n * tp + th * 32);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) part[j] = (r < M && q + 4 * j < n) ? __ldcg(pg.ssq_in + (size_t)(q + 4 * j) * 64 + r) : 0.0f;
-                float ss = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) ss += part[j];
-                ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-                ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-                if (q == 0 && r < M) sm.rms[r] = rsqrtf(ss / (float)K + eps);
-            }
-            mbar_wait(&sm.a_full[a_cnt & 1u], (a_cnt >> 1) & 1u, wc, CL_DEV_TIMEOUT);
-            a_slot = (a_cnt & 1u) * slot_bytes;
-            ++a_cnt;
-            const uint8_t *As = sm.arena + a_slot;
-            if (use_rms == RMS_LOCAL) {  // four threads per row, interleaved 16-byte chunks
-                const int r = tid >> 2, q = tid & 3;
-                float s0 = 0.0f, s1 = 0.0f;
-                if (r < M) {
-                    const uint4 *rowp = reinterpret_cast<const uint4 *>(As + (size_t)r * astride);
-                    for (int cc = q; cc < (kslice >> 3); cc += 8) {
-                        const uint4 v0 = rowp[cc], v1 = cc + 4 < (kslice >> 3) ? rowp[cc + 4] : make_uint4(0, 0, 0, 0);
-                        const __nv_bfloat162 *h0 = reinterpret_cast<const __nv_bfloat162 *>(&v0), *h1 = reinterpret_cast<const __nv_bfloat162 *>(&v1);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 f0 = __bfloat1622float2(h0[e]), f1 = __bfloat1622float2(h1[e]);
-                            s0 = fmaf(f0.x, f0.x, s0); s0 = fmaf(f0.y, f0.y, s0);
-                            s1 = fmaf(f1.x, f1.x, s1); s1 = fmaf(f1.y, f1.y, s1);
-                        }
-                    }
-                }
-                float ss = s0 + s1;
-                ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-                ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-                if (q == 0 && r < M) sm.rms[r] = rsqrtf(ss / (float)K + eps);
+                for (int e = 0; e < 8; ++e)
+                    if (th * 32 + e * 4 < M) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
             }
         }
-        const unsigned stage = cons % CL_STAGES;
-        mbar_wait(&sm.full[stage], (cons / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
-        const uint32_t w_addr = smem_u32(sm.ring + (size_t)stage * CL_STAGE_BYTES) + b_lane;
-        if (c == 0) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < NG; ++j)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0f;
+        tc_fence_before();
+        fence_proxy_async_smem();
+        cons_sync();  // staged; and the partial sums of squares are in place
+        if (lane == 0) {
+            if (a_bytes) mbar_arrive(sm.acc_free);
+            if (warp < kd) {  // warp w sends rank w of the group its columns
+                const int b = w8p * warp >> sh, oN = (w8p * (warp + 1) >> sh) - b;
+                const uint32_t bytes = (uint32_t)(oN * 8 * tp) * 4u;
+                if (oN > 0)
+                    bulk_s2rank(map_rank(smem_u32(sm.arena + recv_off + (uint32_t)pass * recv_bytes), base_rank + warp) + (uint32_t)kr * bytes,
+                                smem_u32(stg) + (uint32_t)(b * 8 * tp) * 4u, bytes, map_rank(smem_u32(&sm.x_full[pass]), base_rank + warp));
+            }
         }
-        const uint32_t a_k = a_slot + (uint32_t)cs * (uint32_t)kchunk * 2u;
+        const float rms = use_rms ? rsqrtf(((sm.red[row] + sm.red[64 + row]) + (sm.red[128 + row] + sm.red[192 + row])) / (float)K + pg.eps) : 1.0f;
+        mbar_wait_cluster(&sm.x_full[pass], par_bit(par, PAR_X + pass), wc, CL_DEV_TIMEOUT);
+        par ^= 1u << (PAR_X + pass);
+        if (row < M) {
+            const float *recv = reinterpret_cast<const float *>(sm.arena + recv_off + (uint32_t)pass * recv_bytes) + row;
+            const int ld = ownN * 8 * tp;
+            for (int jl = cg; jl < ownN; jl += 4) {
+                const int n8 = gp.j0 + p0 + own0 + jl;
+                if (jl != cg || pass > 0) {
+                    epi_static(pg, pre, step, n8, row);
+                    epi_dynamic(pg, pre, n8, row);
+                }
+                const float *src = recv + (size_t)jl * 8 * tp;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f), w = v;
 #pragma unroll 2
-        for (int ks = ks0; ks < ks1; ++ks) {
-            uint32_t a[2][4];
-#pragma unroll
-            for (int mtl = 0; mtl < 2; ++mtl) ldsm4(a[mtl], a_off[mtl] + a_k + (uint32_t)ks * 32u);
-#pragma unroll
-            for (int gp = 0; gp < NG / 2; ++gp) {
-                uint32_t b[4];
-                ldsm4(b, w_addr + (uint32_t)gp * 16u * wstride + (uint32_t)ks * 32u);
-#pragma unroll
-                for (int mtl = 0; mtl < 2; ++mtl) {
-                    if (!mt_ok[mtl]) continue;
-                    mma_bf16(acc[mtl][2 * gp], a[mtl], b[0], b[1]);
-                    mma_bf16(acc[mtl][2 * gp + 1], a[mtl], b[2], b[3]);
+                for (int s = 0; s < kd; ++s, src += ld) {
+                    v.x += src[0]; v.y += src[tp]; v.z += src[2 * tp]; v.w += src[3 * tp];
+                    w.x += src[4 * tp]; w.y += src[5 * tp]; w.z += src[6 * tp]; w.w += src[7 * tp];
                 }
+                if (use_rms) {
+                    v.x *= rms; v.y *= rms; v.z *= rms; v.w *= rms;
+                    w.x *= rms; w.y *= rms; w.z *= rms; w.w *= rms;
+                }
+                const float ssq = epi_item(pg, pre, n8, row, v, w);
+                if (pg.ssq_out) __stcg(pg.ssq_out + (size_t)n8 * 64 + row + pg.row_off, ssq);
             }
         }
-        __syncwarp();  // every lane's fragments of this stage have been consumed by its products
-        if (lane == 0) mbar_arrive(&sm.empty[stage]);
-        ++cons;
-        if (c + 1 < n_chunks) continue;  // more of this unit's K follows: keep accumulating
-        cons_sync();  // the previous unit's epilogue has read the scratch tile
-        // ---- epilogue: NG / 2 blocks of 16 columns through the scratch tile
-#pragma unroll
-        for (int blk = 0; blk < NG / 2; ++blk) {
-            if (blk > 0) cons_sync();  // the previous block's sums have been read
-            float *dst = sc + (size_t)kq * M * CL_SC_LD;
-#pragma unroll
-            for (int mtl = 0; mtl < 2; ++mtl)
-#pragma unroll
-                for (int hr = 0; hr < 2; ++hr) {
-                    const int row = (2 * mh + mtl) * 16 + g + hr * 8;
-                    if (row >= M) continue;
-                    float *rp = dst + (size_t)row * CL_SC_LD + q2;
-                    *reinterpret_cast<float2 *>(rp) = make_float2(acc[mtl][2 * blk][2 * hr], acc[mtl][2 * blk][2 * hr + 1]);
-                    *reinterpret_cast<float2 *>(rp + 8) = make_float2(acc[mtl][2 * blk + 1][2 * hr], acc[mtl][2 * blk + 1][2 * hr + 1]);
-                }
-            cons_sync();
-            gemm_epilogue(pg, sm, sc, u * (NG / 2) + blk, step, M, N, half, out_mode, use_rms, act, erow, ec4);
-        }
     }
-    a_cnt_ref = a_cnt;
+    return par;
 }
 
 // ----------------------------------------------------------------------------------------------- EMBED
-__device__ __noinline__ void embed_phase(const LoopPhase &p, const LoopParams &lp, int step) {
+__device__ __noinline__ void embed_phase(const LoopPhase &p, const LoopParams &lp, int step, unsigned target) {
     const Smem sm = get_smem();
+    grid_wait(lp, target, sm);
     float *xs = reinterpret_cast<float *>(sm.arena);
     const int A = p.A_dim, H = p.H, chunk = p.chunk, sd = p.sd;
-    cons_sync();
     for (int i = threadIdx.x; i < chunk * A; i += CL_THREADS) xs[i] = __ldcg(p.x + i);
     float *ss = xs + chunk * A;
     for (int i = threadIdx.x; i < sd; i += CL_THREADS) ss[i] = lp.state[i];
@@ -580,13 +676,13 @@ __device__ __noinline__ void embed_phase(const LoopPhase &p, const LoopParams &l
                 }
             }
             if (!p.scale_next) {
-                *reinterpret_cast<__nv_bfloat16 *>(p.outp + pad_off(chunk, H, r, o)) = __float2bfloat16(acc);
+                *reinterpret_cast<__nv_bfloat16 *>(p.outp + sw_off((chunk + 7) & ~7, r, o)) = __float2bfloat16(acc);
             } else {
                 // pi0.5: the embedding IS the residual stream (rows = action tokens); mirror with the first norm's (1 + scale),
                 // sums of squares per 32 columns (a warp holds 32 consecutive columns of one row block)
                 __stcg(p.h + (size_t)r * H + o, acc);
                 const float sn = p.scale_next[(size_t)step * p.mod_stride + o];
-                *reinterpret_cast<__nv_bfloat16 *>(p.hbp + pad_off(p.S, H, r, o)) = __float2bfloat16(acc + acc * sn);
+                *reinterpret_cast<__nv_bfloat16 *>(p.hbp + sw_off((p.S + 7) & ~7, r, o)) = __float2bfloat16(acc + acc * sn);
                 float sq = acc * acc;
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
@@ -594,19 +690,27 @@ __device__ __noinline__ void embed_phase(const LoopPhase &p, const LoopParams &l
             }
         }
     }
-    if (sd > 0)  // pi0: the state token is row 0 of the residual stream
-        for (int o = gt; o < H; o += gn) {
-            const __nv_bfloat16 *wr = p.w2 + (size_t)o * sd;
-            float acc = p.b2 ? p.b2[o] : 0.0f;
-            for (int k = 0; k < sd; ++k) acc = fmaf(__bfloat162float(wr[k]), ss[k], acc);
-            __stcg(p.h + o, acc);
-            *reinterpret_cast<__nv_bfloat16 *>(p.hbp + pad_off(p.S, H, 0, o)) = __float2bfloat16(acc);
+    if (sd > 0)  // pi0: the state token is row 0 of the residual stream; a warp holds 32 consecutive columns
+        for (int o = gt; o - (int)(threadIdx.x & 31) < H; o += gn) {
+            float sq = 0.0f;
+            if (o < H) {
+                const __nv_bfloat16 *wr = p.w2 + (size_t)o * sd;
+                float acc = p.b2 ? p.b2[o] : 0.0f;
+                for (int k = 0; k < sd; ++k) acc = fmaf(__bfloat162float(wr[k]), ss[k], acc);
+                __stcg(p.h + o, acc);
+                const __nv_bfloat16 hb = __float2bfloat16(acc);
+                *reinterpret_cast<__nv_bfloat16 *>(p.hbp + sw_off((p.S + 7) & ~7, 0, o)) = hb;
+                sq = __bfloat162float(hb) * __bfloat162float(hb);
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+            if ((threadIdx.x & 31) == 0) __stcg(p.ssq_out + (size_t)(o >> 5) * 64, sq);
         }
 }
 
 // ------------------------------------------------------------------------------------------- ATTENTION
 template <int HD>
-__device__ __noinline__ void att_phase(const LoopPhase &pg, const LoopParams &lp, unsigned &a_cnt) {
+__device__ __noinline__ unsigned att_phase(const LoopPhase &pg, const LoopParams &lp, unsigned par, unsigned target) {
     const Smem sm = get_smem();
     const WaitCtx wc{sm.abort_flag, lp.status};
     constexpr int SQ = HD * 2 + 16;   // bytes per staged row
@@ -614,41 +718,81 @@ __device__ __noinline__ void att_phase(const LoopPhase &pg, const LoopParams &lp
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int mt = warp & 1, kp = warp >> 1;
     const int mi = lane >> 3, lr = lane & 7, g = lane >> 2, q2 = (lane & 3) * 2;
-    const int ks = pg.ks, ns = pg.ns, n_rt = pg.n_rt, kv_len = pg.kv_len, R = pg.R, S = pg.S, P = pg.P, cap = pg.cap, mask_mode = pg.mask_mode;
+    const int ks = pg.ks, n_rt = pg.n_rt, kv_len = pg.kv_len, R = pg.R, S = pg.S, P = pg.P, cap = pg.cap, mask_mode = pg.mask_mode;
+    const int ad = pg.kd, rpo = 32 / ad;  // key ranges = CTAs per unit; query rows each of them merges
+    const int grp = blockIdx.x / ad, ar = blockIdx.x - grp * ad, base_rank = (int)(blockIdx.x % CL_CLUSTER) - ar;
     const int gq = pg.g;
     const float scale_log2 = pg.scale_log2;
-    uint8_t *Qs = sm.arena, *Ks = Qs + 32 * SQ, *Vs = Ks + (size_t)ks * SQ, *Ps = Vs + (size_t)ks * SQ;
-    const int SP = (ks + 8) * 2;
-    const int n_units = pg.n_kv * n_rt * ns;
+    constexpr int OP = HD + 8;        // floats per exchanged row: O, maximum and sum behind it
+    uint8_t *Qs = sm.arena, *Ks = Qs + pg.k_off, *Vs = Ks + (size_t)ks * SQ, *Ps = sm.arena + pg.p_off, *recv = sm.arena + pg.recv_off;
+    const int SP = (((ks + 15) & ~15) + 8) * 2;
+    const int n_units = pg.n_kv * n_rt;
     int pad_lo = 0, pad_hi = 0;
     if (lp.pad) {
         pad_lo = lp.pad[0];
         pad_hi = lp.pad[1];
     }
-    for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
-        const int kvh = u / (n_rt * ns), rem = u - kvh * (n_rt * ns), rt = rem / ns, s = rem - rt * ns;
-        const int key0 = s * ks, nkeys = min(ks, kv_len - key0), ks16 = (nkeys + 15) & ~15;
+    const int n_grp = gridDim.x / ad, k_begin = ar * pg.per, k_end = min(kv_len, k_begin + pg.per);
+    // Before the barrier: the rows of the first key block that lie in the prefix (they do not change during the loop).
+    const int nk0 = max(0, min(ks, k_end - k_begin)), n_prefix = max(0, min(nk0, P - k_begin));
+    const int n_early_k = pg.early_k ? n_prefix : 0, n_early = pg.early_v ? n_prefix : 0;
+    if (tid == 0) {
+        const bool work = grp < n_units && nk0 > 0;
+        const int kvh = grp / n_rt, row0 = (grp - kvh * n_rt) * 32;
+        const uint32_t q_bytes = (uint32_t)min(32, R - row0) * SQ;
+        const uint8_t *kp0 = pg.kpp + ((size_t)kvh * cap + k_begin) * SQ, *vp0 = pg.vpp + ((size_t)kvh * cap + k_begin) * SQ;
+        if (work) {
+            fence_proxy_async_all();
+            mbar_expect_tx(sm.k_full, q_bytes + (uint32_t)nk0 * SQ);
+            mbar_expect_tx(sm.v_full, (uint32_t)nk0 * SQ);
+            if (n_early_k > 0) bulk_g2s(Ks, kp0, (uint32_t)n_early_k * SQ, sm.k_full);
+            if (n_early > 0) bulk_g2s(Vs, vp0, (uint32_t)n_early * SQ, sm.v_full);
+        }
+        if (grid_poll(lp, target, sm) && work) {
+            fence_proxy_async_all();
+            bulk_g2s(Qs, pg.qp + ((size_t)kvh * gq * S + row0) * SQ, q_bytes, sm.k_full);
+            if (n_early_k < nk0) bulk_g2s(Ks + (size_t)n_early_k * SQ, kp0 + (size_t)n_early_k * SQ, (uint32_t)(nk0 - n_early_k) * SQ, sm.k_full);
+            if (n_early < nk0) bulk_g2s(Vs + (size_t)n_early * SQ, vp0 + (size_t)n_early * SQ, (uint32_t)(nk0 - n_early) * SQ, sm.v_full);
+        }
+    }
+    cons_sync();
+    for (int u = grp; u < n_units; u += n_grp) {  // several units per group only when ad == 1
+        const int kvh = u / n_rt, rt = u - kvh * n_rt;
         const int row0 = rt * 32, nrows = min(32, R - row0);
-        cons_sync();  // the arena is free
-        if (tid == 0) {
-            uint64_t *bar = &sm.a_full[a_cnt & 1u];
-            mbar_expect_tx(bar, (uint32_t)(nrows + 2 * nkeys) * SQ);
-            bulk_g2s(Qs, pg.qp + ((size_t)kvh * gq * S + row0) * SQ, (uint32_t)nrows * SQ, bar);
-            bulk_g2s(Ks, pg.kpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, bar);
-            bulk_g2s(Vs, pg.vpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, bar);
+        const int vrows = max(0, min(rpo, nrows - ar * rpo));  // rows this CTA merges
+        if (u != grp) cons_sync();  // the unit before has been merged: the arena is free
+        if (tid == 0) mbar_expect_tx(sm.xa_full, (uint32_t)(ad * rpo * OP) * 4u);
+        float oacc[2][NGV][4], ms[2] = {-INFINITY, -INFINITY}, mo[2][2] = {{-INFINITY, -INFINITY}, {-INFINITY, -INFINITY}}, sum[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < NGV; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) oacc[i][j][e] = 0.0f;
+        const int c0 = warp * (HD / 8);
+        for (int key0 = k_begin; key0 < k_end; key0 += ks) {
+        const int nkeys = min(ks, k_end - key0), ks16 = (nkeys + 15) & ~15;
+        if (key0 != k_begin) cons_sync();  // the block before has been consumed
+        if (tid == 0 && (u != grp || key0 != k_begin)) {
+            fence_proxy_async_all();
+            const uint32_t q_bytes = key0 == k_begin ? (uint32_t)nrows * SQ : 0u;
+            mbar_expect_tx(sm.k_full, q_bytes + (uint32_t)nkeys * SQ);
+            if (q_bytes) bulk_g2s(Qs, pg.qp + ((size_t)kvh * gq * S + row0) * SQ, q_bytes, sm.k_full);
+            bulk_g2s(Ks, pg.kpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, sm.k_full);
+            mbar_expect_tx(sm.v_full, (uint32_t)nkeys * SQ);
+            bulk_g2s(Vs, pg.vpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, sm.v_full);
         }
         for (int i = tid; i < (ks16 - nkeys) * (HD / 8); i += CL_THREADS) {
             const int r = nkeys + i / (HD / 8), c = i % (HD / 8);
             *reinterpret_cast<uint4 *>(Vs + (size_t)r * SQ + c * 16) = make_uint4(0, 0, 0, 0);
         }
-        mbar_wait(&sm.a_full[a_cnt & 1u], (a_cnt >> 1) & 1u, wc, CL_DEV_TIMEOUT);
-        ++a_cnt;
-        cons_sync();
+        mbar_wait(sm.k_full, par_bit(par, PAR_K), wc, CL_DEV_TIMEOUT);
+        par ^= 1u << PAR_K;
         // ---- S = Q K^T for this warp's 16 rows and its share of the 8-key groups
-        const int ng = ks16 >> 3, g0 = kp * ng / 4, g1 = (kp + 1) * ng / 4, n_g = g1 - g0;  // n_g <= 3
-        float sacc[3][4];
+        const int ng = ks16 >> 3, g0 = kp * ng / 4, g1 = (kp + 1) * ng / 4, n_g = g1 - g0;  // n_g <= 4
+        float sacc[4][4];
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int e = 0; e < 4; ++e) sacc[i][e] = 0.0f;
         {
@@ -661,7 +805,7 @@ __device__ __noinline__ void att_phase(const LoopPhase &pg, const LoopParams &lp
                 ldsm4(a0, q_addr + kk * 64);
                 ldsm4(a1, q_addr + kk * 64 + 32);
 #pragma unroll
-                for (int gi = 0; gi < 3; ++gi) {
+                for (int gi = 0; gi < 4; ++gi) {
                     if (gi >= n_g) break;
                     uint32_t b[4];
                     ldsm4(b, k_addr + (uint32_t)gi * 8u * SQ + kk * 64);
@@ -684,7 +828,7 @@ __device__ __noinline__ void att_phase(const LoopPhase &pg, const LoopParams &lp
         }
         float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-        for (int gi = 0; gi < 3; ++gi) {
+        for (int gi = 0; gi < 4; ++gi) {
             if (gi >= n_g) break;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -700,16 +844,19 @@ __device__ __noinline__ void att_phase(const LoopPhase &pg, const LoopParams &lp
             mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 2));
             if ((lane & 3) == 0) sm.red_max[rl[hr] * 4 + kp] = mx[hr];
         }
-        cons_sync();
-        float sum[2] = {0.0f, 0.0f};
+        cons_sync();  // the maxima are in place; Q (P may lie over it) and K have been read
+        if (key0 + ks >= k_end && tid < ad) arrive_rank(map_rank(smem_u32(sm.rdy), base_rank + tid));
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
             const float *rm = sm.red_max + rl[hr] * 4;
-            const float m = fmaxf(fmaxf(rm[0], rm[1]), fmaxf(rm[2], rm[3]));
+            const float m = fmaxf(ms[hr], fmaxf(fmaxf(rm[0], rm[1]), fmaxf(rm[2], rm[3])));
             mx[hr] = m == -INFINITY ? 0.0f : m;
+            sum[hr] *= ex2f(ms[hr] - mx[hr]);  // 0 before the first block
+            ms[hr] = m;
+            if (kp == 0 && (lane & 3) == 0) sm.row_m[rl[hr]] = m;
         }
 #pragma unroll
-        for (int gi = 0; gi < 3; ++gi) {
+        for (int gi = 0; gi < 4; ++gi) {
             if (gi >= n_g) break;
             float pv[4];
 #pragma unroll
@@ -723,20 +870,29 @@ __device__ __noinline__ void att_phase(const LoopPhase &pg, const LoopParams &lp
         }
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
-            sum[hr] += __shfl_xor_sync(0xffffffffu, sum[hr], 1);
-            sum[hr] += __shfl_xor_sync(0xffffffffu, sum[hr], 2);
-            if ((lane & 3) == 0) sm.red_sum[rl[hr] * 4 + kp] = sum[hr];
+            float s = sum[hr];
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if ((lane & 3) == 0) sm.red_sum[rl[hr] * 4 + kp] = s;
         }
+        mbar_wait(sm.v_full, par_bit(par, PAR_V), wc, CL_DEV_TIMEOUT);
+        par ^= 1u << PAR_V;
         cons_sync();
         // ---- O = P V: this warp's HD / 8 output columns, all 32 rows
-        float oacc[2][NGV][4];
+        if (pg.per > ks) {  // several key blocks: earlier sums follow the running maximum
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+            for (int m2 = 0; m2 < 2; ++m2)
 #pragma unroll
-            for (int j = 0; j < NGV; ++j)
+                for (int hr = 0; hr < 2; ++hr) {
+                    const float m = sm.row_m[m2 * 16 + g + hr * 8], f = ex2f(mo[m2][hr] - (m == -INFINITY ? 0.0f : m));
+                    mo[m2][hr] = m;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) oacc[i][j][e] = 0.0f;
-        const int c0 = warp * (HD / 8);
+                    for (int j = 0; j < NGV; ++j) {
+                        oacc[m2][j][2 * hr] *= f;
+                        oacc[m2][j][2 * hr + 1] *= f;
+                    }
+                }
+        }
         {
             const uint32_t p_addr = smem_u32(Ps) + (uint32_t)(lr + (mi & 1) * 8) * SP + (uint32_t)(mi >> 1) * 16u;
             const uint32_t v_addr = smem_u32(Vs) + (uint32_t)(lr + (mi & 1) * 8) * SQ + (uint32_t)(c0 + (NGV > 1 ? (mi >> 1) * 8 : 0)) * 2u;
@@ -762,67 +918,61 @@ __device__ __noinline__ void att_phase(const LoopPhase &pg, const LoopParams &lp
                 }
             }
         }
-        float *wo = pg.ws_o + (size_t)u * 32 * HD;
+        }
+        if (k_begin >= k_end) {  // no keys in this CTA's range: it contributes nothing, but its peers count on its arrival
+            if (tid < ad) arrive_rank(map_rank(smem_u32(sm.rdy), base_rank + tid));
+            if (tid < 128) sm.red_sum[tid] = 0.0f;
+            if (tid < 32) sm.row_m[tid] = -INFINITY;
+            cons_sync();
+        }
+        // ---- un-normalised O rows, maximum and row sum: staged over V (read by everyone), then one copy per CTA that merges rows
+        cons_sync();
+        float *stg = reinterpret_cast<float *>(sm.arena + pg.stage_off);
 #pragma unroll
         for (int m2 = 0; m2 < 2; ++m2)
 #pragma unroll
             for (int hr = 0; hr < 2; ++hr) {
-                const int row = m2 * 16 + g + hr * 8;
-                if (row >= nrows) continue;
+                float *rp = stg + (size_t)(m2 * 16 + g + hr * 8) * OP + c0 + q2;
 #pragma unroll
-                for (int j = 0; j < NGV; ++j)
-                    __stcg(reinterpret_cast<float2 *>(wo + (size_t)row * HD + c0 + j * 8 + q2), make_float2(oacc[m2][j][2 * hr], oacc[m2][j][2 * hr + 1]));
+                for (int j = 0; j < NGV; ++j) *reinterpret_cast<float2 *>(rp + j * 8) = make_float2(oacc[m2][j][2 * hr], oacc[m2][j][2 * hr + 1]);
             }
-        if (tid < 32 && tid < nrows) {
-            const float *rm = sm.red_max + tid * 4, *rs = sm.red_sum + tid * 4;
-            const float m = fmaxf(fmaxf(rm[0], rm[1]), fmaxf(rm[2], rm[3]));
-            const float l = ((rs[0] + rs[1]) + rs[2]) + rs[3];
-            __stcg(reinterpret_cast<float2 *>(pg.ws_ml + ((size_t)u * 32 + tid) * 2), make_float2(m, l));
+        if (tid < 32) {
+            const float *rs = sm.red_sum + tid * 4;
+            *reinterpret_cast<float2 *>(stg + (size_t)tid * OP + HD) = make_float2(sm.row_m[tid], ((rs[0] + rs[1]) + rs[2]) + rs[3]);
+        }
+        fence_proxy_async_smem();
+        cons_sync();
+        const uint32_t xblk = (uint32_t)(rpo * OP) * 4u;
+        if (lane == 0 && warp < ad && mbar_wait_cluster(sm.rdy, par_bit(par, PAR_RDY), wc, CL_DEV_TIMEOUT))  // the group has read its K blocks, where the rows may land
+            bulk_s2rank(map_rank(smem_u32(recv), base_rank + warp) + (uint32_t)ar * xblk, smem_u32(stg) + (uint32_t)warp * xblk, xblk,
+                        map_rank(smem_u32(sm.xa_full), base_rank + warp));
+        par ^= 1u << PAR_RDY;
+        // ---- merge
+        mbar_wait_cluster(sm.xa_full, par_bit(par, PAR_XA), wc, CL_DEV_TIMEOUT);
+        par ^= 1u << PAR_XA;
+        if (vrows <= 0) continue;
+        for (int it = tid; it < vrows * (HD / 4); it += CL_THREADS) {
+            const int c4 = it % (HD / 4), lrow = it / (HD / 4);
+            const float *rv = reinterpret_cast<const float *>(recv) + (size_t)lrow * OP;
+            float mmax = -INFINITY, L = 0.0f;
+            for (int s = 0; s < ad; ++s) mmax = fmaxf(mmax, rv[(size_t)s * rpo * OP + HD]);
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int s = 0; s < ad; ++s) {
+                const float2 m = *reinterpret_cast<const float2 *>(rv + (size_t)s * rpo * OP + HD);
+                if (m.x == -INFINITY) continue;
+                const float4 v = *reinterpret_cast<const float4 *>(rv + (size_t)s * rpo * OP + c4 * 4);
+                const float w = ex2f(m.x - mmax);
+                o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w);
+                L = fmaf(w, m.y, L);
+            }
+            const float inv = L > 0.0f ? 1.0f / L : 0.0f;
+            const int r = row0 + ar * rpo + lrow, head_l = r / S, tok = r - head_l * S, col = (kvh * gq + head_l) * HD + c4 * 4;
+            __stcg(reinterpret_cast<uint2 *>(pg.outp + sw_off(pg.out_rows8, tok, col)),
+                   make_uint2(pack_bf16(o.x * inv, o.y * inv), pack_bf16(o.z * inv, o.w * inv)));
         }
     }
-}
-
-template <int HD>
-__device__ __forceinline__ void combine_phase(const LoopPhase &p) {
-    const int R = p.R, S = p.S, ns = p.ns, n_rt = p.n_rt, gq = p.g, out_rows = p.out_rows, out_kslice = p.out_kslice;
-    const int items = p.n_kv * R * (HD / 4);
-    const float2 *ml = reinterpret_cast<const float2 *>(p.ws_ml);
-    for (int it = blockIdx.x * CL_THREADS + threadIdx.x; it < items; it += gridDim.x * CL_THREADS) {
-        const int c4 = it % (HD / 4), rr = it / (HD / 4);
-        const int kvh = rr / R, r = rr - kvh * R, rt = r >> 5, rl = r & 31;
-        const int u0 = (kvh * n_rt + rt) * ns;
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-        float L = 0.0f, mmax = -INFINITY;
-        for (int s0 = 0; s0 < ns; s0 += 8) {
-            float2 m[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) m[j] = s0 + j < ns ? __ldcg(ml + (size_t)(u0 + s0 + j) * 32 + rl) : make_float2(-INFINITY, 0.0f);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) mmax = fmaxf(mmax, m[j].x);
-        }
-        for (int s0 = 0; s0 < ns; s0 += 8) {
-            float2 m[8];
-            float4 v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (s0 + j < ns) {
-                    m[j] = __ldcg(ml + (size_t)(u0 + s0 + j) * 32 + rl);
-                    v[j] = __ldcg(reinterpret_cast<const float4 *>(p.ws_o + ((size_t)(u0 + s0 + j) * 32 + rl) * HD) + c4);
-                }
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (s0 + j < ns && m[j].x != -INFINITY) {
-                    const float w = ex2f(m[j].x - mmax);
-                    o.x = fmaf(w, v[j].x, o.x); o.y = fmaf(w, v[j].y, o.y); o.z = fmaf(w, v[j].z, o.z); o.w = fmaf(w, v[j].w, o.w);
-                    L = fmaf(w, m[j].y, L);
-                }
-        }
-        const float inv = L > 0.0f ? 1.0f / L : 0.0f;
-        const int head_l = r / S, tok = r - head_l * S;
-        const int col = (kvh * gq + head_l) * HD + c4 * 4;
-        __stcg(reinterpret_cast<uint2 *>(p.outp + pad_off(out_rows, out_kslice, tok, col)),
-               make_uint2(pack_bf16(o.x * inv, o.y * inv), pack_bf16(o.z * inv, o.w * inv)));
-    }
+    return par;
 }
 
 // prefix rows of the engine's K / V pages (observation 0) -> the padded pages the attention tiles are copied from
@@ -848,86 +998,121 @@ __device__ __noinline__ void pages_prologue(const LoopParams &lp) {
 // and what does not fit the SM's instruction cache is fetched from L2 every time).
 template <int HD>
 __global__ void __launch_bounds__(CL_BLOCK, 1) chunk_loop_kernel(const __grid_constant__ LoopParams lp) {
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    if (threadIdx.x == 0) *reinterpret_cast<int *>(smem_raw + 124) = lp.n_wtab;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    if (threadIdx.x == 0) *reinterpret_cast<int *>(smem_raw + 228) = lp.n_wtab;
     __syncthreads();
     const Smem sm = get_smem();
     WEntry *wtab = reinterpret_cast<WEntry *>(smem_raw + CL_WTAB_OFF);
     if (threadIdx.x == 0) {
         for (int i = 0; i < CL_STAGES; ++i) {
             mbar_init(&sm.full[i], 1);
-            mbar_init(&sm.empty[i], CL_THREADS / 32);
+            mbar_init(&sm.empty[i], 1);
         }
-        mbar_init(&sm.a_full[0], 1);
-        mbar_init(&sm.a_full[1], 1);
-        mbar_init(sm.done, 1);
-        *sm.abort_flag = 0;
+        mbar_init(sm.a_full, 1);
+        mbar_init(sm.acc_full, 1);
+        mbar_init(sm.acc_free, CL_THREADS / 32);
+        mbar_init(sm.k_full, 1);
+        mbar_init(sm.v_full, 1);
+        for (int i = 0; i < CL_PASSES; ++i) mbar_init(&sm.x_full[i], 1);
+        mbar_init(sm.xa_full, 1);
+        mbar_init(sm.rdy, lp.att_cta);
+        mbar_init(sm.done, 2);
+        *sm.abort_flag = smem_u32(smem_raw) & 1023u ? 1 : 0;  // the swizzled tiles count on it; an unaligned base is reported like a time-out
+        if (*sm.abort_flag) atomicCAS(lp.status, 0, CL_DEV_TIMEOUT);
+        *sm.issued = 0;
+        *sm.consumed = 0;
         fence_barrier_init();
+    }
+    if (threadIdx.x < 32) {
+        tmem_alloc(sm.tmem_slot, CL_TMEM_COLS);
+        tmem_relinquish();
     }
     for (int i = threadIdx.x; i < lp.n_wtab * 8; i += CL_BLOCK)
         reinterpret_cast<uint32_t *>(wtab)[i] = reinterpret_cast<const uint32_t *>(lp.wtab)[i];
     // descriptor of phase 0 into slot 0; from then on every phase fetches its successor's while it works
     for (int i = threadIdx.x; i < (int)(sizeof(LoopPhase) / 4); i += CL_BLOCK)
         reinterpret_cast<uint32_t *>(smem_raw + CL_DESC_OFF)[i] = reinterpret_cast<const uint32_t *>(lp.phases)[i];
+    tc_fence_before();
     __syncthreads();
-    if (threadIdx.x >= CL_THREADS) {  // the feeder warp: lane 0 works, the warp takes no part in any later barrier
+    cluster_sync_all();  // every CTA's barriers exist before another CTA of the cluster signals them
+    tc_fence_after();
+    const uint32_t tmem = *sm.tmem_slot;
+    if (threadIdx.x >= CL_THREADS) {  // the feeder and the issuer warp: lane 0 works, the warps take no part in any barrier of the computing ones
         if (threadIdx.x == CL_THREADS) feeder_loop(lp);
-        return;
-    }
-    const WaitCtx wc{sm.abort_flag, lp.status};
-    unsigned cons = 0, a_cnt = 0, barriers = 0, seq = 0;
-    pages_prologue(lp);
-    ++barriers;
-    bool ok = grid_barrier(lp, barriers * gridDim.x, sm, wc);
-    for (int step = 0; ok && step < lp.steps; ++step) {
-        for (int ph = 0; ok && ph < lp.n_phases; ++ph, ++seq) {
-            const LoopPhase &p = *reinterpret_cast<const LoopPhase *>(smem_raw + CL_DESC_OFF + (seq & 1u) * CL_DESC_BYTES);
-            if (threadIdx.x < (int)(sizeof(LoopPhase) / 16)) {  // the next phase's descriptor: asynchronous 16-byte copies
-                const int nx = ph + 1 == lp.n_phases ? 0 : ph + 1;
-                const uint32_t dst = smem_u32(smem_raw + CL_DESC_OFF + ((seq + 1) & 1u) * CL_DESC_BYTES) + threadIdx.x * 16u;
-                const uint8_t *src = reinterpret_cast<const uint8_t *>(lp.phases + nx) + threadIdx.x * 16u;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-                asm volatile("cp.async.commit_group;" ::: "memory");
-            }
-            switch (p.type) {
-            case PH_GEMM:
-                gemm_phase<2>(p, lp, step, cons, a_cnt);
-                break;
-            case PH_EMBED: embed_phase(p, lp, step); break;
-            case PH_ATT:
-                att_phase<HD>(p, lp, a_cnt);
-                break;
-            default:
-                combine_phase<HD>(p);
-                break;
-            }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            ++barriers;
-            ok = grid_barrier(lp, barriers * gridDim.x, sm, wc);
-            if (lp.trace && blockIdx.x == 0 && threadIdx.x == 0) {
-                unsigned long long t;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-                lp.trace[barriers - 2] = t;
+        if (threadIdx.x == CL_THREADS + 32) issuer_loop(lp, tmem);
+        __syncwarp();
+    } else {
+        const WaitCtx wc{sm.abort_flag, lp.status};
+        unsigned target = gridDim.x, seq = 0, par = 0;
+        pages_prologue(lp);
+        grid_arrive(lp);
+        bool ok = true;
+        for (int step = 0; ok && step < lp.steps; ++step) {
+            for (int ph = 0; ok && ph < lp.n_phases; ++ph, ++seq) {
+                const LoopPhase &p = *reinterpret_cast<const LoopPhase *>(smem_raw + CL_DESC_OFF + (seq & 1u) * CL_DESC_BYTES);
+                if (threadIdx.x < (int)(sizeof(LoopPhase) / 16)) {  // the next phase's descriptor: asynchronous 16-byte copies
+                    const int nx = ph + 1 == lp.n_phases ? 0 : ph + 1;
+                    const uint32_t dst = smem_u32(smem_raw + CL_DESC_OFF + ((seq + 1) & 1u) * CL_DESC_BYTES) + threadIdx.x * 16u;
+                    const uint8_t *src = reinterpret_cast<const uint8_t *>(lp.phases + nx) + threadIdx.x * 16u;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                }
+                switch (p.type) {  // every phase waits for `target` arrivals once it has prepared what it can
+                case PH_GEMM: par = gemm_phase(p, lp, step, par, target, tmem); break;
+                case PH_EMBED: embed_phase(p, lp, step, target); break;
+                default: par = att_phase<HD>(p, lp, par, target); break;
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                target += gridDim.x;
+                grid_arrive(lp);  // (and every warp's part of the next descriptor is in place)
+                ok = *sm.abort_flag == 0;
+                if (lp.trace && blockIdx.x == 0 && threadIdx.x == 0) {
+                    unsigned long long t;
+                    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+                    lp.trace[seq] = t;
+                }
             }
         }
+        grid_wait(lp, target, sm);
+        // Weight chunks still on their way must land before the CTA gives its shared memory back (only after a failure are
+        // there any: the feeder stops with the computation).
+        if (threadIdx.x == 0 && mbar_wait(sm.done, 0u, wc, CL_DEV_TIMEOUT))
+            for (unsigned i = *sm.consumed, n = *sm.issued; i < n; ++i) mbar_wait(&sm.full[i % CL_STAGES], (i / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
+        if (*sm.abort_flag) __nanosleep(1000000);  // after a failure: products in flight, peers that may still be writing
+        tc_fence_before();
+        __syncwarp();
     }
-    // Weight chunks still on their way must land before the CTA gives its shared memory back (only after a failure are
-    // there any: the feeder stops with the computation).
-    if (threadIdx.x == 0 && mbar_wait(sm.done, 0u, wc, CL_DEV_TIMEOUT)) {
-        const unsigned issued = *reinterpret_cast<volatile unsigned *>(smem_raw + 384);
-        for (unsigned i = cons; i < issued; ++i) mbar_wait(&sm.full[i % CL_STAGES], (i / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
+    __syncthreads();
+    cluster_sync_all();  // no CTA leaves while another of its cluster may still write into its shared memory
+    if (threadIdx.x < 32) {
+        tc_fence_after();
+        tmem_dealloc(tmem, CL_TMEM_COLS);
     }
-    cons_sync();
 }
 
-// dense [rows][K] bf16 -> padded image with K slices of `kslice` columns (the pad bytes stay zero)
-__global__ void pad_image_kernel(const __nv_bfloat16 *__restrict__ src, uint8_t *__restrict__ dst, int rows, int K, int kslice) {
-    const size_t total = (size_t)rows * (K / 8);
+// dense [N][K] bf16 -> weight image for G CTA groups: [group][pass][64-column block][8-column group][8 rows x 128 bytes, 16-byte
+// chunks permuted by the row]; zeros beyond K.
+// half > 0 (q|k|v): a group's 8 columns are dims 4 j .. 4 j + 3 of a head and their rotation partners, `half` further on.
+__global__ void weight_image_kernel(const __nv_bfloat16 *__restrict__ src, uint4 *__restrict__ dst, int N8, int K, int G, int half) {
+    const int kb = (K + 63) >> 6;
+    const size_t total = (size_t)N8 * kb * 64;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int row = (int)(i / (K / 8)), col = (int)(i % (K / 8)) * 8;
-        *reinterpret_cast<uint4 *>(dst + pad_off(rows, kslice, row, col)) = *reinterpret_cast<const uint4 *>(src + (size_t)row * K + col);
+        const int c16 = (int)(i & 7), c = (int)(i >> 3) & 7;
+        size_t r = i >> 6;
+        const int b = (int)(r % kb), n8 = (int)(r / kb);
+        const int grp = (int)((((long long)n8 + 1) * G - 1) / N8), j0 = (int)((long long)N8 * grp / G), w8 = (int)((long long)N8 * (grp + 1) / G) - j0;
+        const int p0 = (n8 - j0) / CL_PASS_N8 * CL_PASS_N8, w8p = min(CL_PASS_N8, w8 - p0), j = n8 - j0 - p0;
+        int row = n8 * 8 + c;
+        if (half > 0) {
+            const int per = half >> 2, head = n8 / per, jj = n8 - head * per;
+            row = head * 2 * half + 4 * jj + (c & 3) + (c >= 4 ? half : 0);
+        }
+        const int k = b * 64 + c16 * 8;
+        const uint4 v = k < K ? *reinterpret_cast<const uint4 *>(src + (size_t)row * K + k) : make_uint4(0u, 0u, 0u, 0u);
+        dst[((size_t)(j0 + p0) * kb + (size_t)b * w8p + j) * 64 + c * 8 + (c16 ^ c)] = v;
     }
 }
+
 
 // pi0.5: the adaptive norm's shift passes through the projection as a per-column constant,
 // out[s][n] = (add ? add[n] : 0) + sum_k W[n][k] shift_s[k]   (shift_s = shift + s * stride; one warp per (s, n))
@@ -951,40 +1136,72 @@ __global__ void shift_bias_kernel(const __nv_bfloat16 *__restrict__ W, const flo
 // ------------------------------------------------------------------------------------------------ host
 struct ChunkLoop {
     const void *kernel = nullptr;
-    DevBuf phases, wtab, counter, ws_o, ws_ml, trace;
+    DevBuf phases, wtab, counter, trace;
     DevBuf hbp, ap, m1p, attp, gp, qp, kpp, vpp;  // padded activations and pages
-    DevBuf ssq;                                    // [H / 16][64] partial sums of squares of the residual mirror
+    DevBuf ssq0, ssq;                              // [H / 8][64] partial sums of squares of the residual mirror: embedding's, residual updates'
     std::vector<DevBuf> cvec;                      // pi0.5: the shift terms of every norm, [steps][N] each
-    std::vector<DevBuf> wp;                        // padded weights
+    std::vector<DevBuf> wp;                        // weight images
     int n_phases = 0, steps = 0, n_cta = 0;
     LoopParams lp{};
 };
 
 namespace {
 
-// K slices of a projection's A operand: one when all of K (<= 1024 columns) fits the arena beside the scratch tile, else the
-// fewest of at most 512 columns such that TWO of them fit (they alternate: the next slice loads while this one is
-// multiplied).  The slices of a unit run back to back on one CTA and accumulate in registers.
-int choose_kslices(int K, int M) {
-    if (K <= CL_MAX_KSLICE && K % 16 == 0 && (size_t)M * (K * 2 + 16) + (size_t)4 * M * CL_SC_ROW <= (size_t)CL_ARENA) return 1;
-    for (int ks = 2; ks <= 64; ++ks) {
-        if (K % ks) continue;
-        const int kslice = K / ks;
-        if (kslice % 16 || kslice > 512) continue;
-        if ((size_t)2 * M * (kslice * 2 + 16) + (size_t)4 * M * CL_SC_ROW > (size_t)CL_ARENA) continue;
-        return ks;
+// one CTA per SM in clusters, all co-resident (the kernel's CTAs wait for one another)
+void loop_launch_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int n_cta, cudaStream_t stream) {
+    cfg->gridDim = dim3(n_cta);
+    cfg->blockDim = dim3(CL_BLOCK);
+    cfg->dynamicSmemBytes = CL_SMEM;
+    cfg->stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 2;
+}
+
+int round_up(int v, int m) { return (v + m - 1) / m * m; }
+size_t image_bytes(int rows, int K) { return (size_t)round_up(rows, 8) * 128 * ((K + 63) / 64); }
+
+// one pass of a group: kd parts of the most columns one CTA owns
+size_t exchange_bytes(int M, int w8, int kd) { return (size_t)round_up(std::min(w8, CL_PASS_N8), kd) * 8 * token_pitch(M) * 4; }
+
+// Does a product fit the arena when kd CTAs share its K?  A of one CTA + what the group sends it + its own sums, staged.
+bool gemm_fits(int M, int N8, int K, int kd, int n_cta) {
+    const int G = n_cta / kd, w8 = (N8 + G - 1) / G, passes = (w8 + CL_PASS_N8 - 1) / CL_PASS_N8, kb = (K + 63) / 64;
+    if (passes > CL_PASSES) return false;
+    const size_t a = (size_t)((kb + kd - 1) / kd) * round_up(M, 8) * 128, x = exchange_bytes(M, w8, kd);
+    return a + x * (passes == 1 ? (x <= a ? 1 : 2) : 2 * CL_PASSES) <= (size_t)CL_ARENA;
+}
+
+// End of the arena range in which a product's own sums are staged (gemm_phase: over A when they fit there in one pass).
+size_t staged_end(int M, int w8, int K, int kd) {
+    const int kb = (K + 63) / 64, passes = (w8 + CL_PASS_N8 - 1) / CL_PASS_N8;
+    const size_t a = (size_t)((kb + kd - 1) / kd) * round_up(M, 8) * 128, x = exchange_bytes(M, w8, kd);
+    return passes == 1 && x <= a ? x : a + (passes == 1 ? 2 : 2 * CL_PASSES) * x;
+}
+
+// CTAs that share a product's K: least (A in at ~50 B/ns and SM, partial sums out at ~20 B/ns, products at ~48 clocks per 128 x 64 x
+// 16).  More CTAs per group read less of A and send more partial sums.
+int choose_kd(int M, int N8, int K, int n_cta) {
+    int best = 0;
+    double best_cost = 0;
+    for (int kd = 1; kd <= CL_CLUSTER; kd *= 2) {
+        if ((kd > 1 && (K + 63) / 64 < kd) || !gemm_fits(M, N8, K, kd, n_cta)) continue;
+        const int G = n_cta / kd, w8 = (N8 + G - 1) / G, kb = ((K + 63) / 64 + kd - 1) / kd;
+        const double a = (double)M * kb * 128 / 50.0, x = (double)M * w8 * 32 * (kd - 1) / kd / 20.0;
+        double mma = 0;
+        for (int p = 0; p < w8; p += CL_PASS_N8) mma += kb * 4 * (std::min(CL_PASS_N8, w8 - p) > 16 ? 2 : 1) * 48 / 1.9;
+        const double cost = a + x + mma;
+        if (!best || cost < best_cost) {
+            best = kd;
+            best_cost = cost;
+        }
     }
-    return 0;
+    return best;
 }
-
-// columns per weight chunk of a unit of `ng` groups: the largest divisor of the A slice that is a multiple of 16 and fits a ring stage
-int pick_kchunk(int kslice, int ng) {
-    for (int kc = std::min(kslice, CL_MAX_KSLICE); kc >= 16; --kc)
-        if (kslice % kc == 0 && kc % 16 == 0 && (size_t)ng * 8 * (kc * 2 + 16) <= (size_t)CL_STAGE_BYTES) return kc;
-    return 0;
-}
-
-size_t image_bytes(int rows, int K, int kslices) { return (size_t)kslices * rows * ((size_t)(K / kslices) * 2 + 16); }
 
 }  // namespace
 
@@ -995,23 +1212,32 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
     const int hd = d.hd, half = hd / 2, qf = d.n_q * hd, H = d.H, S = d.S;
     if (d.model < 0 || d.model > 2 || (d.model == 2 && (!d.mods || H % 32))) return VLAB200_ERR_UNSUPPORTED;
     if (hd != 64 && hd != 128 && hd != 256) return VLAB200_ERR_UNSUPPORTED;
-    if (S > 64 || H % 16 || H > CL_MAX_KSLICE || d.A % 16 || (2 * d.I) % 16 || qf % 16 || d.I % 16) return VLAB200_ERR_UNSUPPORTED;
-    if ((size_t)S * (H * 2 + 16) + (size_t)4 * S * CL_SC_ROW > (size_t)CL_ARENA) return VLAB200_ERR_UNSUPPORTED;
+    if (S > 64 || H % 16 || d.A % 16 || (2 * d.I) % 16 || qf % 16 || d.I % 16) return VLAB200_ERR_UNSUPPORTED;
     if ((size_t)(d.chunk * d.A + 64) * 4 > (size_t)CL_ARENA || d.A > 64) return VLAB200_ERR_UNSUPPORTED;
-    int occ = 0;
     const void *kernel = hd == 64    ? reinterpret_cast<const void *>(chunk_loop_kernel<64>)
                          : hd == 128 ? reinterpret_cast<const void *>(chunk_loop_kernel<128>)
                                      : reinterpret_cast<const void *>(chunk_loop_kernel<256>);
     if (ensure_dyn_smem(kernel, CL_SMEM)) return VLAB200_ERR_CUDA;
-    VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, CL_BLOCK, CL_SMEM));
-    int coop = 0, dev = 0;
+    int coop = 0, dev = 0, n_clusters = 0;
     VB_CUDA(cudaGetDevice(&dev));
     VB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (occ < 1 || !coop) return VLAB200_ERR_UNSUPPORTED;
-    const int n_cta = n_sm;
+    {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr[2];
+        loop_launch_config(&cfg, attr, n_sm / CL_CLUSTER * CL_CLUSTER, nullptr);
+        VB_CUDA(cudaOccupancyMaxActiveClusters(&n_clusters, kernel, &cfg));
+    }
+    n_clusters = std::min(n_clusters, n_sm / CL_CLUSTER);
+    if (n_clusters < 1 || !coop) return VLAB200_ERR_UNSUPPORTED;
+    const int n_cta = n_clusters * CL_CLUSTER;
     const int g = d.n_q / d.n_kv, R = g * S, n_rt = (R + 31) / 32;
-    const int ks_o = choose_kslices(qf, S), ks_d = choose_kslices(d.I, S);
-    if (!ks_o || !ks_d) return VLAB200_ERR_UNSUPPORTED;
+    const int qkv_n8 = (d.n_q + 2 * d.n_kv) * hd / 8;
+    const int kd_qkv = choose_kd(S, qkv_n8, H, n_cta), kd_gu = choose_kd(S, 2 * d.I / 8, H, n_cta), kd_o = choose_kd(S, H / 8, qf, n_cta);
+    const int kd_d = choose_kd(S, H / 8, d.I, n_cta), kd_m = choose_kd(d.chunk, H / 8, H, n_cta), kd_h = choose_kd(S, d.A / 8, H, n_cta);
+    if (!kd_qkv || !kd_gu || !kd_o || !kd_d || !kd_m || !kd_h) return VLAB200_ERR_UNSUPPORTED;
+    // attention units of 32 query rows: as many CTAs each as there are for one round (they split the keys)
+    int att_cta = 1;
+    while (att_cta < CL_CLUSTER && d.n_kv * n_rt <= n_cta / (2 * att_cta)) att_cta *= 2;
 
     ChunkLoop *cl = new (std::nothrow) ChunkLoop();
     if (!cl) return VLAB200_ERR_CUDA;
@@ -1022,27 +1248,24 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
     };
     const uint32_t sq = (uint32_t)hd * 2u + 16u;
     const size_t page_layer = (size_t)d.n_kv * d.cap * sq;
-    if ((rc = cl->hbp.alloc(image_bytes(S, H, 1))) || (rc = cl->ap.alloc(image_bytes(d.chunk, H, 1))) ||
-        (rc = cl->m1p.alloc(image_bytes(d.chunk, H, 1))) || (rc = cl->attp.alloc(image_bytes(S, qf, ks_o))) ||
-        (rc = cl->gp.alloc(image_bytes(S, d.I, ks_d))) || (rc = cl->qp.alloc((size_t)d.n_q * S * sq)) ||
-        (rc = cl->kpp.alloc(page_layer * d.L)) || (rc = cl->vpp.alloc(page_layer * d.L)) || (rc = cl->ssq.alloc((size_t)(H / 16) * 64 * 4)))
-        return fail(rc);
-    for (DevBuf *b : {&cl->hbp, &cl->ap, &cl->m1p, &cl->attp, &cl->gp, &cl->qp})
-        if (cudaMemset(b->p, 0, 16) != cudaSuccess) return fail(VLAB200_ERR_CUDA);
-    if (cudaMemset(cl->hbp.p, 0, image_bytes(S, H, 1)) != cudaSuccess || cudaMemset(cl->ap.p, 0, image_bytes(d.chunk, H, 1)) != cudaSuccess ||
-        cudaMemset(cl->m1p.p, 0, image_bytes(d.chunk, H, 1)) != cudaSuccess || cudaMemset(cl->attp.p, 0, image_bytes(S, qf, ks_o)) != cudaSuccess ||
-        cudaMemset(cl->gp.p, 0, image_bytes(S, d.I, ks_d)) != cudaSuccess || cudaMemset(cl->qp.p, 0, (size_t)d.n_q * S * sq) != cudaSuccess ||
-        cudaMemset(cl->kpp.p, 0, page_layer * d.L) != cudaSuccess || cudaMemset(cl->vpp.p, 0, page_layer * d.L) != cudaSuccess)
-        return fail(VLAB200_ERR_CUDA);
-    // padded weight images
-    auto pad_weight = [&](const void *w, int rows, int K, int kslices, const uint8_t **image) -> int {
+    struct {
+        DevBuf *b;
+        size_t bytes;
+    } const zeroed[] = {{&cl->hbp, image_bytes(S, H)},     {&cl->ap, image_bytes(d.chunk, H)}, {&cl->m1p, image_bytes(d.chunk, H)},
+                        {&cl->attp, image_bytes(S, qf)},   {&cl->gp, image_bytes(S, d.I)},     {&cl->qp, (size_t)d.n_q * S * sq},
+                        {&cl->kpp, page_layer * d.L},            {&cl->vpp, page_layer * d.L},             {&cl->ssq0, (size_t)(H / 8) * 64 * 4},
+                        {&cl->ssq, (size_t)(H / 8) * 64 * 4}};
+    for (const auto &z : zeroed) {
+        if ((rc = z.b->alloc(z.bytes))) return fail(rc);
+        if (cudaMemset(z.b->p, 0, z.bytes) != cudaSuccess) return fail(VLAB200_ERR_CUDA);
+    }
+    // weights as tcgen05 reads them, in the order of the CTA groups
+    auto weight_image = [&](const void *w, int N8, int K, int kd, int half_, const uint8_t **image) -> int {
         cl->wp.emplace_back();
         DevBuf &b = cl->wp.back();
-        const size_t bytes = image_bytes(rows, K, kslices);
-        int r = b.alloc(bytes);
+        int r = b.alloc((size_t)N8 * ((K + 63) / 64) * 1024);
         if (r) return r;
-        VB_CUDA(cudaMemset(b.p, 0, bytes));
-        pad_image_kernel<<<n_sm * 4, 256>>>(static_cast<const __nv_bfloat16 *>(w), b.as<uint8_t>(), rows, K, K / kslices);
+        weight_image_kernel<<<n_sm * 4, 256>>>(static_cast<const __nv_bfloat16 *>(w), b.as<uint4>(), N8, K, n_cta / kd, half_);
         VB_CUDA(cudaGetLastError());
         *image = b.as<uint8_t>();
         return VLAB200_OK;
@@ -1051,17 +1274,17 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
 
     std::vector<LoopPhase> ph;
     bool bad = false;
-    auto gemm = [&](const uint8_t *Ap, int M, const void *w_dense, int N, int K, int kslices, int out_mode) {
+    auto gemm = [&](const uint8_t *Ap, int M, const void *w_dense, int N, int K, int kd, int out_mode) {
         LoopPhase p{};
-        p.type = PH_GEMM; p.out_mode = out_mode; p.Ap = Ap; p.M = M; p.N = N; p.K = K; p.kslices = kslices;
-        p.ng = 2;  // units of 4 groups (half as many, twice the weight bytes each) measured 2-5 % slower, and their code costs instruction cache
-        p.kchunk = pick_kchunk(K / kslices, p.ng);
-        p.n_sub = N / (8 * p.ng);
+        p.type = PH_GEMM; p.out_mode = out_mode; p.Ap = Ap; p.M = M; p.N8 = N / 8; p.K = K; p.kd = kd;
+        p.half = out_mode == OUT_QKV ? half : 0;
         p.eps = d.rms_eps; p.S = S; p.chunk = d.chunk;
-        if (!p.kchunk || pad_weight(w_dense, N, K, K / p.kchunk, &p.Wp)) bad = true;
+        if (weight_image(w_dense, N / 8, K, kd, p.half, &p.Wp)) bad = true;
         return p;
     };
-    size_t ws_units = 0;
+    auto to_mirror = [&](LoopPhase &p) {  // the phase writes the residual mirror
+        p.outp = cl->hbp.as<uint8_t>(); p.out_rows8 = round_up(S, 8);
+    };
     const bool ada = d.model == 2;
     const size_t mod_step = (size_t)3 * H, mod_block = (size_t)d.steps * mod_step;  // one norm's vectors for every step
     auto mod_in = [&](int l) { return d.mods + (size_t)(2 * l) * mod_block; };
@@ -1088,17 +1311,18 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
         p.outp = cl->ap.as<uint8_t>(); p.chunk = d.chunk; p.A_dim = d.A; p.H = H; p.S = S;
         p.sd = d.model == 0 ? d.sd : 0; p.w2 = static_cast<const __nv_bfloat16 *>(d.w_sp); p.b2 = d.b_sp; p.h = d.h;
         p.hbp = cl->hbp.as<uint8_t>();
+        p.ssq_out = cl->ssq0.as<float>();
         if (ada) {  // the embedding is the residual stream; its mirror carries the first norm's (1 + scale)
-            p.scale_next = mod_in(0); p.mod_stride = (long long)mod_step; p.ssq_out = cl->ssq.as<float>();
+            p.scale_next = mod_in(0); p.mod_stride = (long long)mod_step;
         }
         ph.push_back(p);
         if (!ada) {
-            LoopPhase m1 = gemm(cl->ap.as<uint8_t>(), d.chunk, d.w_at1l, H, H, 1, OUT_BIAS_ACT);
-            m1.act = ACT_SILU; m1.bias = d.tvec; m1.bias_step_stride = H; m1.outp = cl->m1p.as<uint8_t>(); m1.out_rows = d.chunk; m1.out_kslice = H;
+            LoopPhase m1 = gemm(cl->ap.as<uint8_t>(), d.chunk, d.w_at1l, H, H, kd_m, OUT_BIAS_ACT);
+            m1.act = ACT_SILU; m1.bias = d.tvec; m1.bias_step_stride = H; m1.outp = cl->m1p.as<uint8_t>(); m1.out_rows8 = round_up(d.chunk, 8);
             ph.push_back(m1);
-            LoopPhase m2 = gemm(cl->m1p.as<uint8_t>(), d.chunk, d.w_at2, H, H, 1, OUT_BIAS_ACT);
-            m2.act = ACT_NONE; m2.bias = d.b_at2; m2.outp = cl->hbp.as<uint8_t>(); m2.out_rows = S; m2.out_kslice = H; m2.out_f32 = d.h;
-            m2.row_off = S - d.chunk;
+            LoopPhase m2 = gemm(cl->m1p.as<uint8_t>(), d.chunk, d.w_at2, H, H, kd_m, OUT_BIAS_ACT);
+            m2.act = ACT_NONE; m2.bias = d.b_at2; m2.out_f32 = d.h; m2.row_off = S - d.chunk; m2.ssq_out = cl->ssq0.as<float>();
+            to_mirror(m2);
             ph.push_back(m2);
         }
     }
@@ -1106,9 +1330,9 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
         const bool self = d.is_self[l];
         uint8_t *kp = cl->kpp.as<uint8_t>() + (size_t)l * page_layer, *vp = cl->vpp.as<uint8_t>() + (size_t)l * page_layer;
         const int n_heads = d.n_q + (self ? 2 * d.n_kv : 0);
-        LoopPhase qkv = gemm(cl->hbp.as<uint8_t>(), S, d.wqkv[l], n_heads * hd, H, 1, OUT_QKV);
-        qkv.use_rms = (l == 0 && !ada) ? RMS_LOCAL : RMS_PARTS; qkv.ssq_in = cl->ssq.as<float>(); qkv.ssq_n = (l == 0 && ada) ? H / 32 : H / 16;
-        qkv.half = half; qkv.qp = cl->qp.as<uint8_t>();
+        LoopPhase qkv = gemm(cl->hbp.as<uint8_t>(), S, d.wqkv[l], n_heads * hd, H, kd_qkv, OUT_QKV);
+        qkv.use_rms = 1; qkv.ssq_in = l == 0 ? cl->ssq0.as<float>() : cl->ssq.as<float>(); qkv.ssq_n = (l == 0 && ada) ? H / 32 : H / 8;
+        qkv.qp = cl->qp.as<uint8_t>();
         if (ada) {
             if ((rc = shift_bias(d.wqkv[l], n_heads * hd, mod_in(l), nullptr, &qkv.bias))) return fail(rc);
             qkv.bias_step_stride = n_heads * hd;
@@ -1117,57 +1341,74 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
         qkv.cap = d.cap; qkv.P = d.P;
         ph.push_back(qkv);
         LoopPhase at{};
-        at.type = PH_ATT; at.hd = hd; at.qp = cl->qp.as<uint8_t>(); at.kpp = kp; at.vpp = vp; at.n_kv = d.n_kv; at.g = g;
+        at.type = PH_ATT; at.qp = cl->qp.as<uint8_t>(); at.kpp = kp; at.vpp = vp; at.n_kv = d.n_kv; at.g = g;
         at.S = S; at.R = R; at.n_rt = n_rt; at.kv_len = self ? d.P + S : d.P; at.P = d.P; at.cap = d.cap; at.n_q = d.n_q;
         at.mask_mode = (self && !ada) ? (d.model == 0 ? 1 : 2) : 0;  // pi0.5: every action token sees the prefix and every action token
         at.scale_log2 = 1.4426950408889634f / std::sqrt((float)hd);
-        {   // keys per slice: the fewest rounds over the CTAs, then the cheapest unit
-            int best = 0;
-            double best_cost = 0;
-            for (int ks = 16; ks <= 96; ks += 16) {
-                if ((size_t)32 * sq + (size_t)2 * ks * sq + (size_t)32 * (ks + 8) * 2 > (size_t)CL_ARENA) continue;
-                const int ns = (at.kv_len + ks - 1) / ks;
-                if (ns > 64) continue;
-                const int units = d.n_kv * n_rt * ns;
-                const double cost = (double)((units + n_cta - 1) / n_cta) * (600.0 + (double)ks * hd * 0.07) + 10.0 * ns;
-                if (!best || cost < best_cost) {
-                    best = ks;
-                    best_cost = cost;
+        at.kd = att_cta;
+        at.per = (at.kv_len + att_cta - 1) / att_cta;  // keys per CTA
+        at.outp = cl->attp.as<uint8_t>(); at.out_rows8 = round_up(S, 8);
+        {   // the fewest key blocks whose tiles fit: Q | K | V | probabilities (over Q when there is one block) | exchanged rows
+            // (over K when there is no room behind: a CTA sends only after its group has read K)
+            // Own rows are staged over V, or behind.  K and V may be copied before the grid barrier where they lie behind q|k|v's
+            // staged sums, which may still be on their way to its group.
+            const int rows = 32 * (hd + 8) * 4, q_bytes = 32 * (int)sq;
+            const int w8q = (n_heads * hd / 8 + n_cta / kd_qkv - 1) / (n_cta / kd_qkv), stg_end = (int)staged_end(S, w8q, H, kd_qkv);
+            bool found = false;
+            for (int nb = 1; !found && nb <= at.per; ++nb) {
+                const int ks = (at.per + nb - 1) / nb, ks16 = round_up(ks, 16), pbytes = 32 * (ks16 + 8) * 2;
+                if (ks > 128) continue;
+                for (int apart = 1; !found && apart >= 0; --apart) {
+                    const int k_off = apart ? std::max(q_bytes, round_up(stg_end, 16)) : q_bytes, v_off = k_off + ks * (int)sq, v_end = v_off + ks16 * (int)sq;
+                    const bool p_over_q = nb == 1 && pbytes <= k_off;
+                    int end = v_end + (p_over_q ? 0 : pbytes);
+                    at.p_off = p_over_q ? 0 : v_end;
+                    at.k_off = at.recv_off = k_off;
+                    at.stage_off = v_off;
+                    if (rows > ks16 * (int)sq) {
+                        at.stage_off = end;
+                        end += rows;
+                    }
+                    if (end + rows <= CL_ARENA || rows > ks * (int)sq) {
+                        at.recv_off = end;
+                        end += rows;
+                    }
+                    if (end > CL_ARENA) continue;
+                    at.ks = ks;
+                    at.early_k = k_off >= stg_end;
+                    at.early_v = v_off >= stg_end;
+                    found = true;
                 }
             }
-            if (!best) bad = true;
-            at.ks = best ? best : 16;
-            at.ns = (at.kv_len + at.ks - 1) / at.ks;
+            if (!found) bad = true;
         }
-        ws_units = std::max(ws_units, (size_t)d.n_kv * n_rt * at.ns);
         ph.push_back(at);
-        LoopPhase cb = at;
-        cb.type = PH_COMBINE; cb.outp = cl->attp.as<uint8_t>(); cb.out_rows = S; cb.out_kslice = qf / ks_o;
-        ph.push_back(cb);
-        LoopPhase o = gemm(cl->attp.as<uint8_t>(), S, d.wo[l], H, qf, ks_o, OUT_RESID);
-        o.h = d.h; o.hbp = cl->hbp.as<uint8_t>(); o.ssq_out = cl->ssq.as<float>();
+        LoopPhase o = gemm(cl->attp.as<uint8_t>(), S, d.wo[l], H, qf, kd_o, OUT_RESID);
+        to_mirror(o);
+        o.h = d.h; o.ssq_out = cl->ssq.as<float>();
         if (ada) {
             o.colscale = mod_in(l) + 2 * H; o.scale_next = mod_post(l); o.mod_stride = (long long)mod_step;
         }
         ph.push_back(o);
-        LoopPhase gu = gemm(cl->hbp.as<uint8_t>(), S, d.wgu[l], 2 * d.I, H, 1, OUT_GATED);
-        gu.use_rms = RMS_PARTS; gu.ssq_in = cl->ssq.as<float>(); gu.ssq_n = H / 16;
-        gu.act = d.act; gu.outp = cl->gp.as<uint8_t>(); gu.out_rows = S; gu.out_kslice = d.I / ks_d;
+        LoopPhase gu = gemm(cl->hbp.as<uint8_t>(), S, d.wgu[l], 2 * d.I, H, kd_gu, OUT_GATED);
+        gu.use_rms = 1; gu.ssq_in = cl->ssq.as<float>(); gu.ssq_n = H / 8;
+        gu.act = d.act; gu.outp = cl->gp.as<uint8_t>(); gu.out_rows8 = round_up(S, 8);
         if (ada) {
             if ((rc = shift_bias(d.wgu[l], 2 * d.I, mod_post(l), nullptr, &gu.bias))) return fail(rc);
             gu.bias_step_stride = 2 * d.I;
         }
         ph.push_back(gu);
-        LoopPhase dn = gemm(cl->gp.as<uint8_t>(), S, d.wdown[l], H, d.I, ks_d, OUT_RESID);
-        dn.h = d.h; dn.hbp = cl->hbp.as<uint8_t>(); dn.ssq_out = cl->ssq.as<float>();
+        LoopPhase dn = gemm(cl->gp.as<uint8_t>(), S, d.wdown[l], H, d.I, kd_d, OUT_RESID);
+        to_mirror(dn);
+        dn.h = d.h; dn.ssq_out = cl->ssq.as<float>();
         if (ada) {
             dn.colscale = mod_post(l) + 2 * H; dn.scale_next = l + 1 < d.L ? mod_in(l + 1) : mod_final; dn.mod_stride = (long long)mod_step;
         }
         ph.push_back(dn);
     }
     {
-        LoopPhase hdp = gemm(cl->hbp.as<uint8_t>(), S, d.w_aout, d.A, H, 1, OUT_EULER);
-        hdp.use_rms = RMS_PARTS; hdp.ssq_in = cl->ssq.as<float>(); hdp.ssq_n = H / 16; hdp.bias = d.b_aout; hdp.x = d.x; hdp.dt = -1.0f / (float)d.steps;
+        LoopPhase hdp = gemm(cl->hbp.as<uint8_t>(), S, d.w_aout, d.A, H, kd_h, OUT_EULER);
+        hdp.use_rms = 1; hdp.ssq_in = cl->ssq.as<float>(); hdp.ssq_n = H / 8; hdp.bias = d.b_aout; hdp.x = d.x; hdp.dt = -1.0f / (float)d.steps;
         if (ada) {
             if ((rc = shift_bias(d.w_aout, d.A, mod_final, d.b_aout, &hdp.bias))) return fail(rc);
             hdp.bias_step_stride = d.A;
@@ -1175,27 +1416,19 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
         ph.push_back(hdp);
     }
     if (bad) return fail(VLAB200_ERR_UNSUPPORTED);
-    if ((rc = cl->ws_o.alloc(ws_units * 32 * hd * 4)) || (rc = cl->ws_ml.alloc(ws_units * 32 * 2 * 4)) ||
-        (rc = cl->phases.alloc(ph.size() * sizeof(LoopPhase))) || (rc = cl->counter.alloc(64)))
-        return fail(rc);
-    for (LoopPhase &p : ph)
-        if (p.type == PH_ATT || p.type == PH_COMBINE) {
-            p.ws_o = cl->ws_o.as<float>();
-            p.ws_ml = cl->ws_ml.as<float>();
-        }
+    if ((rc = cl->phases.alloc(ph.size() * sizeof(LoopPhase))) || (rc = cl->counter.alloc(64))) return fail(rc);
     std::vector<WEntry> wt;
     for (const LoopPhase &p : ph)
         if (p.type == PH_GEMM) {
             WEntry w{};
-            w.Wp = p.Wp; w.n_units = p.n_sub; w.n_chunks = p.K / p.kchunk; w.N = p.N; w.half = p.half; w.ng = p.ng;
-            w.stride = (uint32_t)p.kchunk * 2u + 16u;
+            w.Wp = p.Wp; w.N8 = p.N8; w.K = p.K; w.kd = p.kd; w.M = p.M;
             wt.push_back(w);
         }
     if ((int)wt.size() > CL_WTAB_MAX) return fail(VLAB200_ERR_UNSUPPORTED);
     if ((rc = cl->wtab.alloc(wt.size() * sizeof(WEntry)))) return fail(rc);
     cudaError_t ce = cudaMemcpy(cl->wtab.p, wt.data(), wt.size() * sizeof(WEntry), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemcpy(cl->phases.p, ph.data(), ph.size() * sizeof(LoopPhase), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess) ce = cudaDeviceSynchronize();  // the padded weight images are complete
+    if (ce == cudaSuccess) ce = cudaDeviceSynchronize();  // the weight images are complete
     if (ce != cudaSuccess) {
         delete cl;
         return cuda_fail(ce, "chunk loop: phase table / weight images");
@@ -1209,6 +1442,7 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
     lp.n_phases = cl->n_phases;
     lp.wtab = cl->wtab.p;
     lp.n_wtab = (int)wt.size();
+    lp.att_cta = att_cta;
     lp.steps = d.steps;
     lp.counter = cl->counter.as<unsigned>();
     lp.status = device_status_ptr();
@@ -1238,12 +1472,15 @@ int chunk_loop_run(ChunkLoop *cl, const float *state, const int32_t *pad, cudaSt
         lp.trace = cl->trace.as<unsigned long long>();
     }
     void *args[] = {&lp};
-    const cudaError_t le = cudaLaunchCooperativeKernel(cl->kernel, dim3(cl->n_cta), dim3(CL_BLOCK), args, CL_SMEM, stream);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    loop_launch_config(&cfg, attr, cl->n_cta, stream);
+    const cudaError_t le = cudaLaunchKernelExC(&cfg, cl->kernel, args);
     if (le == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device reports are ours (a partitioned GPU): not an error of the call
         cudaGetLastError();
         return VLAB200_ERR_UNSUPPORTED;
     }
-    if (le != cudaSuccess) return cuda_fail(le, "cudaLaunchCooperativeKernel");
+    if (le != cudaSuccess) return cuda_fail(le, "cudaLaunchKernelExC");
     if (lp.trace) {
         const size_t n = (size_t)cl->n_phases * cl->steps;
         std::vector<unsigned long long> t(n);
