@@ -23,6 +23,7 @@
 
 #include <cstdlib>
 
+#include <algorithm>
 #include <atomic>
 
 #include "gemm.h"
@@ -216,7 +217,9 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             uint32_t st = 0, ph = 0;
             bool ok = true;
             for (int tile = t_begin; ok && tile < t_end; ++tile) {
-                for (int kt = 0; kt < ksteps; ++kt) {
+                const int ks = SPLIT ? tile % ks_n : 0;
+                const int kbeg = SPLIT ? ks * ksteps / ks_n : 0, kend = SPLIT ? (ks + 1) * ksteps / ks_n : ksteps;
+                for (int kt = kbeg; kt < kend; ++kt) {
                     ok = mbar_wait(&full[st], ph, wc, DEV_TIMEOUT_FULL);
                     if (!ok) break;
                     mbar_arrive_cluster(&full[st], 0);
@@ -450,6 +453,12 @@ dense_gemm_splitk_kernel(const __grid_constant__ CUtensorMap a_map, const __grid
     dense_gemm_body<64, false, true>(a_map, w_map, p, tiles_m, tiles_n);
 }
 
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1)
+dense_gemm_pair_splitk_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap w_map,
+                              const GemmParams p, int tiles_m, int tiles_n) {
+    dense_gemm_body<256, true, true>(a_map, w_map, p, tiles_m, tiles_n);
+}
+
 // h[m][n] += (sum over the K slices, in slice order) (* colscale[n]) (+ bias[n]); hb = bf16(h).  Four columns per thread.
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ partial, int ksplit, int M, int N,
                                                             const float *__restrict__ colscale, const float *__restrict__ bias,
@@ -512,6 +521,18 @@ static float tiling_cost(int M, int N, int n_sm, int *variant_out) {
 
 static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, cudaStream_t stream, int forced_variant);
 
+// K slices as separate work items (variant 5: 128 x 64 tiles, 6: pair tiles), then their sum in slice order with the residual epilogue.
+static int split_residual(const void *A, int lda, const void *W, const GemmParams &p, int ksplit, int variant, int n_sm, cudaStream_t stream) {
+    GemmParams ps = p;
+    ps.ksplit = ksplit;
+    int rc = dense_gemm_one(A, lda, W, ps, stream, variant);
+    if (rc) return rc;
+    const size_t total4 = (size_t)p.M * p.N / 4;
+    const int blocks = (int)((total4 + 255) / 256 < (size_t)n_sm * 4 ? (total4 + 255) / 256 : (size_t)n_sm * 4);
+    return launch_pdl(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const float *>(p.partial), ksplit, p.M, p.N,
+                      p.colscale, p.bias, p.h, p.out_bf, p.ld_out);
+}
+
 // Launches the GEMM.  A: bf16 [M][K] (row stride lda elements), W: bf16 [N][K].
 //
 // Rows are independent, so a problem whose tiles fill the machine unevenly is cut in two along M: the first rows as
@@ -529,16 +550,27 @@ int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t
         int ksplit = n_sm / tiles;
         if (ksplit > ksteps / 4) ksplit = ksteps / 4;  // at least four 64-wide k-steps per slice
         if (ksplit > p.partial_slices) ksplit = p.partial_slices;
-        if (ksplit >= 2) {
-            GemmParams ps = p;
-            ps.ksplit = ksplit;
-            int rc = dense_gemm_one(A, lda, W, ps, stream, 5);
-            if (rc) return rc;
-            const size_t total4 = (size_t)p.M * p.N / 4;
-            const int blocks = (int)((total4 + 255) / 256 < (size_t)n_sm * 4 ? (total4 + 255) / 256 : (size_t)n_sm * 4);
-            return launch_pdl(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const float *>(p.partial), ksplit,
-                              p.M, p.N, p.colscale, p.bias, p.h, p.out_bf, p.ld_out);
+        if (ksplit >= 2) return split_residual(A, lda, W, p, ksplit, 5, n_sm, stream);
+    }
+    // Some hundred rows, long K (Wdown of a backbone, fc2 of a vision tower): one wave of narrow tiles streams all of K through each SM
+    // at about 0.35 us a 64-wide step, pair tiles would fill a fraction of the machine at 0.42 us.  K slices of pair tiles do both; the
+    // float sums and the second launch cost about 8 us + 1 us per 2.5 MB.  816 x 2048 x 16384: 97 us as 112 tiles of 128 x 128.
+    if (p.partial && p.epi == EPI_RESIDUAL && dense_gemm_variant() == 0 && p.M > 2 * G_BM && p.M <= p.partial_rows && p.rows_in == 0 &&
+        p.scatter_hd == 0 && !p.use_rms && p.N % 4 == 0 && n_sm >= 2) {
+        const int pairs = n_sm / 2, ksteps = (p.K + G_BK - 1) / G_BK, units = ((p.M + 2 * G_BM - 1) / (2 * G_BM)) * ((p.N + 255) / 256);
+        auto waves = [](int tiles, int u) { return (tiles + u - 1) / u; };
+        const int tm = (p.M + G_BM - 1) / G_BM, w64 = waves(tm * ((p.N + 63) / 64), n_sm), w128 = waves(tm * ((p.N + 127) / 128), n_sm);
+        const float whole = (float)ksteps * std::min(0.35f * (float)std::min(w64, w128), 0.42f * (float)waves(units, pairs));
+        float best = 0.9f * whole;
+        int slices = 0;
+        for (int s = 2; s <= p.partial_slices && ksteps / s >= 8; ++s) {
+            const float c = 0.42f * (float)(waves(units * s, pairs) * waves(ksteps, s)) + 8.0f + (float)(s + 2) * (float)p.M * (float)p.N * 4.0f / 2.5e6f;
+            if (c < best) {
+                best = c;
+                slices = s;
+            }
         }
+        if (slices) return split_residual(A, lda, W, p, slices, 6, n_sm, stream);
     }
     static const bool split_off = std::getenv("VLAB200_NO_GEMM_SPLIT") != nullptr;  // measurement knob
     if (!split_off && dense_gemm_variant() == 0 && n_sm >= 2 && p.rows_in == 0 && p.scatter_hd == 0 && p.M > 2 * G_BM) {
@@ -623,11 +655,17 @@ static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, c
         return launch_pdl(dense_gemm_splitk_kernel, dim3(nt < n_sm ? nt : n_sm), dim3(G_THREADS), GemmCfg<64, false>::SMEM, stream,
                           amap, wmap, p, tiles_m, tn64);
     }
-    if (variant == 3) {
+    if (variant == 3 || variant == 6) {
         const uint32_t box[2] = {G_BK, 128};  // each CTA of a pair stages half of the 256 weight rows
         int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, wdims, wstrides, box,
                                  CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
+        if (variant == 6) {
+            if (int rc = ensure_dyn_smem(dense_gemm_pair_splitk_kernel, GemmCfg<256, true>::SMEM)) return rc;
+            const int nt = tiles_mp * tn256 * p.ksplit;
+            return launch_pdl(dense_gemm_pair_splitk_kernel, dim3(2 * (nt < pairs ? nt : pairs)), dim3(G_THREADS), GemmCfg<256, true>::SMEM,
+                              stream, amap, wmap, p, tiles_mp, tn256);
+        }
         if (int rc = ensure_dyn_smem(dense_gemm_pair_kernel, GemmCfg<256, true>::SMEM)) return rc;
         const int nt = tiles_mp * tn256;
         return launch_pdl(dense_gemm_pair_kernel, dim3(2 * (nt < pairs ? nt : pairs)), dim3(G_THREADS), GemmCfg<256, true>::SMEM,

@@ -36,6 +36,9 @@ int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t
 int rope_split(const void *qkv, const float *cos_t, const float *sin_t, void *q_out, void *k_pages, void *v_pages,
                int M, int seq, int n_q, int n_kv_proj, int n_kv_store, int hd, int cap, int row0, cudaStream_t st);
 
+// Workspace of callers with some hundred rows (a prefix, the views of a vision tower): K slices and rows it is sized for.
+constexpr int kSplitSlices = 4, kSplitRows = 1024;
+
 // 0 = choose the tiling by cost (default); 1 / 2 / 3 / 4 force 128 x 256, 128 x 128, CTA pairs, 128 x 64.
 void dense_gemm_set_variant(int v);
 int dense_gemm_variant();

@@ -31,6 +31,8 @@ struct vlab200_vision {
     vb::DevBuf patch_w, posb, post_w, post_b, connector, connector_b;
     std::vector<vb::DevBuf> wqkv, bqkv, wo, bo, w1, b1, w2, b2, ln1w, ln1b, ln2w, ln2b;
     vb::DevBuf a_patch, h, hb, nb, qkv, q, kpg, vpg, att, f, shuf, ident;
+    vb::DevBuf splitk;  // float32 K slices of Wo / fc2
+    int split_rows = 0;
 };
 
 namespace vb {
@@ -310,6 +312,8 @@ vlab200_vision *vlab200_vision_create(const vlab200_vision_config *cfg, const vl
         if ((rc = v->att.alloc(M * qf * 2))) break;
         if ((rc = v->f.alloc(M * I * 2))) break;
         if ((rc = v->shuf.alloc(M * H * 2))) break;
+        v->split_rows = (int)(M < (size_t)vb::kSplitRows ? M : (size_t)vb::kSplitRows);
+        if ((rc = v->splitk.alloc((size_t)vb::kSplitSlices * v->split_rows * H * 4))) break;
         const int nrot = v->np * (hd_pad / 2);
         if ((rc = v->ident.alloc((size_t)2 * nrot * 4))) break;
         vb::fill_identity_rotation_kernel<<<(nrot + 127) / 128, 128>>>(v->ident.as<float>(), v->ident.as<float>() + nrot, nrot);
@@ -344,6 +348,7 @@ int32_t vlab200_vision_run(vlab200_vision *v, const void *pixels, int32_t pixels
         vb::GemmParams g{};
         g.M = M; g.N = H; g.K = K; g.epi = vb::EPI_RESIDUAL; g.bias = bias;
         g.h = v->h.as<float>(); g.out_bf = v->hb.as<__nv_bfloat16>(); g.ld_out = H;
+        g.partial = v->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = v->split_rows;
         return vb::dense_gemm(A, K, W, g, cs);
     };
     auto layernorm = [&](const float *w, const float *b, __nv_bfloat16 *out, int shuffle) {
