@@ -178,7 +178,9 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        // The whole warp walks the tiles and one elected lane issues: control that is the same for the warp lets the descriptors stay in
+        // uniform registers, which the instruction reads; from one lane of a diverged warp every product pays for moving them.
+        if (rank == 0) {
             constexpr uint32_t idesc = make_idesc(1, 1, 1, 0, 0, TILE_M, G_BN);
             // descriptors differ between stages and k sub-steps only in the 14-bit start address
             const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
@@ -187,30 +189,34 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             bool ok = true;
             for (int tile = t_begin; ok && tile < t_end; ++tile, ++j) {
                 const uint32_t buf = j & 1u;
-                ok = mbar_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
+                ok = warp_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * G_BN;
                 const int ks = SPLIT ? tile % ks_n : 0;
                 const int kbeg = SPLIT ? ks * ksteps / ks_n : 0, kend = SPLIT ? (ks + 1) * ksteps / ks_n : ksteps;
                 for (int kt = kbeg; kt < kend; ++kt) {
-                    ok = mbar_wait(&full[st], ph, wc, DEV_TIMEOUT_FULL);
+                    ok = warp_wait(&full[st], ph, wc, DEV_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t off = (uint64_t)(st * (G_STAGE_BYTES >> 4));
+                    if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < G_BK / 16; ++k) {
                         const uint32_t acc = (kt != kbeg || k != 0) ? 1u : 0u;  // the first MMA of a tile overwrites the accumulator
                         if (PAIR) mma_f16_pair(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, acc);
                         else mma_f16(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, acc);
                     }
-                    if (PAIR) tc_commit_pair(&empty[st], 3);
-                    else tc_commit(&empty[st]);
+                        if (PAIR) tc_commit_pair(&empty[st], 3);
+                        else tc_commit(&empty[st]);
+                    }
                     if (++st == G_STAGES) { st = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
-                if (PAIR) tc_commit_pair(&accum_full[buf], 3);
-                else tc_commit(&accum_full[buf]);
+                if (elect_one()) {
+                    if (PAIR) tc_commit_pair(&accum_full[buf], 3);
+                    else tc_commit(&accum_full[buf]);
+                }
             }
         } else if (PAIR && lane == 0) {
             // odd CTA of a pair: tell the even CTA when this CTA's stage has landed

@@ -105,6 +105,11 @@ __device__ __forceinline__ bool mbar_wait_backoff(uint64_t *bar, uint32_t parity
     }
 }
 
+// The same answer for every lane of a converged warp (elect.sync counts on all of them).
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, const WaitCtx &w, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, w, code)) != 0;
+}
+
 // Releases a TMA-filled stage that the warp has READ with ordinary loads: one arrival per warp.
 // TMA refills the stage through the async proxy as soon as the barrier completes.  An mbarrier
 // arrive orders the generic-proxy loads only against other generic-proxy accesses; without
