@@ -316,3 +316,21 @@ def test_ternarize_pack_on_device_matches_oracle(oracle, n, k, scale):
     assert api.device_status() == 0
     assert sc.cpu().numpy()[0] == np.float32(absmean)
     assert np.array_equal(packed.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("m", [9, 128, 129, 300])
+@pytest.mark.parametrize("n,k", [(64, 128), (144, 384), (1152, 1152), (2560, 640), (4304, 256)])
+def test_few_rows_default_tiling_accumulators_exact(oracle, m, n, k):
+    """The tiling the library picks by itself for few rows (narrow tiles, ragged last tile, one to several K steps): the int32
+    accumulators are whole numbers, so any tiling gives exactly the oracle's."""
+    torch = require_cuda()
+    import vla_cpp_b200 as vb
+
+    rng = np.random.default_rng(m + n + k)
+    tern = rng.integers(-1, 2, (n, k)).astype(np.int8)
+    a = rng.integers(-127, 128, (m, k)).astype(np.int8)
+    acc = torch.zeros((m, n), dtype=torch.int32, device="cuda")
+    vb.ternary_linear(torch.from_numpy(a).cuda(), torch.from_numpy(oracle.pack_ladder_int2(tern)).cuda(),
+                      torch.full((m,), 50.0, device="cuda"), torch.tensor([0.02], device="cuda"), n, acc_out=acc)
+    assert vb.device_status() == 0
+    assert np.array_equal(acc.cpu().numpy(), oracle.gemm_i8_i32(a, tern))

@@ -273,6 +273,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
+    constexpr bool HALF = BN < 128;  // fewer than eight 16-row weight blocks: four warps decode even K steps, four odd ones
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ksteps = K / GEMM_BK;
     const int n_tiles = tiles_m * tiles_n;
@@ -284,7 +285,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
             mbar_init(&empty_a[i], 1);
         }
         for (int i = 0; i < GEMM_SW; ++i) {
-            mbar_init(&full_w[i], 8);  // one arrival per decode warp
+            mbar_init(&full_w[i], HALF ? 4 : 8);  // one arrival per decode warp of the step
             mbar_init(&empty_w[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -323,21 +324,22 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {  // the whole warp walks the tiles, one elected lane issues (uniform control: see gemm.cu)
             constexpr uint32_t idesc = make_idesc(2, 1, 1, 0, 0, GEMM_BM, BN);
             uint32_t st = 0, ph = 0, sw = 0, pw = 0, j = 0;
             bool ok = true;
             for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x, ++j) {
                 const uint32_t buf = j & 1u;
-                ok = mbar_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
+                ok = warp_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int kt = 0; kt < ksteps; ++kt) {
-                    ok = mbar_wait(&full_a[st], ph, wc, DEV_TIMEOUT_FULL);
-                    if (ok) ok = mbar_wait(&full_w[sw], pw, wc, DEV_TIMEOUT_FULL);
+                    ok = warp_wait(&full_a[st], ph, wc, DEV_TIMEOUT_FULL);
+                    if (ok) ok = warp_wait(&full_w[sw], pw, wc, DEV_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
+                    if (elect_one()) {
                     const uint32_t a_addr = smem_u32(smem + st * L::A_BYTES);
                     const uint32_t w_addr = smem_u32(smem + L::W_OFFSET + sw * L::W_BYTES);
 #pragma unroll
@@ -346,18 +348,20 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
                                smem_desc_sw128(w_addr + k * 32, 16, 1024), idesc, (kt | k) != 0 ? 1u : 0u);
                     tc_commit(&empty_a[st]);
                     tc_commit(&empty_w[sw]);
+                    }
                     if (++st == GEMM_SA) { st = 0; ph ^= 1u; }
                     if (++sw == GEMM_SW) { sw = 0; pw ^= 1u; }
                 }
                 if (!ok) break;
-                tc_commit(&accum_full[buf]);
+                if (elect_one()) tc_commit(&accum_full[buf]);
             }
         }
     } else if (warp < 10) {
         // ---- decode warps: ladder slots -> swizzled K-major int8 tile ----
         const int dw = warp - 2;                  // 0..7
         constexpr int NBLK = BN / 16;             // 16-row weight blocks in the tile
-        constexpr int PER_WARP = NBLK / 8;
+        constexpr int PER_WARP = HALF ? 1 : NBLK / 8;
+        const int blk0 = HALF ? dw & 3 : dw;
         const int nblk_total = N / 16;
         // lane geometry inside one 512-byte chunk (lane t holds the 4 slots at byte offset 16 t)
         const int row_in_blk = 8 * ((lane & 7) >> 2) + 4 * (lane & 1);  // + slot 0..3
@@ -377,7 +381,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
             const int nb0 = (tile / tiles_m) * NBLK;
 #pragma unroll
             for (int i = 0; i < PER_WARP; ++i) {
-                const int nb = nb0 + dw + 8 * i;
+                const int nb = nb0 + blk0 + 8 * i;
                 dst[i] = (g < total && nb < nblk_total)
                              ? __ldg(reinterpret_cast<const uint4 *>(Wp + (size_t)nb * 4 * K + (size_t)kt * 512) + lane)
                              : make_uint4(0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu);
@@ -386,7 +390,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
         auto decode_store = [&](const uint4 (&cur)[PER_WARP], uint8_t *wt) {
 #pragma unroll
             for (int i = 0; i < PER_WARP; ++i) {
-                const int blk = dw + 8 * i;
+                const int blk = blk0 + 8 * i;
                 const uint32_t words[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
 #pragma unroll
                 for (int sl = 0; sl < 4; ++sl) {
@@ -398,26 +402,27 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
                 }
             }
         };
-        uint32_t st = 0, ph = 0;
+        constexpr int STEP = HALF ? 2 : 1;  // this warp decodes steps first, first + STEP, ...
+        const int first = HALF ? dw >> 2 : 0;
         bool ok = true;
 #pragma unroll
-        for (int i = 0; i < PF; ++i) fetch(i, pf[i]);
-        for (int g0 = 0; ok && g0 < total; g0 += PF) {
+        for (int i = 0; i < PF; ++i) fetch(first + i * STEP, pf[i]);
+        for (int g0 = first; ok && g0 < total; g0 += PF * STEP) {
 #pragma unroll
             for (int u = 0; u < PF; ++u) {
-                const int g = g0 + u;
+                const int g = g0 + u * STEP;
                 if (g >= total) break;
                 uint4 cur[PER_WARP];
 #pragma unroll
                 for (int i = 0; i < PER_WARP; ++i) cur[i] = pf[u][i];
-                fetch(g + PF, pf[u]);
+                fetch(g + PF * STEP, pf[u]);
+                const uint32_t st = (uint32_t)g % GEMM_SW, ph = ((uint32_t)g / GEMM_SW) & 1u;
                 ok = mbar_wait(&empty_w[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 decode_store(cur, smem + L::W_OFFSET + st * L::W_BYTES);
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full_w[st]);
-                if (++st == GEMM_SW) { st = 0; ph ^= 1u; }
             }
         }
     } else {
@@ -596,7 +601,7 @@ ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {  // the whole warp walks the tiles, one elected lane issues (uniform control: see gemm.cu)
             constexpr uint32_t idesc = make_idesc(2, 1, 1, 0, 0, 256, BN);
             // descriptors differ between stages and k sub-steps only in the 14-bit start address
             const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
@@ -605,23 +610,25 @@ ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_
             bool ok = true;
             for (int tile = cid; ok && tile < n_tiles; tile += ncl, ++j) {
                 const uint32_t buf = j & 1u;
-                ok = mbar_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
+                ok = warp_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int kt = 0; kt < ksteps; ++kt) {
-                    ok = mbar_wait(&full[st], ph, wc, DEV_TIMEOUT_FULL);
+                    ok = warp_wait(&full[st], ph, wc, DEV_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t off = (uint64_t)(st * (L::STAGE_BYTES >> 4));
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < GEMM_BK / 32; ++k)
-                        mma_i8_pair(d_tmem, a_desc0 + off + 2 * k, w_desc0 + off + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
-                    tc_commit_pair(&empty[st], 3);
+                        for (int k = 0; k < GEMM_BK / 32; ++k)
+                            mma_i8_pair(d_tmem, a_desc0 + off + 2 * k, w_desc0 + off + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
+                        tc_commit_pair(&empty[st], 3);
+                    }
                     if (++st == PAIR_STAGES) { st = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
-                tc_commit_pair(&accum_full[buf], 3);
+                if (elect_one()) tc_commit_pair(&accum_full[buf], 3);
             }
         } else if (lane == 0) {
             // odd CTA: tell the even CTA when this CTA's stage is in shared memory
@@ -862,9 +869,21 @@ static int ternary_linear(const int8_t *A, const uint8_t *W, __nv_bfloat16 *out,
         return VLAB200_ERR_ARG;
     // a 32-column epilogue chunk must not straddle two weight-scale groups; with one group N % 16 == 0 is enough
     if (ws_num > 1 && (N / ws_num) % 32) return VLAB200_ERR_UNSUPPORTED;
-    // CTA pairs measured faster than one CTA per tile on every BitVLA shape from M = 300 up
-    if (force_path == 3 || (force_path == 0 && N >= 256))
-        return launch_gemm_pair(A, W, out, acc, s, ws, ws_num, M, N, K, st);
+    if (force_path == 3) return launch_gemm_pair(A, W, out, acc, s, ws, ws_num, M, N, K, st);
+    if (force_path == 0) {
+        // ns of a launch (measured back to back, 64 <= M <= 2000): set-up and epilogue, plus waves times 128-wide K steps.  Pair tiles
+        // move the fewest bytes per product and win as soon as there are enough of them; with few rows (one image, one prompt) they
+        // leave most SMs without work and narrow tiles win: 256 x 1152 x 1152 9.7 -> 7.0 us, 300 x 2560 x 2560 13.8 -> 11.3 us,
+        // 256 x 1152 (K 4352) 18.5 -> 16.0 us; 300 x 13824 x 2560 takes 22.2 us in pairs and 33.1 / 41.5 us in tiles of 128 / 64.
+        const int n_sm = sm_count(), tm = (M + 127) / 128, tp = (M + 255) / 256, ks = K / 128;
+        if (n_sm <= 0) return cuda_fail(cudaGetLastError(), "sm_count");
+        auto waves = [](int tiles, int units) { return (tiles + units - 1) / units; };
+        const int c64 = 3600 + 370 * ks * waves(tm * ((N + 63) / 64), n_sm), c128 = 4400 + 460 * ks * waves(tm * ((N + 127) / 128), n_sm);
+        const int cpair = N >= 256 && n_sm >= 2 ? 6400 + 360 * ks * waves(tp * ((N + 255) / 256), n_sm / 2) : c64 + c128;
+        if (cpair <= c64 && cpair <= c128) return launch_gemm_pair(A, W, out, acc, s, ws, ws_num, M, N, K, st);
+        if (c64 < c128) return launch_gemm_tc<64, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
+        return launch_gemm_tc<128, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
+    }
     if (N >= 256) return launch_gemm_tc<256, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
     return launch_gemm_tc<128, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
 }
