@@ -355,7 +355,7 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {  // the whole warp walks the tiles, one elected lane issues (uniform control: see gemm.cu)
             constexpr uint32_t idesc = make_idesc(1, 1, 1, 0, 0, TILE_M, QKV_BN);
             // descriptors differ between stages and k sub-steps only in the 14-bit start address
             const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
@@ -364,15 +364,16 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
             bool ok = true;
             for (int tile = t_begin; ok && tile < t_end; ++tile, ++j) {
                 const uint32_t buf = j & 1u;
-                ok = mbar_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
+                ok = warp_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * QKV_BN;
                 for (int kt = 0; kt < ksteps; ++kt) {
-                    ok = mbar_wait(&full[st], ph, wc, DEV_TIMEOUT_FULL);
+                    ok = warp_wait(&full[st], ph, wc, DEV_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t off = (uint64_t)(st * (STAGE_BYTES >> 4));
+                    if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < QKV_BK / 16; ++k) {
                         if (PAIR) mma_f16_pair(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
@@ -380,11 +381,14 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
                     }
                     if (PAIR) tc_commit_pair(&empty[st], 3);
                     else tc_commit(&empty[st]);
+                    }
                     if (++st == (uint32_t)nst) { st = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
-                if (PAIR) tc_commit_pair(&accum_full[buf], 3);
-                else tc_commit(&accum_full[buf]);
+                if (elect_one()) {
+                    if (PAIR) tc_commit_pair(&accum_full[buf], 3);
+                    else tc_commit(&accum_full[buf]);
+                }
             }
         } else if (PAIR && lane == 0) {
             // odd CTA of a pair: tell the even CTA when this CTA's stage has landed
