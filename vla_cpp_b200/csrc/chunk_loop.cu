@@ -21,10 +21,8 @@
 //            [CTA group][pass][64-column block][row], so that any range of blocks is one contiguous cp.async.bulk (a bulk copy costs
 //            its issuing thread 40-60 ns whatever its size; 51 row copies of 2 KB took 3 us).  They arrive in a ring that one
 //            thread feeds from a cursor which runs AHEAD of the computation, across phase boundaries and barriers (weights do
-//            not depend on anything the loop computes), so HBM streams while the CTAs wait for each other; another thread
-//            issues the products as soon as the A tile and the next ring stage have landed.  Products of 64 columns that
-//            accumulate into ONE place follow each other at 130 clocks (each waits for the sums of the one before); dealt to
-//            four accumulators, added when they are read, they do not.
+//            not depend on anything the loop computes), so HBM streams while the CTAs wait for each other; another warp
+//            issues the products as soon as the A tile and the next ring stage have landed.
 //            (mma.sync on the same tiles ran at 410 - 460 multiply-adds per clock and SM, a ninth of tcgen05's rate: 2840
 //            clocks for Wo's 64 x 72 x 256, 5755 for Wdown's.)
 //   ATT      units of (kv head, 32 stacked query rows), a group of CTAs each, the keys split between its CTAs: S = Q K^T and P V
@@ -57,14 +55,13 @@ enum { PH_GEMM = 0, PH_ATT = 2, PH_EMBED = 4 };
 enum { OUT_RESID = 0, OUT_GATED = 1, OUT_QKV = 2, OUT_BIAS_ACT = 3, OUT_EULER = 4 };
 
 constexpr int CL_THREADS = 256;   // the eight computing warps
-constexpr int CL_BLOCK = 320;     // + one warp whose lane 0 feeds the weight ring, one whose lane 0 issues the products
+constexpr int CL_BLOCK = 320;     // + one warp whose lane 0 feeds the weight ring, one that issues the products
 constexpr int CL_CLUSTER = 8;     // CTAs per cluster (the portable maximum)
 constexpr int CL_STAGES = 4;
 constexpr int CL_STAGE_BYTES = 22528;                             // 22 tiles (8 columns x 64 K) of 1 KB
 constexpr int CL_PASS_N8 = 22;                                    // 8-column groups a CTA group works on at once: 176 weight rows, two tiles of 128
 constexpr int CL_PASSES = 2;                                      // at most two passes per group: the exchange has a buffer for each
-constexpr int CL_ACC = 4;                                         // accumulators per tile: consecutive products go to different ones
-constexpr int CL_TMEM_COLS = 2 * CL_ACC * 64;                     // [tile][accumulator] of 64 columns
+constexpr int CL_TMEM_COLS = 128;                                 // an accumulator of 64 columns (tokens) per tile of 128 weight rows
 constexpr int CL_DESC_BYTES = 352;                                // one phase descriptor slot (two of them: this phase, the next)
 constexpr int CL_DESC_OFF = 1536;
 constexpr int CL_WTAB_OFF = 2304;                                 // weight feeder table: one 32-byte entry per GEMM phase of a step
@@ -215,8 +212,8 @@ __device__ __forceinline__ Smem get_smem() {
     sm.full = reinterpret_cast<uint64_t *>(smem_raw);  // [CL_STAGES]
     sm.empty = sm.full + CL_STAGES;                    // [CL_STAGES]
     sm.a_full = sm.empty + CL_STAGES;                  // a product's A tile has landed
-    sm.acc_full = sm.a_full + 1;                       // its accumulators are complete
-    sm.acc_free = sm.acc_full + 1;                     // they have been read
+    sm.acc_full = sm.a_full + 1;                       // its accumulator is complete
+    sm.acc_free = sm.acc_full + 1;                     // it has been read
     sm.k_full = sm.acc_free + 1;                       // attention: Q and K, V
     sm.v_full = sm.k_full + 1;
     sm.x_full = sm.v_full + 1;                         // [CL_PASSES]: the group's partial sums have arrived
@@ -289,7 +286,9 @@ __device__ __noinline__ void feeder_loop(const LoopParams &lp) {
     mbar_arrive(sm.done);
 }
 
-// The issuer: one thread walks the same list and issues the products of a chunk as soon as it and the phase's A tile have landed
+// The issuer: one warp walks the same list and issues the products of a chunk as soon as it and the phase's A tile have landed.  The whole
+// warp runs the loop and one elected lane issues: control that is the same for the warp lets the descriptors stay in uniform
+// registers, which the instruction reads; from one lane of a diverged warp each product paid for moving them (pi0 6924 -> 6712 us).
 // (A is copied after the grid barrier before the phase, so the accumulator of the phase before has been read by then).
 __device__ __noinline__ void issuer_loop(const LoopParams &lp, uint32_t tmem) {
     const Smem sm = get_smem();
@@ -299,23 +298,25 @@ __device__ __noinline__ void issuer_loop(const LoopParams &lp, uint32_t tmem) {
     const uint64_t a_desc0 = smem_desc_sw128(smem_u32(sm.ring), 16, 1024), b_desc0 = smem_desc_sw128(smem_u32(sm.arena), 16, 1024);
     for (int step = 0; ok && step < lp.steps; ++step)
         for (int gi = 0; ok && gi < sm.n_wtab; ++gi) {
-            const WEntry w = sm.wtab[gi];
+            WEntry w = sm.wtab[gi];
+            w.N8 = __shfl_sync(0xffffffffu, w.N8, 0); w.K = __shfl_sync(0xffffffffu, w.K, 0);
+            w.kd = __shfl_sync(0xffffffffu, w.kd, 0); w.M = __shfl_sync(0xffffffffu, w.M, 0);
             const GemmPart gp = gemm_part(w.N8, w.K, w.kd);
             if (gp.w8 <= 0 || gp.kb0 >= gp.kb1) continue;
             const uint32_t idesc = make_idesc(1, 1, 1, 0, 0, 128, (w.M + 15) & ~15);
             const uint32_t b_blk = (uint32_t)((w.M + 7) & ~7) * 8u;  // one 64-column block of A, in descriptor units of 16 bytes
-            ok = mbar_wait(sm.a_full, a_cnt & 1u, wc, CL_DEV_TIMEOUT);
+            ok = warp_wait(sm.a_full, a_cnt & 1u, wc, CL_DEV_TIMEOUT);
             ++a_cnt;
             tc_fence_after();
             for (int p0 = 0; ok && p0 < gp.w8; p0 += CL_PASS_N8, ++acc_cnt) {
                 const int w8p = min(CL_PASS_N8, gp.w8 - p0), kc = CL_STAGE_BYTES / (w8p * 1024);
                 if (p0 > 0) {  // (before a phase's first pass the grid barrier has seen to it)
-                    ok = mbar_wait(sm.acc_free, (acc_cnt & 1u) ^ 1u, wc, CL_DEV_TIMEOUT);
+                    ok = warp_wait(sm.acc_free, (acc_cnt & 1u) ^ 1u, wc, CL_DEV_TIMEOUT);
                     tc_fence_after();
                 }
                 for (int k0 = gp.kb0; k0 < gp.kb1; k0 += kc, ++cons) {
                     const unsigned stage = cons % CL_STAGES;
-                    ok = mbar_wait(&sm.full[stage], (cons / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
+                    ok = warp_wait(&sm.full[stage], (cons / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
                     if (!ok) break;
                     tc_fence_after();
                     const int nk = min(kc, gp.kb1 - k0);
@@ -323,24 +324,23 @@ __device__ __noinline__ void issuer_loop(const LoopParams &lp, uint32_t tmem) {
                         const uint64_t a = a_desc0 + (uint64_t)(stage * (CL_STAGE_BYTES / 16) + (unsigned)(kk * w8p) * 64u);
                         const uint64_t b = b_desc0 + (uint64_t)((uint32_t)(k0 + kk - gp.kb0) * b_blk);
                         const uint32_t acc = k0 + kk > gp.kb0 ? 1u : 0u;
-                        if (w8p > 16) {
+                        if (elect_one()) {
 #pragma unroll
-                            for (int k = 0; k < CL_ACC; ++k) {
-                                mma_f16(tmem + k * 64u, a + 2 * k, b + 2 * k, idesc, acc);
-                                mma_f16(tmem + (CL_ACC + k) * 64u, a + 1024 + 2 * k, b + 2 * k, idesc, acc);
+                            for (int k = 0; k < 4; ++k) {
+                                mma_f16(tmem, a + 2 * k, b + 2 * k, idesc, k ? 1u : acc);
+                                if (w8p > 16) mma_f16(tmem + 64u, a + 1024 + 2 * k, b + 2 * k, idesc, k ? 1u : acc);
                             }
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < CL_ACC; ++k) mma_f16(tmem + k * 64u, a + 2 * k, b + 2 * k, idesc, acc);
                         }
                     }
-                    tc_commit(&sm.empty[stage]);
+                    if (elect_one()) tc_commit(&sm.empty[stage]);
                 }
-                if (ok) tc_commit(sm.acc_full);
+                if (ok && elect_one()) tc_commit(sm.acc_full);
             }
         }
-    *sm.consumed = cons;
-    mbar_arrive(sm.done);
+    if (elect_one()) {
+        *sm.consumed = cons;
+        mbar_arrive(sm.done);
+    }
 }
 
 // Grid-wide barrier in two halves, so that what a phase can prepare without the phase before is done between them.
@@ -574,27 +574,21 @@ __device__ __noinline__ unsigned gemm_phase(const LoopPhase &pg, const LoopParam
         // ---- this CTA's K part into its staging area, [column][token]: a lane holds one column, 32 tokens
         float *stg = reinterpret_cast<float *>(sm.arena + stage_off + (uint32_t)pass * recv_bytes);
         for (int n0 = hw * 32; n0 < w8p * 8; n0 += 128) {
-            float v[32];
-#pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = 0.0f;
+            uint32_t v[32];
             if (a_bytes) {
-                const uint32_t ta = tmem + (uint32_t)((n0 >> 7) * CL_ACC * 64 + th * 32) + ((uint32_t)(hw * 32) << 16);
+                tmem_ld32(tmem + (uint32_t)((n0 >> 7) * 64 + th * 32) + ((uint32_t)(hw * 32) << 16), v);
+                tmem_ld_wait();
+            } else {
 #pragma unroll
-                for (int k = 0; k < CL_ACC; k += 2) {
-                    uint32_t r0[32], r1[32];
-                    tmem_ld32(ta + (uint32_t)k * 64u, r0);
-                    tmem_ld32(ta + (uint32_t)(k + 1) * 64u, r1);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) v[e] += __uint_as_float(r0[e]) + __uint_as_float(r1[e]);
-                }
+                for (int e = 0; e < 32; ++e) v[e] = 0u;
             }
             const int n = n0 + lane;
             if (n < w8p * 8) {
                 float4 *dst = reinterpret_cast<float4 *>(stg + (size_t)n * tp + th * 32);
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
-                    if (th * 32 + e * 4 < M) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                    if (th * 32 + e * 4 < M)
+                        dst[e] = make_float4(__uint_as_float(v[4 * e]), __uint_as_float(v[4 * e + 1]), __uint_as_float(v[4 * e + 2]), __uint_as_float(v[4 * e + 3]));
             }
         }
         tc_fence_before();
@@ -1037,9 +1031,9 @@ __global__ void __launch_bounds__(CL_BLOCK, 1) chunk_loop_kernel(const __grid_co
     cluster_sync_all();  // every CTA's barriers exist before another CTA of the cluster signals them
     tc_fence_after();
     const uint32_t tmem = *sm.tmem_slot;
-    if (threadIdx.x >= CL_THREADS) {  // the feeder and the issuer warp: lane 0 works, the warps take no part in any barrier of the computing ones
+    if (threadIdx.x >= CL_THREADS) {  // the feeder (lane 0) and the issuer warp; they take no part in any barrier of the computing ones
         if (threadIdx.x == CL_THREADS) feeder_loop(lp);
-        if (threadIdx.x == CL_THREADS + 32) issuer_loop(lp, tmem);
+        if (threadIdx.x >= CL_THREADS + 32) issuer_loop(lp, tmem);
         __syncwarp();
     } else {
         const WaitCtx wc{sm.abort_flag, lp.status};
