@@ -160,7 +160,7 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         }
     } else if (warp == 5) {
         // ----------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        {  // the whole warp walks the units, one elected lane issues (uniform control: see gemm.cu)
             constexpr uint32_t idesc_s = make_idesc(1, 1, 1, 0, 0, 128, FA_BKV);
             constexpr uint32_t idesc_o = make_idesc(1, 1, 1, 0, 1, 128, HD);
             const uint32_t q_addr = smem_u32(smem);
@@ -171,6 +171,7 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 const uint32_t st = jbx & 1u;
                 const uint32_t k_addr = k_base + st * L::KV_BYTES;
                 const uint32_t d = tmem_base + L::O_COLS + st * 64;
+                if (!elect_one()) return;
 #pragma unroll
                 for (int kk = 0; kk < HD / 16; ++kk)
                     mma_f16(d, smem_desc_sw128(q_addr + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
@@ -182,32 +183,33 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             for (int wu = blockIdx.x; ok && wu < n_work; wu += gridDim.x, ++ui) {
                 const int sp = SPLIT ? wu % ns : 0;
                 const int j0 = SPLIT ? sp * nb / ns : 0, j1 = SPLIT ? (sp + 1) * nb / ns : nb;
-                ok = mbar_wait(q_full, ui & 1u, wc, DEV_TIMEOUT_FULL);
+                ok = warp_wait(q_full, ui & 1u, wc, DEV_TIMEOUT_FULL);
                 if (!ok) break;
                 // first S block of the unit: its TMEM buffer was last read by the P V of block jb-2, which this thread
                 // issued earlier -- the tensor pipe runs a thread's MMAs in issue order, so there is nothing to wait for
-                ok = mbar_wait(&k_full[jb & 1u], (jb >> 1) & 1u, wc, DEV_TIMEOUT_FULL);
+                ok = warp_wait(&k_full[jb & 1u], (jb >> 1) & 1u, wc, DEV_TIMEOUT_FULL);
                 if (!ok) break;
                 tc_fence_after();
                 issue_s(jb);
-                if (j1 - j0 == 1) tc_commit(q_free);
+                if (j1 - j0 == 1 && elect_one()) tc_commit(q_free);
                 for (int j = j0; j < j1; ++j, ++jb) {
                     const uint32_t st = jb & 1u, ph = (jb >> 1) & 1u;
                     if (j + 1 < j1) {
                         const uint32_t jn = jb + 1;
-                        ok = mbar_wait(&k_full[jn & 1u], (jn >> 1) & 1u, wc, DEV_TIMEOUT_FULL);
+                        ok = warp_wait(&k_full[jn & 1u], (jn >> 1) & 1u, wc, DEV_TIMEOUT_FULL);
                         if (!ok) break;
                         tc_fence_after();
                         issue_s(jn);
-                        if (j + 2 == j1) tc_commit(q_free);  // the unit's last S block has been issued
+                        if (j + 2 == j1 && elect_one()) tc_commit(q_free);  // the unit's last S block has been issued
                     }
-                    ok = mbar_wait(&p_full[st], ph, wc, DEV_TIMEOUT_FULL);
-                    if (ok) ok = mbar_wait(&v_full[st], ph, wc, DEV_TIMEOUT_FULL);
-                    if (ok && j == j0) ok = mbar_wait(o_free, (ui & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
+                    ok = warp_wait(&p_full[st], ph, wc, DEV_TIMEOUT_FULL);
+                    if (ok) ok = warp_wait(&v_full[st], ph, wc, DEV_TIMEOUT_FULL);
+                    if (ok && j == j0) ok = warp_wait(o_free, (ui & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t v_addr = v_base + st * L::KV_BYTES;
                     const uint32_t p_tmem = tmem_base + L::O_COLS + st * 64;
+                    if (elect_one()) {
 #pragma unroll
                     for (int k16 = 0; k16 < FA_BKV / 16; ++k16)
                         mma_f16_tmem_a(tmem_base, p_tmem + (uint32_t)(k16 * 8),
@@ -215,9 +217,10 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                                        (j != j0 || k16 != 0) ? 1u : 0u);
                     tc_commit(&pv_done[st]);
                     tc_commit(&v_free[st]);
+                    }
                 }
                 if (!ok) break;
-                tc_commit(o_done);
+                if (elect_one()) tc_commit(o_done);
             }
         }
     } else {
@@ -540,7 +543,7 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             }
         }
     } else if (warp == FP_MMA_WARP) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {  // the whole warp walks the units, one elected lane issues (uniform control: see gemm.cu)
             // ------------------------------------------------------------- MMA issuer (even CTA)
             constexpr uint32_t idesc_s = make_idesc(1, 1, 1, 0, 0, 256, FP_BKV);
             const uint32_t q_addr = smem_u32(smem);
@@ -552,6 +555,7 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 const uint32_t st = jbx % FP_STAGES;
                 const uint64_t k_desc = k_desc0 + (uint64_t)(st * (L::K_BYTES >> 4));
                 const uint32_t d = tmem_base + L::O_COLS + (jbx % FP_NS) * FP_BKV;
+                if (!elect_one()) return;
 #pragma unroll
                 for (int kk = 0; kk < HD / 16; ++kk)
                     mma_f16_pair(d, q_desc0 + (uint64_t)((kk >> 2) * 1024 + (kk & 3) * 2),
@@ -585,16 +589,16 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 return r;
             };
             for (int unit = cid; ok && unit < n_units; unit += ncl, ++ui) {
-                ok = mbar_wait(q_full, ui & 1u, wc, DEV_TIMEOUT_FULL);
+                ok = warp_wait(q_full, ui & 1u, wc, DEV_TIMEOUT_FULL);
                 if (!ok) break;
                 for (int j = 0; j < nb; ++j, ++jb) {
-                    ok = ready_s(jb);
+                    ok = __all_sync(0xffffffffu, ready_s(jb)) != 0;
                     if (!ok) break;
                     tc_fence_after();
                     issue_s(jb);
                 }
                 if (!ok) break;
-                tc_commit_pair(q_free, 3);  // the unit's last S block has been issued
+                if (elect_one()) tc_commit_pair(q_free, 3);  // the unit's last S block has been issued
             }
         } else if (lane == 0) {
             // ------------------------------------------------------------- odd CTA: forward "landed" to the even CTA
@@ -616,7 +620,7 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             }
         }
     } else if (warp == FP_PV_WARP) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {  // the whole warp walks the units, one elected lane issues (uniform control: see gemm.cu)
             // ------------------------------------------------------------- P V issuer (even CTA)
             constexpr uint32_t idesc_o = make_idesc(1, 1, 1, 0, 1, 256, HD);
             const uint64_t v_desc0 = smem_desc_sw128(smem_u32(smem) + L::V_OFF, FP_BKV * 128, 1024);
@@ -626,13 +630,14 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 for (int j = 0; j < nb; ++j, ++jb) {
                     const uint32_t sb = jb % FP_NS, sph = (jb / FP_NS) & 1u;         // S / P buffer and its phase
                     const uint32_t st = jb % FP_STAGES, ph = (jb / FP_STAGES) & 1u;  // K / V stage and its phase
-                    ok = mbar_wait(&p_full[sb], sph, wc, DEV_TIMEOUT_FULL);
-                    if (ok) ok = mbar_wait(&v_full[st], ph, wc, DEV_TIMEOUT_FULL);
-                    if (ok && j == 0) ok = mbar_wait(o_free, (ui & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
+                    ok = warp_wait(&p_full[sb], sph, wc, DEV_TIMEOUT_FULL);
+                    if (ok) ok = warp_wait(&v_full[st], ph, wc, DEV_TIMEOUT_FULL);
+                    if (ok && j == 0) ok = warp_wait(o_free, (ui & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t v_desc = v_desc0 + (uint64_t)(st * (L::V_BYTES >> 4));
                     const uint32_t p_tmem = tmem_base + L::O_COLS + sb * FP_BKV;
+                    if (elect_one()) {
 #pragma unroll
                     for (int k16 = 0; k16 < FP_BKV / 16; ++k16)
                         mma_f16_tmem_a_pair(tmem_base, p_tmem + (uint32_t)(k16 * 8), v_desc + (uint64_t)(k16 * 128), idesc_o,
@@ -640,9 +645,10 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     *pv_issued = jb + 1u;
                     tc_commit_pair(&pv_done[sb], 3);
                     tc_commit_pair(&v_free[st], 3);
+                    }
                 }
                 if (!ok) break;
-                tc_commit_pair(o_done, 3);
+                if (elect_one()) tc_commit_pair(o_done, 3);
             }
         }
     } else {
