@@ -126,3 +126,11 @@ def test_pi0_backbone_at_full_width(oracle):
                             vlm_dims=(4, 2048, 8, 1, 256, 16384),
                             expert_kw=dict(H=1024, inter=4096, chunk=50, A=32, sd=32, T=2), act=2)
     print(f"pi0 full-width prefill: worst K/V rel_l2 {w:.3e}, chunk rel_l2 {o:.3e}")
+
+
+def test_prefill_long_k_in_slices_of_pair_tiles(oracle):
+    """520 rows, width 1064, MLP 12288: Wdown runs as K slices of CTA-pair tiles, the last row and column tile mostly empty."""
+    w, _ = run_prefill_case(oracle, 5, model=0, n_obs=1, P=520, pos=None, mask_mode=0, pad=None,
+                            vlm_dims=(2, 1064, 4, 1, 64, 12288),
+                            expert_kw=dict(H=128, inter=256, chunk=10, A=32, sd=32, T=1), act=2, check_denoise=False)
+    print(f"long-K prefill: worst K/V rel_l2 {w:.3e}")
