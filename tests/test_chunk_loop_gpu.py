@@ -45,6 +45,23 @@ def test_loop_kernel_matches_operator_path(policy):
     assert torch.equal(out, again)  # every sum has a fixed order
 
 
+@pytest.mark.parametrize("policy", ["pi0", "pi05"])
+def test_loop_kernel_rows_exchanged_over_k(policy):
+    """816 prefix keys at head_dim 256: the attention rows a CTA group exchanges land where its K tiles were.  A row that arrived before
+    its reader had finished would change some of the runs."""
+    torch = require_cuda()
+    import vla_cpp_b200 as vb
+
+    eng, x0, state = _engine(torch, vb, policy, seed=11)
+    assert eng.prefix_len == 816
+    ref = _with_loop("0", lambda: eng.denoise(x0, state))
+    outs = _with_loop("1", lambda: [eng.denoise(x0, state) for _ in range(40)])
+    torch.cuda.synchronize()
+    assert vb.device_status() == 0
+    assert ((outs[0] - ref).norm() / ref.norm()).item() <= 1e-2  # both paths round activations to bf16 at different points
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+
+
 def test_loop_kernel_hidden_key_range_and_prefix_length():
     """SmolVLA-shaped: a pad range hides prefix keys; then the prefix in use shrinks (the phase table is rebuilt)."""
     torch = require_cuda()

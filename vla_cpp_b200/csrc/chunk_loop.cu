@@ -742,8 +742,9 @@ __device__ __noinline__ unsigned att_phase(const LoopPhase &pg, const LoopParams
             if (n_early_k > 0) bulk_g2s(Ks, kp0, (uint32_t)n_early_k * SQ, sm.k_full);
             if (n_early > 0) bulk_g2s(Vs, vp0, (uint32_t)n_early * SQ, sm.v_full);
         }
-        if (grid_poll(lp, target, sm) && work) {
-            fence_proxy_async_all();
+        const bool open = grid_poll(lp, target, sm);
+        if (grp < n_units) fence_proxy_async_all();  // also for the rows that a CTA without keys sends
+        if (open && work) {
             bulk_g2s(Qs, pg.qp + ((size_t)kvh * gq * S + row0) * SQ, q_bytes, sm.k_full);
             if (n_early_k < nk0) bulk_g2s(Ks + (size_t)n_early_k * SQ, kp0 + (size_t)n_early_k * SQ, (uint32_t)(nk0 - n_early_k) * SQ, sm.k_full);
             if (n_early < nk0) bulk_g2s(Vs + (size_t)n_early * SQ, vp0 + (size_t)n_early * SQ, (uint32_t)(nk0 - n_early) * SQ, sm.v_full);
@@ -838,6 +839,9 @@ __device__ __noinline__ unsigned att_phase(const LoopPhase &pg, const LoopParams
             mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 2));
             if ((lane & 3) == 0) sm.red_max[rl[hr] * 4 + kp] = mx[hr];
         }
+        // K's last block has been read.  Where the rows of the group's CTAs land over it, they do so by bulk copies, which an arrival
+        // alone does not order behind these loads (see stage_release in tc5.cuh)
+        if (key0 + ks >= k_end && pg.recv_off == pg.k_off) fence_proxy_async_smem();
         cons_sync();  // the maxima are in place; Q (P may lie over it) and K have been read
         if (key0 + ks >= k_end && tid < ad) arrive_rank(map_rank(smem_u32(sm.rdy), base_rank + tid));
 #pragma unroll
