@@ -347,6 +347,13 @@ VLAB200_API int32_t vlab200_engines_denoise_host(vlab200_engine *const *engines,
 VLAB200_API int32_t vlab200_engine_run_stage(vlab200_engine *e, int32_t layer, int32_t stage, int32_t n_obs,
                                              int32_t reps, void *stream);
 
+/* Which path calls with one observation take.  vlab200_engine_loop_phases: phases (= grid-wide barriers) per Euler step of the
+ * loop kernel that the engine holds for them since its last such call, 0 if they run a launch per operator (or there was
+ * none).  vlab200_loop_kernel_phases: the same for an expert of these sizes on a device with room for n_cta co-resident
+ * CTAs (whole clusters of eight), from the sizes alone; needs no GPU.  No counterpart in the reference. */
+VLAB200_API int32_t vlab200_engine_loop_phases(const vlab200_engine *e);
+VLAB200_API int32_t vlab200_loop_kernel_phases(const vlab200_policy_config *cfg, int32_t n_cta);
+
 /* Tiling of the bf16 GEMMs (the fused QKV projection, and inside the engine the O-projection, MLP,
  * embedding MLPs and action head):
  * 0 = chosen per call from the problem size (default), 1 = one CTA per 128 x 256 tile,

@@ -28,6 +28,25 @@ def _with_loop(flag, fn):
             os.environ["VLAB200_CHUNK_LOOP"] = old
 
 
+@pytest.fixture(autouse=True)
+def loop_phases(monkeypatch):
+    """Every one-observation call that these tests make with the loop kernel on must have run it, not the launch-per-operator path:
+    both meet the same bounds.  -> phases per Euler step of each such call."""
+    import vla_cpp_b200 as vb
+
+    phases, denoise = [], vb.PolicyEngine.denoise
+
+    def checked(self, x0, *a, **kw):
+        out = denoise(self, x0, *a, **kw)
+        if x0.shape[0] == 1 and os.environ.get("VLAB200_CHUNK_LOOP", "1") != "0":
+            phases.append(self.loop_phases)
+            assert phases[-1] > 0
+        return out
+
+    monkeypatch.setattr(vb.PolicyEngine, "denoise", checked)
+    return phases
+
+
 @pytest.mark.parametrize("policy", ["pi0", "smolvla", "pi05"])
 def test_loop_kernel_matches_operator_path(policy):
     torch = require_cuda()
@@ -127,3 +146,31 @@ def test_loop_kernel_work_split_edges(oracle, kw):
 
     w, d = _with_loop("1", lambda: run_case(oracle, 81, n_obs=1, **kw))
     assert w < 1e-2 and d < 3e-2, (w, d)
+
+
+WIDE = dict(model=0, L=1, H=1024, n_q=8, n_kv=1, hd=256, chunk=50, A=32, sd=32, T=2)
+
+
+@pytest.mark.parametrize("kw", [
+    # gate/up in two parts of its columns, Wdown in one; then both in parts, and a part of K that ends within a 64-column block
+    dict(P=40, inter=6144, **WIDE),
+    dict(P=40, inter=8192, **WIDE),
+    dict(P=40, inter=12304, **WIDE),
+    # 320 attention units (three rounds of them per CTA), q|k|v in parts of its columns, Wo in parts of K
+    dict(P=70, model=1, L=2, H=128, n_q=160, n_kv=160, hd=64, inter=256, chunk=50, A=32, sd=32, T=2, self_every=2),
+], ids=["inter6144", "inter8192", "inter12304", "heads160"])
+def test_loop_kernel_products_in_several_phases(oracle, loop_phases, kw):
+    from tests.test_engine_gpu import run_case
+
+    w, d = _with_loop("1", lambda: run_case(oracle, 83, n_obs=1, **kw))
+    assert loop_phases[-1] > 5 * kw["L"] + 4  # more than one phase per product
+    assert w < 1e-2 and d < 3e-2, (w, d)
+
+
+def test_loop_kernel_gated_residual_in_parts_of_k(oracle, loop_phases):
+    """pi0.5: the gate scales every part of Wdown's K on its way into the residual stream."""
+    from tests.test_pi05_gpu import run_pi05
+
+    err = _with_loop("1", lambda: run_pi05(oracle, 84, 1, 40, L=2, H=1024, n_q=8, n_kv=1, hd=256, inter=9216, chunk=50, A=32, T=2))
+    assert loop_phases[-1] > 5 * 2 + 2
+    assert err <= 1e-2, err

@@ -79,6 +79,7 @@ EXPORTS = [
     "vlab200_denoise_attn_loop_static",
     "vlab200_engine_create", "vlab200_engine_free", "vlab200_engine_set_prefix", "vlab200_engine_denoise",
     "vlab200_engine_denoise_host", "vlab200_engine_run_stage", "vlab200_engine_set_prefix_len",
+    "vlab200_engine_loop_phases", "vlab200_loop_kernel_phases",
     "vlab200_engine_get_prefix", "vlab200_shard_range", "vlab200_engines_denoise_host",
     "vlab200_prefill_create", "vlab200_prefill_free", "vlab200_prefill_run", "vlab200_set_gemm_tiling",
     "vlab200_vision_create", "vlab200_vision_free", "vlab200_vision_tokens_per_view", "vlab200_vision_run",
@@ -398,6 +399,16 @@ class _PolicyConfig(C.Structure):
         ("cond_dim", C.c_int32)]
 
 
+def _policy_config(cfg):
+    return _PolicyConfig(**{k: cfg.get(k, 0) if k == "cond_dim" else cfg[k] for k, _ in _PolicyConfig._fields_})
+
+
+def loop_kernel_phases(cfg, n_cta):
+    """Phases per Euler step of the one-observation loop kernel for an expert of these sizes with n_cta resident CTAs (whole clusters
+    of eight); 0: such calls run a launch per operator.  Needs no GPU."""
+    return lib().vlab200_loop_kernel_phases(C.byref(_policy_config(cfg)), int(n_cta))
+
+
 _PER_LAYER = ("wq", "wk", "wv", "wo", "wgate", "wup", "wdown", "ln_in", "ln_post")
 _GLOBAL = ("w_sp", "b_sp", "w_ain", "b_ain", "w_at1", "b_at1", "w_at2", "b_at2", "out_norm", "w_aout", "b_aout")
 # pi0.5 (model 2): adaptive-norm dense maps per layer and the time MLP, all float32
@@ -421,7 +432,7 @@ class PolicyEngine:
         import torch
 
         self.cfg = dict(cfg)
-        c = _PolicyConfig(**{k: cfg.get(k, 0) if k == "cond_dim" else cfg[k] for k, _ in _PolicyConfig._fields_})
+        c = _policy_config(cfg)
         w = _PolicyWeights()
         keep = []
         ada = cfg["model"] == 2
@@ -528,6 +539,12 @@ class PolicyEngine:
         """Prefix rows in use from now on (<= the length the engine was created with)."""
         _check(lib().vlab200_engine_set_prefix_len(C.c_void_p(self.h), int(prefix_len)), "vlab200_engine_set_prefix_len")
         self.prefix_len = int(prefix_len)
+
+    @property
+    def loop_phases(self):
+        """Phases per Euler step of the loop kernel the engine holds for calls with one observation; 0: they run a launch per operator
+        (or there was none yet)."""
+        return lib().vlab200_engine_loop_phases(C.c_void_p(self.h))
 
     STAGES = {"qkv": 0, "attention": 1, "o_proj": 2, "gate_up": 3, "down": 4}
 

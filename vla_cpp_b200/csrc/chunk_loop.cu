@@ -16,9 +16,10 @@
 //            projection with the bf16 mirror and sums of squares (the consumer's RMS factor), act(gate) * up, RMS factor + NeoX
 //            rotation + append of q|k|v, bias + activation, the Euler update.  A CTA so reads M x K / kd of the activations
 //            instead of all of them: without the split the 148 copies of A alone were 2 us of L2 traffic per phase (4 x that
-//            for Wdown), and Wo / Wdown kept 64 of 148 SMs busy.  kd is chosen per product by choose_kd.
+//            for Wdown), and Wo / Wdown kept 64 of 148 SMs busy.  kd is chosen per product by choose_kd; a product too wide for
+//            the shared memory of one phase (an MLP above about 5,700 columns at a width of 1024) is cut into several by plan_gemm.
 //            Weights and activations lie as tcgen05 reads them (K-major, SWIZZLE_128B blocks of 64 columns), weights as
-//            [CTA group][pass][64-column block][row], so that any range of blocks is one contiguous cp.async.bulk (a bulk copy costs
+//            [CTA group][64-column block][row], so that any range of blocks is one contiguous cp.async.bulk (a bulk copy costs
 //            its issuing thread 40-60 ns whatever its size; 51 row copies of 2 KB took 3 us).  They arrive in a ring that one
 //            thread feeds from a cursor which runs AHEAD of the computation, across phase boundaries and barriers (weights do
 //            not depend on anything the loop computes), so HBM streams while the CTAs wait for each other; another warp
@@ -59,13 +60,13 @@ constexpr int CL_BLOCK = 320;     // + one warp whose lane 0 feeds the weight ri
 constexpr int CL_CLUSTER = 8;     // CTAs per cluster (the portable maximum)
 constexpr int CL_STAGES = 4;
 constexpr int CL_STAGE_BYTES = 22528;                             // 22 tiles (8 columns x 64 K) of 1 KB
-constexpr int CL_PASS_N8 = 22;                                    // 8-column groups a CTA group works on at once: 176 weight rows, two tiles of 128
-constexpr int CL_PASSES = 2;                                      // at most two passes per group: the exchange has a buffer for each
+constexpr int CL_GROUP_N8 = 22;                                   // most 8-column groups of a CTA group in one phase: 176 weight rows, two tiles of 128
+constexpr int CL_LAYER_PRODUCTS = 7;                              // most phases of a layer beside attention (make_plan)
 constexpr int CL_TMEM_COLS = 128;                                 // an accumulator of 64 columns (tokens) per tile of 128 weight rows
 constexpr int CL_DESC_BYTES = 352;                                // one phase descriptor slot (two of them: this phase, the next)
 constexpr int CL_DESC_OFF = 1536;
-constexpr int CL_WTAB_OFF = 2304;                                 // weight feeder table: one 32-byte entry per GEMM phase of a step
-constexpr int CL_WTAB_MAX = 104;
+constexpr int CL_WTAB_OFF = 2304;                                 // weight feeder table: one 16-byte entry per GEMM phase of a step
+constexpr int CL_WTAB_MAX = 240;
 constexpr int CL_HEADER = 6144;                                   // barriers, abort flag, small float arrays, descriptors, feeder table
 constexpr int CL_RING_OFF = CL_HEADER;
 constexpr int CL_ARENA_OFF = CL_RING_OFF + CL_STAGES * CL_STAGE_BYTES;
@@ -83,6 +84,7 @@ __host__ __device__ __forceinline__ uint32_t sw_off(int rows8, int row, int col)
 struct alignas(16) LoopPhase {
     int type, out_mode, act, use_rms;
     int M, N8, K, kd;                   // N8: 8-column groups; kd: CTAs that share a product's K / an attention unit's keys
+    int n8_0, N;                        // the phase's first 8-column group, columns of the whole product
     int half, ssq_n, row_off, out_rows8;  // half = head_dim / 2 (q|k|v)
     float eps, scale_log2, dt;
     int bias_step_stride;
@@ -185,16 +187,16 @@ __device__ __forceinline__ void arrive_rank(uint32_t bar) {
 
 struct WEntry {  // what the weight feeder and the product issuer need to know about one GEMM phase
     const uint8_t *Wp;
-    int N8, K, kd, M, unused[2];
+    uint32_t n8_kb, kd_m;  // 8-column groups | 64-column blocks of K << 16, CTAs that share K | tokens << 16
 };
 static_assert(sizeof(LoopPhase) <= CL_DESC_BYTES && sizeof(LoopPhase) % 16 == 0, "descriptor slot");
-static_assert(sizeof(WEntry) == 32, "feeder table entry");
+static_assert(sizeof(WEntry) == 16 && CL_WTAB_OFF + CL_WTAB_MAX * 16 <= CL_HEADER, "feeder table");
 
 // barrier of the computing warps (the feeder warp is not part of it)
 __device__ __forceinline__ void cons_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 struct Smem {
-    uint64_t *full, *empty, *a_full, *acc_full, *acc_free, *k_full, *v_full, *x_full, *xa_full, *rdy, *done;
+    uint64_t *full, *empty, *a_full, *acc_full, *k_full, *v_full, *x_full, *xa_full, *rdy, *done;
     const WEntry *wtab;
     int n_wtab;
     volatile int *abort_flag;
@@ -213,11 +215,10 @@ __device__ __forceinline__ Smem get_smem() {
     sm.empty = sm.full + CL_STAGES;                    // [CL_STAGES]
     sm.a_full = sm.empty + CL_STAGES;                  // a product's A tile has landed
     sm.acc_full = sm.a_full + 1;                       // its accumulator is complete
-    sm.acc_free = sm.acc_full + 1;                     // it has been read
-    sm.k_full = sm.acc_free + 1;                       // attention: Q and K, V
+    sm.k_full = sm.acc_full + 1;                       // attention: Q and K, V
     sm.v_full = sm.k_full + 1;
-    sm.x_full = sm.v_full + 1;                         // [CL_PASSES]: the group's partial sums have arrived
-    sm.xa_full = sm.x_full + CL_PASSES;                // attention: its rows have
+    sm.x_full = sm.v_full + 1;                         // the group's partial sums have arrived
+    sm.xa_full = sm.x_full + 1;                        // attention: its rows have
     sm.rdy = sm.xa_full + 1;
     sm.done = sm.rdy + 1;
     sm.abort_flag = reinterpret_cast<volatile int *>(smem_raw + 224);
@@ -236,15 +237,15 @@ __device__ __forceinline__ Smem get_smem() {
 }
 
 // The computing warps' barrier parities, one bit each, carried from phase to phase.
-constexpr unsigned PAR_K = 0, PAR_V = 1, PAR_RDY = 2, PAR_XA = 3, PAR_ACC = 4, PAR_X = 5 /* + pass */;
+constexpr unsigned PAR_K = 0, PAR_V = 1, PAR_RDY = 2, PAR_XA = 3, PAR_ACC = 4, PAR_X = 5;
 __device__ __forceinline__ uint32_t par_bit(unsigned par, unsigned which) { return (par >> which) & 1u; }
 
 // This CTA's part of a product: its group's 8-column groups [j0, j0 + w8) and the 64-column blocks [kb0, kb1) of K it multiplies.
 struct GemmPart {
     int kr, j0, w8, kb0, kb1;
 };
-__device__ __forceinline__ GemmPart gemm_part(int N8, int K, int kd) {
-    const int sh = 31 - __clz(kd), G = gridDim.x >> sh, grp = blockIdx.x >> sh, kb = (K + 63) >> 6;
+__device__ __forceinline__ GemmPart gemm_part(int N8, int kb, int kd) {
+    const int sh = 31 - __clz(kd), G = gridDim.x >> sh, grp = blockIdx.x >> sh;
     GemmPart r;
     r.kr = blockIdx.x & (kd - 1);
     r.j0 = (int)((unsigned)(N8 * grp) / (unsigned)G);
@@ -265,21 +266,20 @@ __device__ __noinline__ void feeder_loop(const LoopParams &lp) {
     for (int step = 0; ok && step < lp.steps; ++step)
         for (int gi = 0; ok && gi < sm.n_wtab; ++gi) {
             const WEntry w = sm.wtab[gi];
-            const GemmPart gp = gemm_part(w.N8, w.K, w.kd);
-            const int kb = (w.K + 63) >> 6;
-            for (int p0 = 0; ok && p0 < gp.w8; p0 += CL_PASS_N8) {
-                const int w8p = min(CL_PASS_N8, gp.w8 - p0), kc = CL_STAGE_BYTES / (w8p * 1024);
-                const uint8_t *src = w.Wp + (size_t)(gp.j0 + p0) * kb * 1024;
-                for (int k0 = gp.kb0; k0 < gp.kb1; k0 += kc, ++issued) {
-                    const unsigned stage = issued % CL_STAGES;
-                    if (issued >= CL_STAGES && !mbar_wait_backoff(&sm.empty[stage], ((issued / CL_STAGES) - 1u) & 1u, wc, CL_DEV_TIMEOUT, 20)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t bytes = (uint32_t)(min(kc, gp.kb1 - k0) * w8p) * 1024u;
-                    mbar_expect_tx(&sm.full[stage], bytes);
-                    bulk_g2s(sm.ring + (size_t)stage * CL_STAGE_BYTES, src + (size_t)k0 * w8p * 1024, bytes, &sm.full[stage]);
+            const int kb = (int)(w.n8_kb >> 16);
+            const GemmPart gp = gemm_part((int)(w.n8_kb & 0xffffu), kb, (int)(w.kd_m & 0xffffu));
+            if (gp.w8 <= 0) continue;
+            const int kc = CL_STAGE_BYTES / (gp.w8 * 1024);
+            const uint8_t *src = w.Wp + (size_t)gp.j0 * kb * 1024;
+            for (int k0 = gp.kb0; k0 < gp.kb1; k0 += kc, ++issued) {
+                const unsigned stage = issued % CL_STAGES;
+                if (issued >= CL_STAGES && !mbar_wait_backoff(&sm.empty[stage], ((issued / CL_STAGES) - 1u) & 1u, wc, CL_DEV_TIMEOUT, 20)) {
+                    ok = false;
+                    break;
                 }
+                const uint32_t bytes = (uint32_t)(min(kc, gp.kb1 - k0) * gp.w8) * 1024u;
+                mbar_expect_tx(&sm.full[stage], bytes);
+                bulk_g2s(sm.ring + (size_t)stage * CL_STAGE_BYTES, src + (size_t)k0 * gp.w8 * 1024, bytes, &sm.full[stage]);
             }
         }
     *sm.issued = issued;
@@ -293,49 +293,45 @@ __device__ __noinline__ void feeder_loop(const LoopParams &lp) {
 __device__ __noinline__ void issuer_loop(const LoopParams &lp, uint32_t tmem) {
     const Smem sm = get_smem();
     const WaitCtx wc{sm.abort_flag, lp.status};
-    unsigned cons = 0, a_cnt = 0, acc_cnt = 0;
+    unsigned cons = 0, a_cnt = 0;
     bool ok = true;
     const uint64_t a_desc0 = smem_desc_sw128(smem_u32(sm.ring), 16, 1024), b_desc0 = smem_desc_sw128(smem_u32(sm.arena), 16, 1024);
     for (int step = 0; ok && step < lp.steps; ++step)
         for (int gi = 0; ok && gi < sm.n_wtab; ++gi) {
-            WEntry w = sm.wtab[gi];
-            w.N8 = __shfl_sync(0xffffffffu, w.N8, 0); w.K = __shfl_sync(0xffffffffu, w.K, 0);
-            w.kd = __shfl_sync(0xffffffffu, w.kd, 0); w.M = __shfl_sync(0xffffffffu, w.M, 0);
-            const GemmPart gp = gemm_part(w.N8, w.K, w.kd);
-            if (gp.w8 <= 0 || gp.kb0 >= gp.kb1) continue;
-            const uint32_t idesc = make_idesc(1, 1, 1, 0, 0, 128, (w.M + 15) & ~15);
-            const uint32_t b_blk = (uint32_t)((w.M + 7) & ~7) * 8u;  // one 64-column block of A, in descriptor units of 16 bytes
+            const WEntry &w = sm.wtab[gi];
+            const uint32_t n8_kb = __shfl_sync(0xffffffffu, w.n8_kb, 0), kd_m = __shfl_sync(0xffffffffu, w.kd_m, 0);
+            const GemmPart gp = gemm_part((int)(n8_kb & 0xffffu), (int)(n8_kb >> 16), (int)(kd_m & 0xffffu));
+            const int M = (int)(kd_m >> 16);
+            if (gp.w8 <= 0) continue;
+            const uint32_t idesc = make_idesc(1, 1, 1, 0, 0, 128, (M + 15) & ~15);
+            const uint32_t b_blk = (uint32_t)((M + 7) & ~7) * 8u;  // one 64-column block of A, in descriptor units of 16 bytes
             ok = warp_wait(sm.a_full, a_cnt & 1u, wc, CL_DEV_TIMEOUT);
             ++a_cnt;
+            if (!ok) break;
             tc_fence_after();
-            for (int p0 = 0; ok && p0 < gp.w8; p0 += CL_PASS_N8, ++acc_cnt) {
-                const int w8p = min(CL_PASS_N8, gp.w8 - p0), kc = CL_STAGE_BYTES / (w8p * 1024);
-                if (p0 > 0) {  // (before a phase's first pass the grid barrier has seen to it)
-                    ok = warp_wait(sm.acc_free, (acc_cnt & 1u) ^ 1u, wc, CL_DEV_TIMEOUT);
-                    tc_fence_after();
-                }
-                for (int k0 = gp.kb0; k0 < gp.kb1; k0 += kc, ++cons) {
-                    const unsigned stage = cons % CL_STAGES;
-                    ok = warp_wait(&sm.full[stage], (cons / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const int nk = min(kc, gp.kb1 - k0);
-                    for (int kk = 0; kk < nk; ++kk) {
-                        const uint64_t a = a_desc0 + (uint64_t)(stage * (CL_STAGE_BYTES / 16) + (unsigned)(kk * w8p) * 64u);
-                        const uint64_t b = b_desc0 + (uint64_t)((uint32_t)(k0 + kk - gp.kb0) * b_blk);
-                        const uint32_t acc = k0 + kk > gp.kb0 ? 1u : 0u;
-                        if (elect_one()) {
+            const int kc = CL_STAGE_BYTES / (gp.w8 * 1024);
+            for (int k0 = gp.kb0; k0 < gp.kb1; k0 += kc, ++cons) {
+                const unsigned stage = cons % CL_STAGES;
+                ok = warp_wait(&sm.full[stage], (cons / CL_STAGES) & 1u, wc, CL_DEV_TIMEOUT);
+                if (!ok) break;
+                tc_fence_after();
+                const int nk = min(kc, gp.kb1 - k0);
+#pragma unroll 1  // unrolled, its code does not stay in the instruction cache beside the phases' (pi0 6,715 -> 6,497 us)
+                for (int kk = 0; kk < nk; ++kk) {
+                    const uint64_t a = a_desc0 + (uint64_t)(stage * (CL_STAGE_BYTES / 16) + (unsigned)(kk * gp.w8) * 64u);
+                    const uint64_t b = b_desc0 + (uint64_t)((uint32_t)(k0 + kk - gp.kb0) * b_blk);
+                    const uint32_t acc = k0 + kk > gp.kb0 ? 1u : 0u;
+                    if (elect_one()) {
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                mma_f16(tmem, a + 2 * k, b + 2 * k, idesc, k ? 1u : acc);
-                                if (w8p > 16) mma_f16(tmem + 64u, a + 1024 + 2 * k, b + 2 * k, idesc, k ? 1u : acc);
-                            }
+                        for (int k = 0; k < 4; ++k) {
+                            mma_f16(tmem, a + 2 * k, b + 2 * k, idesc, k ? 1u : acc);
+                            if (gp.w8 > 16) mma_f16(tmem + 64u, a + 1024 + 2 * k, b + 2 * k, idesc, k ? 1u : acc);
                         }
                     }
-                    if (elect_one()) tc_commit(&sm.empty[stage]);
                 }
-                if (ok && elect_one()) tc_commit(sm.acc_full);
+                if (elect_one()) tc_commit(&sm.empty[stage]);
             }
+            if (ok && elect_one()) tc_commit(sm.acc_full);
         }
     if (elect_one()) {
         *sm.consumed = cons;
@@ -405,7 +401,7 @@ __device__ __forceinline__ void epi_static(const LoopPhase &pg, EpiPre &e, int s
 }
 // what they wrote
 __device__ __forceinline__ void epi_dynamic(const LoopPhase &pg, EpiPre &e, int n8, int row) {
-    const int col = n8 * 8, N = pg.N8 * 8;
+    const int col = n8 * 8, N = pg.N;
     if (pg.out_mode == OUT_RESID) {
         const float *h = pg.h + (size_t)row * N + col;
         e.a0 = ldcg4(h); e.a1 = ldcg4(h + 4);
@@ -430,7 +426,7 @@ __device__ __forceinline__ float bf2_sq(uint32_t v) {
 __device__ __forceinline__ float sq8(uint4 v) { return (bf2_sq(v.x) + bf2_sq(v.y)) + (bf2_sq(v.z) + bf2_sq(v.w)); }
 // v, w: the products of the group's columns 0 .. 3 and 4 .. 7, RMS factor applied.  Returns the sum of squares of what the next norm reads.
 __device__ __forceinline__ float epi_item(const LoopPhase &pg, const EpiPre &e, int n8, int row, float4 v, float4 w) {
-    const int N = pg.N8 * 8, col = n8 * 8;
+    const int N = pg.N, col = n8 * 8;
     switch (pg.out_mode) {
     case OUT_RESID: {  // residual stream += projection; bf16 mirror; sums of squares of the mirror
         if (pg.colscale) {
@@ -513,34 +509,31 @@ __device__ __noinline__ unsigned gemm_phase(const LoopPhase &pg, const LoopParam
     const Smem sm = get_smem();
     const WaitCtx wc{sm.abort_flag, lp.status};
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int M = pg.M, K = pg.K, kd = pg.kd;
-    const GemmPart gp = gemm_part(pg.N8, K, kd);
-    if (gp.w8 <= 0) {
+    const int M = pg.M, K = pg.K, kd = pg.kd, kb = (K + 63) >> 6;
+    const GemmPart gp = gemm_part(pg.N8, kb, kd);
+    const int w8 = gp.w8;
+    if (w8 <= 0) {
         grid_wait(lp, target, sm);
         return par;
     }
     const int sh = 31 - __clz(kd), kr = gp.kr, base_rank = (int)(blockIdx.x % CL_CLUSTER) - kr;
     const uint32_t blk_bytes = (uint32_t)((M + 7) & ~7) * 128u, a_bytes = (uint32_t)(gp.kb1 - gp.kb0) * blk_bytes;
-    // arena: A (the longest of the group) | what the group sends, per pass [source][owned column][token]; this CTA's own sums are staged
-    // over A when one pass does it all (A has been multiplied by then), else behind
-    const int tp = token_pitch(M), w8m = min(CL_PASS_N8, gp.w8), row = tid & 63, cg = tid >> 6;
-    const uint32_t recv_bytes = (uint32_t)((((w8m + kd - 1) >> sh) << sh) * 8 * tp) * 4u;  // kd parts of the most columns one CTA owns
-    const uint32_t recv_off = (uint32_t)((((K + 63) >> 6) + kd - 1) >> sh) * blk_bytes;
-    const bool one_pass = gp.w8 <= CL_PASS_N8;
-    const uint32_t stage_off = one_pass && recv_bytes <= recv_off ? 0u : recv_off + (one_pass ? 1u : (uint32_t)CL_PASSES) * recv_bytes;
+    // arena: A (the longest of the group) | what the group sends, [source][owned column][token]; this CTA's own sums are staged over A
+    // where they fit (A has been multiplied by then), else behind
+    const int tp = token_pitch(M), row = tid & 63, cg = tid >> 6;
+    const uint32_t recv_bytes = (uint32_t)((((w8 + kd - 1) >> sh) << sh) * 8 * tp) * 4u;  // kd parts of the most columns one CTA owns
+    const uint32_t recv_off = (uint32_t)((kb + kd - 1) >> sh) * blk_bytes;
+    const uint32_t stage_off = recv_bytes <= recv_off ? 0u : recv_off + recv_bytes;
     const int hw = warp & 3, th = warp >> 2;  // this warp's quarter of the TMEM lanes and half of the tokens
     // ---- before the barrier: everything that does not depend on the phase before
-    const int own00 = w8m * kr >> sh, oN0 = (w8m * (kr + 1) >> sh) - own00;
+    const int own0 = w8 * kr >> sh, ownN = (w8 * (kr + 1) >> sh) - own0, n8_own = pg.n8_0 + gp.j0 + own0;
     EpiPre pre;
     pre.a0 = pre.a1 = pre.b0 = pre.b1 = pre.c0 = pre.c1 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool first = row < M && cg < oN0;
-    if (first) epi_static(pg, pre, step, gp.j0 + own00 + cg, row);
+    const bool first = row < M && cg < ownN;
+    if (first) epi_static(pg, pre, step, n8_own + cg, row);
     if (tid == 0) {
-        for (int p0 = 0, pass = 0; p0 < gp.w8; p0 += CL_PASS_N8, ++pass) {
-            const int w8p = min(CL_PASS_N8, gp.w8 - p0), oN = (w8p * (kr + 1) >> sh) - (w8p * kr >> sh);
-            mbar_expect_tx(&sm.x_full[pass], (uint32_t)(kd * oN * 8 * tp) * 4u);
-        }
-        if (grid_poll(lp, target, sm) && a_bytes) {
+        mbar_expect_tx(sm.x_full, (uint32_t)(kd * ownN * 8 * tp) * 4u);
+        if (grid_poll(lp, target, sm)) {
             fence_proxy_async_all();
             mbar_expect_tx(sm.a_full, a_bytes);
             bulk_g2s(sm.arena, pg.Ap + (size_t)gp.kb0 * blk_bytes, a_bytes, sm.a_full);
@@ -548,7 +541,7 @@ __device__ __noinline__ unsigned gemm_phase(const LoopPhase &pg, const LoopParam
     }
     cons_sync();
     // ---- after it
-    if (first) epi_dynamic(pg, pre, gp.j0 + own00 + cg, row);
+    if (first) epi_dynamic(pg, pre, n8_own + cg, row);
     const bool use_rms = pg.use_rms != 0;
     if (use_rms) {  // row sums of squares from the producer's partial sums, fixed order
         const int n = pg.ssq_n;
@@ -563,73 +556,59 @@ __device__ __noinline__ unsigned gemm_phase(const LoopPhase &pg, const LoopParam
         }
         sm.red[cg * 64 + row] = ss;
     }
-    for (int p0 = 0, pass = 0; p0 < gp.w8; p0 += CL_PASS_N8, ++pass) {
-        const int w8p = min(CL_PASS_N8, gp.w8 - p0);
-        const int own0 = w8p * kr >> sh, ownN = (w8p * (kr + 1) >> sh) - own0;
-        if (a_bytes) {
-            mbar_wait(sm.acc_full, par_bit(par, PAR_ACC), wc, CL_DEV_TIMEOUT);
-            par ^= 1u << PAR_ACC;
-            tc_fence_after();
-        }
-        // ---- this CTA's K part into its staging area, [column][token]: a lane holds one column, 32 tokens
-        float *stg = reinterpret_cast<float *>(sm.arena + stage_off + (uint32_t)pass * recv_bytes);
-        for (int n0 = hw * 32; n0 < w8p * 8; n0 += 128) {
-            uint32_t v[32];
-            if (a_bytes) {
-                tmem_ld32(tmem + (uint32_t)((n0 >> 7) * 64 + th * 32) + ((uint32_t)(hw * 32) << 16), v);
-                tmem_ld_wait();
-            } else {
+    mbar_wait(sm.acc_full, par_bit(par, PAR_ACC), wc, CL_DEV_TIMEOUT);
+    par ^= 1u << PAR_ACC;
+    tc_fence_after();
+    // ---- this CTA's K part into its staging area, [column][token]: a lane holds one column, 32 tokens
+    float *stg = reinterpret_cast<float *>(sm.arena + stage_off);
+    for (int n0 = hw * 32; n0 < w8 * 8; n0 += 128) {
+        uint32_t v[32];
+        tmem_ld32(tmem + (uint32_t)((n0 >> 7) * 64 + th * 32) + ((uint32_t)(hw * 32) << 16), v);
+        tmem_ld_wait();
+        const int n = n0 + lane;
+        if (n < w8 * 8) {
+            float4 *dst = reinterpret_cast<float4 *>(stg + (size_t)n * tp + th * 32);
 #pragma unroll
-                for (int e = 0; e < 32; ++e) v[e] = 0u;
-            }
-            const int n = n0 + lane;
-            if (n < w8p * 8) {
-                float4 *dst = reinterpret_cast<float4 *>(stg + (size_t)n * tp + th * 32);
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (th * 32 + e * 4 < M)
-                        dst[e] = make_float4(__uint_as_float(v[4 * e]), __uint_as_float(v[4 * e + 1]), __uint_as_float(v[4 * e + 2]), __uint_as_float(v[4 * e + 3]));
-            }
+            for (int e = 0; e < 8; ++e)
+                if (th * 32 + e * 4 < M)
+                    dst[e] = make_float4(__uint_as_float(v[4 * e]), __uint_as_float(v[4 * e + 1]), __uint_as_float(v[4 * e + 2]), __uint_as_float(v[4 * e + 3]));
         }
-        tc_fence_before();
-        fence_proxy_async_smem();
-        cons_sync();  // staged; and the partial sums of squares are in place
-        if (lane == 0) {
-            if (a_bytes) mbar_arrive(sm.acc_free);
-            if (warp < kd) {  // warp w sends rank w of the group its columns
-                const int b = w8p * warp >> sh, oN = (w8p * (warp + 1) >> sh) - b;
-                const uint32_t bytes = (uint32_t)(oN * 8 * tp) * 4u;
-                if (oN > 0)
-                    bulk_s2rank(map_rank(smem_u32(sm.arena + recv_off + (uint32_t)pass * recv_bytes), base_rank + warp) + (uint32_t)kr * bytes,
-                                smem_u32(stg) + (uint32_t)(b * 8 * tp) * 4u, bytes, map_rank(smem_u32(&sm.x_full[pass]), base_rank + warp));
+    }
+    tc_fence_before();
+    fence_proxy_async_smem();
+    cons_sync();  // staged; and the partial sums of squares are in place
+    if (lane == 0 && warp < kd) {  // warp w sends rank w of the group its columns
+        const int b = w8 * warp >> sh, oN = (w8 * (warp + 1) >> sh) - b;
+        const uint32_t bytes = (uint32_t)(oN * 8 * tp) * 4u;
+        if (oN > 0)
+            bulk_s2rank(map_rank(smem_u32(sm.arena + recv_off), base_rank + warp) + (uint32_t)kr * bytes, smem_u32(stg) + (uint32_t)(b * 8 * tp) * 4u,
+                        bytes, map_rank(smem_u32(sm.x_full), base_rank + warp));
+    }
+    const float rms = use_rms ? rsqrtf(((sm.red[row] + sm.red[64 + row]) + (sm.red[128 + row] + sm.red[192 + row])) / (float)K + pg.eps) : 1.0f;
+    mbar_wait_cluster(sm.x_full, par_bit(par, PAR_X), wc, CL_DEV_TIMEOUT);
+    par ^= 1u << PAR_X;
+    if (row < M) {
+        const float *recv = reinterpret_cast<const float *>(sm.arena + recv_off) + row;
+        const int ld = ownN * 8 * tp;
+        for (int jl = cg; jl < ownN; jl += 4) {
+            const int n8 = n8_own + jl;
+            if (jl != cg) {
+                epi_static(pg, pre, step, n8, row);
+                epi_dynamic(pg, pre, n8, row);
             }
-        }
-        const float rms = use_rms ? rsqrtf(((sm.red[row] + sm.red[64 + row]) + (sm.red[128 + row] + sm.red[192 + row])) / (float)K + pg.eps) : 1.0f;
-        mbar_wait_cluster(&sm.x_full[pass], par_bit(par, PAR_X + pass), wc, CL_DEV_TIMEOUT);
-        par ^= 1u << (PAR_X + pass);
-        if (row < M) {
-            const float *recv = reinterpret_cast<const float *>(sm.arena + recv_off + (uint32_t)pass * recv_bytes) + row;
-            const int ld = ownN * 8 * tp;
-            for (int jl = cg; jl < ownN; jl += 4) {
-                const int n8 = gp.j0 + p0 + own0 + jl;
-                if (jl != cg || pass > 0) {
-                    epi_static(pg, pre, step, n8, row);
-                    epi_dynamic(pg, pre, n8, row);
-                }
-                const float *src = recv + (size_t)jl * 8 * tp;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f), w = v;
+            const float *src = recv + (size_t)jl * 8 * tp;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f), w = v;
 #pragma unroll 2
-                for (int s = 0; s < kd; ++s, src += ld) {
-                    v.x += src[0]; v.y += src[tp]; v.z += src[2 * tp]; v.w += src[3 * tp];
-                    w.x += src[4 * tp]; w.y += src[5 * tp]; w.z += src[6 * tp]; w.w += src[7 * tp];
-                }
-                if (use_rms) {
-                    v.x *= rms; v.y *= rms; v.z *= rms; v.w *= rms;
-                    w.x *= rms; w.y *= rms; w.z *= rms; w.w *= rms;
-                }
-                const float ssq = epi_item(pg, pre, n8, row, v, w);
-                if (pg.ssq_out) __stcg(pg.ssq_out + (size_t)n8 * 64 + row + pg.row_off, ssq);
+            for (int s = 0; s < kd; ++s, src += ld) {
+                v.x += src[0]; v.y += src[tp]; v.z += src[2 * tp]; v.w += src[3 * tp];
+                w.x += src[4 * tp]; w.y += src[5 * tp]; w.z += src[6 * tp]; w.w += src[7 * tp];
             }
+            if (use_rms) {
+                v.x *= rms; v.y *= rms; v.z *= rms; v.w *= rms;
+                w.x *= rms; w.y *= rms; w.z *= rms; w.w *= rms;
+            }
+            const float ssq = epi_item(pg, pre, n8, row, v, w);
+            if (pg.ssq_out) __stcg(pg.ssq_out + (size_t)n8 * 64 + row + pg.row_off, ssq);
         }
     }
     return par;
@@ -1008,10 +987,9 @@ __global__ void __launch_bounds__(CL_BLOCK, 1) chunk_loop_kernel(const __grid_co
         }
         mbar_init(sm.a_full, 1);
         mbar_init(sm.acc_full, 1);
-        mbar_init(sm.acc_free, CL_THREADS / 32);
         mbar_init(sm.k_full, 1);
         mbar_init(sm.v_full, 1);
-        for (int i = 0; i < CL_PASSES; ++i) mbar_init(&sm.x_full[i], 1);
+        mbar_init(sm.x_full, 1);
         mbar_init(sm.xa_full, 1);
         mbar_init(sm.rdy, lp.att_cta);
         mbar_init(sm.done, 2);
@@ -1025,7 +1003,7 @@ __global__ void __launch_bounds__(CL_BLOCK, 1) chunk_loop_kernel(const __grid_co
         tmem_alloc(sm.tmem_slot, CL_TMEM_COLS);
         tmem_relinquish();
     }
-    for (int i = threadIdx.x; i < lp.n_wtab * 8; i += CL_BLOCK)
+    for (int i = threadIdx.x; i < lp.n_wtab * 4; i += CL_BLOCK)
         reinterpret_cast<uint32_t *>(wtab)[i] = reinterpret_cast<const uint32_t *>(lp.wtab)[i];
     // descriptor of phase 0 into slot 0; from then on every phase fetches its successor's while it works
     for (int i = threadIdx.x; i < (int)(sizeof(LoopPhase) / 4); i += CL_BLOCK)
@@ -1088,10 +1066,11 @@ __global__ void __launch_bounds__(CL_BLOCK, 1) chunk_loop_kernel(const __grid_co
     }
 }
 
-// dense [N][K] bf16 -> weight image for G CTA groups: [group][pass][64-column block][8-column group][8 rows x 128 bytes, 16-byte
-// chunks permuted by the row]; zeros beyond K.
+// Columns n8_0 * 8 .. (n8_0 + N8) * 8 and K range [k0, k0 + K) of a dense [N][ld] bf16 matrix -> weight image for G CTA groups: [group]
+// [64-column block][8-column group][8 rows x 128 bytes, 16-byte chunks permuted by the row]; zeros beyond K.
 // half > 0 (q|k|v): a group's 8 columns are dims 4 j .. 4 j + 3 of a head and their rotation partners, `half` further on.
-__global__ void weight_image_kernel(const __nv_bfloat16 *__restrict__ src, uint4 *__restrict__ dst, int N8, int K, int G, int half) {
+__global__ void weight_image_kernel(const __nv_bfloat16 *__restrict__ src, uint4 *__restrict__ dst, int n8_0, int N8, int k0, int K, int ld, int G,
+                                    int half) {
     const int kb = (K + 63) >> 6;
     const size_t total = (size_t)N8 * kb * 64;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -1099,15 +1078,14 @@ __global__ void weight_image_kernel(const __nv_bfloat16 *__restrict__ src, uint4
         size_t r = i >> 6;
         const int b = (int)(r % kb), n8 = (int)(r / kb);
         const int grp = (int)((((long long)n8 + 1) * G - 1) / N8), j0 = (int)((long long)N8 * grp / G), w8 = (int)((long long)N8 * (grp + 1) / G) - j0;
-        const int p0 = (n8 - j0) / CL_PASS_N8 * CL_PASS_N8, w8p = min(CL_PASS_N8, w8 - p0), j = n8 - j0 - p0;
-        int row = n8 * 8 + c;
+        int row = (n8_0 + n8) * 8 + c;
         if (half > 0) {
-            const int per = half >> 2, head = n8 / per, jj = n8 - head * per;
+            const int per = half >> 2, head = (n8_0 + n8) / per, jj = n8_0 + n8 - head * per;
             row = head * 2 * half + 4 * jj + (c & 3) + (c >= 4 ? half : 0);
         }
         const int k = b * 64 + c16 * 8;
-        const uint4 v = k < K ? *reinterpret_cast<const uint4 *>(src + (size_t)row * K + k) : make_uint4(0u, 0u, 0u, 0u);
-        dst[((size_t)(j0 + p0) * kb + (size_t)b * w8p + j) * 64 + c * 8 + (c16 ^ c)] = v;
+        const uint4 v = k < K ? *reinterpret_cast<const uint4 *>(src + (size_t)row * ld + k0 + k) : make_uint4(0u, 0u, 0u, 0u);
+        dst[((size_t)j0 * kb + (size_t)b * w8 + (n8 - j0)) * 64 + c * 8 + (c16 ^ c)] = v;
     }
 }
 
@@ -1163,55 +1141,113 @@ void loop_launch_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int 
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
 size_t image_bytes(int rows, int K) { return (size_t)round_up(rows, 8) * 128 * ((K + 63) / 64); }
 
-// one pass of a group: kd parts of the most columns one CTA owns
-size_t exchange_bytes(int M, int w8, int kd) { return (size_t)round_up(std::min(w8, CL_PASS_N8), kd) * 8 * token_pitch(M) * 4; }
+// kd parts of the most columns one CTA owns
+size_t exchange_bytes(int M, int w8, int kd) { return (size_t)round_up(w8, kd) * 8 * token_pitch(M) * 4; }
 
-// Does a product fit the arena when kd CTAs share its K?  A of one CTA + what the group sends it + its own sums, staged.
-bool gemm_fits(int M, int N8, int K, int kd, int n_cta) {
-    const int G = n_cta / kd, w8 = (N8 + G - 1) / G, passes = (w8 + CL_PASS_N8 - 1) / CL_PASS_N8, kb = (K + 63) / 64;
-    if (passes > CL_PASSES) return false;
+// Arena bytes of a product of kb 64-column blocks shared by kd CTAs: A of one CTA + what the group sends it + its own sums (over A
+// where they fit there).
+size_t gemm_arena(int M, int w8, int kb, int kd) {
     const size_t a = (size_t)((kb + kd - 1) / kd) * round_up(M, 8) * 128, x = exchange_bytes(M, w8, kd);
-    return a + x * (passes == 1 ? (x <= a ? 1 : 2) : 2 * CL_PASSES) <= (size_t)CL_ARENA;
+    return a + x * (x <= a ? 1 : 2);
 }
 
-// End of the arena range in which a product's own sums are staged (gemm_phase: over A when they fit there in one pass).
-size_t staged_end(int M, int w8, int K, int kd) {
-    const int kb = (K + 63) / 64, passes = (w8 + CL_PASS_N8 - 1) / CL_PASS_N8;
+// End of the arena range in which its own sums are staged (gemm_phase).
+size_t staged_end(int M, int w8, int kb, int kd) {
     const size_t a = (size_t)((kb + kd - 1) / kd) * round_up(M, 8) * 128, x = exchange_bytes(M, w8, kd);
-    return passes == 1 && x <= a ? x : a + (passes == 1 ? 2 : 2 * CL_PASSES) * x;
+    return x <= a ? x : a + 2 * x;
 }
+
+// How a product runs: kd CTAs share K; `cols` phases each take a part of the columns, `ks` phases each a part of K (only where the
+// output is added to).
+struct GemmPlan {
+    int kd, cols, ks;
+};
 
 // CTAs that share a product's K: least (A in at ~50 B/ns and SM, partial sums out at ~20 B/ns, products at ~48 clocks per 128 x 64 x
-// 16).  More CTAs per group read less of A and send more partial sums.
-int choose_kd(int M, int N8, int K, int n_cta) {
+// 16).  More CTAs per group read less of A and send more partial sums.  0: no number of them fits.  kb_min: blocks of the shortest part.
+int choose_kd(int M, int N8, int kb, int kb_min, int n_cta, double *cost_out) {
     int best = 0;
-    double best_cost = 0;
-    for (int kd = 1; kd <= CL_CLUSTER; kd *= 2) {
-        if ((kd > 1 && (K + 63) / 64 < kd) || !gemm_fits(M, N8, K, kd, n_cta)) continue;
-        const int G = n_cta / kd, w8 = (N8 + G - 1) / G, kb = ((K + 63) / 64 + kd - 1) / kd;
-        const double a = (double)M * kb * 128 / 50.0, x = (double)M * w8 * 32 * (kd - 1) / kd / 20.0;
-        double mma = 0;
-        for (int p = 0; p < w8; p += CL_PASS_N8) mma += kb * 4 * (std::min(CL_PASS_N8, w8 - p) > 16 ? 2 : 1) * 48 / 1.9;
-        const double cost = a + x + mma;
-        if (!best || cost < best_cost) {
+    for (int kd = 1; kd <= CL_CLUSTER && kd <= kb_min; kd *= 2) {
+        const int G = n_cta / kd, w8 = (N8 + G - 1) / G, kbc = (kb + kd - 1) / kd;
+        // (a shorter part may have to stage its sums behind A where the longest does not)
+        if (w8 > CL_GROUP_N8 || std::max(gemm_arena(M, w8, kb, kd), gemm_arena(M, w8, kb_min, kd)) > (size_t)CL_ARENA) continue;
+        const double a = (double)M * kbc * 128 / 50.0, x = (double)M * w8 * 32 * (kd - 1) / kd / 20.0;
+        const double cost = a + x + kbc * 4 * (w8 > 16 ? 2 : 1) * 48 / 1.9;
+        if (!best || cost < *cost_out) {
             best = kd;
-            best_cost = cost;
+            *cost_out = cost;
         }
     }
     return best;
 }
 
+// The fewest phases in which the product fits (each costs a round of its own: barrier, A, exchange), then the cheapest way to cut it.
+// kd == 0: none.
+GemmPlan plan_gemm(int M, int N8, int K, bool adds, int n_cta) {
+    const int kb = (K + 63) / 64;
+    GemmPlan best{0, 1, 1};
+    if (N8 > 65535 || kb > 65535) return best;
+    double best_cost = 0;
+    for (int parts = 1; parts < CL_LAYER_PRODUCTS && !best.kd; ++parts)
+        for (int ks = 1; ks <= parts; ++ks) {
+            const int cols = parts / ks;
+            if (cols * ks != parts || (ks > 1 && !adds) || ks > kb || cols > N8) continue;
+            double cost = 0;
+            const int kd = choose_kd(M, (N8 + cols - 1) / cols, (kb + ks - 1) / ks, kb / ks, n_cta, &cost);
+            if (kd && (!best.kd || cost < best_cost)) {
+                best = {kd, cols, ks};
+                best_cost = cost;
+            }
+        }
+    return best;
+}
+
+// What the kernel does for an expert of these sizes with n_cta CTAs resident.
+struct LoopPlan {
+    GemmPlan qkv, gu, o, dn, mlp, head;  // qkv: of self layers, cross layers have fewer columns; mlp: the two products of the suffix embedding
+    int att_cta, n_phases, n_wtab;  // CTAs per attention unit; phases and products per Euler step
+};
+
+bool make_plan(const ChunkLoopDesc &d, int n_cta, LoopPlan *out) {
+    const int hd = d.hd, qf = d.n_q * hd, H = d.H, S = d.S;
+    if (n_cta < CL_CLUSTER || n_cta % CL_CLUSTER || d.model < 0 || d.model > 2 || (d.model == 2 && H % 32)) return false;
+    if (hd != 64 && hd != 128 && hd != 256) return false;
+    if (S > 64 || H % 16 || d.A % 16 || qf % 16 || d.I % 16) return false;
+    if ((size_t)(d.chunk * d.A + 64) * 4 > (size_t)CL_ARENA || d.A > 64) return false;
+    LoopPlan &p = *out;
+    p.qkv = plan_gemm(S, (d.n_q + 2 * d.n_kv) * hd / 8, H, false, n_cta);
+    p.gu = plan_gemm(S, 2 * d.I / 8, H, false, n_cta);
+    p.o = plan_gemm(S, H / 8, qf, true, n_cta);
+    p.dn = plan_gemm(S, H / 8, d.I, true, n_cta);
+    p.mlp = plan_gemm(d.chunk, H / 8, H, false, n_cta);
+    p.head = plan_gemm(S, d.A / 8, H, false, n_cta);
+    for (const GemmPlan *g : {&p.qkv, &p.gu, &p.o, &p.dn, &p.mlp, &p.head})
+        if (!g->kd) return false;
+    // attention units of 32 query rows: as many CTAs each as there are for one round (they split the keys)
+    const int units = d.n_kv * ((d.n_q / d.n_kv * S + 31) / 32);
+    p.att_cta = 1;
+    while (p.att_cta < CL_CLUSTER && units <= n_cta / (2 * p.att_cta)) p.att_cta *= 2;
+    // With nine phases a layer a launch per operator is as fast (pi0's depth and width, ms per chunk here and there: MLP width 4096
+    // 6.4 and 10.7, 8192 9.2 and 11.4, 12288 11.2 and 13.7, 14336 in eight phases 11.6 and 12.7, 16384 in nine 13.4 and 13.2).
+    const int layer = p.qkv.cols + p.gu.cols + p.o.cols * p.o.ks + p.dn.cols * p.dn.ks;
+    p.n_wtab = d.L * layer + p.head.cols + (d.model == 2 ? 0 : 2 * p.mlp.cols);
+    p.n_phases = p.n_wtab + d.L + 1;
+    return layer <= CL_LAYER_PRODUCTS && p.n_wtab <= CL_WTAB_MAX;
+}
+
 }  // namespace
+
+int chunk_loop_plan_phases(const ChunkLoopDesc &d, int n_cta) {
+    LoopPlan plan;
+    return make_plan(d, n_cta, &plan) ? plan.n_phases : 0;
+}
 
 int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
     *out = nullptr;
     const int n_sm = sm_count();
     if (n_sm <= 0) return VLAB200_ERR_CUDA;
     const int hd = d.hd, half = hd / 2, qf = d.n_q * hd, H = d.H, S = d.S;
-    if (d.model < 0 || d.model > 2 || (d.model == 2 && (!d.mods || H % 32))) return VLAB200_ERR_UNSUPPORTED;
-    if (hd != 64 && hd != 128 && hd != 256) return VLAB200_ERR_UNSUPPORTED;
-    if (S > 64 || H % 16 || d.A % 16 || (2 * d.I) % 16 || qf % 16 || d.I % 16) return VLAB200_ERR_UNSUPPORTED;
-    if ((size_t)(d.chunk * d.A + 64) * 4 > (size_t)CL_ARENA || d.A > 64) return VLAB200_ERR_UNSUPPORTED;
+    if ((hd != 64 && hd != 128 && hd != 256) || (d.model == 2 && !d.mods)) return VLAB200_ERR_UNSUPPORTED;
     const void *kernel = hd == 64    ? reinterpret_cast<const void *>(chunk_loop_kernel<64>)
                          : hd == 128 ? reinterpret_cast<const void *>(chunk_loop_kernel<128>)
                                      : reinterpret_cast<const void *>(chunk_loop_kernel<256>);
@@ -1228,14 +1264,9 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
     n_clusters = std::min(n_clusters, n_sm / CL_CLUSTER);
     if (n_clusters < 1 || !coop) return VLAB200_ERR_UNSUPPORTED;
     const int n_cta = n_clusters * CL_CLUSTER;
-    const int g = d.n_q / d.n_kv, R = g * S, n_rt = (R + 31) / 32;
-    const int qkv_n8 = (d.n_q + 2 * d.n_kv) * hd / 8;
-    const int kd_qkv = choose_kd(S, qkv_n8, H, n_cta), kd_gu = choose_kd(S, 2 * d.I / 8, H, n_cta), kd_o = choose_kd(S, H / 8, qf, n_cta);
-    const int kd_d = choose_kd(S, H / 8, d.I, n_cta), kd_m = choose_kd(d.chunk, H / 8, H, n_cta), kd_h = choose_kd(S, d.A / 8, H, n_cta);
-    if (!kd_qkv || !kd_gu || !kd_o || !kd_d || !kd_m || !kd_h) return VLAB200_ERR_UNSUPPORTED;
-    // attention units of 32 query rows: as many CTAs each as there are for one round (they split the keys)
-    int att_cta = 1;
-    while (att_cta < CL_CLUSTER && d.n_kv * n_rt <= n_cta / (2 * att_cta)) att_cta *= 2;
+    LoopPlan plan;
+    if (!make_plan(d, n_cta, &plan)) return VLAB200_ERR_UNSUPPORTED;
+    const int g = d.n_q / d.n_kv, R = g * S, n_rt = (R + 31) / 32, att_cta = plan.att_cta;
 
     ChunkLoop *cl = new (std::nothrow) ChunkLoop();
     if (!cl) return VLAB200_ERR_CUDA;
@@ -1257,27 +1288,38 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
         if ((rc = z.b->alloc(z.bytes))) return fail(rc);
         if (cudaMemset(z.b->p, 0, z.bytes) != cudaSuccess) return fail(VLAB200_ERR_CUDA);
     }
-    // weights as tcgen05 reads them, in the order of the CTA groups
-    auto weight_image = [&](const void *w, int N8, int K, int kd, int half_, const uint8_t **image) -> int {
-        cl->wp.emplace_back();
-        DevBuf &b = cl->wp.back();
-        int r = b.alloc((size_t)N8 * ((K + 63) / 64) * 1024);
-        if (r) return r;
-        weight_image_kernel<<<n_sm * 4, 256>>>(static_cast<const __nv_bfloat16 *>(w), b.as<uint4>(), N8, K, n_cta / kd, half_);
-        VB_CUDA(cudaGetLastError());
-        *image = b.as<uint8_t>();
+    cl->wp.reserve((size_t)plan.n_wtab);
+    auto no_room = [&] {  // for a second copy of the weights: not an error of the call
+        cudaGetLastError();
+        return fail(VLAB200_ERR_UNSUPPORTED);
+    };
+    std::vector<LoopPhase> ph;
+    // One product: p says what goes in (Ap, M) and out; its weights as tcgen05 reads them, in the order of the CTA groups.
+    auto push_gemm = [&](LoopPhase p, const void *w_dense, int N, int K, const GemmPlan &gp) -> int {
+        const int N8 = N / 8, kb = (K + 63) / 64;
+        p.type = PH_GEMM; p.N = N; p.kd = gp.kd; p.half = p.out_mode == OUT_QKV ? half : 0; p.eps = d.rms_eps; p.S = S; p.chunk = d.chunk;
+        const uint8_t *a_image = p.Ap;
+        for (int ci = 0; ci < gp.cols; ++ci)
+            for (int ki = 0; ki < gp.ks; ++ki) {
+                const int kb0 = kb * ki / gp.ks, kb1 = kb * (ki + 1) / gp.ks;
+                p.n8_0 = N8 * ci / gp.cols; p.N8 = N8 * (ci + 1) / gp.cols - p.n8_0;
+                p.K = std::min(K, kb1 * 64) - kb0 * 64;
+                p.Ap = a_image + (size_t)kb0 * round_up(p.M, 8) * 128;
+                cl->wp.emplace_back();
+                DevBuf &b = cl->wp.back();
+                const int r = b.alloc((size_t)p.N8 * (kb1 - kb0) * 1024);
+                if (r) return r;
+                weight_image_kernel<<<n_sm * 4, 256>>>(static_cast<const __nv_bfloat16 *>(w_dense), b.as<uint4>(), p.n8_0, p.N8, kb0 * 64, p.K, K,
+                                                       n_cta / gp.kd, p.half);
+                VB_CUDA(cudaGetLastError());
+                p.Wp = b.as<uint8_t>();
+                ph.push_back(p);
+            }
         return VLAB200_OK;
     };
-    cl->wp.reserve((size_t)d.L * 4 + 8);
-
-    std::vector<LoopPhase> ph;
-    bool bad = false;
-    auto gemm = [&](const uint8_t *Ap, int M, const void *w_dense, int N, int K, int kd, int out_mode) {
+    auto product = [&](const uint8_t *Ap, int M, int out_mode) {
         LoopPhase p{};
-        p.type = PH_GEMM; p.out_mode = out_mode; p.Ap = Ap; p.M = M; p.N8 = N / 8; p.K = K; p.kd = kd;
-        p.half = out_mode == OUT_QKV ? half : 0;
-        p.eps = d.rms_eps; p.S = S; p.chunk = d.chunk;
-        if (weight_image(w_dense, N / 8, K, kd, p.half, &p.Wp)) bad = true;
+        p.Ap = Ap; p.M = M; p.out_mode = out_mode;
         return p;
     };
     auto to_mirror = [&](LoopPhase &p) {  // the phase writes the residual mirror
@@ -1315,20 +1357,20 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
         }
         ph.push_back(p);
         if (!ada) {
-            LoopPhase m1 = gemm(cl->ap.as<uint8_t>(), d.chunk, d.w_at1l, H, H, kd_m, OUT_BIAS_ACT);
+            LoopPhase m1 = product(cl->ap.as<uint8_t>(), d.chunk, OUT_BIAS_ACT);
             m1.act = ACT_SILU; m1.bias = d.tvec; m1.bias_step_stride = H; m1.outp = cl->m1p.as<uint8_t>(); m1.out_rows8 = round_up(d.chunk, 8);
-            ph.push_back(m1);
-            LoopPhase m2 = gemm(cl->m1p.as<uint8_t>(), d.chunk, d.w_at2, H, H, kd_m, OUT_BIAS_ACT);
+            if (push_gemm(m1, d.w_at1l, H, H, plan.mlp)) return no_room();
+            LoopPhase m2 = product(cl->m1p.as<uint8_t>(), d.chunk, OUT_BIAS_ACT);
             m2.act = ACT_NONE; m2.bias = d.b_at2; m2.out_f32 = d.h; m2.row_off = S - d.chunk; m2.ssq_out = cl->ssq0.as<float>();
             to_mirror(m2);
-            ph.push_back(m2);
+            if (push_gemm(m2, d.w_at2, H, H, plan.mlp)) return no_room();
         }
     }
     for (int l = 0; l < d.L; ++l) {
         const bool self = d.is_self[l];
         uint8_t *kp = cl->kpp.as<uint8_t>() + (size_t)l * page_layer, *vp = cl->vpp.as<uint8_t>() + (size_t)l * page_layer;
         const int n_heads = d.n_q + (self ? 2 * d.n_kv : 0);
-        LoopPhase qkv = gemm(cl->hbp.as<uint8_t>(), S, d.wqkv[l], n_heads * hd, H, kd_qkv, OUT_QKV);
+        LoopPhase qkv = product(cl->hbp.as<uint8_t>(), S, OUT_QKV);
         qkv.use_rms = 1; qkv.ssq_in = l == 0 ? cl->ssq0.as<float>() : cl->ssq.as<float>(); qkv.ssq_n = (l == 0 && ada) ? H / 32 : H / 8;
         qkv.qp = cl->qp.as<uint8_t>();
         if (ada) {
@@ -1337,7 +1379,7 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
         }
         qkv.kpp = kp; qkv.vpp = vp; qkv.rope = self ? d.rope_self : d.rope_cross; qkv.n_q = d.n_q; qkv.n_kvp = self ? d.n_kv : 0;
         qkv.cap = d.cap; qkv.P = d.P;
-        ph.push_back(qkv);
+        if (push_gemm(qkv, d.wqkv[l], n_heads * hd, H, plan.qkv)) return no_room();
         LoopPhase at{};
         at.type = PH_ATT; at.qp = cl->qp.as<uint8_t>(); at.kpp = kp; at.vpp = vp; at.n_kv = d.n_kv; at.g = g;
         at.S = S; at.R = R; at.n_rt = n_rt; at.kv_len = self ? d.P + S : d.P; at.P = d.P; at.cap = d.cap; at.n_q = d.n_q;
@@ -1351,7 +1393,8 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
             // Own rows are staged over V, or behind.  K and V may be copied before the grid barrier where they lie behind q|k|v's
             // staged sums, which may still be on their way to its group.
             const int rows = 32 * (hd + 8) * 4, q_bytes = 32 * (int)sq;
-            const int w8q = (n_heads * hd / 8 + n_cta / kd_qkv - 1) / (n_cta / kd_qkv), stg_end = (int)staged_end(S, w8q, H, kd_qkv);
+            const int n8q = (n_heads * hd / 8 + plan.qkv.cols - 1) / plan.qkv.cols, gq = n_cta / plan.qkv.kd;
+            const int stg_end = (int)staged_end(S, (n8q + gq - 1) / gq, (H + 63) / 64, plan.qkv.kd);
             bool found = false;
             for (int nb = 1; !found && nb <= at.per; ++nb) {
                 const int ks = (at.per + nb - 1) / nb, ks16 = round_up(ks, 16), pbytes = 32 * (ks16 + 8) * 2;
@@ -1378,51 +1421,49 @@ int chunk_loop_create(const ChunkLoopDesc &d, ChunkLoop **out) {
                     found = true;
                 }
             }
-            if (!found) bad = true;
+            if (!found) return fail(VLAB200_ERR_UNSUPPORTED);
         }
         ph.push_back(at);
-        LoopPhase o = gemm(cl->attp.as<uint8_t>(), S, d.wo[l], H, qf, kd_o, OUT_RESID);
+        LoopPhase o = product(cl->attp.as<uint8_t>(), S, OUT_RESID);
         to_mirror(o);
         o.h = d.h; o.ssq_out = cl->ssq.as<float>();
         if (ada) {
             o.colscale = mod_in(l) + 2 * H; o.scale_next = mod_post(l); o.mod_stride = (long long)mod_step;
         }
-        ph.push_back(o);
-        LoopPhase gu = gemm(cl->hbp.as<uint8_t>(), S, d.wgu[l], 2 * d.I, H, kd_gu, OUT_GATED);
+        if (push_gemm(o, d.wo[l], H, qf, plan.o)) return no_room();
+        LoopPhase gu = product(cl->hbp.as<uint8_t>(), S, OUT_GATED);
         gu.use_rms = 1; gu.ssq_in = cl->ssq.as<float>(); gu.ssq_n = H / 8;
         gu.act = d.act; gu.outp = cl->gp.as<uint8_t>(); gu.out_rows8 = round_up(S, 8);
         if (ada) {
             if ((rc = shift_bias(d.wgu[l], 2 * d.I, mod_post(l), nullptr, &gu.bias))) return fail(rc);
             gu.bias_step_stride = 2 * d.I;
         }
-        ph.push_back(gu);
-        LoopPhase dn = gemm(cl->gp.as<uint8_t>(), S, d.wdown[l], H, d.I, kd_d, OUT_RESID);
+        if (push_gemm(gu, d.wgu[l], 2 * d.I, H, plan.gu)) return no_room();
+        LoopPhase dn = product(cl->gp.as<uint8_t>(), S, OUT_RESID);
         to_mirror(dn);
         dn.h = d.h; dn.ssq_out = cl->ssq.as<float>();
         if (ada) {
             dn.colscale = mod_post(l) + 2 * H; dn.scale_next = l + 1 < d.L ? mod_in(l + 1) : mod_final; dn.mod_stride = (long long)mod_step;
         }
-        ph.push_back(dn);
+        if (push_gemm(dn, d.wdown[l], H, d.I, plan.dn)) return no_room();
     }
     {
-        LoopPhase hdp = gemm(cl->hbp.as<uint8_t>(), S, d.w_aout, d.A, H, kd_h, OUT_EULER);
+        LoopPhase hdp = product(cl->hbp.as<uint8_t>(), S, OUT_EULER);
         hdp.use_rms = 1; hdp.ssq_in = cl->ssq.as<float>(); hdp.ssq_n = H / 8; hdp.bias = d.b_aout; hdp.x = d.x; hdp.dt = -1.0f / (float)d.steps;
         if (ada) {
             if ((rc = shift_bias(d.w_aout, d.A, mod_final, d.b_aout, &hdp.bias))) return fail(rc);
             hdp.bias_step_stride = d.A;
         }
-        ph.push_back(hdp);
+        if (push_gemm(hdp, d.w_aout, d.A, H, plan.head)) return no_room();
     }
-    if (bad) return fail(VLAB200_ERR_UNSUPPORTED);
     if ((rc = cl->phases.alloc(ph.size() * sizeof(LoopPhase))) || (rc = cl->counter.alloc(64))) return fail(rc);
     std::vector<WEntry> wt;
     for (const LoopPhase &p : ph)
         if (p.type == PH_GEMM) {
             WEntry w{};
-            w.Wp = p.Wp; w.N8 = p.N8; w.K = p.K; w.kd = p.kd; w.M = p.M;
+            w.Wp = p.Wp; w.n8_kb = (uint32_t)p.N8 | (uint32_t)((p.K + 63) / 64) << 16; w.kd_m = (uint32_t)p.kd | (uint32_t)p.M << 16;
             wt.push_back(w);
         }
-    if ((int)wt.size() > CL_WTAB_MAX) return fail(VLAB200_ERR_UNSUPPORTED);
     if ((rc = cl->wtab.alloc(wt.size() * sizeof(WEntry)))) return fail(rc);
     cudaError_t ce = cudaMemcpy(cl->wtab.p, wt.data(), wt.size() * sizeof(WEntry), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemcpy(cl->phases.p, ph.data(), ph.size() * sizeof(LoopPhase), cudaMemcpyHostToDevice);

@@ -463,13 +463,22 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
     return dense_gemm(e->g.p, I, e->wdown[l].p, p, cs);
 }
 
+// suffix rows per observation: pi0 alone carries the state as a suffix token
+static int suffix_rows(const vlab200_policy_config &c) { return c.chunk + (c.model == 0 ? 1 : 0); }
+
+static ChunkLoopDesc loop_sizes(const vlab200_policy_config &c, int P) {
+    ChunkLoopDesc d{};
+    d.model = c.model; d.L = c.n_layers; d.H = c.H; d.I = c.inter; d.n_q = c.n_q; d.n_kv = c.n_kv; d.hd = c.head_dim; d.S = suffix_rows(c);
+    d.chunk = c.chunk; d.A = c.action_dim; d.sd = c.state_dim; d.steps = c.steps; d.P = P;
+    d.act = c.model == 1 ? ACT_SILU : ACT_GELU_TANH; d.rms_eps = c.rms_eps;
+    return d;
+}
+
 // The persistent loop kernel for calls with one observation, on the engine's own buffers.
 static int engine_chunk_loop(vlab200_engine *e) {
     const vlab200_policy_config &c = e->c;
-    ChunkLoopDesc d{};
-    d.model = c.model; d.L = c.n_layers; d.H = c.H; d.I = c.inter; d.n_q = c.n_q; d.n_kv = c.n_kv; d.hd = c.head_dim; d.S = e->S;
-    d.chunk = c.chunk; d.A = c.action_dim; d.sd = c.state_dim; d.steps = c.steps; d.cap = e->cap; d.P = e->P;
-    d.act = c.model == 1 ? ACT_SILU : ACT_GELU_TANH; d.rms_eps = c.rms_eps;
+    ChunkLoopDesc d = loop_sizes(c, e->P);
+    d.cap = e->cap;
     d.is_self = e->is_self.data();
     std::vector<const void *> wqkv(c.n_layers), wo(c.n_layers), wgu(c.n_layers), wdown(c.n_layers);
     for (int l = 0; l < c.n_layers; ++l) {
@@ -490,6 +499,15 @@ static int engine_chunk_loop(vlab200_engine *e) {
 }  // namespace vb
 
 extern "C" {
+
+int32_t vlab200_loop_kernel_phases(const vlab200_policy_config *cfg, int32_t n_cta) {
+    if (!cfg || cfg->n_layers <= 0 || cfg->H <= 0 || cfg->n_q <= 0 || cfg->n_kv <= 0 || cfg->n_q % cfg->n_kv || cfg->inter <= 0 || cfg->chunk <= 0 ||
+        cfg->action_dim <= 0)
+        return 0;
+    return vb::chunk_loop_plan_phases(vb::loop_sizes(*cfg, 0), n_cta);
+}
+
+int32_t vlab200_engine_loop_phases(const vlab200_engine *e) { return e ? vb::chunk_loop_phases(e->loop) : 0; }
 
 vlab200_engine *vlab200_engine_create(const vlab200_policy_config *cfg, const vlab200_policy_weights *w,
                                       int32_t max_obs, int32_t prefix_len) {
@@ -522,7 +540,7 @@ vlab200_engine *vlab200_engine_create(const vlab200_policy_config *cfg, const vl
     e->max_obs = max_obs;
     e->P = prefix_len;
     e->P_max = prefix_len;
-    e->S = c.chunk + (c.model == 0 ? 1 : 0);  // pi0 alone carries the state as a suffix token
+    e->S = vb::suffix_rows(c);
     e->cap = e->P + e->S;
     e->qf = c.n_q * c.head_dim;
     e->kvf = c.n_kv * c.head_dim;
