@@ -558,9 +558,10 @@ int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t
         if (ksplit > p.partial_slices) ksplit = p.partial_slices;
         if (ksplit >= 2) return split_residual(A, lda, W, p, ksplit, 5, n_sm, stream);
     }
-    // Some hundred rows, long K (Wdown of a backbone, fc2 of a vision tower): one wave of narrow tiles streams all of K through each SM
-    // at about 0.35 us a 64-wide step, pair tiles would fill a fraction of the machine at 0.42 us.  K slices of pair tiles do both; the
-    // float sums and the second launch cost about 8 us + 1 us per 2.5 MB.  816 x 2048 x 16384: 97 us as 112 tiles of 128 x 128.
+    // Some hundred rows, long K (Wdown of a backbone): one wave of narrow tiles streams all of K through each SM at about 0.35 us a 64-wide
+    // step, pair tiles would fill a fraction of the machine at 0.42 us.  K slices of pair tiles do both; the float sums and the second
+    // launch cost about 8 us + 1 us per 2.5 MB.  816 x 2048 x 16384: 97 us as 112 tiles of 128 x 128.  (fc2 of a vision tower, K up to 4304,
+    // stays whole.)
     if (p.partial && p.epi == EPI_RESIDUAL && dense_gemm_variant() == 0 && p.M > 2 * G_BM && p.M <= p.partial_rows && p.rows_in == 0 &&
         p.scatter_hd == 0 && !p.use_rms && p.N % 4 == 0 && n_sm >= 2) {
         const int pairs = n_sm / 2, ksteps = (p.K + G_BK - 1) / G_BK, units = ((p.M + 2 * G_BM - 1) / (2 * G_BM)) * ((p.N + 255) / 256);

@@ -354,9 +354,9 @@ int32_t vlab200_vision_run(vlab200_vision *v, const void *pixels, int32_t pixels
     auto layernorm = [&](const float *w, const float *b, __nv_bfloat16 *out, int shuffle) {
         const float *h = v->h.as<float>();
         const dim3 rows4((M + 3) / 4), warps4(128);
-        if (H % 4 == 0 && H <= 768)
+        if (H <= 768)  // (widths are multiples of 8)
             return vb::launch_pdl(vb::layernorm_vec_kernel<6>, rows4, warps4, 0, cs, h, w, b, out, M, H, c.ln_eps, np, v->grid, shuffle);
-        if (H % 4 == 0 && H <= 1536)
+        if (H <= 1536)
             return vb::launch_pdl(vb::layernorm_vec_kernel<12>, rows4, warps4, 0, cs, h, w, b, out, M, H, c.ln_eps, np, v->grid, shuffle);
         vb::layernorm_kernel<<<(M + 7) / 8, 256, 0, cs>>>(v->h.as<float>(), w, b, out, M, H, c.ln_eps, np, v->grid, shuffle);
         return cudaGetLastError() == cudaSuccess ? VLAB200_OK : vb::cuda_fail(cudaGetLastError(), "layernorm_kernel");
