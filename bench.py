@@ -969,8 +969,7 @@ def measure_policy(torch, vb, dist, dev, args, rank, world, barrier):
         line["roofline"] = {"kernel": "chunk_loop_kernel (whole Euler loop of one observation, one cooperative launch per chunk)",
                             "bound": "hbm", "achieved": gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"],
                             "peak_kind": f"of {peaks['kind']}",
-                            # ncu: 2,010 MB read + 15.7 MB written per launch for the SmolVLA-shaped expert (profiles/chunk_loop_smolvla_b1.md)
-                            "traffic": 2026.1e6 if workload == "smolvla" else None,
+                            "traffic": None,  # no counters: the kernel's launch fails under the profiler (profiles/chunk_loop_smolvla_b1.md)
                             "us_per_launch": ms * 1e3, "algorithmic_bytes_per_launch": wbytes}
     del eng, x0, state
     torch.cuda.empty_cache()
