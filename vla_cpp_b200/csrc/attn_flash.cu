@@ -211,12 +211,12 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                     const uint32_t p_tmem = tmem_base + L::O_COLS + st * 64;
                     if (elect_one()) {
 #pragma unroll
-                    for (int k16 = 0; k16 < FA_BKV / 16; ++k16)
-                        mma_f16_tmem_a(tmem_base, p_tmem + (uint32_t)(k16 * 8),
-                                       smem_desc_sw128(v_addr + k16 * 2048, 8192, 1024), idesc_o,
-                                       (j != j0 || k16 != 0) ? 1u : 0u);
-                    tc_commit(&pv_done[st]);
-                    tc_commit(&v_free[st]);
+                        for (int k16 = 0; k16 < FA_BKV / 16; ++k16)
+                            mma_f16_tmem_a(tmem_base, p_tmem + (uint32_t)(k16 * 8),
+                                           smem_desc_sw128(v_addr + k16 * 2048, 8192, 1024), idesc_o,
+                                           (j != j0 || k16 != 0) ? 1u : 0u);
+                        tc_commit(&pv_done[st]);
+                        tc_commit(&v_free[st]);
                     }
                 }
                 if (!ok) break;
@@ -639,12 +639,12 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     const uint32_t p_tmem = tmem_base + L::O_COLS + sb * FP_BKV;
                     if (elect_one()) {
 #pragma unroll
-                    for (int k16 = 0; k16 < FP_BKV / 16; ++k16)
-                        mma_f16_tmem_a_pair(tmem_base, p_tmem + (uint32_t)(k16 * 8), v_desc + (uint64_t)(k16 * 128), idesc_o,
-                                            (j | k16) != 0 ? 1u : 0u);
-                    *pv_issued = jb + 1u;
-                    tc_commit_pair(&pv_done[sb], 3);
-                    tc_commit_pair(&v_free[st], 3);
+                        for (int k16 = 0; k16 < FP_BKV / 16; ++k16)
+                            mma_f16_tmem_a_pair(tmem_base, p_tmem + (uint32_t)(k16 * 8), v_desc + (uint64_t)(k16 * 128), idesc_o,
+                                                (j | k16) != 0 ? 1u : 0u);
+                        *pv_issued = jb + 1u;
+                        tc_commit_pair(&pv_done[sb], 3);
+                        tc_commit_pair(&v_free[st], 3);
                     }
                 }
                 if (!ok) break;

@@ -745,156 +745,156 @@ __device__ __noinline__ unsigned att_phase(const LoopPhase &pg, const LoopParams
                 for (int e = 0; e < 4; ++e) oacc[i][j][e] = 0.0f;
         const int c0 = warp * (HD / 8);
         for (int key0 = k_begin; key0 < k_end; key0 += ks) {
-        const int nkeys = min(ks, k_end - key0), ks16 = (nkeys + 15) & ~15;
-        if (key0 != k_begin) cons_sync();  // the block before has been consumed
-        if (tid == 0 && (u != grp || key0 != k_begin)) {
-            fence_proxy_async_all();
-            const uint32_t q_bytes = key0 == k_begin ? (uint32_t)nrows * SQ : 0u;
-            mbar_expect_tx(sm.k_full, q_bytes + (uint32_t)nkeys * SQ);
-            if (q_bytes) bulk_g2s(Qs, pg.qp + ((size_t)kvh * gq * S + row0) * SQ, q_bytes, sm.k_full);
-            bulk_g2s(Ks, pg.kpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, sm.k_full);
-            mbar_expect_tx(sm.v_full, (uint32_t)nkeys * SQ);
-            bulk_g2s(Vs, pg.vpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, sm.v_full);
-        }
-        for (int i = tid; i < (ks16 - nkeys) * (HD / 8); i += CL_THREADS) {
-            const int r = nkeys + i / (HD / 8), c = i % (HD / 8);
-            *reinterpret_cast<uint4 *>(Vs + (size_t)r * SQ + c * 16) = make_uint4(0, 0, 0, 0);
-        }
-        mbar_wait(sm.k_full, par_bit(par, PAR_K), wc, CL_DEV_TIMEOUT);
-        par ^= 1u << PAR_K;
-        // ---- S = Q K^T for this warp's 16 rows and its share of the 8-key groups
-        const int ng = ks16 >> 3, g0 = kp * ng / 4, g1 = (kp + 1) * ng / 4, n_g = g1 - g0;  // n_g <= 4
-        float sacc[4][4];
+            const int nkeys = min(ks, k_end - key0), ks16 = (nkeys + 15) & ~15;
+            if (key0 != k_begin) cons_sync();  // the block before has been consumed
+            if (tid == 0 && (u != grp || key0 != k_begin)) {
+                fence_proxy_async_all();
+                const uint32_t q_bytes = key0 == k_begin ? (uint32_t)nrows * SQ : 0u;
+                mbar_expect_tx(sm.k_full, q_bytes + (uint32_t)nkeys * SQ);
+                if (q_bytes) bulk_g2s(Qs, pg.qp + ((size_t)kvh * gq * S + row0) * SQ, q_bytes, sm.k_full);
+                bulk_g2s(Ks, pg.kpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, sm.k_full);
+                mbar_expect_tx(sm.v_full, (uint32_t)nkeys * SQ);
+                bulk_g2s(Vs, pg.vpp + ((size_t)kvh * cap + key0) * SQ, (uint32_t)nkeys * SQ, sm.v_full);
+            }
+            for (int i = tid; i < (ks16 - nkeys) * (HD / 8); i += CL_THREADS) {
+                const int r = nkeys + i / (HD / 8), c = i % (HD / 8);
+                *reinterpret_cast<uint4 *>(Vs + (size_t)r * SQ + c * 16) = make_uint4(0, 0, 0, 0);
+            }
+            mbar_wait(sm.k_full, par_bit(par, PAR_K), wc, CL_DEV_TIMEOUT);
+            par ^= 1u << PAR_K;
+            // ---- S = Q K^T for this warp's 16 rows and its share of the 8-key groups
+            const int ng = ks16 >> 3, g0 = kp * ng / 4, g1 = (kp + 1) * ng / 4, n_g = g1 - g0;  // n_g <= 4
+            float sacc[4][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) sacc[i][e] = 0.0f;
-        {
-            const int qrow = min(mt * 16 + lr + (mi & 1) * 8, nrows - 1);
-            const uint32_t q_addr = smem_u32(Qs) + (uint32_t)qrow * SQ + (uint32_t)(mi >> 1) * 16u;
-            const uint32_t k_addr = smem_u32(Ks) + (uint32_t)(g0 * 8 + lr) * SQ + (uint32_t)mi * 16u;
+                for (int e = 0; e < 4; ++e) sacc[i][e] = 0.0f;
+            {
+                const int qrow = min(mt * 16 + lr + (mi & 1) * 8, nrows - 1);
+                const uint32_t q_addr = smem_u32(Qs) + (uint32_t)qrow * SQ + (uint32_t)(mi >> 1) * 16u;
+                const uint32_t k_addr = smem_u32(Ks) + (uint32_t)(g0 * 8 + lr) * SQ + (uint32_t)mi * 16u;
 #pragma unroll 2
-            for (int kk = 0; kk < HD / 32; ++kk) {
-                uint32_t a0[4], a1[4];
-                ldsm4(a0, q_addr + kk * 64);
-                ldsm4(a1, q_addr + kk * 64 + 32);
+                for (int kk = 0; kk < HD / 32; ++kk) {
+                    uint32_t a0[4], a1[4];
+                    ldsm4(a0, q_addr + kk * 64);
+                    ldsm4(a1, q_addr + kk * 64 + 32);
 #pragma unroll
-                for (int gi = 0; gi < 4; ++gi) {
-                    if (gi >= n_g) break;
-                    uint32_t b[4];
-                    ldsm4(b, k_addr + (uint32_t)gi * 8u * SQ + kk * 64);
-                    mma_bf16(sacc[gi], a0, b[0], b[1]);
-                    mma_bf16(sacc[gi], a1, b[2], b[3]);
-                }
-            }
-        }
-        // ---- mask, row maximum over the unit's keys
-        const int rl[2] = {mt * 16 + g, mt * 16 + g + 8};
-        int jmax[2];
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-            const int tok = (row0 + rl[hr]) % S;
-            const int n_suf = kv_len - P;
-            int limit = n_suf;
-            if (mask_mode == 2) limit = min(tok + 1, n_suf);
-            else if (mask_mode == 1) limit = tok == 0 ? min(1, n_suf) : n_suf;
-            jmax[hr] = min(P + limit, key0 + nkeys);
-        }
-        float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int gi = 0; gi < 4; ++gi) {
-            if (gi >= n_g) break;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = key0 + (g0 + gi) * 8 + q2 + (e & 1), hr = e >> 1;
-                const bool vis = j < jmax[hr] && !(j >= pad_lo && j < pad_hi);
-                sacc[gi][e] = vis ? sacc[gi][e] * scale_log2 : -INFINITY;
-                mx[hr] = fmaxf(mx[hr], sacc[gi][e]);
-            }
-        }
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-            mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 1));
-            mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 2));
-            if ((lane & 3) == 0) sm.red_max[rl[hr] * 4 + kp] = mx[hr];
-        }
-        // K's last block has been read.  Where the rows of the group's CTAs land over it, they do so by bulk copies, which an arrival
-        // alone does not order behind these loads (see stage_release in tc5.cuh)
-        if (key0 + ks >= k_end && pg.recv_off == pg.k_off) fence_proxy_async_smem();
-        cons_sync();  // the maxima are in place; Q (P may lie over it) and K have been read
-        if (key0 + ks >= k_end && tid < ad) arrive_rank(map_rank(smem_u32(sm.rdy), base_rank + tid));
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-            const float *rm = sm.red_max + rl[hr] * 4;
-            const float m = fmaxf(ms[hr], fmaxf(fmaxf(rm[0], rm[1]), fmaxf(rm[2], rm[3])));
-            mx[hr] = m == -INFINITY ? 0.0f : m;
-            sum[hr] *= ex2f(ms[hr] - mx[hr]);  // 0 before the first block
-            ms[hr] = m;
-            if (kp == 0 && (lane & 3) == 0) sm.row_m[rl[hr]] = m;
-        }
-#pragma unroll
-        for (int gi = 0; gi < 4; ++gi) {
-            if (gi >= n_g) break;
-            float pv[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                pv[e] = ex2f(sacc[gi][e] - mx[e >> 1]);
-                sum[e >> 1] += pv[e];
-            }
-            const int col = (g0 + gi) * 8 + q2;
-            *reinterpret_cast<uint32_t *>(Ps + (size_t)rl[0] * SP + col * 2) = pack_bf16(pv[0], pv[1]);
-            *reinterpret_cast<uint32_t *>(Ps + (size_t)rl[1] * SP + col * 2) = pack_bf16(pv[2], pv[3]);
-        }
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-            float s = sum[hr];
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            if ((lane & 3) == 0) sm.red_sum[rl[hr] * 4 + kp] = s;
-        }
-        mbar_wait(sm.v_full, par_bit(par, PAR_V), wc, CL_DEV_TIMEOUT);
-        par ^= 1u << PAR_V;
-        cons_sync();
-        // ---- O = P V: this warp's HD / 8 output columns, all 32 rows
-        if (pg.per > ks) {  // several key blocks: earlier sums follow the running maximum
-#pragma unroll
-            for (int m2 = 0; m2 < 2; ++m2)
-#pragma unroll
-                for (int hr = 0; hr < 2; ++hr) {
-                    const float m = sm.row_m[m2 * 16 + g + hr * 8], f = ex2f(mo[m2][hr] - (m == -INFINITY ? 0.0f : m));
-                    mo[m2][hr] = m;
-#pragma unroll
-                    for (int j = 0; j < NGV; ++j) {
-                        oacc[m2][j][2 * hr] *= f;
-                        oacc[m2][j][2 * hr + 1] *= f;
-                    }
-                }
-        }
-        {
-            const uint32_t p_addr = smem_u32(Ps) + (uint32_t)(lr + (mi & 1) * 8) * SP + (uint32_t)(mi >> 1) * 16u;
-            const uint32_t v_addr = smem_u32(Vs) + (uint32_t)(lr + (mi & 1) * 8) * SQ + (uint32_t)(c0 + (NGV > 1 ? (mi >> 1) * 8 : 0)) * 2u;
-            for (int kk = 0; kk < (ks16 >> 4); ++kk) {
-                uint32_t a[2][4];
-                ldsm4(a[0], p_addr + kk * 32);
-                ldsm4(a[1], p_addr + 16 * SP + kk * 32);
-                if (NGV == 1) {
-                    uint32_t b[2];
-                    ldsm2_t(b, v_addr + (uint32_t)kk * 16u * SQ);
-                    mma_bf16(oacc[0][0], a[0], b[0], b[1]);
-                    mma_bf16(oacc[1][0], a[1], b[0], b[1]);
-                } else {
-#pragma unroll
-                    for (int gp = 0; gp < NGV / 2; ++gp) {
+                    for (int gi = 0; gi < 4; ++gi) {
+                        if (gi >= n_g) break;
                         uint32_t b[4];
-                        ldsm4_t(b, v_addr + (uint32_t)kk * 16u * SQ + gp * 32);
-                        mma_bf16(oacc[0][2 * gp], a[0], b[0], b[1]);
-                        mma_bf16(oacc[1][2 * gp], a[1], b[0], b[1]);
-                        mma_bf16(oacc[0][2 * gp + 1], a[0], b[2], b[3]);
-                        mma_bf16(oacc[1][2 * gp + 1], a[1], b[2], b[3]);
+                        ldsm4(b, k_addr + (uint32_t)gi * 8u * SQ + kk * 64);
+                        mma_bf16(sacc[gi], a0, b[0], b[1]);
+                        mma_bf16(sacc[gi], a1, b[2], b[3]);
                     }
                 }
             }
-        }
+            // ---- mask, row maximum over the unit's keys
+            const int rl[2] = {mt * 16 + g, mt * 16 + g + 8};
+            int jmax[2];
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                const int tok = (row0 + rl[hr]) % S;
+                const int n_suf = kv_len - P;
+                int limit = n_suf;
+                if (mask_mode == 2) limit = min(tok + 1, n_suf);
+                else if (mask_mode == 1) limit = tok == 0 ? min(1, n_suf) : n_suf;
+                jmax[hr] = min(P + limit, key0 + nkeys);
+            }
+            float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+            for (int gi = 0; gi < 4; ++gi) {
+                if (gi >= n_g) break;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = key0 + (g0 + gi) * 8 + q2 + (e & 1), hr = e >> 1;
+                    const bool vis = j < jmax[hr] && !(j >= pad_lo && j < pad_hi);
+                    sacc[gi][e] = vis ? sacc[gi][e] * scale_log2 : -INFINITY;
+                    mx[hr] = fmaxf(mx[hr], sacc[gi][e]);
+                }
+            }
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 1));
+                mx[hr] = fmaxf(mx[hr], __shfl_xor_sync(0xffffffffu, mx[hr], 2));
+                if ((lane & 3) == 0) sm.red_max[rl[hr] * 4 + kp] = mx[hr];
+            }
+            // K's last block has been read.  Where the rows of the group's CTAs land over it, they do so by bulk copies, which an arrival
+            // alone does not order behind these loads (see stage_release in tc5.cuh)
+            if (key0 + ks >= k_end && pg.recv_off == pg.k_off) fence_proxy_async_smem();
+            cons_sync();  // the maxima are in place; Q (P may lie over it) and K have been read
+            if (key0 + ks >= k_end && tid < ad) arrive_rank(map_rank(smem_u32(sm.rdy), base_rank + tid));
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                const float *rm = sm.red_max + rl[hr] * 4;
+                const float m = fmaxf(ms[hr], fmaxf(fmaxf(rm[0], rm[1]), fmaxf(rm[2], rm[3])));
+                mx[hr] = m == -INFINITY ? 0.0f : m;
+                sum[hr] *= ex2f(ms[hr] - mx[hr]);  // 0 before the first block
+                ms[hr] = m;
+                if (kp == 0 && (lane & 3) == 0) sm.row_m[rl[hr]] = m;
+            }
+#pragma unroll
+            for (int gi = 0; gi < 4; ++gi) {
+                if (gi >= n_g) break;
+                float pv[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    pv[e] = ex2f(sacc[gi][e] - mx[e >> 1]);
+                    sum[e >> 1] += pv[e];
+                }
+                const int col = (g0 + gi) * 8 + q2;
+                *reinterpret_cast<uint32_t *>(Ps + (size_t)rl[0] * SP + col * 2) = pack_bf16(pv[0], pv[1]);
+                *reinterpret_cast<uint32_t *>(Ps + (size_t)rl[1] * SP + col * 2) = pack_bf16(pv[2], pv[3]);
+            }
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                float s = sum[hr];
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                if ((lane & 3) == 0) sm.red_sum[rl[hr] * 4 + kp] = s;
+            }
+            mbar_wait(sm.v_full, par_bit(par, PAR_V), wc, CL_DEV_TIMEOUT);
+            par ^= 1u << PAR_V;
+            cons_sync();
+            // ---- O = P V: this warp's HD / 8 output columns, all 32 rows
+            if (pg.per > ks) {  // several key blocks: earlier sums follow the running maximum
+#pragma unroll
+                for (int m2 = 0; m2 < 2; ++m2)
+#pragma unroll
+                    for (int hr = 0; hr < 2; ++hr) {
+                        const float m = sm.row_m[m2 * 16 + g + hr * 8], f = ex2f(mo[m2][hr] - (m == -INFINITY ? 0.0f : m));
+                        mo[m2][hr] = m;
+#pragma unroll
+                        for (int j = 0; j < NGV; ++j) {
+                            oacc[m2][j][2 * hr] *= f;
+                            oacc[m2][j][2 * hr + 1] *= f;
+                        }
+                    }
+            }
+            {
+                const uint32_t p_addr = smem_u32(Ps) + (uint32_t)(lr + (mi & 1) * 8) * SP + (uint32_t)(mi >> 1) * 16u;
+                const uint32_t v_addr = smem_u32(Vs) + (uint32_t)(lr + (mi & 1) * 8) * SQ + (uint32_t)(c0 + (NGV > 1 ? (mi >> 1) * 8 : 0)) * 2u;
+                for (int kk = 0; kk < (ks16 >> 4); ++kk) {
+                    uint32_t a[2][4];
+                    ldsm4(a[0], p_addr + kk * 32);
+                    ldsm4(a[1], p_addr + 16 * SP + kk * 32);
+                    if (NGV == 1) {
+                        uint32_t b[2];
+                        ldsm2_t(b, v_addr + (uint32_t)kk * 16u * SQ);
+                        mma_bf16(oacc[0][0], a[0], b[0], b[1]);
+                        mma_bf16(oacc[1][0], a[1], b[0], b[1]);
+                    } else {
+#pragma unroll
+                        for (int gp = 0; gp < NGV / 2; ++gp) {
+                            uint32_t b[4];
+                            ldsm4_t(b, v_addr + (uint32_t)kk * 16u * SQ + gp * 32);
+                            mma_bf16(oacc[0][2 * gp], a[0], b[0], b[1]);
+                            mma_bf16(oacc[1][2 * gp], a[1], b[0], b[1]);
+                            mma_bf16(oacc[0][2 * gp + 1], a[0], b[2], b[3]);
+                            mma_bf16(oacc[1][2 * gp + 1], a[1], b[2], b[3]);
+                        }
+                    }
+                }
+            }
         }
         if (k_begin >= k_end) {  // no keys in this CTA's range: it contributes nothing, but its peers count on its arrival
             if (tid < ad) arrive_rank(map_rank(smem_u32(sm.rdy), base_rank + tid));

@@ -202,11 +202,11 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
                     const uint64_t off = (uint64_t)(st * (G_STAGE_BYTES >> 4));
                     if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < G_BK / 16; ++k) {
-                        const uint32_t acc = (kt != kbeg || k != 0) ? 1u : 0u;  // the first MMA of a tile overwrites the accumulator
-                        if (PAIR) mma_f16_pair(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, acc);
-                        else mma_f16(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, acc);
-                    }
+                        for (int k = 0; k < G_BK / 16; ++k) {
+                            const uint32_t acc = (kt != kbeg || k != 0) ? 1u : 0u;  // the first MMA of a tile overwrites the accumulator
+                            if (PAIR) mma_f16_pair(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, acc);
+                            else mma_f16(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, acc);
+                        }
                         if (PAIR) tc_commit_pair(&empty[st], 3);
                         else tc_commit(&empty[st]);
                     }

@@ -375,12 +375,12 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
                     const uint64_t off = (uint64_t)(st * (STAGE_BYTES >> 4));
                     if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < QKV_BK / 16; ++k) {
-                        if (PAIR) mma_f16_pair(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
-                        else mma_f16(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
-                    }
-                    if (PAIR) tc_commit_pair(&empty[st], 3);
-                    else tc_commit(&empty[st]);
+                        for (int k = 0; k < QKV_BK / 16; ++k) {
+                            if (PAIR) mma_f16_pair(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
+                            else mma_f16(d_tmem, a_desc0 + off + 2 * k, b_desc0 + off + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
+                        }
+                        if (PAIR) tc_commit_pair(&empty[st], 3);
+                        else tc_commit(&empty[st]);
                     }
                     if (++st == (uint32_t)nst) { st = 0; ph ^= 1u; }
                 }

@@ -340,14 +340,14 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                    const uint32_t a_addr = smem_u32(smem + st * L::A_BYTES);
-                    const uint32_t w_addr = smem_u32(smem + L::W_OFFSET + sw * L::W_BYTES);
+                        const uint32_t a_addr = smem_u32(smem + st * L::A_BYTES);
+                        const uint32_t w_addr = smem_u32(smem + L::W_OFFSET + sw * L::W_BYTES);
 #pragma unroll
-                    for (int k = 0; k < GEMM_BK / 32; ++k)
-                        mma_i8(d_tmem, smem_desc_sw128(a_addr + k * 32, 16, 1024),
-                               smem_desc_sw128(w_addr + k * 32, 16, 1024), idesc, (kt | k) != 0 ? 1u : 0u);
-                    tc_commit(&empty_a[st]);
-                    tc_commit(&empty_w[sw]);
+                        for (int k = 0; k < GEMM_BK / 32; ++k)
+                            mma_i8(d_tmem, smem_desc_sw128(a_addr + k * 32, 16, 1024),
+                                   smem_desc_sw128(w_addr + k * 32, 16, 1024), idesc, (kt | k) != 0 ? 1u : 0u);
+                        tc_commit(&empty_a[st]);
+                        tc_commit(&empty_w[sw]);
                     }
                     if (++st == GEMM_SA) { st = 0; ph ^= 1u; }
                     if (++sw == GEMM_SW) { sw = 0; pw ^= 1u; }
