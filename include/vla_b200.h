@@ -237,7 +237,8 @@ VLAB200_API int32_t vlab200_engine_set_prefix(vlab200_engine *e, int32_t layer, 
  * A call with ONE observation runs the whole loop as one persistent cooperative kernel (the reference's
  * answer to per-operator cost is one cached graph per predict, src/scratch_ctx.h:34-141); its first use builds a second copy
  * of the expert's weights on the engine's device.  Environment VLAB200_CHUNK_LOOP=0 keeps a launch per operator.  The two
- * paths round activations to bf16 at different points: results agree to ~3e-3 rel-L2, each is reproducible bit for bit. */
+ * paths round activations to bf16 at different points: results agree to ~3e-3 rel-L2, each is reproducible bit for bit on
+ * one GPU (how many CTA clusters of the loop kernel fit a GPU decides how its sums are cut). */
 VLAB200_API int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *state, const float *x0,
                                            float *x_out, int32_t pos_base, const int32_t *pad_ranges,
                                            void *stream);
@@ -271,7 +272,9 @@ VLAB200_API int32_t vlab200_engine_set_prefix_len(vlab200_engine *e, int32_t pre
  * (smolvla.cpp:1362-1369, pi0.cpp:553-555).  pos_host: int32 [P] RoPE positions (HOST; NULL = 0..P-1).
  * mask_mode 0 = every prefix token sees every other (pi0), 3 = the last token (state) is seen only by itself
  * (smolvla.cpp:1637-1645); pad_ranges as in vlab200_attention.  P must equal the engine's prefix length in
- * use.  Replaces the prefill loops of smolvla.cpp:1374-1391 and pi0.cpp:557-566. */
+ * use.  The number of rows of a call (n_obs * P) decides how its residual products are tiled: a call is reproducible
+ * bit for bit, an observation's pages may have other last bits in calls with another n_obs.
+ * Replaces the prefill loops of smolvla.cpp:1374-1391 and pi0.cpp:557-566. */
 typedef struct {
     int32_t n_layers, hidden, n_q, n_kv, head_dim, inter, act;
     float rms_eps, rope_base;
@@ -304,7 +307,9 @@ VLAB200_API int32_t vlab200_prefill_run(vlab200_prefill *p, vlab200_engine *e, i
  * next of them in the prepared weights.
  * vlab200_vision_run: pixels = DEVICE buffer [n_views][image][image][3], uint8 (0..255) or float32 (0..1) in
  * H, W, C order (vla_image's layout); x -> x / 255 (uint8 only) -> 2 x - 1.  img_emb: float32 device
- * [n_views * tokens_per_view][out_dim], the tensor vla_inputs.precomputed_img_emb would carry. */
+ * [n_views * tokens_per_view][out_dim], the tensor vla_inputs.precomputed_img_emb would carry.  The number of rows of
+ * a call (n_views patch grids) decides how its residual products are tiled: a call is reproducible bit for bit, a picture's
+ * embeddings may have other last bits in calls with another n_views. */
 typedef struct {
     int32_t image, patch, hidden, n_layers, n_heads, inter, shuffle, out_dim;
     float ln_eps, out_scale;
@@ -359,7 +364,9 @@ VLAB200_API int32_t vlab200_loop_kernel_phases(const vlab200_policy_config *cfg,
  * 0 = chosen per call from the problem size (default), 1 = one CTA per 128 x 256 tile,
  * 2 = one CTA per 128 x 128 tile (QKV: same as 1), 3 = CTA pairs (tcgen05 cta_group::2) on 256 x 256 tiles,
  * 4 = one CTA per 128 x 64 tile (QKV: same as 1).
- * All tilings give the same results bit for bit; the knob exists for tests and measurements.
+ * The forced tilings 1 - 4 give the same results bit for bit.  Tiling 0 may also cut K of a residual product of some
+ * hundred rows at most into slices (Wo, Wdown, fc2), whose float32 sums are added in a fixed order: the same from run to run,
+ * but with other last bits than a forced tiling.  The knob exists for tests and measurements.
  * Process-wide, not thread-safe against concurrent engine calls.  No counterpart in the reference. */
 VLAB200_API int32_t vlab200_set_gemm_tiling(int32_t tiling);
 

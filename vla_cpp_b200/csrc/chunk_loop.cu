@@ -2,7 +2,7 @@
 //
 // With a single observation the suffix is 50 / 51 rows: every product of the loop streams its weights once and does
 // almost no arithmetic, and a launch per operator spends most of its time between kernels (about 1,600 launches per
-// chunk for a pi0-shaped expert).  Here one persistent cooperative kernel (clusters of eight CTAs, one CTA of 256 + 32
+// chunk for a pi0-shaped expert).  Here one persistent cooperative kernel (clusters of eight CTAs, one CTA of 256 + 64
 // threads per SM) walks a table of PHASES -- the operators of one Euler step, src/models/pi0.cpp:570-588,
 // src/models/smolvla.cpp:1393-1418 -- and separates them with a grid-wide barrier (one atomic arrival + a bounded acquire
 // spin per CTA).  Per layer: q|k|v, attention, Wo + residual, gate/up, Wdown + residual = five phases.
@@ -32,7 +32,8 @@
 //   EMBED    action-in projection (+ pi0's state token) on CUDA cores.
 // Everything one CTA writes for another outside its cluster goes through L2 (st / ld .cg, bulk copies), never through L1.  Phase
 // descriptors are fetched one phase ahead into shared memory (cp.async), the weight feeder's table sits there too.
-// Results do not depend on the run: every sum has a fixed order.
+// Results do not depend on the run: every sum has a fixed order.  They may differ in rounding between GPUs, where another number of clusters
+// fits: the order follows from the number of CTAs.
 // What bounds a phase here is a chain of round trips (barrier arrival + poll, A tile, products, exchange, store drain),
 // not the tensor pipe and not HBM.
 #include <cuda_bf16.h>

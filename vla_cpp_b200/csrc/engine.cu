@@ -602,8 +602,8 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
     if ((rc = vlab200_rope_table(rs, rs + (size_t)S * half, pos_base, S, hd, c.rope_base, cs))) return rc;
     if ((rc = vlab200_rope_table(rx, rx + (size_t)S * half, 0, S, hd, c.rope_base, cs))) return rc;
     VB_CUDA(cudaMemcpyAsync(e->x.p, x0, (size_t)Mc * A * 4, cudaMemcpyDeviceToDevice, cs));
-    // One observation: the whole loop as one persistent kernel (6.7 vs 11.4 ms per chunk for a pi0-shaped expert, 4.6 vs
-    // 7.6 ms SmolVLA-shaped); VLAB200_CHUNK_LOOP=0 keeps the launch-per-operator path.
+    // One observation: the whole loop as one persistent kernel (6.5 vs 10.9 ms per chunk for a pi0-shaped expert, 6.4 vs 12.2 ms
+    // pi0.5-shaped, 816 prefix keys; 4.2 vs 7.3 ms SmolVLA-shaped, 177); VLAB200_CHUNK_LOOP=0 keeps the launch-per-operator path.
     const char *loop_env = std::getenv("VLAB200_CHUNK_LOOP");
     const bool want_loop = !loop_env || loop_env[0] != '0';
     if (n_obs == 1 && want_loop) {
