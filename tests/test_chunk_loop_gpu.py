@@ -140,7 +140,10 @@ def test_loop_kernel_other_shapes_against_oracle(oracle):
     dict(P=3, pos_base=3, model=1, L=3, H=208, n_q=5, n_kv=5, hd=64, inter=336, chunk=1, A=16, sd=32, T=2, self_every=2),
     # more attention units than CTA groups of two
     dict(P=70, pos_base=70, model=1, L=2, H=320, n_q=32, n_kv=32, hd=64, inter=640, chunk=50, A=48, sd=32, T=1, self_every=2),
-], ids=["key_blocks", "rows64", "ragged", "many_units"])
+    # a deep expert: 164 products in the phase table.  N(0, 0.02) weights as in the other deep cases: at unit scale this narrow stack
+    # amplifies roundings over 40 layers until either path is 1.4e-2 from the oracle
+    dict(P=20, model=0, L=40, H=128, n_q=2, n_kv=1, hd=64, inter=256, chunk=10, A=32, sd=32, T=2, sigma=0.02),
+], ids=["key_blocks", "rows64", "ragged", "many_units", "deep"])
 def test_loop_kernel_work_split_edges(oracle, kw):
     from tests.test_engine_gpu import run_case
 
