@@ -384,8 +384,10 @@ VLAB200_API int32_t vlab200_act_quant(const void *x_bf16, int8_t *q, float *scal
  * reference's 2-bit "ladder" pack (N*K/4 bytes; N % 16 == 0, K % 128 == 0).
  * acc_out (optional, int32 [M][N]) receives the raw accumulators.
  * path: 0 = automatic (M <= 8: HBM-bound GEMV on the packed weights; larger M: tcgen05
- * int8 MMA, on CTA pairs when N >= 256), 1 = force GEMV, 2 = force the one-CTA-per-tile
- * tensor-core kernel, 3 = force the CTA-pair kernel (with ws_num > 1, 2 and 3 need (N / ws_num) % 32 == 0).
+ * int8 MMA, tiling by cost), 1 = force GEMV, 2 = force the one-CTA-per-tile tensor-core kernel (128 columns),
+ * 3 = force the CTA-pair kernel (with ws_num > 1, 2 and 3 need (N / ws_num) % 32 == 0); 64 or 128, plus 256 times 2 or 4:
+ * one-CTA tiles of so many columns, with their K cut over so many CTAs of a cluster (K / 128 at least as many).  The same
+ * accumulators by every path and the same bits in out by every path but 1.
  * Replaces bitlinear_int8xint2 / bitlinear_int8xint2_m
  * (src/kernels/bitvla/bitnet_kernels.cu:31-116, kernels bitnet_kernels.h:108-409). */
 VLAB200_API int32_t vlab200_ternary_linear(const int8_t *A, const uint8_t *W_ladder, void *out_bf16,

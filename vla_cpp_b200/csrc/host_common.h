@@ -60,6 +60,30 @@ int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cud
     return e == cudaSuccess ? VLAB200_OK : cuda_fail(e, "cudaLaunchKernelEx");
 }
 
+// The same with clusters of `cluster` CTAs along x (the grid is a multiple of it).
+template <typename... KArgs, typename... Args>
+static inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+    return e == cudaSuccess ? VLAB200_OK : cuda_fail(e, "cudaLaunchKernelEx");
+}
+
+// How many clusters of `cluster` CTAs of a kernel (its shared memory already opted into) the current device holds at once; 0 on failure.
+// Asked of the driver once per (device, kernel, cluster).
+int max_active_clusters(const void *kernel, int threads, int smem, int cluster);
+
 // Owning device allocation (move-only).
 struct DevBuf {
     void *p = nullptr;
@@ -87,6 +111,21 @@ struct DevBuf {
         return static_cast<T *>(p);
     }
 };
+
+// The ternary linear as the kernels of this library call it (ternary.cu): vlab200_ternary_linear, and what its epilogue adds.
+struct TernaryCall {
+    const int8_t *A;
+    const uint8_t *W;  // ladder pack
+    void *out;         // bf16
+    int32_t *acc;
+    const float *s, *ws;
+    int ws_num, M, N, K, path;
+    const void *bias;  // bf16 [N], added to the rounded result and rounded again (bitvla_add_bias_bf16), or nullptr
+    int gelu;          // tanh-GELU behind the bias
+    int gate_up;       // out [M][N / 2] = relu(column n)^2 * column N / 2 + n
+    int w_early;       // the packed weights were complete before any kernel that may still run: they are read before the dependency wait
+};
+int ternary_linear(const TernaryCall &c, cudaStream_t st);
 
 // A checkpoint tensor ([d1][d0], d1 == 1 for vectors, d1 < 0: d0 elements of any shape; f32 / f16 / bf16 in the file) uploaded as bf16 or float32,
 // optionally with the Gemma-norm "+1" (gguf.cu).  VLAB200_OK or an error with the last-error text set.

@@ -236,56 +236,194 @@ __global__ void __launch_bounds__(GEMV_THREADS) ternary_gemv_kernel(const int8_t
 //   warp 1      tcgen05.mma issuer
 //   warps 2-9   decoders: 2-bit ladder slots -> int8, written into the swizzled B tile
 //   warps 10-13 epilogue (one per TMEM lane quarter): acc / s[m] * ws -> bf16
+//
+// This is the kernel for few rows, where a launch is a chain of latencies.  Two things shorten it:
+//   * The packed weights do not depend on the kernel before this one, so (e.w_early) the decoders fill their ring while that kernel
+//     is still running; at K = 1152 the ring of the 64-column form holds all of a tile's weights.  What is left behind the
+//     dependency wait is the activation tile, the products and the epilogue.
+//   * `slices` CTAs of a cluster share a tile's K range.  The sums are whole numbers, so they add up to the same result in any
+//     order: every CTA of the cluster finishes BN / slices of the tile's columns and gets the others' sums for them through
+//     distributed shared memory.
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 128;
 constexpr int GEMM_THREADS = 448;
 
-// Separate rings: the activation ring is deep (TMA latency from L2 is several main-loop steps),
-// the decoded-weight ring shallow (its producers are warps of this CTA).
-constexpr int GEMM_SA = 7, GEMM_SW = 3;
-
-template <int BN, int STAGES>
-struct GemmSmem {
-    static constexpr int A_BYTES = GEMM_BM * GEMM_BK;
-    static constexpr int W_BYTES = BN * GEMM_BK;
-    static constexpr int W_OFFSET = GEMM_SA * A_BYTES;
-    static constexpr int BAR_OFFSET = W_OFFSET + GEMM_SW * W_BYTES;
-    static constexpr int STAGING_OFFSET = BAR_OFFSET + 256;  // 4 epilogue warps x 32 rows x 128 bytes
-    static constexpr int TOTAL = STAGING_OFFSET + 4 * 4096 + 1024;  // + alignment slack
+// What the epilogue does behind bf16(acc * ws / s): nothing, [+ bias, rounded] [tanh-GELU, rounded], or with gate_up
+// relu(gate)^2 * up of columns n and N / 2 + n (the output then has N / 2 columns).
+struct TernEpi {
+    const __nv_bfloat16 *bias;
+    int gelu, gate_up, w_early;
 };
 
-template <int BN, int STAGES>
+// tanh.approx: what the reference's tanhf becomes under its --use_fast_math build
+__device__ __forceinline__ float gelu_tanh_fast(float v) {
+    const float u = 0.7978845608028654f * (v + 0.044715f * v * v * v);
+    float th;
+    asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(u));
+    return 0.5f * v * (1.0f + th);
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// NV accumulators of consecutive columns -> packed bf16 of the linear's output, bias (float, in shared memory) and GELU included.
+template <int NV>
+__device__ __forceinline__ void tern_finish(const uint32_t (&r)[NV], float cs, const float *bias, int gelu, uint32_t (&w)[NV / 2]) {
+#pragma unroll
+    for (int e = 0; e < NV / 2; ++e) w[e] = pack_bf16((float)(int)r[2 * e] * cs, (float)(int)r[2 * e + 1] * cs);
+    if (!bias) return;
+#pragma unroll
+    for (int e = 0; e < NV / 2; ++e) {
+        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[e]));
+        w[e] = pack_bf16(v.x + bias[2 * e], v.y + bias[2 * e + 1]);
+    }
+    if (!gelu) return;
+#pragma unroll
+    for (int e = 0; e < NV / 2; ++e) {
+        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[e]));
+        w[e] = pack_bf16(gelu_tanh_fast(v.x), gelu_tanh_fast(v.y));
+    }
+}
+
+// relu(bf16(g))^2 * bf16(u) -> packed bf16 (gate_up_fused_sqrelu_mul_bf16_kernel, bitvla_lm_cuda.cu:527-542)
+__device__ __forceinline__ void tern_gate_up(const uint32_t (&g)[32], const uint32_t (&u)[32], float csg, float csu, uint32_t (&w)[16]) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        const uint32_t gp = pack_bf16((float)(int)g[2 * e] * csg, (float)(int)g[2 * e + 1] * csg);
+        const uint32_t up = pack_bf16((float)(int)u[2 * e] * csu, (float)(int)u[2 * e + 1] * csu);
+        const float2 gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&gp));
+        const float2 uf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&up));
+        const float g0 = fmaxf(gf.x, 0.f), g1 = fmaxf(gf.y, 0.f);
+        w[e] = pack_bf16(g0 * g0 * uf.x, g1 * g1 * uf.y);
+    }
+}
+
+// A lane's 32 columns (packed bf16) into half `hf` of its 128-byte line of the staging area.
+__device__ __forceinline__ void tern_stage(uint8_t *line, int hf, uint32_t sw, const uint32_t (&w)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4 *>(line + (((uint32_t)(4 * hf + i) ^ sw) << 4)) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+}
+
+// A warp's 32 rows x up to 64 columns (bf16), staged by rows in swizzled 128-byte lines, out to global memory as whole lines.
+__device__ __forceinline__ void tern_store_rows(const uint8_t *stg, __nv_bfloat16 *out, int m_first, int M, size_t ld, int n, int cols, int lane) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int rr = (lane >> 3) + 4 * i, ch = lane & 7;
+        const uint4 v = *reinterpret_cast<const uint4 *>(stg + rr * 128 + (((uint32_t)ch ^ (uint32_t)(rr & 7)) << 4));
+        if (m_first + rr < M && ch * 8 < cols) *reinterpret_cast<uint4 *>(out + (size_t)(m_first + rr) * ld + n + ch * 8) = v;
+    }
+}
+
+// One warp's part of a tile's epilogue: 32 rows from m_first (this lane's is m_first + lane, at TMEM address lane_addr), BN accumulator
+// columns.  A thread owns one accumulator row; writing its 128 bytes straight to global memory would scatter 16-byte pieces over 32 rows
+// per instruction, so 32 rows x 64 columns at a time are staged in shared memory (stg) and written as whole 128-byte lines.
+// acc / s * ws is evaluated as acc * (ws / s): at most one float ulp from the two-step form.  A 32-column chunk never straddles a scale
+// group (the group size is a multiple of 32).
+template <int BN>
+__device__ __forceinline__ void tern_epilogue_tile(uint32_t lane_addr, uint8_t *stg, const float *bias, const TernEpi &e, __nv_bfloat16 *out,
+                                                   int32_t *acc_out, const float *ws, int group, float sm, int m_first, int M, int N, int n0, int lane) {
+    uint8_t *mine = stg + lane * 128;
+    const uint32_t sw = (uint32_t)(lane & 7);
+    const int m = m_first + lane;
+    if (e.gate_up) {
+        const int n_out = N / 2;
+        constexpr int STEP = BN / 2 < 64 ? BN / 2 : 64;
+#pragma unroll 1
+        for (int c = 0; c < BN / 2; c += STEP) {
+            const int n = n0 + c;
+            if (n >= n_out) break;
+#pragma unroll 1
+            for (int hf = 0; hf < STEP / 32; ++hf) {
+                uint32_t g[32], u[32], w[16];
+                tmem_ld32(lane_addr + (uint32_t)(c + 32 * hf), g);
+                tmem_ld32(lane_addr + (uint32_t)(BN / 2 + c + 32 * hf), u);
+                tmem_ld_wait();
+                const int nh = min(n + 32 * hf, n_out - 1);
+                tern_gate_up(g, u, __fdiv_rn(ws[nh / group], sm), __fdiv_rn(ws[(n_out + nh) / group], sm), w);
+                tern_stage(mine, hf, sw, w);
+            }
+            __syncwarp();
+            tern_store_rows(stg, out, m_first, M, (size_t)n_out, n, min(STEP, n_out - n), lane);
+            __syncwarp();
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 64) {
+        const int n = n0 + c;
+        if (n >= N) break;  // uniform; N % 16 == 0, so the chunk may be cut after any multiple of 16 columns
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+            uint32_t r[32], w[16];
+            const int ch = c + 32 * hf, nh = n + 32 * hf;
+            tmem_ld32(lane_addr + (uint32_t)ch, r);
+            tmem_ld_wait();
+            if (acc_out && m < M) {
+                int4 *dst = reinterpret_cast<int4 *>(acc_out + (size_t)m * N + nh);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (nh + 4 * i < N) dst[i] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
+            }
+            tern_finish<32>(r, __fdiv_rn(ws[min(nh, N - 1) / group], sm), bias ? bias + ch : nullptr, e.gelu, w);
+            tern_stage(mine, hf, sw, w);
+        }
+        __syncwarp();
+        tern_store_rows(stg, out, m_first, M, (size_t)N, n, min(64, N - n), lane);
+        __syncwarp();
+    }
+}
+
+// Separate rings: SA activation tiles (TMA latency from L2 is several main-loop steps), SW decoded weight tiles.
+template <int BN>
+struct GemmSmem {
+    static constexpr int SA = BN == 64 ? 6 : 5, SW = BN == 64 ? 12 : 5;
+    static constexpr int A_BYTES = GEMM_BM * GEMM_BK;
+    static constexpr int W_BYTES = BN * GEMM_BK;
+    static constexpr int W_OFFSET = SA * A_BYTES;
+    static constexpr int EPI_OFFSET = W_OFFSET + SW * W_BYTES;  // 4 warps x 32 rows x 128 bytes, or the other slices' sums
+    static constexpr int EPI_BYTES = 3 * GEMM_BM * (BN / 4) * 4;
+    static constexpr int BIAS_OFFSET = EPI_OFFSET + EPI_BYTES;  // 4 warps x BN floats
+    static constexpr int BAR_OFFSET = BIAS_OFFSET + 4 * BN * 4;
+    static constexpr int TOTAL = BAR_OFFSET + 512 + 1024;  // + alignment slack
+};
+
+template <int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t *__restrict__ Wp,
                        __nv_bfloat16 *__restrict__ out, int32_t *__restrict__ acc_out,
                        const float *__restrict__ s, const float *__restrict__ ws, int ws_num, int M, int N, int K,
-                       int tiles_m, int tiles_n, int *status) {
-    using L = GemmSmem<BN, STAGES>;
+                       int tiles_m, int tiles_n, int slices, const TernEpi e, int *status) {
+    using L = GemmSmem<BN>;
     extern __shared__ uint8_t gemm_smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) &
                                                 ~static_cast<uintptr_t>(1023));
     uint64_t *full_a = reinterpret_cast<uint64_t *>(smem + L::BAR_OFFSET);
-    uint64_t *empty_a = full_a + GEMM_SA;
-    uint64_t *full_w = empty_a + GEMM_SA;
-    uint64_t *empty_w = full_w + GEMM_SW;
-    uint64_t *accum_full = empty_w + GEMM_SW;
+    uint64_t *empty_a = full_a + L::SA;
+    uint64_t *full_w = empty_a + L::SA;
+    uint64_t *empty_w = full_w + L::SW;
+    uint64_t *accum_full = empty_w + L::SW;
     uint64_t *accum_empty = accum_full + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    constexpr bool HALF = BN < 128;  // fewer than eight 16-row weight blocks: four warps decode even K steps, four odd ones
+    constexpr int WPS = BN / 64;  // decode warps per step
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ksteps = K / GEMM_BK;
+    const int rank = slices > 1 ? (int)cluster_ctarank() : 0;  // this CTA's slice of the K steps
+    const int unit = (int)blockIdx.x / slices, n_units = (int)gridDim.x / slices;
+    const int kbeg = rank * (K / GEMM_BK) / slices, ksteps = (rank + 1) * (K / GEMM_BK) / slices - kbeg;
     const int n_tiles = tiles_m * tiles_n;
     const WaitCtx wc{abort_flag, status};
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < GEMM_SA; ++i) {
+        for (int i = 0; i < L::SA; ++i) {
             mbar_init(&full_a[i], 1);
             mbar_init(&empty_a[i], 1);
         }
-        for (int i = 0; i < GEMM_SW; ++i) {
-            mbar_init(&full_w[i], HALF ? 4 : 8);  // one arrival per decode warp of the step
+        for (int i = 0; i < L::SW; ++i) {
+            mbar_init(&full_w[i], WPS);  // one arrival per decode warp of the step
             mbar_init(&empty_w[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -301,10 +439,12 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
     }
     tc_fence_before();
     __syncthreads();
+    if (slices > 1) cluster_sync_all();  // every CTA of the cluster runs before another one writes to its shared memory
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
-    pdl_wait();  // the set-up above overlapped the previous kernel's tail
+    // the set-up above overlapped the previous kernel's tail; the decoders go on without waiting for it if they may
+    if (warp < 2 || warp >= 10 || !e.w_early) pdl_wait();
 
     // tiles are ordered m-fastest so that CTAs running at the same time share a weight slab
     if (warp == 0) {
@@ -312,23 +452,24 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
             tma_prefetch_desc(&a_map);
             uint32_t st = 0, ph = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x) {
+            for (int tile = unit; ok && tile < n_tiles; tile += n_units) {
                 const int m0 = (tile % tiles_m) * GEMM_BM;
-                for (int kt = 0; kt < ksteps; ++kt) {
+                for (int kt = kbeg; kt < kbeg + ksteps; ++kt) {
                     ok = mbar_wait(&empty_a[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                     if (!ok) break;
                     mbar_expect_tx(&full_a[st], L::A_BYTES);
                     tma_load_2d(smem + st * L::A_BYTES, &a_map, &full_a[st], kt * GEMM_BK, m0);
-                    if (++st == GEMM_SA) { st = 0; ph ^= 1u; }
+                    if (++st == L::SA) { st = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
         {  // the whole warp walks the tiles, one elected lane issues (uniform control: see gemm.cu)
             constexpr uint32_t idesc = make_idesc(2, 1, 1, 0, 0, GEMM_BM, BN);
+            const uint64_t a_desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024), w_desc0 = smem_desc_sw128(smem_u32(smem + L::W_OFFSET), 16, 1024);
             uint32_t st = 0, ph = 0, sw = 0, pw = 0, j = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x, ++j) {
+            for (int tile = unit; ok && tile < n_tiles; tile += n_units, ++j) {
                 const uint32_t buf = j & 1u;
                 ok = warp_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
@@ -339,18 +480,15 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
                     if (ok) ok = warp_wait(&full_w[sw], pw, wc, DEV_TIMEOUT_FULL);
                     if (!ok) break;
                     tc_fence_after();
+                    const uint64_t a_desc = a_desc0 + (uint64_t)(st * (L::A_BYTES >> 4)), w_desc = w_desc0 + (uint64_t)(sw * (L::W_BYTES >> 4));
                     if (elect_one()) {
-                        const uint32_t a_addr = smem_u32(smem + st * L::A_BYTES);
-                        const uint32_t w_addr = smem_u32(smem + L::W_OFFSET + sw * L::W_BYTES);
 #pragma unroll
-                        for (int k = 0; k < GEMM_BK / 32; ++k)
-                            mma_i8(d_tmem, smem_desc_sw128(a_addr + k * 32, 16, 1024),
-                                   smem_desc_sw128(w_addr + k * 32, 16, 1024), idesc, (kt | k) != 0 ? 1u : 0u);
+                        for (int k = 0; k < GEMM_BK / 32; ++k) mma_i8(d_tmem, a_desc + 2 * k, w_desc + 2 * k, idesc, (kt | k) != 0 ? 1u : 0u);
                         tc_commit(&empty_a[st]);
                         tc_commit(&empty_w[sw]);
                     }
-                    if (++st == GEMM_SA) { st = 0; ph ^= 1u; }
-                    if (++sw == GEMM_SW) { sw = 0; pw ^= 1u; }
+                    if (++st == L::SA) { st = 0; ph ^= 1u; }
+                    if (++sw == L::SW) { sw = 0; pw ^= 1u; }
                 }
                 if (!ok) break;
                 if (elect_one()) tc_commit(&accum_full[buf]);
@@ -358,11 +496,10 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
         }
     } else if (warp < 10) {
         // ---- decode warps: ladder slots -> swizzled K-major int8 tile ----
-        const int dw = warp - 2;                  // 0..7
-        constexpr int NBLK = BN / 16;             // 16-row weight blocks in the tile
-        constexpr int PER_WARP = HALF ? 1 : NBLK / 8;
-        const int blk0 = HALF ? dw & 3 : dw;
-        const int nblk_total = N / 16;
+        // A step is four weight blocks (64 rows) per warp, BN / 64 warps; the warps take steps round-robin, so a warp has several steps
+        // of time for one and the barrier wait, the proxy fence and the arrival are paid once per 64 decoded rows.
+        const int dw = warp - 2;  // 0..7
+        const int first = dw / WPS, blk0 = (dw % WPS) * 4;  // steps first, first + STEP, ...; blocks blk0 .. blk0 + 3 of the tile
         // lane geometry inside one 512-byte chunk (lane t holds the 4 slots at byte offset 16 t)
         const int row_in_blk = 8 * ((lane & 7) >> 2) + 4 * (lane & 1);  // + slot 0..3
         const int chunk16 = 2 * (lane >> 3) + ((lane & 3) >> 1);        // 16-byte column 0..7
@@ -370,135 +507,148 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
         // write rows 8 apart (same banks); the upper one walks its slots in the order 2, 3, 0, 1 so that
         // the two never hit the same 16-byte column in the same instruction.
         const bool swap_slots = (lane & 4) != 0;
-        // Packed weights are prefetched three main-loop steps ahead into registers: one step is
-        // shorter than the latency of a load that misses L2.
-        constexpr int PF = 3;
-        uint4 pf[PF][PER_WARP];
-        const int my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+        constexpr int NBLK = BN / 16, STEP = 8 / WPS;
+        const int my_tiles = unit < n_tiles ? (n_tiles - 1 - unit) / n_units + 1 : 0;
         const int total = my_tiles * ksteps;
-        auto fetch = [&](int g, uint4 (&dst)[PER_WARP]) {  // g: flat step index over this CTA's tiles
-            const int tile = blockIdx.x + (g / ksteps) * gridDim.x, kt = g % ksteps;
-            const int nb0 = (tile / tiles_m) * NBLK;
+        auto fetch = [&](int g, uint4 (&dst)[4]) {  // g: flat step index over this CTA's tiles
+            const int tn = (unit + (g / ksteps) * n_units) / tiles_m, kt = kbeg + g % ksteps;
 #pragma unroll
-            for (int i = 0; i < PER_WARP; ++i) {
-                const int nb = nb0 + blk0 + 8 * i;
-                dst[i] = (g < total && nb < nblk_total)
-                             ? __ldg(reinterpret_cast<const uint4 *>(Wp + (size_t)nb * 4 * K + (size_t)kt * 512) + lane)
-                             : make_uint4(0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu);
+            for (int i = 0; i < 4; ++i) {
+                const int blk = blk0 + i;
+                int nb = tn * NBLK + blk, end = N / 16;
+                if (e.gate_up) {  // half of the tile's rows are gate rows, half the up rows of the same columns
+                    nb = tn * (NBLK / 2) + (blk & (NBLK / 2 - 1));
+                    end = N / 32;
+                }
+                const bool in = g < total && nb < end;
+                if (e.gate_up && blk >= NBLK / 2) nb += N / 32;
+                dst[i] = in ? __ldg(reinterpret_cast<const uint4 *>(Wp + (size_t)nb * 4 * K + (size_t)kt * 512) + lane)
+                            : make_uint4(0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu);
             }
         };
-        auto decode_store = [&](const uint4 (&cur)[PER_WARP], uint8_t *wt) {
+        uint4 nxt[4];
+        if (ksteps > 0) fetch(first, nxt);
+        uint32_t st = (uint32_t)first, ph = 0;
+        bool ok = true;
+        for (int g = first; ok && g < total; g += STEP) {
+            uint4 cur[4];
 #pragma unroll
-            for (int i = 0; i < PER_WARP; ++i) {
-                const int blk = blk0 + 8 * i;
+            for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
+            fetch(g + STEP, nxt);
+            uint8_t *wt = smem + L::W_OFFSET + st * L::W_BYTES;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
                 const uint32_t words[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+                uint32_t d[4][4];
+#pragma unroll
+                for (int sl = 0; sl < 4; ++sl) decode_slot(swap_slots ? words[sl ^ 2] : words[sl], d[sl]);
+                if (i == 0) {  // the first block is decoded before the stage is known to be free
+                    ok = mbar_wait(&empty_w[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
+                    if (!ok) break;
+                }
 #pragma unroll
                 for (int sl = 0; sl < 4; ++sl) {
-                    uint32_t d[4];
-                    decode_slot(swap_slots ? words[sl ^ 2] : words[sl], d);
-                    const int r = blk * 16 + row_in_blk + (swap_slots ? (sl ^ 2) : sl);  // row inside the BN tile
+                    const int r = (blk0 + i) * 16 + row_in_blk + (swap_slots ? (sl ^ 2) : sl);  // row inside the BN tile
                     uint8_t *dst = wt + (r >> 3) * 1024 + (r & 7) * 128 + ((chunk16 ^ (r & 7)) << 4);
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(d[0], d[1], d[2], d[3]);
+                    *reinterpret_cast<uint4 *>(dst) = make_uint4(d[sl][0], d[sl][1], d[sl][2], d[sl][3]);
                 }
             }
-        };
-        constexpr int STEP = HALF ? 2 : 1;  // this warp decodes steps first, first + STEP, ...
-        const int first = HALF ? dw >> 2 : 0;
-        bool ok = true;
-#pragma unroll
-        for (int i = 0; i < PF; ++i) fetch(first + i * STEP, pf[i]);
-        for (int g0 = first; ok && g0 < total; g0 += PF * STEP) {
-#pragma unroll
-            for (int u = 0; u < PF; ++u) {
-                const int g = g0 + u * STEP;
-                if (g >= total) break;
-                uint4 cur[PER_WARP];
-#pragma unroll
-                for (int i = 0; i < PER_WARP; ++i) cur[i] = pf[u][i];
-                fetch(g + PF * STEP, pf[u]);
-                const uint32_t st = (uint32_t)g % GEMM_SW, ph = ((uint32_t)g / GEMM_SW) & 1u;
-                ok = mbar_wait(&empty_w[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
-                if (!ok) break;
-                decode_store(cur, smem + L::W_OFFSET + st * L::W_BYTES);
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full_w[st]);
-            }
+            if (!ok) break;
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full_w[st]);
+            st += STEP;
+            if (st >= L::SW) { st -= L::SW; ph ^= 1u; }
         }
-    } else {
-        // ---- epilogue warps 10..13: TMEM -> registers -> shared-memory transpose -> global ----
-        // A thread owns one accumulator row; writing its 128 bytes straight to global memory would
-        // scatter 16-byte pieces over 32 rows per instruction.  Each warp instead stages 32 rows x 64
-        // columns (bf16) in shared memory and writes them back as whole 128-byte lines.
+    } else if (slices == 1) {
+        // ---- epilogue warps 10..13 ----
         const int q = warp & 3;  // TMEM lane quarter this warp may read
-        const int group = N / ws_num;
-        uint8_t *stg = smem + L::STAGING_OFFSET + (warp - 10) * 4096;
-        const uint32_t my_sw = (uint32_t)(lane & 7);
+        uint8_t *stg = smem + L::EPI_OFFSET + (warp - 10) * 4096;
+        float *bias = e.bias ? reinterpret_cast<float *>(smem + L::BIAS_OFFSET) + (warp - 10) * BN : nullptr;
+        const int cols_tile = e.gate_up ? BN / 2 : BN;
         uint32_t j = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x, ++j) {
+        for (int tile = unit; ok && tile < n_tiles; tile += n_units, ++j) {
             const uint32_t buf = j & 1u;
-            const int m0 = (tile % tiles_m) * GEMM_BM, n0 = (tile / tiles_m) * BN;
-            const int m = m0 + q * 32 + lane;
+            const int m_first = (tile % tiles_m) * GEMM_BM + q * 32, n0 = (tile / tiles_m) * cols_tile;
+            const float sm = (m_first + lane < M) ? s[m_first + lane] : 1.0f;
+            if (bias) {
+                for (int c = lane; c < BN; c += 32) bias[c] = n0 + c < N ? __bfloat162float(e.bias[n0 + c]) : 0.0f;
+                __syncwarp();
+            }
             ok = mbar_wait(&accum_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM);
             if (!ok) break;
             tc_fence_after();
-            const float sm = (m < M) ? s[m] : 1.0f;
-            const uint32_t lane_addr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-#pragma unroll 1
-            for (int c = 0; c < BN; c += 64) {
-                uint32_t r0[32], r1[32];
-                tmem_ld32(lane_addr + (uint32_t)c, r0);
-                tmem_ld32(lane_addr + (uint32_t)(c + 32), r1);
-                tmem_ld_wait();
-                const int n = n0 + c;
-                if (n >= N) break;  // uniform; N % 16 == 0, so the chunk may be cut after any multiple of 16 columns
-                if (acc_out && m < M) {
-                    int4 *dst = reinterpret_cast<int4 *>(acc_out + (size_t)m * N + n);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (n + 4 * e < N)
-                            dst[e] = make_int4((int)r0[4 * e], (int)r0[4 * e + 1], (int)r0[4 * e + 2], (int)r0[4 * e + 3]);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (n + 32 + 4 * e < N)
-                            dst[8 + e] = make_int4((int)r1[4 * e], (int)r1[4 * e + 1], (int)r1[4 * e + 2], (int)r1[4 * e + 3]);
-                }
-                // acc / s * ws evaluated as acc * (ws / s): at most one float ulp from the two-step form.
-                // A 32-column chunk never straddles a scale group (the group size is a multiple of 32).
-                const float cs0 = __fdiv_rn(ws[n / group], sm);
-                const float cs1 = __fdiv_rn(ws[min(n + 32, N - 1) / group], sm);
-                uint8_t *mine = stg + lane * 128;
-#pragma unroll
-                for (int e4 = 0; e4 < 4; ++e4) {
-                    uint32_t pa[4], pb[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const __nv_bfloat162 ha = __floats2bfloat162_rn((float)(int)r0[8 * e4 + 2 * e] * cs0,
-                                                                        (float)(int)r0[8 * e4 + 2 * e + 1] * cs0);
-                        const __nv_bfloat162 hb = __floats2bfloat162_rn((float)(int)r1[8 * e4 + 2 * e] * cs1,
-                                                                        (float)(int)r1[8 * e4 + 2 * e + 1] * cs1);
-                        pa[e] = *reinterpret_cast<const uint32_t *>(&ha);
-                        pb[e] = *reinterpret_cast<const uint32_t *>(&hb);
-                    }
-                    *reinterpret_cast<uint4 *>(mine + (((uint32_t)e4 ^ my_sw) << 4)) = make_uint4(pa[0], pa[1], pa[2], pa[3]);
-                    *reinterpret_cast<uint4 *>(mine + (((uint32_t)(4 + e4) ^ my_sw) << 4)) = make_uint4(pb[0], pb[1], pb[2], pb[3]);
-                }
-                __syncwarp();
-                const int cols_valid = min(64, N - n);  // 32 or 64
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int rr = (lane >> 3) + 4 * i;
-                    const int ch = lane & 7;
-                    const uint4 v = *reinterpret_cast<const uint4 *>(stg + rr * 128 + (((uint32_t)ch ^ (uint32_t)(rr & 7)) << 4));
-                    const int mr = m0 + q * 32 + rr;
-                    if (mr < M && ch * 8 < cols_valid)
-                        *reinterpret_cast<uint4 *>(out + (size_t)mr * N + n + ch * 8) = v;
-                }
-                __syncwarp();
-            }
+            tern_epilogue_tile<BN>(tmem_base + buf * BN + ((uint32_t)(q * 32) << 16), stg, bias, e, out, acc_out, ws, N / ws_num, sm, m_first, M, N,
+                                   n0, lane);
             tc_fence_before();
             mbar_arrive(&accum_empty[buf]);
+        }
+    }
+    if (slices > 1) {
+        // One tile per cluster.  The sums of the columns that another CTA finishes go into its shared memory, [sender][4 columns][row] so
+        // that a warp writes 512 contiguous bytes; then each CTA adds what it received to its own sums and finishes its columns.
+        const int q = warp & 3, width = BN / slices;
+        const int m0 = (unit % tiles_m) * GEMM_BM, n0 = (unit / tiles_m) * BN + rank * width;
+        const int row = q * 32 + lane, m = m0 + row;
+        const bool epi = warp >= 10;
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+        uint8_t *recv = smem + L::EPI_OFFSET;
+        const int slot_bytes = width * GEMM_BM * 4;
+        float *bias = e.bias ? reinterpret_cast<float *>(smem + L::BIAS_OFFSET) + (warp & 3) * BN : nullptr;
+        bool ok = epi;
+        float sm = 1.0f;
+        if (epi) {
+            if (m < M) sm = s[m];
+            if (bias) {
+                for (int c = lane; c < width; c += 32) bias[c] = n0 + c < N ? __bfloat162float(e.bias[n0 + c]) : 0.0f;
+                __syncwarp();
+            }
+            ok = mbar_wait(&accum_full[0], 0u, wc, DEV_TIMEOUT_ACCUM);
+            tc_fence_after();
+            if (ok) {
+                for (int r = 0; r < slices; ++r) {
+                    if (r == rank) continue;
+                    const uint32_t dst = cluster_addr(smem_u32(recv) + (uint32_t)((rank < r ? rank : rank - 1) * slot_bytes + row * 16), (uint32_t)r);
+                    for (int c = 0; c < width; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld16(lane_addr + (uint32_t)(r * width + c), v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            st_cluster_v4(dst + (uint32_t)((c / 4 + i) * GEMM_BM * 16), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    }
+                }
+            }
+        }
+        __syncwarp();  // the cluster barrier is for converged warps
+        cluster_sync_all();
+        if (ok) {
+            const int group = N / ws_num;
+            for (int c = 0; c < width; c += 16) {
+                const int n = n0 + c;
+                if (n >= N) break;  // N % 16 == 0: a piece of 16 columns is inside or outside
+                uint32_t v[16], w[8];
+                tmem_ld16(lane_addr + (uint32_t)(rank * width + c), v);
+                tmem_ld_wait();
+                for (int t = 0; t < slices - 1; ++t)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint4 o = *reinterpret_cast<const uint4 *>(recv + t * slot_bytes + (c / 4 + i) * GEMM_BM * 16 + row * 16);
+                        v[4 * i] += o.x; v[4 * i + 1] += o.y; v[4 * i + 2] += o.z; v[4 * i + 3] += o.w;
+                    }
+                tern_finish<16>(v, __fdiv_rn(ws[n / group], sm), bias ? bias + c : nullptr, e.gelu, w);
+                if (m < M) {
+                    if (acc_out) {
+                        int4 *dst = reinterpret_cast<int4 *>(acc_out + (size_t)m * N + n);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) dst[i] = make_int4((int)v[4 * i], (int)v[4 * i + 1], (int)v[4 * i + 2], (int)v[4 * i + 3]);
+                    }
+                    uint4 *dst = reinterpret_cast<uint4 *>(out + (size_t)m * N + n);
+                    dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                    dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                }
+            }
         }
     }
     tc_fence_before();
@@ -525,14 +675,15 @@ struct PairSmem {
     static constexpr int STAGE_BYTES = A_BYTES + W_BYTES;
     static constexpr int BAR_OFFSET = PAIR_STAGES * STAGE_BYTES;
     static constexpr int STAGING_OFFSET = BAR_OFFSET + 256;
-    static constexpr int TOTAL = STAGING_OFFSET + 4 * 4096 + 1024;
+    static constexpr int BIAS_OFFSET = STAGING_OFFSET + 4 * 4096;  // 4 warps x 256 floats
+    static constexpr int TOTAL = BIAS_OFFSET + 4 * 256 * 4 + 1024;
 };
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t *__restrict__ Wp,
                          __nv_bfloat16 *__restrict__ out, int32_t *__restrict__ acc_out,
                          const float *__restrict__ s, const float *__restrict__ ws, int ws_num, int M, int N, int K,
-                         int tiles_mp, int tiles_n, int *status) {
+                         int tiles_mp, int tiles_n, const TernEpi e, int *status) {
     using L = PairSmem;
     constexpr int BN = 256;
     extern __shared__ uint8_t gemm_smem_raw[];
@@ -650,7 +801,8 @@ ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_
         // wait, proxy fence and arrival are paid once per 64 decoded rows.
         const int dw = warp - 2;
         const int pi = dw >> 1, hb = dw & 1;
-        const int nblk_total = N / 16;
+        // gate_up: the even CTA decodes 128 gate rows, the odd one the up rows of the same columns
+        const int nblk_tile = e.gate_up ? 8 : BN / 16, nblk_total = e.gate_up ? N / 32 : N / 16;
         const int row_in_blk = 8 * ((lane & 7) >> 2) + 4 * (lane & 1);  // + slot 0..3
         const int chunk16 = 2 * (lane >> 3) + ((lane & 3) >> 1);        // 16-byte column 0..7
         const bool swap_slots = (lane & 4) != 0;  // see ternary_gemm_tc_kernel: avoids 2-way bank conflicts
@@ -658,11 +810,11 @@ ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_
         const int total = my_tiles * ksteps;
         auto fetch = [&](int g, uint4 (&dst)[4]) {
             const int tile = cid + (g / ksteps) * ncl, kt = g % ksteps;
-            const int nb0 = (tile / tiles_mp) * (BN / 16) + (int)rank * 8 + hb * 4;
+            const int nb0 = (tile / tiles_mp) * nblk_tile + (e.gate_up ? 0 : (int)rank * 8) + hb * 4, up0 = e.gate_up && rank ? nblk_total : 0;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 dst[i] = (g < total && nb0 + i < nblk_total)
-                             ? __ldg(reinterpret_cast<const uint4 *>(Wp + (size_t)(nb0 + i) * 4 * K + (size_t)kt * 512) + lane)
+                             ? __ldg(reinterpret_cast<const uint4 *>(Wp + (size_t)(up0 + nb0 + i) * 4 * K + (size_t)kt * 512) + lane)
                              : make_uint4(0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu, 0xAAAAAAAAu);
         };
         uint4 nxt[4];
@@ -703,72 +855,24 @@ ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_
     } else {
         // ---- epilogue warps 10..13: this CTA's 128 rows of the pair tile ----
         const int q = warp & 3;
-        const int group = N / ws_num;
         uint8_t *stg = smem + L::STAGING_OFFSET + (warp - 10) * 4096;
-        const uint32_t my_sw = (uint32_t)(lane & 7);
+        float *bias = e.bias ? reinterpret_cast<float *>(smem + L::BIAS_OFFSET) + (warp - 10) * BN : nullptr;
         uint32_t j = 0;
         bool ok = true;
         for (int tile = cid; ok && tile < n_tiles; tile += ncl, ++j) {
             const uint32_t buf = j & 1u;
-            const int m0 = (tile % tiles_mp) * 256 + (int)rank * 128, n0 = (tile / tiles_mp) * BN;
-            const int m = m0 + q * 32 + lane;
+            const int m0 = (tile % tiles_mp) * 256 + (int)rank * 128, m_first = m0 + q * 32, n0 = (tile / tiles_mp) * (e.gate_up ? BN / 2 : BN);
+            const float sm = (m_first + lane < M) ? s[m_first + lane] : 1.0f;
+            if (bias) {
+                for (int c = lane; c < BN; c += 32) bias[c] = n0 + c < N ? __bfloat162float(e.bias[n0 + c]) : 0.0f;
+                __syncwarp();
+            }
             ok = mbar_wait_backoff(&accum_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM, 256);
             if (!ok) break;
             tc_fence_after();
-            const float sm = (m < M) ? s[m] : 1.0f;
-            const uint32_t lane_addr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-            if (m0 < M) {  // warp-uniform: the odd CTA's rows may all lie past M
-#pragma unroll 1
-                for (int c = 0; c < BN; c += 64) {
-                    uint32_t r0[32], r1[32];
-                    tmem_ld32(lane_addr + (uint32_t)c, r0);
-                    tmem_ld32(lane_addr + (uint32_t)(c + 32), r1);
-                    tmem_ld_wait();
-                    const int n = n0 + c;
-                    if (n >= N) break;
-                    if (acc_out && m < M) {
-                        int4 *dst = reinterpret_cast<int4 *>(acc_out + (size_t)m * N + n);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (n + 4 * e < N)
-                                dst[e] = make_int4((int)r0[4 * e], (int)r0[4 * e + 1], (int)r0[4 * e + 2], (int)r0[4 * e + 3]);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (n + 32 + 4 * e < N)
-                                dst[8 + e] = make_int4((int)r1[4 * e], (int)r1[4 * e + 1], (int)r1[4 * e + 2], (int)r1[4 * e + 3]);
-                    }
-                    const float cs0 = __fdiv_rn(ws[n / group], sm);
-                    const float cs1 = __fdiv_rn(ws[min(n + 32, N - 1) / group], sm);
-                    uint8_t *mine = stg + lane * 128;
-#pragma unroll
-                    for (int e4 = 0; e4 < 4; ++e4) {
-                        uint32_t pa[4], pb[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const __nv_bfloat162 ha = __floats2bfloat162_rn((float)(int)r0[8 * e4 + 2 * e] * cs0,
-                                                                            (float)(int)r0[8 * e4 + 2 * e + 1] * cs0);
-                            const __nv_bfloat162 hb = __floats2bfloat162_rn((float)(int)r1[8 * e4 + 2 * e] * cs1,
-                                                                            (float)(int)r1[8 * e4 + 2 * e + 1] * cs1);
-                            pa[e] = *reinterpret_cast<const uint32_t *>(&ha);
-                            pb[e] = *reinterpret_cast<const uint32_t *>(&hb);
-                        }
-                        *reinterpret_cast<uint4 *>(mine + (((uint32_t)e4 ^ my_sw) << 4)) = make_uint4(pa[0], pa[1], pa[2], pa[3]);
-                        *reinterpret_cast<uint4 *>(mine + (((uint32_t)(4 + e4) ^ my_sw) << 4)) = make_uint4(pb[0], pb[1], pb[2], pb[3]);
-                    }
-                    __syncwarp();
-                    const int cols_valid = min(64, N - n);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int rr = (lane >> 3) + 4 * i;
-                        const int ch = lane & 7;
-                        const uint4 v = *reinterpret_cast<const uint4 *>(stg + rr * 128 + (((uint32_t)ch ^ (uint32_t)(rr & 7)) << 4));
-                        const int mr = m0 + q * 32 + rr;
-                        if (mr < M && ch * 8 < cols_valid)
-                            *reinterpret_cast<uint4 *>(out + (size_t)mr * N + n + ch * 8) = v;
-                    }
-                    __syncwarp();
-                }
-            }
+            if (m0 < M)  // warp-uniform: the odd CTA's rows may all lie past M
+                tern_epilogue_tile<BN>(tmem_base + buf * BN + ((uint32_t)(q * 32) << 16), stg, bias, e, out, acc_out, ws, N / ws_num, sm, m_first, M,
+                                       N, n0, lane);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
@@ -804,9 +908,16 @@ static int launch_gemv(const int8_t *A, const uint8_t *W, __nv_bfloat16 *out, in
     return launch_pdl(ternary_gemv_kernel<MT>, dim3(N / 16), dim3(GEMV_THREADS), smem, st, A, W, out, acc, s, ws, ws_num, M, N, K, m0);
 }
 
-template <int BN, int STAGES>
+// How many clusters of `cluster` CTAs of the kernel the device holds at once (0: none).
+template <int BN>
+static int tc_clusters(int cluster) {
+    if (ensure_dyn_smem(ternary_gemm_tc_kernel<BN>, GemmSmem<BN>::TOTAL) != VLAB200_OK) return 0;
+    return max_active_clusters(reinterpret_cast<const void *>(ternary_gemm_tc_kernel<BN>), GEMM_THREADS, GemmSmem<BN>::TOTAL, cluster);
+}
+
+template <int BN>
 static int launch_gemm_tc(const int8_t *A, const uint8_t *W, __nv_bfloat16 *out, int32_t *acc, const float *s,
-                          const float *ws, int ws_num, int M, int N, int K, cudaStream_t st) {
+                          const float *ws, int ws_num, int M, int N, int K, const TernEpi &e, int slices, cudaStream_t st) {
     int *status = device_status_ptr();
     if (!status) return cuda_fail(cudaGetLastError(), "device_status_ptr");
     CUtensorMap amap;
@@ -816,18 +927,22 @@ static int launch_gemm_tc(const int8_t *A, const uint8_t *W, __nv_bfloat16 *out,
     int rc = make_tensor_map(&amap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, A, dims, strides, box,
                              CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    using L = GemmSmem<BN, STAGES>;
-    if ((rc = ensure_dyn_smem(ternary_gemm_tc_kernel<BN, STAGES>, L::TOTAL))) return rc;
+    using L = GemmSmem<BN>;
+    if ((rc = ensure_dyn_smem(ternary_gemm_tc_kernel<BN>, L::TOTAL))) return rc;
     const int n_sm = sm_count();
     if (n_sm <= 0) return cuda_fail(cudaGetLastError(), "sm_count");
-    const int tiles_m = (M + GEMM_BM - 1) / GEMM_BM, tiles_n = (N + BN - 1) / BN;
+    const int bn_out = e.gate_up ? BN / 2 : BN, n_out = e.gate_up ? N / 2 : N;
+    const int tiles_m = (M + GEMM_BM - 1) / GEMM_BM, tiles_n = (n_out + bn_out - 1) / bn_out;
     const int nt = tiles_m * tiles_n;
-    return launch_pdl(ternary_gemm_tc_kernel<BN, STAGES>, dim3(nt < n_sm ? nt : n_sm), dim3(GEMM_THREADS), L::TOTAL, st, amap, W, out,
-                      acc, s, ws, ws_num, M, N, K, tiles_m, tiles_n, status);
+    if (slices > 1)
+        return launch_pdl_cluster(ternary_gemm_tc_kernel<BN>, dim3(nt * slices), dim3(GEMM_THREADS), L::TOTAL, slices, st, amap, W, out, acc, s, ws,
+                                  ws_num, M, N, K, tiles_m, tiles_n, slices, e, status);
+    return launch_pdl(ternary_gemm_tc_kernel<BN>, dim3(nt < n_sm ? nt : n_sm), dim3(GEMM_THREADS), L::TOTAL, st, amap, W, out,
+                      acc, s, ws, ws_num, M, N, K, tiles_m, tiles_n, 1, e, status);
 }
 
 static int launch_gemm_pair(const int8_t *A, const uint8_t *W, __nv_bfloat16 *out, int32_t *acc, const float *s,
-                            const float *ws, int ws_num, int M, int N, int K, cudaStream_t st) {
+                            const float *ws, int ws_num, int M, int N, int K, const TernEpi &e, cudaStream_t st) {
     int *status = device_status_ptr();
     if (!status) return cuda_fail(cudaGetLastError(), "device_status_ptr");
     CUtensorMap amap;
@@ -840,52 +955,87 @@ static int launch_gemm_pair(const int8_t *A, const uint8_t *W, __nv_bfloat16 *ou
     if ((rc = ensure_dyn_smem(ternary_gemm_pair_kernel, PairSmem::TOTAL))) return rc;
     const int n_sm = sm_count();
     if (n_sm <= 0) return cuda_fail(cudaGetLastError(), "sm_count");
-    const int tiles_mp = (M + 255) / 256, tiles_n = (N + 255) / 256;
+    const int tiles_mp = (M + 255) / 256, tiles_n = e.gate_up ? (N / 2 + 127) / 128 : (N + 255) / 256;
     const int nt = tiles_mp * tiles_n, pairs = n_sm / 2;
     return launch_pdl(ternary_gemm_pair_kernel, dim3(2 * (nt < pairs ? nt : pairs)), dim3(GEMM_THREADS), PairSmem::TOTAL, st, amap,
-                      W, out, acc, s, ws, ws_num, M, N, K, tiles_mp, tiles_n, status);
+                      W, out, acc, s, ws, ws_num, M, N, K, tiles_mp, tiles_n, e, status);
 }
 
-static int ternary_linear(const int8_t *A, const uint8_t *W, __nv_bfloat16 *out, int32_t *acc, const float *s,
-                          const float *ws, int ws_num, int M, int N, int K, cudaStream_t st, int force_path) {
-    int rc = check_gemm_args(A, W, out, s, ws, ws_num, M, N, K);
+// The tiling of a call with more than eight rows, by ns of a launch: set-up and epilogue, plus waves times 128-wide K steps.  Pair tiles
+// move the fewest bytes per product and win as soon as there are enough of them; with few rows (one image, one prompt) they leave
+// most SMs without work and narrow tiles win, and where even those are few, K slices over a cluster.
+struct TernTiling {
+    int bn, slices;  // bn 256: pair tiles
+};
+static TernTiling choose_tiling(int M, int N, int K, bool gate_up, int n_sm) {
+    const int tm = (M + 127) / 128, tp = (M + 255) / 256, ks = K / 128;
+    auto waves = [](int tiles, int units) { return (tiles + units - 1) / units; };
+    TernTiling best{64, 1};
+    int cost = 0x7fffffff;
+    auto consider = [&](int bn, int slices, int c) {
+        if (c < cost) {
+            cost = c;
+            best = {bn, slices};
+        }
+    };
+    const int t64 = tm * ((N + 63) / 64), t128 = tm * ((N + 127) / 128);
+    consider(64, 1, 3600 + 370 * ks * waves(t64, n_sm));
+    consider(128, 1, 4400 + 460 * ks * waves(t128, n_sm));
+    if (N >= 256 && n_sm >= 2) consider(256, 1, 6400 + 360 * ks * waves(tp * ((N + 255) / 256), n_sm / 2));
+    if (!gate_up)
+        for (int sl = 2; sl <= 4 && ks >= 4 * sl; sl *= 2) {
+            if (t64 * sl <= n_sm && t64 <= tc_clusters<64>(sl)) consider(64, sl, 5000 + 370 * waves(ks, sl));
+            if (t128 * sl <= n_sm && t128 <= tc_clusters<128>(sl)) consider(128, sl, 5800 + 460 * waves(ks, sl));
+        }
+    return best;
+}
+
+int ternary_linear(const TernaryCall &c, cudaStream_t st) {
+    const int8_t *A = c.A;
+    const uint8_t *W = c.W;
+    __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(c.out);
+    const int ws_num = c.ws_num, M = c.M, N = c.N, K = c.K, path = c.path;
+    int rc = check_gemm_args(A, W, out, c.s, c.ws, ws_num, M, N, K);
     if (rc) return rc;
     if (M == 0) return VLAB200_OK;
-    const bool gemv = force_path == 1 || (force_path == 0 && M <= 8);
+    const bool gemv = path == 1 || (path == 0 && M <= 8);
+    const TernEpi e{static_cast<const __nv_bfloat16 *>(c.bias), c.gelu, c.gate_up, c.w_early};
     if (gemv) {
+        if (e.bias || e.gelu || e.gate_up) return VLAB200_ERR_UNSUPPORTED;
         if ((size_t)8 * K + 4 * 8 * 16 * sizeof(int) > 200 * 1024) return VLAB200_ERR_UNSUPPORTED;
         for (int m0 = 0; m0 < M; m0 += 8) {
             const int left = M - m0;
-            if (left >= 5) rc = launch_gemv<8>(A, W, out, acc, s, ws, ws_num, M, N, K, m0, st);
-            else if (left >= 3) rc = launch_gemv<4>(A, W, out, acc, s, ws, ws_num, M, N, K, m0, st);
-            else if (left == 2) rc = launch_gemv<2>(A, W, out, acc, s, ws, ws_num, M, N, K, m0, st);
-            else rc = launch_gemv<1>(A, W, out, acc, s, ws, ws_num, M, N, K, m0, st);
+            if (left >= 5) rc = launch_gemv<8>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, m0, st);
+            else if (left >= 3) rc = launch_gemv<4>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, m0, st);
+            else if (left == 2) rc = launch_gemv<2>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, m0, st);
+            else rc = launch_gemv<1>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, m0, st);
             if (rc) return rc;
         }
         return VLAB200_OK;
     }
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(out) & 15) ||
-        (acc && (reinterpret_cast<uintptr_t>(acc) & 15)))
+        (c.acc && (reinterpret_cast<uintptr_t>(c.acc) & 15)))
         return VLAB200_ERR_ARG;
     // a 32-column epilogue chunk must not straddle two weight-scale groups; with one group N % 16 == 0 is enough
     if (ws_num > 1 && (N / ws_num) % 32) return VLAB200_ERR_UNSUPPORTED;
-    if (force_path == 3) return launch_gemm_pair(A, W, out, acc, s, ws, ws_num, M, N, K, st);
-    if (force_path == 0) {
-        // ns of a launch (measured back to back, 64 <= M <= 2000): set-up and epilogue, plus waves times 128-wide K steps.  Pair tiles
-        // move the fewest bytes per product and win as soon as there are enough of them; with few rows (one image, one prompt) they
-        // leave most SMs without work and narrow tiles win: 256 x 1152 x 1152 9.7 -> 7.0 us, 300 x 2560 x 2560 13.8 -> 11.3 us,
-        // 256 x 1152 (K 4352) 18.5 -> 16.0 us; 300 x 13824 x 2560 takes 22.2 us in pairs and 33.1 / 41.5 us in tiles of 128 / 64.
-        const int n_sm = sm_count(), tm = (M + 127) / 128, tp = (M + 255) / 256, ks = K / 128;
-        if (n_sm <= 0) return cuda_fail(cudaGetLastError(), "sm_count");
-        auto waves = [](int tiles, int units) { return (tiles + units - 1) / units; };
-        const int c64 = 3600 + 370 * ks * waves(tm * ((N + 63) / 64), n_sm), c128 = 4400 + 460 * ks * waves(tm * ((N + 127) / 128), n_sm);
-        const int cpair = N >= 256 && n_sm >= 2 ? 6400 + 360 * ks * waves(tp * ((N + 255) / 256), n_sm / 2) : c64 + c128;
-        if (cpair <= c64 && cpair <= c128) return launch_gemm_pair(A, W, out, acc, s, ws, ws_num, M, N, K, st);
-        if (c64 < c128) return launch_gemm_tc<64, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
-        return launch_gemm_tc<128, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
-    }
-    if (N >= 256) return launch_gemm_tc<256, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
-    return launch_gemm_tc<128, 4>(A, W, out, acc, s, ws, ws_num, M, N, K, st);
+    if (e.gate_up && (N % 64 || c.acc || e.bias)) return VLAB200_ERR_UNSUPPORTED;
+    const int n_sm = sm_count();
+    if (n_sm <= 0) return cuda_fail(cudaGetLastError(), "sm_count");
+    TernTiling t{128, 1};  // path 2
+    if (path == 0) t = choose_tiling(M, N, K, e.gate_up != 0, n_sm);
+    else if (path == 3) t = {256, 1};
+    else if ((path & 0xff) == 64 || (path & 0xff) == 128) t = {path & 0xff, (path >> 8) > 1 ? path >> 8 : 1};
+    if (t.slices != 1 && ((t.slices != 2 && t.slices != 4) || K / GEMM_BK < t.slices || e.gate_up)) return VLAB200_ERR_UNSUPPORTED;
+    if (t.bn == 256) return launch_gemm_pair(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, e, st);
+    if (t.bn == 64) return launch_gemm_tc<64>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, e, t.slices, st);
+    return launch_gemm_tc<128>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, e, t.slices, st);
+}
+
+static int ternary_linear(const int8_t *A, const uint8_t *W, void *out, int32_t *acc, const float *s, const float *ws, int ws_num, int M, int N,
+                          int K, cudaStream_t st, int path) {
+    TernaryCall c{};
+    c.A = A; c.W = W; c.out = out; c.acc = acc; c.s = s; c.ws = ws; c.ws_num = ws_num; c.M = M; c.N = N; c.K = K; c.path = path;
+    return ternary_linear(c, st);
 }
 
 // ws_num for the fused projections the reference registers (src/kernels/bitvla/bitnet_kernels.cu:31-116)
@@ -979,8 +1129,7 @@ int32_t vlab200_act_quant(const void *x_bf16, int8_t *q, float *scales, int32_t 
 int32_t vlab200_ternary_linear(const int8_t *A, const uint8_t *W_ladder, void *out_bf16, int32_t *acc_out,
                                const float *s, const float *ws, int32_t ws_num, int32_t M, int32_t N, int32_t K,
                                int32_t path, void *stream) {
-    return vb::ternary_linear(A, W_ladder, static_cast<__nv_bfloat16 *>(out_bf16), acc_out, s, ws, ws_num, M, N, K,
-                              static_cast<cudaStream_t>(stream), path);
+    return vb::ternary_linear(A, W_ladder, out_bf16, acc_out, s, ws, ws_num, M, N, K, static_cast<cudaStream_t>(stream), path);
 }
 
 // Drop-in names of the reference (src/kernels/bitvla/bitnet_kernels.cu:31,76,118).  The
@@ -1005,7 +1154,7 @@ int32_t vlab200_ternarize_pack(const float *W, int64_t N, int64_t K, uint8_t *pa
 void bitlinear_int8xint2(int8_t *input0, int8_t *input1, void *output0, float *s, float *ws, int M, int N, int K,
                          void *stream) {
     const int rc = vb::ternary_linear(input0, reinterpret_cast<const uint8_t *>(input1),
-                                      static_cast<__nv_bfloat16 *>(output0), nullptr, s, ws,
+                                      output0, nullptr, s, ws,
                                       vb::reference_ws_num(N, K), M, N, K, static_cast<cudaStream_t>(stream), 0);
     if (rc) std::fprintf(stderr, "vla_b200: bitlinear_int8xint2(M=%d,N=%d,K=%d) failed: %d %s\n", M, N, K, rc,
                          vlab200_last_error());
