@@ -38,7 +38,7 @@ namespace vb {
 // streaming kernel for wide heads / long key ranges (attn_flash.cu)
 int attention_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len,
                     int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale = 0.0f,
-                    float *ws = nullptr, size_t ws_bytes = 0);
+                    float *ws = nullptr, size_t ws_bytes = 0, int row_major_hd = 0);
 
 constexpr int ATT_SOFTMAX_WARPS = 16;
 constexpr int ATT_THREADS = (ATT_SOFTMAX_WARPS + 3) * 32;  // + loader + 2 MMA issuers
@@ -529,7 +529,7 @@ int vb::attention_ws(const vlab200_kv_store *st, int layer, const void *q, void 
     // streaming kernel spreads them over more SMs
     const bool few = ws && st->n_obs * st->n_kv * 4 <= vb::sm_count() && kv_len > 3 * 64;
     if (st->head_dim != 64 || kv_len > vb::ATT_MAX_KEYS || R > 256 || few)
-        return vb::attention_flash(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, 0.0f, ws, ws_bytes);
+        return vb::attention_flash(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, 0.0f, ws, ws_bytes, 0);
     int *status = vb::device_status_ptr();
     if (!status) return vb::cuda_fail(cudaGetLastError(), "device_status_ptr");
 

@@ -31,7 +31,9 @@ struct FlashParams {
     const int32_t *pad;
     int S, n_q, n_kv, g, kv_len, prefix_len, mask_mode, R, n_mt, n_units, n_blocks, page0;
     float scale_log2;
-    int out_al32;  // out is 32-byte aligned: 256-bit stores
+    int out_al32;  // every output row segment is 32-byte aligned: 256-bit stores
+    int out_hd;    // columns of a head in the output: HD, or the width of the heads that were zero-padded to HD (a multiple of 8)
+    int row_major; // the maps' dimensions are (column, head, row) instead of (column, row, item)
     int *status;
     // key-split mode (few work units): a unit's key blocks are cut into n_split slices that run as separate work items;
     // a slice leaves its un-normalised O rows, running maximum and row sum in the workspace for attn_split_combine_kernel
@@ -133,28 +135,26 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 const int unit = SPLIT ? wu / ns : wu, sp = SPLIT ? wu % ns : 0;
                 const int j0 = SPLIT ? sp * nb / ns : 0, j1 = SPLIT ? (sp + 1) * nb / ns : nb;
                 const int item = unit / p.n_mt, mt = unit % p.n_mt;
-                const int obs = item / p.n_kv, kvh = item % p.n_kv;
-                const int page = p.page0 + item;
-                const int qrow0 = (obs * p.n_q + kvh * p.g) * p.S + mt * 128;
+                const int page = p.page0 + item, head = item % p.n_kv, row0 = item / p.n_kv * p.S;  // the latter two: row_major
                 ok = mbar_wait(q_free, (ui & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 mbar_expect_tx(q_full, L::Q_BYTES);
-                for (int cb = 0; cb < L::CB; ++cb) tma_load_2d(smem + cb * 16384, &q_map, q_full, cb * 64, qrow0);
+                for (int cb = 0; cb < L::CB; ++cb)
+                    tma_load_3d(smem + cb * 16384, &q_map, q_full, cb * 64, p.row_major ? head : mt * 128, p.row_major ? row0 + mt * 128 : item);
                 for (int j = j0; j < j1; ++j, ++jb) {
+                    const int y = p.row_major ? head : j * FA_BKV, z = p.row_major ? row0 + j * FA_BKV : page;
                     const int st = jb & 1;
                     const uint32_t ph = (jb >> 1) & 1u;
                     ok = mbar_wait(&k_free[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                     if (!ok) break;
                     mbar_expect_tx(&k_full[st], L::KV_BYTES);
                     for (int cb = 0; cb < L::CB; ++cb)
-                        tma_load_3d(smem + L::K_OFF + st * L::KV_BYTES + cb * 8192, &k_map, &k_full[st], cb * 64,
-                                    j * FA_BKV, page);
+                        tma_load_3d(smem + L::K_OFF + st * L::KV_BYTES + cb * 8192, &k_map, &k_full[st], cb * 64, y, z);
                     ok = mbar_wait(&v_free[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                     if (!ok) break;
                     mbar_expect_tx(&v_full[st], L::KV_BYTES);
                     for (int cb = 0; cb < L::CB; ++cb)
-                        tma_load_3d(smem + L::V_OFF + st * L::KV_BYTES + cb * 8192, &v_map, &v_full[st], cb * 64,
-                                    j * FA_BKV, page);
+                        tma_load_3d(smem + L::V_OFF + st * L::KV_BYTES + cb * 8192, &v_map, &v_full[st], cb * 64, y, z);
                 }
             }
         }
@@ -363,8 +363,8 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                 continue;
             }
             const float inv = 1.0f / l_sum;
-            __nv_bfloat16 *dst = p.out + ((size_t)obs * p.S + tok) * ((size_t)p.n_q * HD) + (size_t)(kvh * p.g + head_l) * HD;
-            for (int c = 0; c < HD; c += 32) {
+            __nv_bfloat16 *dst = p.out + (((size_t)obs * p.S + tok) * p.n_q + kvh * p.g + head_l) * p.out_hd;
+            for (int c = 0; c < p.out_hd; c += 32) {
                 uint32_t ov[32];
                 tmem_ld32(tmem_base + lane_sel + (uint32_t)c, ov);
                 tmem_ld_wait();
@@ -372,6 +372,7 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 #pragma unroll
                     for (int q8 = 0; q8 < 2; ++q8) {
                         uint32_t w[8];
+                        if (c + 16 * q8 >= p.out_hd) break;
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
                             const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(ov[16 * q8 + 2 * e]) * inv,
@@ -383,7 +384,7 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
                         } else {
                             uint4 *d4 = reinterpret_cast<uint4 *>(dst + c + 16 * q8);
                             d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                            d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                            if (c + 16 * q8 + 8 < p.out_hd) d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
                         }
                     }
                 }
@@ -517,28 +518,28 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             bool ok = true;
             for (int unit = cid; ok && unit < n_units; unit += ncl, ++ui) {
                 const int item = unit / n_mt2, mt = (unit % n_mt2) * 2 + (int)rank;
-                const int obs = item / p.n_kv, kvh = item % p.n_kv;
-                const int page = p.page0 + item;
-                const int qrow0 = (obs * p.n_q + kvh * p.g) * p.S + mt * 128;
+                const int page = p.page0 + item, head = item % p.n_kv, row0 = item / p.n_kv * p.S;  // the latter two: row_major
                 ok = mbar_wait(q_free, (ui & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 mbar_expect_tx(q_full, L::Q_BYTES);
-                for (int cb = 0; cb < L::CB; ++cb) tma_load_2d(smem + cb * 16384, &q_map, q_full, cb * 64, qrow0);
+                for (int cb = 0; cb < L::CB; ++cb)
+                    tma_load_3d(smem + cb * 16384, &q_map, q_full, cb * 64, p.row_major ? head : mt * 128, p.row_major ? row0 + mt * 128 : item);
                 for (int j = 0; j < nb; ++j, ++jb) {
                     const int st = jb % FP_STAGES;
                     const uint32_t ph = (jb / FP_STAGES) & 1u;
                     ok = mbar_wait(&k_free[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                     if (!ok) break;
                     mbar_expect_tx(&k_full[st], L::K_BYTES);
+                    const int key0 = j * FP_BKV + (int)rank * (FP_BKV / 2);
                     for (int cb = 0; cb < L::CB; ++cb)
-                        tma_load_3d(smem + L::K_OFF + st * L::K_BYTES + cb * 8192, &k_map, &k_full[st], cb * 64,
-                                    j * FP_BKV + (int)rank * (FP_BKV / 2), page);
+                        tma_load_3d(smem + L::K_OFF + st * L::K_BYTES + cb * 8192, &k_map, &k_full[st], cb * 64, p.row_major ? head : key0,
+                                    p.row_major ? row0 + key0 : page);
                     ok = mbar_wait(&v_free[st], ph ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                     if (!ok) break;
                     mbar_expect_tx(&v_full[st], L::V_BYTES);
                     for (int cb = 0; cb < L::CBH; ++cb)
                         tma_load_3d(smem + L::V_OFF + st * L::V_BYTES + cb * (FP_BKV * 128), &v_map, &v_full[st],
-                                    ((int)rank * L::CBH + cb) * 64, j * FP_BKV, page);
+                                    ((int)rank * L::CBH + cb) * 64, p.row_major ? head : j * FP_BKV, p.row_major ? row0 + j * FP_BKV : page);
                 }
             }
         }
@@ -694,6 +695,7 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #pragma unroll
                     for (int q8 = 0; q8 < 2; ++q8) {
                         uint32_t w[8];
+                        if (c + 16 * q8 >= p.out_hd) break;
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
                             const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(ov[16 * q8 + 2 * e]) * inv,
@@ -705,7 +707,7 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                         } else {
                             uint4 *d4 = reinterpret_cast<uint4 *>(dst + c + 16 * q8);
                             d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                            d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                            if (c + 16 * q8 + 8 < p.out_hd) d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
                         }
                     }
                 }
@@ -843,7 +845,7 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             if (!ok) break;
             // ---- O / l -> bf16 -> out (each half stores half of the head dimension): after the next unit's first block ----
             prev_l = l_sum;
-            prev_dst = p.out + ((size_t)obs * p.S + tok) * ((size_t)p.n_q * HD) + (size_t)(kvh * p.g + head_l) * HD;
+            prev_dst = p.out + (((size_t)obs * p.S + tok) * p.n_q + kvh * p.g + head_l) * p.out_hd;
             prev_row_ok = row_ok;
             pad_lo = pad_lo_n;
             pad_hi = pad_hi_n;
@@ -896,20 +898,30 @@ __global__ void __launch_bounds__(256) attn_split_combine_kernel(const FlashPara
 template <int HD>
 static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len,
                         int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws,
-                        size_t ws_bytes) {
+                        size_t ws_bytes, int row_major_hd) {
     using L = FlashSmem<HD>;
     int *status = device_status_ptr();
     if (!status) return cuda_fail(cudaGetLastError(), "device_status_ptr");
     CUtensorMap qmap, kmap, vmap;
+    // row_major_hd: q, k and v are column ranges of one [n_obs S][3 n_q row_major_hd] matrix; columns past a head are outside the map
+    const uint64_t rdims[3] = {(uint64_t)row_major_hd, (uint64_t)n_q, (uint64_t)st->n_obs * S};
+    const uint64_t rstrides[2] = {(uint64_t)row_major_hd * 2, (uint64_t)3 * n_q * row_major_hd * 2};
     {
-        const uint64_t dims[2] = {(uint64_t)HD, (uint64_t)st->n_obs * n_q * S};
-        const uint64_t strides[1] = {(uint64_t)HD * 2};
-        const uint32_t box[2] = {64, 128};
-        int rc = make_tensor_map(&qmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, dims, strides, box,
-                                 CU_TENSOR_MAP_SWIZZLE_128B);
+        // an item's g * S stacked query rows; rows past them are outside the map
+        const uint64_t R = (uint64_t)(n_q / st->n_kv) * S;
+        const uint64_t dims[3] = {(uint64_t)HD, R, (uint64_t)st->n_obs * st->n_kv};
+        const uint64_t strides[2] = {(uint64_t)HD * 2, R * HD * 2};
+        const uint32_t box[3] = {64, 128, 1}, rbox[3] = {64, 1, 128};
+        int rc = make_tensor_map(&qmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, q, row_major_hd ? rdims : dims, row_major_hd ? rstrides : strides,
+                                 row_major_hd ? rbox : box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }
-    {
+    if (row_major_hd) {
+        const uint32_t box[3] = {64, 1, FA_BKV};
+        int rc = make_tensor_map(&kmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, st->k_pages, rdims, rstrides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (!rc) rc = make_tensor_map(&vmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, st->v_pages, rdims, rstrides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (rc) return rc;
+    } else {
         // rows >= kv_len are outside the map: TMA zero-fills them
         const uint64_t dims[3] = {(uint64_t)HD, (uint64_t)kv_len, (uint64_t)st->n_layers * st->n_obs * st->n_kv};
         const uint64_t strides[2] = {(uint64_t)HD * 2, (uint64_t)st->cap * HD * 2};
@@ -933,7 +945,9 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
     p.page0 = layer * st->n_obs * st->n_kv;
     // softmax_scale > 0 replaces 1 / sqrt(HD): heads narrower than HD that were zero-padded to it
     p.scale_log2 = 1.4426950408889634f * (softmax_scale > 0.0f ? softmax_scale : 1.0f / sqrtf((float)HD));
-    p.out_al32 = (reinterpret_cast<uintptr_t>(out) & 31) == 0 ? 1 : 0;
+    p.row_major = row_major_hd > 0 ? 1 : 0;
+    p.out_hd = row_major_hd > 0 ? row_major_hd : HD;
+    p.out_al32 = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && p.out_hd % 16 == 0 ? 1 : 0;
     p.status = status;
     const int n_sm = sm_count();
     if constexpr (HD >= 128) {
@@ -947,9 +961,9 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
             CUtensorMap vmap128;
             const uint64_t dims[3] = {(uint64_t)HD, (uint64_t)kv_len, (uint64_t)st->n_layers * st->n_obs * st->n_kv};
             const uint64_t strides[2] = {(uint64_t)HD * 2, (uint64_t)st->cap * HD * 2};
-            const uint32_t box[3] = {64, FP_BKV, 1};
-            int rc = make_tensor_map(&vmap128, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, st->v_pages, dims, strides, box,
-                                     CU_TENSOR_MAP_SWIZZLE_128B);
+            const uint32_t box[3] = {64, FP_BKV, 1}, rbox[3] = {64, 1, FP_BKV};
+            int rc = make_tensor_map(&vmap128, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, st->v_pages, row_major_hd ? rdims : dims,
+                                     row_major_hd ? rstrides : strides, row_major_hd ? rbox : box, CU_TENSOR_MAP_SWIZZLE_128B);
             if (rc) return rc;
             if ((rc = ensure_dyn_smem(attn_flash_pair_kernel<HD>, LP::TOTAL))) return rc;
             const int ncl = n_pair_units < pairs ? n_pair_units : pairs;
@@ -957,7 +971,7 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
         }
     }
     p.n_split = 1;
-    if (ws && p.n_units * 2 <= n_sm && p.n_blocks >= 4) {
+    if (ws && !p.row_major && p.n_units * 2 <= n_sm && p.n_blocks >= 4) {
         // few units (one observation): cut every unit's keys into slices of at least two 64-key blocks so that the slices fill
         // the machine, then merge them (flash-decoding)
         int n_split = n_sm / p.n_units;
@@ -982,13 +996,16 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
 
 int attention_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len,
                     int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws,
-                    size_t ws_bytes) {
+                    size_t ws_bytes, int row_major_hd) {
+    // a key block may reach into the next observation's rows (hidden, but multiplied by 0): several need whole blocks
+    if (row_major_hd && (row_major_hd % 8 || row_major_hd > st->head_dim || n_q != st->n_kv || kv_len != S || (st->n_obs > 1 && S % FP_BKV)))
+        return VLAB200_ERR_UNSUPPORTED;
     if (st->head_dim == 256)
-        return launch_flash<256>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes);
+        return launch_flash<256>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes, row_major_hd);
     if (st->head_dim == 128)
-        return launch_flash<128>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes);
+        return launch_flash<128>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes, row_major_hd);
     if (st->head_dim == 64)
-        return launch_flash<64>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes);
+        return launch_flash<64>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes, row_major_hd);
     return VLAB200_ERR_UNSUPPORTED;
 }
 

@@ -16,8 +16,8 @@
 //   norm_quant_kernel   attn sub-norm -> int8
 //   ternary GEMM        o
 //   norm_quant_kernel   h += o; ffn norm -> int8
-//   ternary GEMM        gate_up
-//   norm_quant_kernel   relu(gate)^2 * up -> ffn sub-norm -> int8
+//   ternary GEMM        gate_up, relu(gate)^2 * up in its epilogue
+//   norm_quant_kernel   ffn sub-norm -> int8
 //   ternary GEMM        down   (its residual add is fused into the next norm_quant_kernel)
 //
 // Sequences of equal length can be batched (n_seq); the reference runs one per call.
@@ -33,6 +33,7 @@
 
 #include "gemm.h"
 #include "host_common.h"
+#include "quant8.cuh"
 #include "tc5.cuh"
 
 namespace vb {
@@ -138,12 +139,18 @@ __global__ void __launch_bounds__(256) norm_quant_vec_kernel(__nv_bfloat16 *__re
                                                              const __nv_bfloat16 *__restrict__ add,
                                                              const __nv_bfloat16 *__restrict__ w, float eps, int K,
                                                              int8_t *__restrict__ q_out, float *__restrict__ s_out,
-                                                             __nv_bfloat16 *__restrict__ out_bf) {
+                                                             __nv_bfloat16 *__restrict__ out_bf, int w_early) {
     __shared__ float red[8];
-    pdl_launch_dependents();
-    pdl_wait();
     const int m = blockIdx.x, tid = threadIdx.x;
     const int K8 = K >> 3;
+    // the norm's weights: ahead of the kernel in front where they cannot be its output (w_early)
+    uint4 wv[NV];
+    if (!w_early) pdl_wait();
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+        if (tid + v * 256 < K8) wv[v] = __ldg(reinterpret_cast<const uint4 *>(w) + tid + v * 256);
+    pdl_launch_dependents();
+    if (w_early) pdl_wait();
     const size_t ld = MODE == NQ_GATE_UP ? 2 * (size_t)K : (size_t)K;
     uint4 *src = reinterpret_cast<uint4 *>(in + m * ld);
     uint4 x[NV];
@@ -191,8 +198,7 @@ __global__ void __launch_bounds__(256) norm_quant_vec_kernel(__nv_bfloat16 *__re
     for (int v = 0; v < NV; ++v) {
         const int i = tid + v * 256;
         if (i >= K8) break;
-        const uint4 wv = __ldg(reinterpret_cast<const uint4 *>(w) + i);
-        const uint32_t *ww = reinterpret_cast<const uint32_t *>(&wv);
+        const uint32_t ww[4] = {wv[v].x, wv[v].y, wv[v].z, wv[v].w};
         uint32_t *xw = reinterpret_cast<uint32_t *>(&x[v]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -215,16 +221,7 @@ __global__ void __launch_bounds__(256) norm_quant_vec_kernel(__nv_bfloat16 *__re
     for (int v = 0; v < NV; ++v) {
         const int i = tid + v * 256;
         if (i >= K8) break;
-        const uint32_t *xw = reinterpret_cast<const uint32_t *>(&x[v]);
-        uint32_t o[2] = {0u, 0u};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 yf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
-            const int a = (int)fminf(fmaxf(rintf(yf.x * qs), -128.f), 127.f);
-            const int b = (int)fminf(fmaxf(rintf(yf.y * qs), -128.f), 127.f);
-            o[e >> 1] |= ((uint32_t)(a & 0xff) | ((uint32_t)(b & 0xff) << 8)) << (16 * (e & 1));
-        }
-        dst[i] = make_uint2(o[0], o[1]);
+        dst[i] = quant8_bf16(x[v], qs);
     }
 }
 
@@ -458,14 +455,14 @@ namespace vb {
 
 template <int MODE>
 static int launch_norm_quant(void *in, const void *add, const void *w, float eps, int M, int K, int8_t *q, float *s,
-                             void *out_bf, cudaStream_t st) {
+                             void *out_bf, cudaStream_t st, int w_early = 0) {
     auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     __nv_bfloat16 *in_b = static_cast<__nv_bfloat16 *>(in);
     const __nv_bfloat16 *add_b = static_cast<const __nv_bfloat16 *>(add), *w_b = static_cast<const __nv_bfloat16 *>(w);
     __nv_bfloat16 *out_b = static_cast<__nv_bfloat16 *>(out_bf);
     if (K % 8 == 0 && K <= 8192 && al16(in) && al16(add) && al16(w) && al16(out_bf) && (reinterpret_cast<uintptr_t>(q) & 7) == 0) {
-        if (K <= 4096) return launch_pdl(norm_quant_vec_kernel<MODE, 2>, dim3(M), dim3(256), 0, st, in_b, add_b, w_b, eps, K, q, s, out_b);
-        return launch_pdl(norm_quant_vec_kernel<MODE, 4>, dim3(M), dim3(256), 0, st, in_b, add_b, w_b, eps, K, q, s, out_b);
+        if (K <= 4096) return launch_pdl(norm_quant_vec_kernel<MODE, 2>, dim3(M), dim3(256), 0, st, in_b, add_b, w_b, eps, K, q, s, out_b, w_early);
+        return launch_pdl(norm_quant_vec_kernel<MODE, 4>, dim3(M), dim3(256), 0, st, in_b, add_b, w_b, eps, K, q, s, out_b, w_early);
     }
     const size_t smem = (size_t)K * 4;
     if (smem > 48 * 1024)
@@ -578,18 +575,30 @@ extern "C" int32_t vlab200_bitvla_lm_forward(vlab200_bitvla_lm *ctx, const void 
     // :523), so the two stacks can be compared stage by stage.  A debugging path: it synchronises, allocates and
     // runs the normalisations a second time without their fused quantisation.
     vb::L0Dump dump(n_seq == 1 ? std::getenv("VLA_BITVLA_DUMP_L0") : nullptr, st, (size_t)M * (size_t)(F > hq ? (F > H ? F : H) : (hq > H ? hq : H)));
+    // the weights were complete before the copy above: the kernels below read them ahead of the kernel in front of them
+    auto linear = [&](const void *packed, void *out, const float *ws, int ws_num, int N, int K, int gate_up) {
+        vb::TernaryCall c{};
+        c.A = a8; c.W = static_cast<const uint8_t *>(packed); c.out = out; c.s = s; c.ws = ws; c.ws_num = ws_num; c.M = M; c.N = N; c.K = K;
+        c.gate_up = gate_up; c.w_early = 1;
+        return vb::ternary_linear(c, st);
+    };
+    // relu(gate)^2 * up in the product's epilogue (the GEMV of a few tokens has none): half of the gate_up traffic in both directions
+    const int fused = M > 8 ? 1 : 0;
     for (int L = 0; L < ctx->n_layers && !rc; ++L) {
         const vb::LmLayer &l = ctx->layers[L];
+        auto sub_norm = [&](int8_t *q, float *sc, void *y) {
+            if (fused) return vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->gate_up.p, nullptr, l.w.ffn_sub_norm_w, ctx->eps, M, F, q, sc, y, st, 1);
+            return vb::launch_norm_quant<vb::NQ_GATE_UP>(ctx->gate_up.p, nullptr, l.w.ffn_sub_norm_w, ctx->eps, M, F, q, sc, y, st, 1);
+        };
         const bool dl = dump.on() && L == 0;
         if (dl) {
             vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->h.p, nullptr, l.w.attn_norm_w, ctx->eps, M, H, nullptr, nullptr, dump.tmp.p, st);
             dump.write("L0_01_attn_norm", dump.tmp.p, (size_t)M * H);
         }
-        if (L == 0) rc = vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->h.p, nullptr, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st);
-        else rc = vb::launch_norm_quant<vb::NQ_ADD>(ctx->h.p, ctx->proj.p, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st);
+        if (L == 0) rc = vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->h.p, nullptr, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st, 1);
+        else rc = vb::launch_norm_quant<vb::NQ_ADD>(ctx->h.p, ctx->proj.p, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st, 1);
         if (rc) break;
-        rc = vlab200_ternary_linear(a8, l.qkv_packed.as<uint8_t>(), ctx->qkv.p, nullptr, s, l.qkv_ws.as<float>(),
-                                    ctx->qkv_ws_num, M, hq + 2 * hkv, H, 0, st);
+        rc = linear(l.qkv_packed.p, ctx->qkv.p, l.qkv_ws.as<float>(), ctx->qkv_ws_num, hq + 2 * hkv, H, 0);
         if (rc) break;
         if (dl) dump.write_qkv("L0_02_qkv_proj", ctx->qkv.p, M, hq, hkv);
         rc = vb::rope_split(ctx->qkv.p, ctx->cos_t.as<float>(), ctx->sin_t.as<float>(), ctx->q.p, ctx->k_pages.p,
@@ -602,30 +611,27 @@ extern "C" int32_t vlab200_bitvla_lm_forward(vlab200_bitvla_lm *ctx, const void 
             vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->att.p, nullptr, l.w.attn_sub_norm_w, ctx->eps, M, hq, nullptr, nullptr, dump.tmp.p, st);
             dump.write("L0_04_attn_sub_norm", dump.tmp.p, (size_t)M * hq);
         }
-        rc = vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->att.p, nullptr, l.w.attn_sub_norm_w, ctx->eps, M, hq, a8, s, nullptr, st);
+        rc = vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->att.p, nullptr, l.w.attn_sub_norm_w, ctx->eps, M, hq, a8, s, nullptr, st, 1);
         if (rc) break;
-        rc = vlab200_ternary_linear(a8, static_cast<const uint8_t *>(l.w.o_packed), ctx->proj.p, nullptr, s,
-                                    static_cast<const float *>(l.w.o_ws), 1, M, H, hq, 0, st);
+        rc = linear(l.w.o_packed, ctx->proj.p, l.w.o_ws, 1, H, hq, 0);
         if (rc) break;
         if (dl) dump.write("L0_05_o_proj_out", ctx->proj.p, (size_t)M * H);
-        rc = vb::launch_norm_quant<vb::NQ_ADD>(ctx->h.p, ctx->proj.p, l.w.ffn_norm_w, ctx->eps, M, H, a8, s, nullptr, st);
+        rc = vb::launch_norm_quant<vb::NQ_ADD>(ctx->h.p, ctx->proj.p, l.w.ffn_norm_w, ctx->eps, M, H, a8, s, nullptr, st, 1);
         if (rc) break;
         if (dl) {
             dump.write("L0_06_after_attn_residual", ctx->h.p, (size_t)M * H);
             vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->h.p, nullptr, l.w.ffn_norm_w, ctx->eps, M, H, nullptr, nullptr, dump.tmp.p, st);
             dump.write("L0_07_ffn_norm", dump.tmp.p, (size_t)M * H);
         }
-        rc = vlab200_ternary_linear(a8, static_cast<const uint8_t *>(l.w.gate_up_packed), ctx->gate_up.p, nullptr, s,
-                                    static_cast<const float *>(l.w.gate_up_ws), 2, M, 2 * F, H, 0, st);
+        rc = linear(l.w.gate_up_packed, ctx->gate_up.p, l.w.gate_up_ws, 2, 2 * F, H, fused);
         if (rc) break;
         if (dl) {
-            vb::launch_norm_quant<vb::NQ_GATE_UP>(ctx->gate_up.p, nullptr, l.w.ffn_sub_norm_w, ctx->eps, M, F, nullptr, nullptr, dump.tmp.p, st);
+            sub_norm(nullptr, nullptr, dump.tmp.p);
             dump.write("L0_08_ffn_sub_norm", dump.tmp.p, (size_t)M * F);
         }
-        rc = vb::launch_norm_quant<vb::NQ_GATE_UP>(ctx->gate_up.p, nullptr, l.w.ffn_sub_norm_w, ctx->eps, M, F, a8, s, nullptr, st);
+        rc = sub_norm(a8, s, nullptr);
         if (rc) break;
-        rc = vlab200_ternary_linear(a8, static_cast<const uint8_t *>(l.w.down_packed), ctx->proj.p, nullptr, s,
-                                    static_cast<const float *>(l.w.down_ws), 1, M, H, F, 0, st);
+        rc = linear(l.w.down_packed, ctx->proj.p, l.w.down_ws, 1, H, F, 0);
         if (dl && !rc) {
             dump.write("L0_09_down_out", ctx->proj.p, (size_t)M * H);
             dump.write_sum("L0_10_final", ctx->h.p, ctx->proj.p, (size_t)M * H);  // the residual add is fused into the next stage
@@ -634,7 +640,7 @@ extern "C" int32_t vlab200_bitvla_lm_forward(vlab200_bitvla_lm *ctx, const void 
     if (rc) return rc;
     // h += down of the last layer, then the output norm (bitvla_lm_cuda.cu:718)
     return vb::launch_norm_quant<vb::NQ_ADD>(ctx->h.p, ctx->proj.p, ctx->output_norm, ctx->eps, M, H, nullptr, nullptr,
-                                             d_out, st);
+                                             d_out, st, 1);
 }
 
 // The reference's own names and signatures for the context API (src/kernels/bitvla/bitvla_lm_cuda.h:247-286),

@@ -17,6 +17,9 @@
 //   vit_gelu_quant_kernel    + bias -> tanh-GELU -> bf16, zero-padded to a multiple of 128 -> act-quant
 //   ternary GEMM             fc2   (its bias and residual add are fused into the next vit_ln_quant_kernel)
 //
+// and, where rows, heads and alignments allow 16-byte accesses (`fast` in the forward), 9: the biases and the GELU in the products' epilogues,
+// the attention straight from the q | k | v matrix (no head split, no merge), row kernels with the row in registers.
+//
 // Every value the reference stores as bf16 is rounded to bf16 here too, in the same order; the patch embedding and the
 // projector run on the bf16 tcgen05 GEMM with the bias (and erf-GELU) in the epilogue.
 #include <cuda_bf16.h>
@@ -28,12 +31,14 @@
 
 #include "gemm.h"
 #include "host_common.h"
+#include "quant8.cuh"
 #include "tc5.cuh"
 
 namespace vb {
 
 int attention_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len,
-                    int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws, size_t ws_bytes);
+                    int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws, size_t ws_bytes,
+                    int row_major_hd);
 
 __device__ __forceinline__ float vit_block_sum(float v, float *red) {
 #pragma unroll
@@ -206,6 +211,156 @@ __global__ void __launch_bounds__(256) vit_gelu_quant_kernel(const __nv_bfloat16
     vit_quant_row(row, amax, F_pad, q_out + (size_t)m * F_pad, s_out + m, red);
 }
 
+// ---- the row stages with 16-byte accesses and rows in registers: the usual route (`fast` below) ----
+__device__ __forceinline__ float2 vit_f2(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w)); }
+__device__ __forceinline__ uint32_t vit_pack(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ float vit_amax8(const uint4 &y, float amax) {
+    const uint32_t w[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 f = vit_f2(w[e]);
+        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+    return amax;
+}
+
+// The sum that vit_block_sum gives for a row of which thread t of its block of 256 holds columns t, t + 256, ..., from a block whose
+// thread 32 w + L holds columns 8 (32 w + L) .. + 7 in x: the same additions in the same order (SQ: of the squares), so both kernels give
+// the same bits.  (The columns of one thread there are those of lane L of every warp here, in the order of the warps.)
+template <bool SQ>
+__device__ __forceinline__ float vit_row_sum(const float (&x)[8], int n_warps, float4 *part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    part[(warp * 2) * 32 + lane] = make_float4(x[0], x[1], x[2], x[3]);
+    part[(warp * 2 + 1) * 32 + lane] = make_float4(x[4], x[5], x[6], x[7]);
+    __syncthreads();
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int w = 0; w < n_warps; ++w) {
+        const float4 a = part[(w * 2) * 32 + lane], b = part[(w * 2 + 1) * 32 + lane];
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] = SQ ? fmaf(v[e], v[e], s[e]) : s[e] + v[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        s[e] += __shfl_xor_sync(0xffffffffu, s[e], 2);
+        s[e] += __shfl_xor_sync(0xffffffffu, s[e], 1);
+    }
+    const float v = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+    float t = __shfl_sync(0xffffffffu, v, 0);
+#pragma unroll
+    for (int w = 1; w < 8; ++w) t += __shfl_sync(0xffffffffu, v, 4 * w);
+    return t;
+}
+
+// vit_ln_quant_kernel with 8 columns a thread in registers (K % 8 == 0, K <= 8 x 32 x VIT_LN_WARPS, just enough warps for a row) and the weights
+// read before the dependency wait (nothing that may still run writes them).  With a whole row in one warp the 1,200 instructions of a
+// lane took longer than the block barriers it saved (5.5 us inside the tower, the scalar kernel 5.0).
+constexpr int VIT_LN_WARPS = 8;
+__global__ void __launch_bounds__(32 * VIT_LN_WARPS) vit_ln_quant_rows_kernel(__nv_bfloat16 *__restrict__ h, const __nv_bfloat16 *__restrict__ add,
+                                                                              const __nv_bfloat16 *__restrict__ add_bias,
+                                                                              const __nv_bfloat16 *__restrict__ ln_w,
+                                                                              const __nv_bfloat16 *__restrict__ ln_b, float eps, int K,
+                                                                              int8_t *__restrict__ q_out, float *__restrict__ s_out) {
+    __shared__ float4 part[2][VIT_LN_WARPS * 2 * 32];
+    __shared__ float red[VIT_LN_WARPS];
+    const int m = blockIdx.x, i = threadIdx.x, n_warps = blockDim.x >> 5;
+    const bool in = i < K >> 3;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    uint4 lw = zero, lb = zero, ab = zero, x = zero, av = zero;
+    if (in) {
+        if (ln_w) {
+            lw = __ldg(reinterpret_cast<const uint4 *>(ln_w) + i);
+            lb = __ldg(reinterpret_cast<const uint4 *>(ln_b) + i);
+        }
+        if (add) ab = __ldg(reinterpret_cast<const uint4 *>(add_bias) + i);
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    uint4 *hr = reinterpret_cast<uint4 *>(h + (size_t)m * K);
+    if (in) {
+        x = hr[i];
+        if (add) av = reinterpret_cast<const uint4 *>(add + (size_t)m * K)[i];
+    }
+    uint32_t *xw = reinterpret_cast<uint32_t *>(&x);
+    if (add) {
+        const uint32_t aw[4] = {av.x, av.y, av.z, av.w}, bw[4] = {ab.x, ab.y, ab.z, ab.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 a = vit_f2(aw[e]), b = vit_f2(bw[e]), r = vit_f2(xw[e]);
+            const float2 o = vit_f2(vit_pack(a.x + b.x, a.y + b.y));
+            xw[e] = vit_pack(r.x + o.x, r.y + o.y);
+        }
+        if (in) hr[i] = x;
+    }
+    if (!ln_w) return;
+    float f[8], t[8];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 v = vit_f2(xw[e]);
+        f[2 * e] = v.x;
+        f[2 * e + 1] = v.y;
+    }
+    const float mean = vit_row_sum<false>(f, n_warps, part[0]) / (float)K;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        f[e] -= mean;
+        t[e] = in ? f[e] : 0.f;
+    }
+    const float inv_std = rsqrtf(vit_row_sum<true>(t, n_warps, part[1]) / (float)K + eps);
+    const uint32_t ww[4] = {lw.x, lw.y, lw.z, lw.w}, bw[4] = {lb.x, lb.y, lb.z, lb.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 w = vit_f2(ww[e]), b = vit_f2(bw[e]);
+        xw[e] = vit_pack(fmaf(f[2 * e] * inv_std, w.x, b.x), fmaf(f[2 * e + 1] * inv_std, w.y, b.y));
+    }
+    float amax = in ? vit_amax8(x, 0.f) : 0.f;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    if ((i & 31) == 0) red[i >> 5] = amax;
+    __syncthreads();
+    for (int w = 0; w < n_warps; ++w) amax = fmaxf(amax, red[w]);
+    amax = amax < 1e-5f ? 1e-5f : amax;
+    const float qs = __fdiv_rn(127.0f, amax);
+    if (i == 0) s_out[m] = qs;
+    if (in) reinterpret_cast<uint2 *>(q_out + (size_t)m * K)[i] = quant8_bf16(x, qs);
+}
+
+// Act-quant of a row of K columns into K_pad int8 (zero past K), WARPS warps per row and NV x 8 columns per lane.
+template <int WARPS, int NV>
+__global__ void __launch_bounds__(32 * WARPS) vit_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int K, int K_pad,
+                                                                    int8_t *__restrict__ q_out, float *__restrict__ s_out) {
+    __shared__ float red[WARPS];
+    constexpr int T = 32 * WARPS;
+    const int m = blockIdx.x, t = threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint4 *xr = reinterpret_cast<const uint4 *>(x + (size_t)m * K);
+    uint4 v[NV];
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = t + T * i < K >> 3 ? xr[t + T * i] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) amax = vit_amax8(v[i], amax);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    if ((t & 31) == 0) red[t >> 5] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < WARPS; ++i) amax = fmaxf(amax, red[i]);
+    amax = amax < 1e-5f ? 1e-5f : amax;
+    const float qs = __fdiv_rn(127.0f, amax);
+    if (t == 0) s_out[m] = qs;
+    uint2 *dst = reinterpret_cast<uint2 *>(q_out + (size_t)m * K_pad);
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+        if (t + T * i < K_pad >> 3) dst[t + T * i] = quant8_bf16(v[i], qs);
+}
+constexpr int VIT_Q_WARPS = 5;                     // rows of the attention: up to 1280 columns, 8 a thread
+constexpr int VIT_FFN_WARPS = 12, VIT_FFN_NV = 2;  // rows of the MLP: up to 6144 columns
+
 // h = bf16(bf16(h + patch_b[k]) + pos[m][k])  (bitvla_vit_cuda.cu:283-284)
 __global__ void vit_embed_finish_kernel(__nv_bfloat16 *__restrict__ h, const __nv_bfloat16 *__restrict__ patch_b,
                                         const __nv_bfloat16 *__restrict__ pos, int H, size_t total) {
@@ -231,7 +386,7 @@ __global__ void vit_bf16_to_f32_kernel(const __nv_bfloat16 *__restrict__ src, fl
 
 struct VitLayer {
     bitvla_vit_layer_cuda w{};
-    DevBuf qkv_packed, qkv_ws;
+    DevBuf qkv_packed, qkv_ws, qkv_b;
     bool set = false;
 };
 
@@ -291,6 +446,7 @@ bitvla_vit_cuda_ctx *bitvla_vit_cuda_init(int n_layers, int hidden, int n_heads,
     for (int l = 0; l < n_layers && !rc; ++l) {
         rc = c->layers[(size_t)l].qkv_packed.alloc(3 * H * H / 4);
         if (!rc) rc = c->layers[(size_t)l].qkv_ws.alloc(3 * sizeof(float));
+        if (!rc) rc = c->layers[(size_t)l].qkv_b.alloc(3 * H * 2);
     }
     if (rc) {
         delete c;
@@ -313,10 +469,13 @@ void bitvla_vit_cuda_set_layer(bitvla_vit_cuda_ctx *ctx, int L, const bitvla_vit
     const size_t bytes = (size_t)ctx->hidden * ctx->hidden / 4;
     const int8_t *packs[3] = {layer->q_packed, layer->k_packed, layer->v_packed};
     const float *wss[3] = {layer->q_ws, layer->k_ws, layer->v_ws};
+    const void *bias[3] = {layer->q_b, layer->k_b, layer->v_b};
+    const size_t bias_bytes = (size_t)ctx->hidden * 2;
     bool ok = true;
     for (int j = 0; j < 3; ++j) {
         ok = ok && cudaMemcpy(static_cast<char *>(dst.qkv_packed.p) + j * bytes, packs[j], bytes, cudaMemcpyDeviceToDevice) == cudaSuccess;
         ok = ok && cudaMemcpy(dst.qkv_ws.as<float>() + j, wss[j], sizeof(float), cudaMemcpyDeviceToDevice) == cudaSuccess;
+        ok = ok && cudaMemcpy(static_cast<char *>(dst.qkv_b.p) + j * bias_bytes, bias[j], bias_bytes, cudaMemcpyDeviceToDevice) == cudaSuccess;
     }
     if (!ok) {
         vb::cuda_fail(cudaGetLastError(), "bitvla_vit_cuda_set_layer");
@@ -385,10 +544,48 @@ int bitvla_vit_cuda_forward(bitvla_vit_cuda_ctx *ctx, const void *d_patches, voi
         if ((rc = vb::ensure_dyn_smem(vb::vit_merge_quant_kernel, (int)row_smem))) return fail("shared memory", rc);
     }
     const __nv_bfloat16 *pend = nullptr, *pend_bias = nullptr;  // a projection whose bias + residual add is still due
-    for (int L = 0; L < ctx->n_layers; ++L) {
+    const auto bf = [](const void *p) { return static_cast<const __nv_bfloat16 *>(p); };
+    // The route with 16-byte accesses needs whole 8-column groups, rows that fit the registers, aligned vectors and more rows than the
+    // GEMV takes (its epilogue adds no bias).
+    bool fast = hd % 8 == 0 && H <= 256 * vb::VIT_Q_WARPS && F % 8 == 0 && FP <= 256 * vb::VIT_FFN_WARPS * vb::VIT_FFN_NV && S > 8;
+    for (const vb::VitLayer &l : ctx->layers)
+        for (const void *p : {l.w.ln1_w, l.w.ln1_b, l.w.ln2_w, l.w.ln2_b, l.w.o_b, l.w.fc2_b}) fast = fast && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+    // weights were complete before the embedding kernels above started: the layers' kernels read them ahead of the kernel in front
+    auto ternary = [&](const int8_t *a, const void *wp, const float *ws, int ws_num, void *out, int N, int K, const void *bias, int gelu) {
+        vb::TernaryCall c{};
+        c.A = a; c.W = static_cast<const uint8_t *>(wp); c.out = out; c.s = s; c.ws = ws; c.ws_num = ws_num; c.M = S; c.N = N; c.K = K;
+        c.bias = bias; c.gelu = gelu; c.w_early = 1;
+        return vb::ternary_linear(c, cs);
+    };
+    for (int L = 0; fast && L < ctx->n_layers; ++L) {
         const vb::VitLayer &lr = ctx->layers[(size_t)L];
         const bitvla_vit_layer_cuda &w = lr.w;
-        const auto bf = [](const void *p) { return static_cast<const __nv_bfloat16 *>(p); };
+        auto ln = [&](const __nv_bfloat16 *add, const __nv_bfloat16 *add_b, const void *lw, const void *lb) {
+            return vb::launch_pdl(vb::vit_ln_quant_rows_kernel, dim3(S), dim3((unsigned)(H / 8 + 31) / 32 * 32), 0, cs, h, add, add_b, bf(lw), bf(lb),
+                                  ctx->ln_eps, H, a8, s);
+        };
+        if ((rc = ln(pend, pend_bias, w.ln1_w, w.ln1_b))) return fail("ln1", rc);
+        if ((rc = ternary(a8, lr.qkv_packed.p, lr.qkv_ws.as<float>(), 3, ctx->qkv.p, 3 * H, H, lr.qkv_b.p, 0))) return fail("qkv projection", rc);
+        // the attention reads q, k and v as column ranges of the projection and leaves packed heads: no head split, no merge
+        __nv_bfloat16 *qkv = ctx->qkv.as<__nv_bfloat16>();
+        vlab200_kv_store view{qkv + H, qkv + 2 * H, 1, 1, heads, hp, S, 0};
+        if ((rc = vb::attention_flash(&view, 0, qkv, ctx->att.p, S, heads, S, 0, nullptr, cs, scale, nullptr, 0, hd))) return fail("attention", rc);
+        if ((rc = vb::launch_pdl(vb::vit_quant_rows_kernel<vb::VIT_Q_WARPS, 1>, dim3(S), dim3(32 * vb::VIT_Q_WARPS), 0, cs, ctx->att.as<__nv_bfloat16>(),
+                                 H, H, a8, s)))
+            return fail("attention quantisation", rc);
+        if ((rc = ternary(a8, w.o_packed, w.o_ws, 1, proj, H, H, nullptr, 0))) return fail("o projection", rc);
+        if ((rc = ln(proj, bf(w.o_b), w.ln2_w, w.ln2_b))) return fail("ln2", rc);
+        if ((rc = ternary(a8, w.fc1_packed, w.fc1_ws, 1, ctx->fc1.p, F, H, w.fc1_b, 1))) return fail("fc1", rc);
+        if ((rc = vb::launch_pdl(vb::vit_quant_rows_kernel<vb::VIT_FFN_WARPS, vb::VIT_FFN_NV>, dim3(S), dim3(32 * vb::VIT_FFN_WARPS), 0, cs,
+                                 ctx->fc1.as<__nv_bfloat16>(), F, FP, a8f, s)))
+            return fail("fc1 quantisation", rc);
+        if ((rc = ternary(a8f, w.fc2_packed, w.fc2_ws, 1, proj, H, FP, nullptr, 0))) return fail("fc2", rc);
+        pend = proj;
+        pend_bias = bf(w.fc2_b);
+    }
+    for (int L = 0; !fast && L < ctx->n_layers; ++L) {
+        const vb::VitLayer &lr = ctx->layers[(size_t)L];
+        const bitvla_vit_layer_cuda &w = lr.w;
         if ((rc = vb::launch_pdl(vb::vit_ln_quant_kernel, dim3(S), dim3(256), (size_t)H * 4, cs, h, pend, pend_bias, bf(w.ln1_w),
                                  bf(w.ln1_b), ctx->ln_eps, H, a8, s)))
             return fail("ln1", rc);
@@ -398,7 +595,7 @@ int bitvla_vit_cuda_forward(bitvla_vit_cuda_ctx *ctx, const void *d_patches, voi
                                  bf(w.v_b), ctx->q.as<__nv_bfloat16>(), ctx->kp.as<__nv_bfloat16>(), ctx->vp.as<__nv_bfloat16>(), S, heads, hd, hp)))
             return fail("head split", rc);
         vlab200_kv_store view{ctx->kp.p, ctx->vp.p, 1, 1, heads, hp, S, 0};
-        if ((rc = vb::attention_flash(&view, 0, ctx->q.p, ctx->att.p, S, heads, S, 0, nullptr, cs, scale, nullptr, 0))) return fail("attention", rc);
+        if ((rc = vb::attention_flash(&view, 0, ctx->q.p, ctx->att.p, S, heads, S, 0, nullptr, cs, scale, nullptr, 0, 0))) return fail("attention", rc);
         if ((rc = vb::launch_pdl(vb::vit_merge_quant_kernel, dim3(S), dim3(256), (size_t)H * 4, cs, ctx->att.as<__nv_bfloat16>(), heads, hd,
                                  hp, a8, s)))
             return fail("merge", rc);
