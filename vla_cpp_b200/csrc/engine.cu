@@ -177,7 +177,6 @@ __global__ void pages_to_f32_kernel(const __nv_bfloat16 *__restrict__ pages, flo
 }
 
 constexpr int kFewRows = 256;  // suffix rows (n_obs * S) up to which the QKV projection takes the narrow-tile path
-constexpr int kFewRowSlices = 8;  // most K slices of a residual GEMM with few rows
 // key-split attention: at most one (unit, slice) per SM, 128 rows of head_dim + 2 floats each
 static size_t kAttnWsBytes(int hd) { return (size_t)160 * 128 * (hd + 2) * sizeof(float); }
 }
@@ -192,7 +191,6 @@ struct vlab200_engine {
     std::vector<vb::DevBuf> wqkv, wo, wgu, wdown, wkx, wvx;
     vb::DevBuf w_ain, b_ain, w_sp, b_sp, w_at1l, tvec, w_at2, b_at2, out_norm, w_aout, b_aout;
     vb::DevBuf attn_ws;  // float32 workspace of the key-split attention path (calls with one or two observations)
-    vb::DevBuf splitk;  // float32 [kFewRowSlices][kFewRows][H]: K slices of Wo / Wdown when a call has few suffix rows
     vb::DevBuf mods;  // pi0.5: float32 [n_layers][2][steps][3H] (scale | shift | gate of the two norms), then [steps][3H] final
     // workspace
     vb::DevBuf k_pages, v_pages, h, hb, q, att, g, a, m1, x, rope_self, rope_cross, tmp_bf, x_stage, state_stage, pad_stage, vbuf;
@@ -323,7 +321,7 @@ static int engine_build(vlab200_engine *e, const vlab200_policy_weights *w) {
         (rc = e->tmp_bf.alloc((size_t)2 * B * e->P * kvf * 2)) || (rc = e->x_stage.alloc(Mc * A * 4)) ||
         (rc = e->state_stage.alloc(B * (size_t)(c.state_dim > 0 ? c.state_dim : 1) * 4)) ||
         (rc = e->pad_stage.alloc(B * 2 * 4)) || (rc = e->vbuf.alloc(M * A * 4)) ||
-        (rc = e->splitk.alloc((size_t)kFewRowSlices * kFewRows * H * 4)) || (rc = e->attn_ws.alloc(kAttnWsBytes(hd))))
+        (rc = e->attn_ws.alloc(kAttnWsBytes(hd))))
         return rc;
     VB_CUDA(cudaMemset(e->h.p, 0, M * H * 4));
     VB_CUDA(cudaMemset(e->hb.p, 0, M * H * 2));
@@ -345,7 +343,16 @@ static vlab200_kv_store engine_store(const vlab200_engine *e, int n_obs_view) {
 }
 
 
-// One expert layer = five launches (six on the few-row path).  Stages, in order:
+// Where the rotated q | k | v of a layer go.
+static RopeParams engine_rope(const vlab200_engine *e, const vlab200_kv_store &live, const float *rope, bool self) {
+    RopeParams r{};
+    r.cos_t = rope; r.sin_t = rope + (size_t)e->S * (e->c.head_dim / 2);
+    r.q_out = e->q.as<__nv_bfloat16>(); r.k_pages = static_cast<__nv_bfloat16 *>(live.k_pages); r.v_pages = static_cast<__nv_bfloat16 *>(live.v_pages);
+    r.seq = e->S; r.n_q = e->c.n_q; r.n_kv_proj = self ? e->c.n_kv : 0; r.n_kv_store = e->c.n_kv; r.hd = e->c.head_dim; r.cap = e->cap; r.row0 = e->P;
+    return r;
+}
+
+// One expert layer = five launches.  Stages, in order:
 //   0 fused RMSNorm + Q/K/V projection + RoPE + KV append   1 attention   2 O-projection + residual
 //   3 fused RMSNorm + gate/up + activation                   4 down projection + residual
 constexpr int kLayerStages = 5;
@@ -356,7 +363,6 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
     const int H = c.H, S = e->S, hd = c.head_dim, I = c.inter, half = hd / 2;
     const int M = n_obs * S;
     const bool self = e->is_self[l];
-    int rc;
     // pages are laid out for max_obs observations per layer; the kernels walk st.n_obs
     // observations from the store base, so hand them a one-layer view of the live ones
     vlab200_kv_store live = engine_store(e, e->max_obs);
@@ -368,17 +374,9 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
     switch (stage) {
     case 0: {
         const float *rope = self ? rs : rx;
-        const int qkv_n = (c.n_q + (self ? 2 * c.n_kv : 0)) * hd;
-        if (M <= kFewRows && qkv_n <= I) {
-            // Few rows: the fused kernel's 128 x 256 tiles leave most SMs idle (10 CTAs for one
-            // observation).  Project with the narrow-tile GEMM (RMS factor in its epilogue) into the
-            // MLP scratch buffer, which is free here, then rotate / split / append in one small kernel.
-            GemmParams p{};
-            p.M = M; p.N = qkv_n; p.K = H; p.epi = EPI_BIAS_ACT; p.act = ACT_NONE; p.use_rms = 1;
-            p.eps = c.rms_eps; p.out_bf = e->g.as<__nv_bfloat16>(); p.ld_out = qkv_n;
-            if ((rc = dense_gemm(e->hb.p, H, e->wqkv[l].p, p, cs))) return rc;
-            return rope_split(e->g.p, rope, rope + (size_t)S * half, e->q.p, live.k_pages, live.v_pages, M, S, c.n_q,
-                              self ? c.n_kv : 0, c.n_kv, hd, e->cap, e->P, cs);
+        if (M <= kFewRows && hd % 64 == 0) {
+            // Few rows: the fused kernel's 128 x 256 tiles leave most SMs idle
+            return qkv_rope_rows(e->hb.p, e->wqkv[l].p, M, H, true, c.rms_eps, engine_rope(e, live, rope, self), cs);
         }
         return vlab200_qkv_rope_append(&live, 0, e->hb.p, 0, nullptr, e->wqkv[l].p, rope, rope + (size_t)S * half,
                                        c.rms_eps, S, H, c.n_q, self ? 1 : 0, e->q.p, cs);
@@ -393,21 +391,21 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
         GemmParams p{};
         p.M = M; p.N = H; p.K = e->qf; p.epi = EPI_RESIDUAL;
         p.h = e->h.as<float>(); p.out_bf = e->hb.as<__nv_bfloat16>(); p.ld_out = H;
-        p.partial = e->splitk.as<float>(); p.partial_slices = kFewRowSlices; p.partial_rows = kFewRows;
+        p.w_early = 1;
         return dense_gemm(e->att.p, e->qf, e->wo[l].p, p, cs);
     }
     case 3: {
         GemmParams p{};
         p.M = M; p.N = 2 * I; p.K = H; p.epi = EPI_GATED; p.use_rms = 1; p.eps = c.rms_eps;
         p.act = c.model == 0 ? ACT_GELU_TANH : ACT_SILU;
-        p.out_bf = e->g.as<__nv_bfloat16>(); p.ld_out = I;
+        p.out_bf = e->g.as<__nv_bfloat16>(); p.ld_out = I; p.w_early = 1;
         return dense_gemm(e->hb.p, H, e->wgu[l].p, p, cs);
     }
     case 4: {
         GemmParams p{};
         p.M = M; p.N = H; p.K = I; p.epi = EPI_RESIDUAL;
         p.h = e->h.as<float>(); p.out_bf = e->hb.as<__nv_bfloat16>(); p.ld_out = H;
-        p.partial = e->splitk.as<float>(); p.partial_slices = kFewRowSlices; p.partial_rows = kFewRows;
+        p.w_early = 1;
         return dense_gemm(e->g.p, I, e->wdown[l].p, p, cs);
     }
     default:
@@ -419,7 +417,7 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
 static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float *rope, cudaStream_t cs) {
     const vlab200_policy_config &c = e->c;
     const int H = c.H, S = e->S, hd = c.head_dim, I = c.inter, half = hd / 2, T = c.steps;
-    const int M = n_obs * S, qkv_n = e->qf + 2 * e->kvf;
+    const int M = n_obs * S;
     const size_t per = (size_t)T * 3 * H;
     const float *mod_in = e->mods.as<float>() + ((size_t)l * 2) * per + (size_t)step * 3 * H;
     const float *mod_post = e->mods.as<float>() + ((size_t)l * 2 + 1) * per + (size_t)step * 3 * H;
@@ -435,12 +433,8 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
     if ((rc = launch_pdl(adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, static_cast<const float *>(h), mod_in, hb, M, H, c.rms_eps)))
         return rc;
     GemmParams p{};
-    if (M <= kFewRows) {  // few rows: narrow-tile GEMM, then rotation / split / append (as in layer_stage)
-        p.M = M; p.N = qkv_n; p.K = H; p.epi = EPI_BIAS_ACT; p.act = ACT_NONE; p.out_bf = e->g.as<__nv_bfloat16>(); p.ld_out = qkv_n;
-        if ((rc = dense_gemm(hb, H, e->wqkv[l].p, p, cs))) return rc;
-        if ((rc = rope_split(e->g.p, rope, rope + (size_t)S * half, e->q.p, live.k_pages, live.v_pages, M, S, c.n_q, c.n_kv, c.n_kv,
-                             hd, e->cap, e->P, cs)))
-            return rc;
+    if (M <= kFewRows && hd % 64 == 0) {  // few rows (as in layer_stage)
+        if ((rc = qkv_rope_rows(hb, e->wqkv[l].p, M, H, false, c.rms_eps, engine_rope(e, live, rope, true), cs))) return rc;
     } else if ((rc = vlab200_qkv_rope_append(&live, 0, hb, 0, nullptr, e->wqkv[l].p, rope, rope + (size_t)S * half, -1.0f, S, H, c.n_q,
                                              1, e->q.p, cs))) {  // the fused kernel without its RMS factor
         return rc;
@@ -450,16 +444,16 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
         return rc;
     p = GemmParams{};
     p.M = M; p.N = H; p.K = e->qf; p.epi = EPI_RESIDUAL; p.colscale = mod_in + 2 * H;
-    p.h = h; p.out_bf = hb; p.ld_out = H; p.partial = e->splitk.as<float>(); p.partial_slices = kFewRowSlices; p.partial_rows = kFewRows;
+    p.h = h; p.out_bf = hb; p.ld_out = H; p.w_early = 1;
     if ((rc = dense_gemm(e->att.p, e->qf, e->wo[l].p, p, cs))) return rc;
     if ((rc = launch_pdl(adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, static_cast<const float *>(h), mod_post, hb, M, H, c.rms_eps)))
         return rc;
     p = GemmParams{};
-    p.M = M; p.N = 2 * I; p.K = H; p.epi = EPI_GATED; p.act = ACT_GELU_TANH; p.out_bf = e->g.as<__nv_bfloat16>(); p.ld_out = I;
+    p.M = M; p.N = 2 * I; p.K = H; p.epi = EPI_GATED; p.act = ACT_GELU_TANH; p.out_bf = e->g.as<__nv_bfloat16>(); p.ld_out = I; p.w_early = 1;
     if ((rc = dense_gemm(hb, H, e->wgu[l].p, p, cs))) return rc;
     p = GemmParams{};
     p.M = M; p.N = H; p.K = I; p.epi = EPI_RESIDUAL; p.colscale = mod_post + 2 * H;
-    p.h = h; p.out_bf = hb; p.ld_out = H; p.partial = e->splitk.as<float>(); p.partial_slices = kFewRowSlices; p.partial_rows = kFewRows;
+    p.h = h; p.out_bf = hb; p.ld_out = H; p.w_early = 1;
     return dense_gemm(e->g.p, I, e->wdown[l].p, p, cs);
 }
 
@@ -639,7 +633,7 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
                 return rc;
             vb::GemmParams p{};
             p.M = M; p.N = A; p.K = H; p.epi = vb::EPI_BIAS_ACT; p.act = vb::ACT_NONE;
-            p.out_f32 = e->vbuf.as<float>(); p.bias = e->b_aout.as<float>(); p.ld_out = A;
+            p.out_f32 = e->vbuf.as<float>(); p.bias = e->b_aout.as<float>(); p.ld_out = A; p.w_early = 1;
             if ((rc = vb::dense_gemm(e->hb.p, H, e->w_aout.p, p, cs))) return rc;
             if ((rc = vb::launch_pdl(vb::euler_kernel, dim3((Mc * A + 255) / 256), dim3(256), 0, cs, e->x.as<float>(),
                                      e->vbuf.as<float>(), Mc * A, A, chunk, S, dt)))
@@ -653,14 +647,14 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
         {
             vb::GemmParams p{};
             p.M = Mc; p.N = H; p.K = H; p.epi = vb::EPI_BIAS_ACT; p.act = vb::ACT_SILU;
-            p.out_bf = e->m1.as<__nv_bfloat16>(); p.bias = e->tvec.as<float>() + (size_t)step * H; p.ld_out = H;
+            p.out_bf = e->m1.as<__nv_bfloat16>(); p.bias = e->tvec.as<float>() + (size_t)step * H; p.ld_out = H; p.w_early = 1;
             if ((rc = vb::dense_gemm(e->a.p, H, e->w_at1l.p, p, cs))) return rc;
         }
         {
             vb::GemmParams p{};
             p.M = Mc; p.N = H; p.K = H; p.epi = vb::EPI_BIAS_ACT; p.act = vb::ACT_NONE;
             p.out_bf = e->hb.as<__nv_bfloat16>(); p.out_f32 = e->h.as<float>(); p.bias = e->b_at2.as<float>();
-            p.ld_out = H; p.rows_in = chunk; p.rows_out = S; p.row_off = S - chunk;
+            p.w_early = 1; p.ld_out = H; p.rows_in = chunk; p.rows_out = S; p.row_off = S - chunk;
             if ((rc = vb::dense_gemm(e->m1.p, H, e->w_at2.p, p, cs))) return rc;
         }
         for (int l = 0; l < c.n_layers; ++l)
@@ -669,7 +663,7 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
         {   // v = W_aout (rms(h) * w_out) + b_aout over every suffix row, then the Euler update on the action rows
             vb::GemmParams p{};
             p.M = M; p.N = A; p.K = H; p.epi = vb::EPI_BIAS_ACT; p.act = vb::ACT_NONE; p.use_rms = 1; p.eps = c.rms_eps;
-            p.out_f32 = e->vbuf.as<float>(); p.bias = e->b_aout.as<float>(); p.ld_out = A;
+            p.out_f32 = e->vbuf.as<float>(); p.bias = e->b_aout.as<float>(); p.ld_out = A; p.w_early = 1;
             if ((rc = vb::dense_gemm(e->hb.p, H, e->w_aout.p, p, cs))) return rc;
             if ((rc = vb::launch_pdl(vb::euler_kernel, dim3((Mc * A + 255) / 256), dim3(256), 0, cs, e->x.as<float>(),
                                      e->vbuf.as<float>(), Mc * A, A, chunk, S, dt)))
@@ -949,9 +943,14 @@ int32_t vlab200_prefill_run(vlab200_prefill *p, vlab200_engine *e, int32_t obs0,
         {   // RMSNorm (factor in the epilogue, weight folded) + q | k | v, then rotation and the page write
             vb::GemmParams g{};
             g.M = M; g.N = qkv_n; g.K = H; g.epi = vb::EPI_BIAS_ACT; g.act = vb::ACT_NONE; g.use_rms = 1; g.eps = c.rms_eps;
-            g.out_bf = p->qkv.as<__nv_bfloat16>(); g.ld_out = qkv_n;
-            if ((rc = vb::dense_gemm(p->hb.p, H, p->wqkv[l].p, g, cs))) return rc;
-            if ((rc = vb::rope_split(p->qkv.p, cos_t, sin_t, p->q.p, kp, vp, M, P, c.n_q, c.n_kv, c.n_kv, hd, e->cap, 0, cs)))
+            g.out_bf = p->qkv.as<__nv_bfloat16>(); g.ld_out = qkv_n; g.w_early = 1;
+            vb::RopeParams r{};
+            r.cos_t = cos_t; r.sin_t = sin_t; r.q_out = p->q.as<__nv_bfloat16>(); r.k_pages = kp; r.v_pages = vp; r.seq = P;
+            r.n_q = c.n_q; r.n_kv_proj = r.n_kv_store = c.n_kv; r.hd = hd; r.cap = e->cap; r.row0 = 0;
+            const bool rows = M <= vb::kSplitRows && (reinterpret_cast<uintptr_t>(sin_t) & 31) == 0;
+            if (rows && (rc = vb::qkv_rope_rows(p->hb.p, p->wqkv[l].p, M, H, true, c.rms_eps, r, cs))) return rc;
+            if (!rows && (rc = vb::dense_gemm(p->hb.p, H, p->wqkv[l].p, g, cs))) return rc;
+            if (!rows && (rc = vb::rope_split(p->qkv.p, cos_t, sin_t, p->q.p, kp, vp, M, P, c.n_q, c.n_kv, c.n_kv, hd, e->cap, 0, cs)))
                 return rc;
         }
         if (l + 1 < c.n_layers) {
@@ -960,16 +959,16 @@ int32_t vlab200_prefill_run(vlab200_prefill *p, vlab200_engine *e, int32_t obs0,
             vb::GemmParams g{};
             g.M = M; g.N = H; g.K = qf; g.epi = vb::EPI_RESIDUAL;
             g.h = p->h.as<float>(); g.out_bf = p->hb.as<__nv_bfloat16>(); g.ld_out = H;
-            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = p->split_rows;
+            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = p->split_rows; g.w_early = 1;
             if ((rc = vb::dense_gemm(p->att.p, qf, p->wo[l].p, g, cs))) return rc;
             g = vb::GemmParams{};
             g.M = M; g.N = 2 * I; g.K = H; g.epi = vb::EPI_GATED; g.use_rms = 1; g.eps = c.rms_eps; g.act = c.act;
-            g.out_bf = p->g.as<__nv_bfloat16>(); g.ld_out = I;
+            g.out_bf = p->g.as<__nv_bfloat16>(); g.ld_out = I; g.w_early = 1;
             if ((rc = vb::dense_gemm(p->hb.p, H, p->wgu[l].p, g, cs))) return rc;
             g = vb::GemmParams{};
             g.M = M; g.N = H; g.K = I; g.epi = vb::EPI_RESIDUAL;
             g.h = p->h.as<float>(); g.out_bf = p->hb.as<__nv_bfloat16>(); g.ld_out = H;
-            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = p->split_rows;
+            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = p->split_rows; g.w_early = 1;
             if ((rc = vb::dense_gemm(p->g.p, I, p->wdown[l].p, g, cs))) return rc;
         }
         if (!e->is_self[l]) {

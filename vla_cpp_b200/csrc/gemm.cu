@@ -27,6 +27,7 @@
 #include <atomic>
 
 #include "gemm.h"
+#include "gemm_epi.cuh"
 #include "host_common.h"
 #include "tc5.cuh"
 
@@ -48,42 +49,6 @@ struct GemmCfg {
     static constexpr int STAGE_BYTES = G_A_BYTES + B_BYTES;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 256 + 1024 + 1024;  // + barriers, statistics, alignment
 };
-
-// Both activations are x * sigmoid(.): SiLU(x) = x / (1 + e^-x) and, since 1 + tanh(u) = 2 / (1 + e^-2u),
-// tanh-GELU(x) = 0.5 x (1 + tanh(u)) = x / (1 + e^-2u) with u = k0 x (1 + k1 x^2) (constants of
-// src/cuda/vla_cuda_bf16.cu:470-474).  One ex2 and one reciprocal each (relative error ~1e-6) keep the
-// epilogue off the critical path; tanhf and an IEEE division cost several times the issue slots.
-template <int ACT>
-__device__ __forceinline__ float act_t(float x) {
-    if (ACT == ACT_SILU) return __fdividef(x, 1.0f + __expf(-x));
-    if (ACT == ACT_GELU_TANH) {
-        const float k0 = 0.79788456080286535587989211986876f, k1 = 0.044715f;
-        const float u = k0 * x * (1.0f + k1 * x * x);
-        return __fdividef(x, 1.0f + __expf(-2.0f * u));
-    }
-    if (ACT == ACT_GELU_ERF) return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f));
-    return x;
-}
-
-// The activation is uniform over a launch: the epilogues branch on it ONCE per 32-column chunk and run a loop compiled
-// for that activation.  (With the activation as a run-time argument of the element function the compiler evaluated
-// every variant for every element and selected: the epilogue of a plain projection paid for SiLU, tanh-GELU and erf.)
-template <int ACT>
-__device__ __forceinline__ void gated_chunk(const uint32_t (&v)[32], float rms, uint32_t (&w)[8]) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const float g0 = act_t<ACT>(__uint_as_float(v[4 * e]) * rms) * (__uint_as_float(v[4 * e + 1]) * rms);
-        const float g1 = act_t<ACT>(__uint_as_float(v[4 * e + 2]) * rms) * (__uint_as_float(v[4 * e + 3]) * rms);
-        const __nv_bfloat162 h2 = __floats2bfloat162_rn(g0, g1);
-        w[e] = *reinterpret_cast<const uint32_t *>(&h2);
-    }
-}
-
-template <int ACT>
-__device__ __forceinline__ void act_chunk(float (&f)[32]) {
-#pragma unroll
-    for (int e = 0; e < 32; ++e) f[e] = act_t<ACT>(f[e]);
-}
 
 // SPLIT: the K loop of every output tile is cut into p.ksplit slices that run as separate work items; a slice stores its
 // float accumulator to p.partial[slice][m][n] and splitk_reduce_kernel adds the slices in a fixed order (few rows and a
@@ -295,8 +260,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             tc_fence_after();
             const float rms = p.use_rms ? rsqrtf(stats[buf * 128 + row] / (float)p.K + p.eps) : 1.0f;
             const uint32_t lane_addr = tmem_base + buf * G_BN + ((uint32_t)(qtr * 32) << 16);
-            size_t mo = (size_t)m;
-            if (p.rows_in > 0 && p.scatter_hd == 0) mo = (size_t)(m / p.rows_in) * p.rows_out + p.row_off + (m % p.rows_in);
+            const size_t mo = mapped_row(p, m);
             for (int c = grp * (G_BN / 2); c < (grp + 1) * (G_BN / 2); c += 32) {
                 const int n = n0 + c;
                 if (n >= p.N) break;  // N % 8 == 0: a chunk may be cut after a multiple of 8 columns
@@ -383,38 +347,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
                         if (n + 16 < p.N) bp[1] = make_uint4(w[4], w[5], w[6], w[7]);
                     }
                 } else {
-                    float f[32];
-#pragma unroll
-                    for (int e = 0; e < 32; ++e)
-                        f[e] = __uint_as_float(v[e]) * rms + ((p.bias && n + e < p.N) ? __ldg(p.bias + n + e) : 0.0f);
-                    if (p.act == ACT_SILU) act_chunk<ACT_SILU>(f);
-                    else if (p.act == ACT_GELU_TANH) act_chunk<ACT_GELU_TANH>(f);
-                    else if (p.act == ACT_GELU_ERF) act_chunk<ACT_GELU_ERF>(f);
-                    if (p.out_f32) {
-                        float4 *fp = reinterpret_cast<float4 *>(p.out_f32 + mo * p.ld_out + n);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (n + 4 * e < p.N) fp[e] = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
-                    }
-                    if (p.out_bf) {
-                        size_t off = mo * p.ld_out + n;
-                        if (p.scatter_hd > 0)  // head-major pages: [obs][head][cap][hd]
-                            off = ((size_t)(m / p.rows_in) * (p.N / p.scatter_hd) + (size_t)(n / p.scatter_hd)) *
-                                      ((size_t)p.scatter_cap * p.scatter_hd) +
-                                  (size_t)(m % p.rows_in) * p.scatter_hd + (n % p.scatter_hd);
-                        uint4 *bp = reinterpret_cast<uint4 *>(p.out_bf + off);
-#pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4) {
-                            if (n + 8 * q4 >= p.N) break;
-                            uint32_t w[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const __nv_bfloat162 h2 = __floats2bfloat162_rn(f[8 * q4 + 2 * e], f[8 * q4 + 2 * e + 1]);
-                                w[e] = *reinterpret_cast<const uint32_t *>(&h2);
-                            }
-                            bp[q4] = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
-                    }
+                    bias_act_chunk(p, v, rms, m, mo, n);
                 }
             }
             tc_fence_before();
@@ -451,12 +384,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1)
 dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap w_map,
                        const GemmParams p, int tiles_m, int tiles_n) {
     dense_gemm_body<256, true>(a_map, w_map, p, tiles_m, tiles_n);
-}
-
-__global__ void __launch_bounds__(G_THREADS, 1)
-dense_gemm_splitk_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap w_map,
-                         const GemmParams p, int tiles_m, int tiles_n) {
-    dense_gemm_body<64, false, true>(a_map, w_map, p, tiles_m, tiles_n);
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1)
@@ -499,6 +426,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restr
 
 // 0 = choose by cost; 1 / 2 / 3 / 4 force the 128 x 256, 128 x 128, CTA-pair and 128 x 64 tilings (testing knob).
 static std::atomic<int> g_gemm_variant{0};
+constexpr int kRowsMax = 4096;
 constexpr float kPairTileFactor = 0.95f;  // time of a pair's 256 x 256 tile relative to a lone CTA's 128 x 256 tile
 
 void dense_gemm_set_variant(int v) { g_gemm_variant.store((v >= 0 && v <= 4) ? v : 0, std::memory_order_relaxed); }
@@ -527,11 +455,44 @@ static float tiling_cost(int M, int N, int n_sm, int *variant_out) {
 
 static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, cudaStream_t stream, int forced_variant);
 
-// K slices as separate work items (variant 5: 128 x 64 tiles, 6: pair tiles), then their sum in slice order with the residual epilogue.
-static int split_residual(const void *A, int lda, const void *W, const GemmParams &p, int ksplit, int variant, int n_sm, cudaStream_t stream) {
+// 256-bit epilogue accesses need every touched row segment on a 32-byte boundary
+static GemmParams with_al32(GemmParams p) {
+    const bool f32_ok = !p.h || ((reinterpret_cast<uintptr_t>(p.h) & 31) == 0 && p.ld_out % 8 == 0);
+    const bool bf_ok = !p.out_bf || ((reinterpret_cast<uintptr_t>(p.out_bf) & 31) == 0 && p.ld_out % 16 == 0);
+    p.al32 = (p.rows_in == 0 && f32_ok && bf_ok) ? 1 : 0;
+    return p;
+}
+
+// Whether a problem goes to the kernel for few rows (gemm_rows.cu), and with which tile width and K slices.  us of a launch inside a
+// chain of launches: what it costs whatever its size, plus 64-wide K steps times what one costs an SM (operand bytes; two resident CTAs
+// share that), against the persistent kernels' tiles.
+static bool choose_rows(const void *A, int lda, const void *W, const GemmParams &p, int n_sm, int *bn_out, int *slices_out) {
+    if (p.N % 8 || (p.epi == EPI_GATED && p.N % 16) || p.K % 8 || lda % 8 || p.ld_out % 8 || p.M > kRowsMax) return false;
+    if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return false;
+    const int nk = (p.K + G_BK - 1) / G_BK, tm = (p.M + G_BM - 1) / G_BM;
+    const bool can_split = p.epi == EPI_RESIDUAL && p.rows_in == 0 && p.scatter_hd == 0;
+    float best = 6.0f + 0.5f * (float)nk * tiling_cost(p.M, p.N, n_sm, nullptr);
+    *bn_out = 0;
+    for (int bn = 64; bn <= 128; bn *= 2)
+        for (int s = 1; s <= (can_split ? 8 : 1); s *= 2) {
+            const int tiles = tm * ((p.N + bn - 1) / bn);
+            if (s > 1 && (nk < 2 * s || tiles * s > 2 * n_sm || tiles > gemm_rows_clusters(bn, s))) break;
+            const float waves = std::max(1.0f, (float)(tiles * s) / (float)n_sm);
+            const float c = 4.0f + (s > 1 ? 1.0f : 0.0f) + (bn == 64 ? 0.28f : 0.38f) * (float)((nk + s - 1) / s) * waves;
+            if (c < best) {
+                best = c;
+                *bn_out = bn;
+                *slices_out = s;
+            }
+        }
+    return *bn_out > 0;
+}
+
+// K slices of pair tiles as separate work items (variant 6), then their sum in slice order with the residual epilogue.
+static int split_residual(const void *A, int lda, const void *W, const GemmParams &p, int ksplit, int n_sm, cudaStream_t stream) {
     GemmParams ps = p;
     ps.ksplit = ksplit;
-    int rc = dense_gemm_one(A, lda, W, ps, stream, variant);
+    int rc = dense_gemm_one(A, lda, W, ps, stream, 6);
     if (rc) return rc;
     const size_t total4 = (size_t)p.M * p.N / 4;
     const int blocks = (int)((total4 + 255) / 256 < (size_t)n_sm * 4 ? (total4 + 255) / 256 : (size_t)n_sm * 4);
@@ -548,15 +509,9 @@ static int split_residual(const void *A, int lda, const void *W, const GemmParam
 int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t stream) {
     if (!A || !W || p.M <= 0 || p.N <= 0 || p.K <= 0) return VLAB200_ERR_ARG;
     const int n_sm = sm_count();
-    // Few rows, narrow N, long K (Wo / Wdown of one to five observations: 16 or 32 tiles of 128 x 64 for N = 1024, each
-    // streaming all of K through one SM): cut K so that the slices fill the machine, then add the slices in a fixed order.
-    if (p.partial && p.epi == EPI_RESIDUAL && dense_gemm_variant() == 0 && p.M <= p.partial_rows && p.rows_in == 0 &&
-        p.scatter_hd == 0 && !p.use_rms && p.N % 4 == 0 && n_sm > 0) {
-        const int tiles = ((p.M + G_BM - 1) / G_BM) * ((p.N + 63) / 64), ksteps = (p.K + G_BK - 1) / G_BK;
-        int ksplit = n_sm / tiles;
-        if (ksplit > ksteps / 4) ksplit = ksteps / 4;  // at least four 64-wide k-steps per slice
-        if (ksplit > p.partial_slices) ksplit = p.partial_slices;
-        if (ksplit >= 2) return split_residual(A, lda, W, p, ksplit, 5, n_sm, stream);
+    {
+        int bn = 0, slices = 1;
+        if (dense_gemm_variant() == 0 && n_sm > 0 && choose_rows(A, lda, W, p, n_sm, &bn, &slices)) return dense_gemm_rows(A, lda, W, with_al32(p), bn, slices, stream);
     }
     // Some hundred rows, long K (Wdown of a backbone): one wave of narrow tiles streams all of K through each SM at about 0.35 us a 64-wide
     // step, pair tiles would fill a fraction of the machine at 0.42 us.  K slices of pair tiles do both; the float sums and the second
@@ -577,7 +532,7 @@ int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t
                 slices = s;
             }
         }
-        if (slices) return split_residual(A, lda, W, p, slices, 6, n_sm, stream);
+        if (slices) return split_residual(A, lda, W, p, slices, n_sm, stream);
     }
     static const bool split_off = std::getenv("VLAB200_NO_GEMM_SPLIT") != nullptr;  // measurement knob
     if (!split_off && dense_gemm_variant() == 0 && n_sm >= 2 && p.rows_in == 0 && p.scatter_hd == 0 && p.M > 2 * G_BM) {
@@ -617,12 +572,7 @@ static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, c
     if (!A || !W || p.M <= 0 || p.N <= 0 || p.K <= 0) return VLAB200_ERR_ARG;
     if (p.N % 8 || (p.epi == EPI_GATED && p.N % 16) || p.K % 8 || lda % 8 || p.ld_out % 8) return VLAB200_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return VLAB200_ERR_ARG;
-    {
-        // 256-bit epilogue accesses need every touched row segment on a 32-byte boundary
-        const bool f32_ok = !p.h || ((reinterpret_cast<uintptr_t>(p.h) & 31) == 0 && p.ld_out % 8 == 0);
-        const bool bf_ok = !p.out_bf || ((reinterpret_cast<uintptr_t>(p.out_bf) & 31) == 0 && p.ld_out % 16 == 0);
-        p.al32 = (p.rows_in == 0 && f32_ok && bf_ok) ? 1 : 0;
-    }
+    p = with_al32(p);
     p.status = device_status_ptr();
     if (!p.status) return cuda_fail(cudaGetLastError(), "device_status_ptr");
     CUtensorMap amap, wmap;
@@ -652,16 +602,6 @@ static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, c
     if (variant == 4 && p.N <= 64) variant = 1;
     const uint64_t wdims[2] = {(uint64_t)p.K, (uint64_t)p.N};
     const uint64_t wstrides[1] = {(uint64_t)p.K * 2};
-    if (variant == 5) {  // split-K slices on 128 x 64 tiles
-        const uint32_t box[2] = {G_BK, 64};
-        int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, wdims, wstrides, box,
-                                 CU_TENSOR_MAP_SWIZZLE_128B);
-        if (rc) return rc;
-        if (int rc = ensure_dyn_smem(dense_gemm_splitk_kernel, GemmCfg<64, false>::SMEM)) return rc;
-        const int nt = tiles_m * tn64 * p.ksplit;
-        return launch_pdl(dense_gemm_splitk_kernel, dim3(nt < n_sm ? nt : n_sm), dim3(G_THREADS), GemmCfg<64, false>::SMEM, stream,
-                          amap, wmap, p, tiles_m, tn64);
-    }
     if (variant == 3 || variant == 6) {
         const uint32_t box[2] = {G_BK, 128};  // each CTA of a pair stages half of the 256 weight rows
         int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, wdims, wstrides, box,

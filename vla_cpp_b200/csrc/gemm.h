@@ -5,7 +5,7 @@
 
 namespace vb {
 
-enum { EPI_RESIDUAL = 0, EPI_GATED = 1, EPI_BIAS_ACT = 2 };
+enum { EPI_RESIDUAL = 0, EPI_GATED = 1, EPI_BIAS_ACT = 2, EPI_ROPE = 3 };
 enum { ACT_NONE = 0, ACT_SILU = 1, ACT_GELU_TANH = 2, ACT_GELU_ERF = 3 };
 
 struct GemmParams {
@@ -25,11 +25,26 @@ struct GemmParams {
     // K slices on separate SMs followed by a fixed-order reduction (ksplit is chosen by dense_gemm)
     float *partial;
     int partial_slices, partial_rows, ksplit;
+    int w_early;  // W was complete before any kernel that may still run in the stream: it may be read before the dependency wait
     int *status;
+};
+
+// EPI_ROPE: where a fused q | k | v projection goes, rotated (rows m = observation * seq + token; see rope_split below).
+struct RopeParams {
+    const float *cos_t, *sin_t;  // [seq][hd / 2]
+    __nv_bfloat16 *q_out, *k_pages, *v_pages;
+    int seq, n_q, n_kv_proj, n_kv_store, hd, cap, row0;
 };
 
 // A: bf16 [M][K] (row stride lda elements), W: bf16 [N][K].
 int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t stream);
+
+// The GEMM for few rows (gemm_rows.cu): tiles of 128 x bn (64 or 128), for a RESIDUAL problem with K cut over `slices` CTAs of a cluster.
+int dense_gemm_rows(const void *A, int lda, const void *W, const GemmParams &p, int bn, int slices, cudaStream_t stream);
+int gemm_rows_clusters(int bn, int slices);  // clusters of that many CTAs the device holds at once
+
+// q | k | v of few rows: A [M][K] times W [(n_q + 2 n_kv_proj) hd][K], RMS factor, rotation, head split and page write in one kernel.
+int qkv_rope_rows(const void *A, const void *W, int M, int K, bool use_rms, float eps, const RopeParams &rp, cudaStream_t stream);
 
 // NeoX rotation + head split of a fused [M][(n_q + 2 n_kv_proj) hd] bf16 projection into the q buffer
 // [M / seq][n_q][seq][hd] and K / V page rows row0 + s (pages [.][n_kv_store][cap][hd]); bitvla_lm.cu.

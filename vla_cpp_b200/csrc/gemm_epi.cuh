@@ -1,0 +1,88 @@
+// Epilogue arithmetic of the bf16 GEMM kernels (gemm.cu, gemm_rows.cu).
+#pragma once
+#include <cuda_bf16.h>
+
+#include "gemm.h"
+#include "tc5.cuh"
+
+namespace vb {
+
+// Both activations are x * sigmoid(.): SiLU(x) = x / (1 + e^-x) and, since 1 + tanh(u) = 2 / (1 + e^-2u),
+// tanh-GELU(x) = 0.5 x (1 + tanh(u)) = x / (1 + e^-2u) with u = k0 x (1 + k1 x^2) (constants of
+// src/cuda/vla_cuda_bf16.cu:470-474).  One ex2 and one reciprocal each (relative error ~1e-6) keep the
+// epilogue off the critical path; tanhf and an IEEE division cost several times the issue slots.
+template <int ACT>
+__device__ __forceinline__ float act_t(float x) {
+    if (ACT == ACT_SILU) return __fdividef(x, 1.0f + __expf(-x));
+    if (ACT == ACT_GELU_TANH) {
+        const float k0 = 0.79788456080286535587989211986876f, k1 = 0.044715f;
+        const float u = k0 * x * (1.0f + k1 * x * x);
+        return __fdividef(x, 1.0f + __expf(-2.0f * u));
+    }
+    if (ACT == ACT_GELU_ERF) return 0.5f * x * (1.0f + erff(x * 0.70710678118654752440f));
+    return x;
+}
+
+// The activation is uniform over a launch: the epilogues branch on it ONCE per 32-column chunk and run a loop compiled
+// for that activation.  (With the activation as a run-time argument of the element function the compiler evaluated
+// every variant for every element and selected: the epilogue of a plain projection paid for SiLU, tanh-GELU and erf.)
+template <int ACT>
+__device__ __forceinline__ void gated_chunk(const uint32_t (&v)[32], float rms, uint32_t (&w)[8]) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float g0 = act_t<ACT>(__uint_as_float(v[4 * e]) * rms) * (__uint_as_float(v[4 * e + 1]) * rms);
+        const float g1 = act_t<ACT>(__uint_as_float(v[4 * e + 2]) * rms) * (__uint_as_float(v[4 * e + 3]) * rms);
+        const __nv_bfloat162 h2 = __floats2bfloat162_rn(g0, g1);
+        w[e] = *reinterpret_cast<const uint32_t *>(&h2);
+    }
+}
+
+template <int ACT>
+__device__ __forceinline__ void act_chunk(float (&f)[32]) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) f[e] = act_t<ACT>(f[e]);
+}
+
+// 32 accumulator columns [n, n + 32) of row m through the BIAS_ACT epilogue; mo: the output row (re-mapped).
+__device__ __forceinline__ void bias_act_chunk(const GemmParams &p, const uint32_t (&v)[32], float rms, int m, size_t mo, int n) {
+    float f[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e)
+        f[e] = __uint_as_float(v[e]) * rms + ((p.bias && n + e < p.N) ? __ldg(p.bias + n + e) : 0.0f);
+    if (p.act == ACT_SILU) act_chunk<ACT_SILU>(f);
+    else if (p.act == ACT_GELU_TANH) act_chunk<ACT_GELU_TANH>(f);
+    else if (p.act == ACT_GELU_ERF) act_chunk<ACT_GELU_ERF>(f);
+    if (p.out_f32) {
+        float4 *fp = reinterpret_cast<float4 *>(p.out_f32 + mo * p.ld_out + n);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (n + 4 * e < p.N) fp[e] = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
+    }
+    if (p.out_bf) {
+        size_t off = mo * p.ld_out + n;
+        if (p.scatter_hd > 0)  // head-major pages: [obs][head][cap][hd]
+            off = ((size_t)(m / p.rows_in) * (p.N / p.scatter_hd) + (size_t)(n / p.scatter_hd)) *
+                      ((size_t)p.scatter_cap * p.scatter_hd) +
+                  (size_t)(m % p.rows_in) * p.scatter_hd + (n % p.scatter_hd);
+        uint4 *bp = reinterpret_cast<uint4 *>(p.out_bf + off);
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {
+            if (n + 8 * q4 >= p.N) break;
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const __nv_bfloat162 h2 = __floats2bfloat162_rn(f[8 * q4 + 2 * e], f[8 * q4 + 2 * e + 1]);
+                w[e] = *reinterpret_cast<const uint32_t *>(&h2);
+            }
+            bp[q4] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+// The row of the output that row m of the problem goes to.
+__device__ __forceinline__ size_t mapped_row(const GemmParams &p, int m) {
+    if (p.rows_in > 0 && p.scatter_hd == 0) return (size_t)(m / p.rows_in) * p.rows_out + p.row_off + (m % p.rows_in);
+    return (size_t)m;
+}
+
+}  // namespace vb

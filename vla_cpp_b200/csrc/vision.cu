@@ -25,9 +25,15 @@
 #include "host_common.h"
 #include "tc5.cuh"
 
+namespace vb {
+int attention_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len, int mask_mode,
+                    const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws, size_t ws_bytes, int row_major_hd);
+}
+
 struct vlab200_vision {
     vlab200_vision_config c;
-    int max_views, np, grid, hd, hd_pad, kp, qf, n_tok, c4;
+    int max_views, np, grid, hd, hd_pad, att_hd, kp, qf, n_tok, c4;  // att_hd: head width of the attention kernel
+    bool packed;
     vb::DevBuf patch_w, posb, post_w, post_b, connector, connector_b;
     std::vector<vb::DevBuf> wqkv, bqkv, wo, bo, w1, b1, w2, b2, ln1w, ln1b, ln2w, ln2b;
     vb::DevBuf a_patch, h, hb, nb, qkv, q, kpg, vpg, att, f, shuf, ident;
@@ -234,7 +240,7 @@ vlab200_vision *vlab200_vision_create(const vlab200_vision_config *cfg, const vl
         return nullptr;
     }
     const int hd = c.hidden / c.n_heads;
-    const int hd_pad = hd <= 64 ? 64 : (hd <= 128 ? 128 : 256);
+    int hd_pad = hd <= 64 ? 64 : (hd <= 128 ? 128 : 256);
     if (hd > 256 || hd % 2) {
         vb::set_last_error("vlab200_vision_create: head_dim %d is not supported", hd);
         return nullptr;
@@ -252,6 +258,11 @@ vlab200_vision *vlab200_vision_create(const vlab200_vision_config *cfg, const vl
     v->grid = c.image / c.patch;
     v->np = v->grid * v->grid;
     v->hd = hd;
+    // The attention reads q, k and v as column ranges of the projection (whole 16-byte pieces of a head; whole key blocks of a view):
+    // heads keep their width.  Otherwise they are zero-padded to the attention kernel's and split into pages.
+    v->packed = hd % 8 == 0 && (v->np % 128 == 0 || max_views == 1);
+    v->att_hd = hd_pad;
+    if (v->packed) hd_pad = hd;
     v->hd_pad = hd_pad;
     v->kp = (3 * c.patch * c.patch + 7) / 8 * 8;
     v->qf = c.n_heads * hd_pad;
@@ -306,9 +317,7 @@ vlab200_vision *vlab200_vision_create(const vlab200_vision_config *cfg, const vl
         if ((rc = v->hb.alloc(M * H * 2))) break;
         if ((rc = v->nb.alloc(M * H * 2))) break;
         if ((rc = v->qkv.alloc(M * (size_t)3 * qf * 2))) break;
-        if ((rc = v->q.alloc(M * qf * 2))) break;
-        if ((rc = v->kpg.alloc(M * qf * 2))) break;
-        if ((rc = v->vpg.alloc(M * qf * 2))) break;
+        if (!v->packed && ((rc = v->q.alloc(M * qf * 2)) || (rc = v->kpg.alloc(M * qf * 2)) || (rc = v->vpg.alloc(M * qf * 2)))) break;
         if ((rc = v->att.alloc(M * qf * 2))) break;
         if ((rc = v->f.alloc(M * I * 2))) break;
         if ((rc = v->shuf.alloc(M * H * 2))) break;
@@ -348,7 +357,7 @@ int32_t vlab200_vision_run(vlab200_vision *v, const void *pixels, int32_t pixels
         vb::GemmParams g{};
         g.M = M; g.N = H; g.K = K; g.epi = vb::EPI_RESIDUAL; g.bias = bias;
         g.h = v->h.as<float>(); g.out_bf = v->hb.as<__nv_bfloat16>(); g.ld_out = H;
-        g.partial = v->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = v->split_rows;
+        g.partial = v->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = v->split_rows; g.w_early = 1;
         return vb::dense_gemm(A, K, W, g, cs);
     };
     auto layernorm = [&](const float *w, const float *b, __nv_bfloat16 *out, int shuffle) {
@@ -367,25 +376,32 @@ int32_t vlab200_vision_run(vlab200_vision *v, const void *pixels, int32_t pixels
         if ((rc = layernorm(v->ln1w[l].as<float>(), v->ln1b[l].as<float>(), v->nb.as<__nv_bfloat16>(), 1))) return rc;
         vb::GemmParams g{};
         g.M = M; g.N = 3 * qf; g.K = H; g.epi = vb::EPI_BIAS_ACT; g.act = vb::ACT_NONE; g.bias = v->bqkv[l].as<float>();
-        g.out_bf = v->qkv.as<__nv_bfloat16>(); g.ld_out = 3 * qf;
+        g.out_bf = v->qkv.as<__nv_bfloat16>(); g.ld_out = 3 * qf; g.w_early = 1;
         if ((rc = vb::dense_gemm(v->nb.p, H, v->wqkv[l].p, g, cs))) return rc;
-        if ((rc = vb::rope_split(v->qkv.p, cos_t, sin_t, v->q.p, v->kpg.p, v->vpg.p, M, np, c.n_heads, c.n_heads, c.n_heads, v->hd_pad,
-                                 np, 0, cs)))
-            return rc;
-        vlab200_kv_store view{v->kpg.p, v->vpg.p, 1, n_views, c.n_heads, v->hd_pad, np, 0};
-        if ((rc = vlab200_attention(&view, 0, v->q.p, v->att.p, np, c.n_heads, np, 0, nullptr, cs))) return rc;
+        if (v->packed) {
+            __nv_bfloat16 *qkv = v->qkv.as<__nv_bfloat16>();
+            vlab200_kv_store view{qkv + qf, qkv + 2 * qf, 1, n_views, c.n_heads, v->att_hd, np, 0};
+            if ((rc = vb::attention_flash(&view, 0, qkv, v->att.p, np, c.n_heads, np, 0, nullptr, cs, 1.0f / std::sqrt((float)v->hd), nullptr, 0, v->hd)))
+                return rc;
+        } else {
+            if ((rc = vb::rope_split(v->qkv.p, cos_t, sin_t, v->q.p, v->kpg.p, v->vpg.p, M, np, c.n_heads, c.n_heads, c.n_heads, v->hd_pad,
+                                     np, 0, cs)))
+                return rc;
+            vlab200_kv_store view{v->kpg.p, v->vpg.p, 1, n_views, c.n_heads, v->hd_pad, np, 0};
+            if ((rc = vlab200_attention(&view, 0, v->q.p, v->att.p, np, c.n_heads, np, 0, nullptr, cs))) return rc;
+        }
         if ((rc = residual(v->att.p, qf, v->wo[l].p, v->bo[l].as<float>()))) return rc;
         if ((rc = layernorm(v->ln2w[l].as<float>(), v->ln2b[l].as<float>(), v->nb.as<__nv_bfloat16>(), 1))) return rc;
         g = vb::GemmParams{};
         g.M = M; g.N = I; g.K = H; g.epi = vb::EPI_BIAS_ACT; g.act = vb::ACT_GELU_TANH; g.bias = v->b1[l].as<float>();
-        g.out_bf = v->f.as<__nv_bfloat16>(); g.ld_out = I;
+        g.out_bf = v->f.as<__nv_bfloat16>(); g.ld_out = I; g.w_early = 1;
         if ((rc = vb::dense_gemm(v->nb.p, H, v->w1[l].p, g, cs))) return rc;
         if ((rc = residual(v->f.p, I, v->w2[l].p, v->b2[l].as<float>()))) return rc;
     }
     if ((rc = layernorm(v->post_w.as<float>(), v->post_b.as<float>(), v->shuf.as<__nv_bfloat16>(), c.shuffle))) return rc;
     vb::GemmParams g{};
     g.M = n_views * v->n_tok; g.N = c.out_dim; g.K = v->c4; g.epi = vb::EPI_BIAS_ACT; g.act = vb::ACT_NONE;
-    g.bias = v->connector_b.as<float>(); g.out_f32 = img_emb; g.ld_out = c.out_dim;
+    g.bias = v->connector_b.as<float>(); g.out_f32 = img_emb; g.ld_out = c.out_dim; g.w_early = 1;
     if ((rc = vb::dense_gemm(v->shuf.p, v->c4, v->connector.p, g, cs))) return rc;
     if (c.out_scale != 0.0f && c.out_scale != 1.0f) {
         const size_t n = (size_t)g.M * c.out_dim;
