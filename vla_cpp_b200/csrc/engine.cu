@@ -64,45 +64,87 @@ __global__ void time_vector_kernel(const __nv_bfloat16 *__restrict__ w_at1, cons
     if (lane == 0) tvec[warp] = acc + (b_at1 ? b_at1[o] : 0.0f);
 }
 
-// a[row][o] = bf16(b_ain[o] + sum_k W_ain[o][k] x[row][k]) for the n_rows = n_obs*chunk action
-// tokens.  One CTA takes AIN_ROWS tokens (their x rows, A <= 64 floats each, sit in shared memory) and one
-// thread one output column: its weight row is read once (16-byte loads) and kept in registers for all the
-// tokens of the CTA, so W_ain crosses L2 -> SM once per AIN_ROWS tokens instead of once per token.
-constexpr int AIN_ROWS = 16;
+// d = a * b + c on two floats at once (each product and sum rounded as by fmaf).
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t pair2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpair2(uint64_t v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+
+// out[o] of EMB_ROWS input rows of A <= 64 floats: bias[o] + sum_k W[o][k] x[row][k], k in order.  One CTA takes EMB_ROWS rows, kept in shared
+// memory as [k][row], one thread one output column.  Bound by issue slots: a value of k costs a thread four 16-byte shared loads and
+// eight two-wide FMAs for sixteen rows (25,600 rows x 1024 columns: 140 us with a row at a time, scalar loads and the weights
+// unpacked for every row).
+constexpr int EMB_ROWS = 16;
+__device__ __forceinline__ void embed_stage(float (*sx)[EMB_ROWS], const float *x, int row0, int rows, int A) {
+    for (int i = threadIdx.x; i < EMB_ROWS * A; i += blockDim.x) sx[i % A][i / A] = i / A < rows ? x[(size_t)row0 * A + i] : 0.0f;
+    __syncthreads();
+}
+__device__ __forceinline__ void embed_column(const float (*sx)[EMB_ROWS], const __nv_bfloat16 *wr, float bias, int A, uint64_t (&acc)[EMB_ROWS / 2]) {
+#pragma unroll
+    for (int r = 0; r < EMB_ROWS / 2; ++r) acc[r] = pair2(bias, bias);
+    const bool vec = A % 8 == 0 && (reinterpret_cast<uintptr_t>(wr) & 15) == 0;
+    for (int k8 = 0; k8 < A; k8 += 8) {
+        float w[8];
+        if (vec) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(wr + k8));
+            const __nv_bfloat162 *h2 = reinterpret_cast<const __nv_bfloat162 *>(&v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __bfloat1622float2(h2[e]);
+                w[2 * e] = f.x;
+                w[2 * e + 1] = f.y;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = k8 + e < A ? __bfloat162float(wr[k8 + e]) : 0.0f;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            if (k8 + e >= A) break;
+            const uint64_t ww = pair2(w[e], w[e]);
+            const ulonglong2 *xs = reinterpret_cast<const ulonglong2 *>(sx[k8 + e]);
+#pragma unroll
+            for (int r = 0; r < EMB_ROWS / 4; ++r) {
+                const ulonglong2 v = xs[r];
+                acc[2 * r] = fma2(ww, v.x, acc[2 * r]);
+                acc[2 * r + 1] = fma2(ww, v.y, acc[2 * r + 1]);
+            }
+        }
+    }
+}
+
+// a[row][o] = bf16(b_ain[o] + sum_k W_ain[o][k] x[row][k]) for the n_rows = n_obs*chunk action tokens
 __global__ void __launch_bounds__(256) action_in_kernel(const float *__restrict__ x,
                                                         const __nv_bfloat16 *__restrict__ w_ain,
                                                         const float *__restrict__ b_ain, __nv_bfloat16 *__restrict__ a,
                                                         float *__restrict__ a_f32, int n_rows, int H, int A) {
-    __shared__ float sx[AIN_ROWS][64];
+    __shared__ __align__(16) float sx[64][EMB_ROWS];
     pdl_launch_dependents();
     pdl_wait();
-    const int row0 = blockIdx.x * AIN_ROWS;
-    const int rows = min(AIN_ROWS, n_rows - row0);
-    for (int i = threadIdx.x; i < rows * A; i += blockDim.x) sx[i / A][i % A] = x[(size_t)row0 * A + i];
-    __syncthreads();
+    const int row0 = blockIdx.x * EMB_ROWS, rows = min(EMB_ROWS, n_rows - row0);
+    embed_stage(sx, x, row0, rows, A);
     const int o = blockIdx.y * blockDim.x + threadIdx.x;
     if (o >= H) return;
-    uint4 wv[8];  // A % 8 == 0, A <= 64
-    const uint4 *wr = reinterpret_cast<const uint4 *>(w_ain + (size_t)o * A);
+    uint64_t acc[EMB_ROWS / 2];
+    embed_column(sx, w_ain + (size_t)o * A, b_ain ? b_ain[o] : 0.0f, A, acc);
 #pragma unroll
-    for (int k8 = 0; k8 < 8; ++k8)
-        if (k8 * 8 < A) wv[k8] = __ldg(wr + k8);
-    const float bias = b_ain ? b_ain[o] : 0.0f;
-    for (int r = 0; r < rows; ++r) {
-        float acc = bias;
-#pragma unroll
-        for (int k8 = 0; k8 < 8; ++k8) {
-            if (k8 * 8 >= A) break;
-            const __nv_bfloat162 *h2 = reinterpret_cast<const __nv_bfloat162 *>(&wv[k8]);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = __bfloat1622float2(h2[e]);
-                acc = fmaf(f.x, sx[r][k8 * 8 + 2 * e], acc);
-                acc = fmaf(f.y, sx[r][k8 * 8 + 2 * e + 1], acc);
-            }
-        }
-        a[(size_t)(row0 + r) * H + o] = __float2bfloat16(acc);
-        if (a_f32) a_f32[(size_t)(row0 + r) * H + o] = acc;  // pi0.5: the embedding is the residual stream itself
+    for (int r = 0; r < EMB_ROWS; ++r) {
+        const float2 f = unpair2(acc[r / 2]);
+        const float v = r & 1 ? f.y : f.x;
+        if (r >= rows) break;
+        a[(size_t)(row0 + r) * H + o] = __float2bfloat16(v);
+        if (a_f32) a_f32[(size_t)(row0 + r) * H + o] = v;  // pi0.5: the embedding is the residual stream itself
     }
 }
 
@@ -130,19 +172,23 @@ __global__ void __launch_bounds__(256) adarms_norm_kernel(const float *__restric
 __global__ void __launch_bounds__(256) state_token_kernel(const float *__restrict__ state,
                                                           const __nv_bfloat16 *__restrict__ w_sp,
                                                           const float *__restrict__ b_sp, float *__restrict__ h,
-                                                          __nv_bfloat16 *__restrict__ hb, int H, int sd, int S) {
-    __shared__ float ss[64];
+                                                          __nv_bfloat16 *__restrict__ hb, int n_obs, int H, int sd, int S) {
+    __shared__ __align__(16) float sx[64][EMB_ROWS];
     pdl_launch_dependents();
     pdl_wait();
-    const int obs = blockIdx.x;
-    if (threadIdx.x < sd) ss[threadIdx.x] = state[(size_t)obs * sd + threadIdx.x];
-    __syncthreads();
-    for (int o = threadIdx.x; o < H; o += blockDim.x) {
-        const __nv_bfloat16 *wr = w_sp + (size_t)o * sd;
-        float acc = b_sp ? b_sp[o] : 0.0f;
-        for (int k = 0; k < sd; ++k) acc = fmaf(__bfloat162float(wr[k]), ss[k], acc);
-        h[(size_t)obs * S * H + o] = acc;
-        hb[(size_t)obs * S * H + o] = __float2bfloat16(acc);
+    const int row0 = blockIdx.x * EMB_ROWS, rows = min(EMB_ROWS, n_obs - row0);
+    embed_stage(sx, state, row0, rows, sd);
+    const int o = blockIdx.y * blockDim.x + threadIdx.x;
+    if (o >= H) return;
+    uint64_t acc[EMB_ROWS / 2];
+    embed_column(sx, w_sp + (size_t)o * sd, b_sp ? b_sp[o] : 0.0f, sd, acc);
+#pragma unroll
+    for (int r = 0; r < EMB_ROWS; ++r) {
+        const float2 f = unpair2(acc[r / 2]);
+        const float v = r & 1 ? f.y : f.x;
+        if (r >= rows) break;
+        h[(size_t)(row0 + r) * S * H + o] = v;
+        hb[(size_t)(row0 + r) * S * H + o] = __float2bfloat16(v);
     }
 }
 
@@ -620,7 +666,7 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
     }
     const float dt = -1.0f / (float)c.steps;
     for (int step = 0; step < c.steps; ++step) {
-        if ((rc = vb::launch_pdl(vb::action_in_kernel, dim3((Mc + vb::AIN_ROWS - 1) / vb::AIN_ROWS, (H + 255) / 256), dim3(256), 0, cs,
+        if ((rc = vb::launch_pdl(vb::action_in_kernel, dim3((Mc + vb::EMB_ROWS - 1) / vb::EMB_ROWS, (H + 255) / 256), dim3(256), 0, cs,
                                  e->x.as<float>(), e->w_ain.as<__nv_bfloat16>(), e->b_ain.as<float>(), e->a.as<__nv_bfloat16>(),
                                  c.model == 2 ? e->h.as<float>() : static_cast<float *>(nullptr), Mc, H, A)))
             return rc;
@@ -641,8 +687,9 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
             continue;
         }
         if (c.model == 0 &&
-            (rc = vb::launch_pdl(vb::state_token_kernel, dim3(n_obs), dim3(256), 0, cs, state, e->w_sp.as<__nv_bfloat16>(),
-                                 e->b_sp.as<float>(), e->h.as<float>(), e->hb.as<__nv_bfloat16>(), H, c.state_dim, S)))
+            (rc = vb::launch_pdl(vb::state_token_kernel, dim3((n_obs + vb::EMB_ROWS - 1) / vb::EMB_ROWS, (H + 255) / 256), dim3(256), 0, cs, state,
+                                 e->w_sp.as<__nv_bfloat16>(), e->b_sp.as<float>(), e->h.as<float>(), e->hb.as<__nv_bfloat16>(), n_obs, H,
+                                 c.state_dim, S)))
             return rc;
         {
             vb::GemmParams p{};

@@ -254,6 +254,10 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             const int m0 = (sp / tiles_n) * TILE_M + (int)rank * G_BM, n0 = (sp % tiles_n) * G_BN;
             const int m = m0 + row;
             const bool row_ok = m < p.M;
+            const int cbeg = grp * (G_BN / 2), cend = (grp + 1) * (G_BN / 2);
+            const bool residual = !SPLIT && p.epi == EPI_RESIDUAL;
+            uint32_t hn[32];
+            if (residual && row_ok) load_h32(p, mapped_row(p, m), n0 + cbeg, hn);
             ok = mbar_wait(&accum_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM);
             if (ok && p.use_rms) ok = mbar_wait(&stats_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM);
             if (!ok) break;
@@ -261,7 +265,20 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             const float rms = p.use_rms ? rsqrtf(stats[buf * 128 + row] / (float)p.K + p.eps) : 1.0f;
             const uint32_t lane_addr = tmem_base + buf * G_BN + ((uint32_t)(qtr * 32) << 16);
             const size_t mo = mapped_row(p, m);
-            for (int c = grp * (G_BN / 2); c < (grp + 1) * (G_BN / 2); c += 32) {
+            if (residual) {
+                for (int c = cbeg; c < cend; c += 32) {
+                    const int n = n0 + c;
+                    if (n >= p.N) break;
+                    uint32_t v[32], h[32];
+                    tmem_ld32(lane_addr + (uint32_t)c, v);
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) h[e] = hn[e];
+                    if (row_ok && c + 32 < cend) load_h32(p, mo, n + 32, hn);
+                    tmem_ld_wait();
+                    if (row_ok) residual_chunk(p, v, h, mo, n);
+                }
+            } else
+            for (int c = cbeg; c < cend; c += 32) {
                 const int n = n0 + c;
                 if (n >= p.N) break;  // N % 8 == 0: a chunk may be cut after a multiple of 8 columns
                 uint32_t v[32];
@@ -277,64 +294,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
                                                  __uint_as_float(v[4 * e + 3]));
                     continue;
                 }
-                if (p.epi == EPI_RESIDUAL) {
-                    if (p.colscale) {  // gated residual: the projection's column n is multiplied by colscale[n] first
-#pragma unroll
-                        for (int e = 0; e < 32; ++e)
-                            if (n + e < p.N) v[e] = __float_as_uint(__uint_as_float(v[e]) * __ldg(p.colscale + n + e));
-                    }
-                    if (p.bias) {
-#pragma unroll
-                        for (int e = 0; e < 32; ++e)
-                            if (n + e < p.N) v[e] = __float_as_uint(__uint_as_float(v[e]) + __ldg(p.bias + n + e));
-                    }
-                    float *hrow = p.h + mo * p.ld_out + n;
-                    __nv_bfloat16 *brow = p.out_bf + mo * p.ld_out + n;
-                    if (p.al32) {
-                        // 8 float32 columns = one 32-byte sector per load / store and thread
-#pragma unroll
-                        for (int q8 = 0; q8 < 2; ++q8) {
-                            if (n + 16 * q8 >= p.N) break;
-                            const bool two = n + 16 * q8 + 8 < p.N;
-                            uint32_t w[8];
-#pragma unroll
-                            for (int hlf = 0; hlf < 2; ++hlf) {
-                                if (hlf && !two) break;
-                                const int c0 = 16 * q8 + 8 * hlf;
-                                uint32_t a[8];
-                                ld_global_v8(hrow + c0, a);
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) a[e] = __float_as_uint(__uint_as_float(a[e]) + __uint_as_float(v[c0 + e]));
-                                st_global_v8(hrow + c0, a);
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(a[2 * e]), __uint_as_float(a[2 * e + 1]));
-                                    w[4 * hlf + e] = *reinterpret_cast<const uint32_t *>(&h2);
-                                }
-                            }
-                            if (two) st_global_v8(brow + 16 * q8, w);
-                            else *reinterpret_cast<uint4 *>(brow + 16 * q8) = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
-                    } else {
-                    float4 *hp = reinterpret_cast<float4 *>(hrow);
-                    uint4 *bp = reinterpret_cast<uint4 *>(brow);
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        if (n + 8 * q4 >= p.N) break;
-                        float4 a = hp[2 * q4], b = hp[2 * q4 + 1];
-                        a.x += __uint_as_float(v[8 * q4]); a.y += __uint_as_float(v[8 * q4 + 1]);
-                        a.z += __uint_as_float(v[8 * q4 + 2]); a.w += __uint_as_float(v[8 * q4 + 3]);
-                        b.x += __uint_as_float(v[8 * q4 + 4]); b.y += __uint_as_float(v[8 * q4 + 5]);
-                        b.z += __uint_as_float(v[8 * q4 + 6]); b.w += __uint_as_float(v[8 * q4 + 7]);
-                        hp[2 * q4] = a;
-                        hp[2 * q4 + 1] = b;
-                        const __nv_bfloat162 h0 = __floats2bfloat162_rn(a.x, a.y), h1 = __floats2bfloat162_rn(a.z, a.w);
-                        const __nv_bfloat162 h2 = __floats2bfloat162_rn(b.x, b.y), h3 = __floats2bfloat162_rn(b.z, b.w);
-                        bp[q4] = make_uint4(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1),
-                                            *reinterpret_cast<const uint32_t *>(&h2), *reinterpret_cast<const uint32_t *>(&h3));
-                    }
-                    }
-                } else if (p.epi == EPI_GATED) {
+                if (p.epi == EPI_GATED) {
                     uint32_t w[8];
                     if (p.act == ACT_SILU) gated_chunk<ACT_SILU>(v, rms, w);
                     else gated_chunk<ACT_GELU_TANH>(v, rms, w);
@@ -470,7 +430,8 @@ static bool choose_rows(const void *A, int lda, const void *W, const GemmParams 
     if (p.N % 8 || (p.epi == EPI_GATED && p.N % 16) || p.K % 8 || lda % 8 || p.ld_out % 8 || p.M > kRowsMax) return false;
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return false;
     const int nk = (p.K + G_BK - 1) / G_BK, tm = (p.M + G_BM - 1) / G_BM;
-    const bool can_split = p.epi == EPI_RESIDUAL && p.rows_in == 0 && p.scatter_hd == 0;
+    if (p.epi == EPI_RESIDUAL && p.rows_in != 0) return false;
+    const bool can_split = p.epi == EPI_RESIDUAL;
     float best = 6.0f + 0.5f * (float)nk * tiling_cost(p.M, p.N, n_sm, nullptr);
     *bn_out = 0;
     for (int bn = 64; bn <= 128; bn *= 2)

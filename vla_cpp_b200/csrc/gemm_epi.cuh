@@ -79,6 +79,75 @@ __device__ __forceinline__ void bias_act_chunk(const GemmParams &p, const uint32
     }
 }
 
+// The 32 float32 columns [n, n + 32) of row m that a RESIDUAL epilogue adds to (those below N).
+__device__ __forceinline__ void load_h32(const GemmParams &p, size_t m, int n, uint32_t (&r)[32]) {
+    const float *src = p.h + m * p.ld_out + n;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (n + 8 * q >= p.N) break;
+        if (p.al32) {
+            uint32_t t[8];
+            ld_global_v8(src + 8 * q, t);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[8 * q + e] = t[e];
+        } else {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const uint4 t = *reinterpret_cast<const uint4 *>(src + 8 * q + 4 * e);
+                r[8 * q + 4 * e] = t.x; r[8 * q + 4 * e + 1] = t.y; r[8 * q + 4 * e + 2] = t.z; r[8 * q + 4 * e + 3] = t.w;
+            }
+        }
+    }
+}
+
+// 32 accumulator columns [n, n + 32) of row m through the RESIDUAL epilogue: h += v (* colscale) (+ bias), the bf16 mirror.  h holds the
+// old values, requested a chunk ahead by the caller: read where they are added, each 8 columns cost a round trip to DRAM and the
+// epilogue of a tile took longer than its products (26,112 x 1024 x 2048: 154 us).
+__device__ __forceinline__ void residual_chunk(const GemmParams &p, uint32_t (&v)[32], const uint32_t (&h)[32], size_t m, int n) {
+    float *hrow = p.h + m * p.ld_out + n;
+    __nv_bfloat16 *brow = p.out_bf + m * p.ld_out + n;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (n + 8 * q >= p.N) break;
+        uint32_t t[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) t[e] = v[8 * q + e];
+        if (p.colscale) {  // gated residual: the projection's column n is multiplied by colscale[n] first
+#pragma unroll
+            for (int e = 0; e < 8; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) * __ldg(p.colscale + n + 8 * q + e));
+        }
+        if (p.bias) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) t[e] = __float_as_uint(__uint_as_float(t[e]) + __ldg(p.bias + n + 8 * q + e));
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) t[e] = __float_as_uint(__uint_as_float(h[8 * q + e]) + __uint_as_float(t[e]));
+        if (p.al32) {
+            st_global_v8(hrow + 8 * q, t);
+        } else {
+            reinterpret_cast<uint4 *>(hrow)[2 * q] = make_uint4(t[0], t[1], t[2], t[3]);
+            reinterpret_cast<uint4 *>(hrow)[2 * q + 1] = make_uint4(t[4], t[5], t[6], t[7]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(t[2 * e]), __uint_as_float(t[2 * e + 1]));
+            v[4 * q + e] = *reinterpret_cast<const uint32_t *>(&b2);  // (columns 4 q .. 4 q + 3 are used up)
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        if (n + 16 * q >= p.N) break;
+        const uint32_t w[8] = {v[8 * q], v[8 * q + 1], v[8 * q + 2], v[8 * q + 3], v[8 * q + 4], v[8 * q + 5], v[8 * q + 6], v[8 * q + 7]};
+        const bool two = n + 16 * q + 8 < p.N;
+        if (p.al32 && two) {
+            st_global_v8(brow + 16 * q, w);
+        } else {
+            reinterpret_cast<uint4 *>(brow)[2 * q] = make_uint4(w[0], w[1], w[2], w[3]);
+            if (two) reinterpret_cast<uint4 *>(brow)[2 * q + 1] = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+    }
+}
+
 // The row of the output that row m of the problem goes to.
 __device__ __forceinline__ size_t mapped_row(const GemmParams &p, int m) {
     if (p.rows_in > 0 && p.scatter_hd == 0) return (size_t)(m / p.rows_in) * p.rows_out + p.row_off + (m % p.rows_in);
