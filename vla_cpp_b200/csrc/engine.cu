@@ -222,7 +222,11 @@ __global__ void pages_to_f32_kernel(const __nv_bfloat16 *__restrict__ pages, flo
     }
 }
 
-constexpr int kFewRows = 256;  // suffix rows (n_obs * S) up to which the QKV projection takes the narrow-tile path
+constexpr int kFewRows = 256;  // suffix rows (n_obs * S) up to which Wo and Wdown may run as K slices
+// Suffix rows up to which q | k | v runs as 64-column tiles (gemm_rows.cu): the fused kernel's 256-column tiles leave SMs idle or a last
+// wave nearly empty there (the same bits from both).
+constexpr int kRopeRows = 4096;
+static bool rope_in_rows(int M, int hd) { return hd % 64 == 0 && (M <= kFewRows || (M <= kRopeRows && dense_gemm_variant() == 0)); }
 // key-split attention: at most one (unit, slice) per SM, 128 rows of head_dim + 2 floats each
 static size_t kAttnWsBytes(int hd) { return (size_t)160 * 128 * (hd + 2) * sizeof(float); }
 }
@@ -420,7 +424,7 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
     switch (stage) {
     case 0: {
         const float *rope = self ? rs : rx;
-        if (M <= kFewRows && hd % 64 == 0) {
+        if (rope_in_rows(M, hd)) {
             // Few rows: the fused kernel's 128 x 256 tiles leave most SMs idle
             return qkv_rope_rows(e->hb.p, e->wqkv[l].p, M, H, true, c.rms_eps, engine_rope(e, live, rope, self), cs);
         }
@@ -437,7 +441,7 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
         GemmParams p{};
         p.M = M; p.N = H; p.K = e->qf; p.epi = EPI_RESIDUAL;
         p.h = e->h.as<float>(); p.out_bf = e->hb.as<__nv_bfloat16>(); p.ld_out = H;
-        p.w_early = 1;
+        p.slice_rows = kFewRows; p.w_early = 1;
         return dense_gemm(e->att.p, e->qf, e->wo[l].p, p, cs);
     }
     case 3: {
@@ -451,7 +455,7 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
         GemmParams p{};
         p.M = M; p.N = H; p.K = I; p.epi = EPI_RESIDUAL;
         p.h = e->h.as<float>(); p.out_bf = e->hb.as<__nv_bfloat16>(); p.ld_out = H;
-        p.w_early = 1;
+        p.slice_rows = kFewRows; p.w_early = 1;
         return dense_gemm(e->g.p, I, e->wdown[l].p, p, cs);
     }
     default:
@@ -479,7 +483,7 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
     if ((rc = launch_pdl(adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, static_cast<const float *>(h), mod_in, hb, M, H, c.rms_eps)))
         return rc;
     GemmParams p{};
-    if (M <= kFewRows && hd % 64 == 0) {  // few rows (as in layer_stage)
+    if (rope_in_rows(M, hd)) {
         if ((rc = qkv_rope_rows(hb, e->wqkv[l].p, M, H, false, c.rms_eps, engine_rope(e, live, rope, true), cs))) return rc;
     } else if ((rc = vlab200_qkv_rope_append(&live, 0, hb, 0, nullptr, e->wqkv[l].p, rope, rope + (size_t)S * half, -1.0f, S, H, c.n_q,
                                              1, e->q.p, cs))) {  // the fused kernel without its RMS factor
@@ -490,7 +494,7 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
         return rc;
     p = GemmParams{};
     p.M = M; p.N = H; p.K = e->qf; p.epi = EPI_RESIDUAL; p.colscale = mod_in + 2 * H;
-    p.h = h; p.out_bf = hb; p.ld_out = H; p.w_early = 1;
+    p.h = h; p.out_bf = hb; p.ld_out = H; p.slice_rows = kFewRows; p.w_early = 1;
     if ((rc = dense_gemm(e->att.p, e->qf, e->wo[l].p, p, cs))) return rc;
     if ((rc = launch_pdl(adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, static_cast<const float *>(h), mod_post, hb, M, H, c.rms_eps)))
         return rc;
@@ -499,7 +503,7 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
     if ((rc = dense_gemm(hb, H, e->wgu[l].p, p, cs))) return rc;
     p = GemmParams{};
     p.M = M; p.N = H; p.K = I; p.epi = EPI_RESIDUAL; p.colscale = mod_post + 2 * H;
-    p.h = h; p.out_bf = hb; p.ld_out = H; p.w_early = 1;
+    p.h = h; p.out_bf = hb; p.ld_out = H; p.slice_rows = kFewRows; p.w_early = 1;
     return dense_gemm(e->g.p, I, e->wdown[l].p, p, cs);
 }
 
@@ -1006,7 +1010,7 @@ int32_t vlab200_prefill_run(vlab200_prefill *p, vlab200_engine *e, int32_t obs0,
             vb::GemmParams g{};
             g.M = M; g.N = H; g.K = qf; g.epi = vb::EPI_RESIDUAL;
             g.h = p->h.as<float>(); g.out_bf = p->hb.as<__nv_bfloat16>(); g.ld_out = H;
-            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = p->split_rows; g.w_early = 1;
+            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = g.slice_rows = p->split_rows; g.w_early = 1;
             if ((rc = vb::dense_gemm(p->att.p, qf, p->wo[l].p, g, cs))) return rc;
             g = vb::GemmParams{};
             g.M = M; g.N = 2 * I; g.K = H; g.epi = vb::EPI_GATED; g.use_rms = 1; g.eps = c.rms_eps; g.act = c.act;
@@ -1015,7 +1019,7 @@ int32_t vlab200_prefill_run(vlab200_prefill *p, vlab200_engine *e, int32_t obs0,
             g = vb::GemmParams{};
             g.M = M; g.N = H; g.K = I; g.epi = vb::EPI_RESIDUAL;
             g.h = p->h.as<float>(); g.out_bf = p->hb.as<__nv_bfloat16>(); g.ld_out = H;
-            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = p->split_rows; g.w_early = 1;
+            g.partial = p->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = g.slice_rows = p->split_rows; g.w_early = 1;
             if ((rc = vb::dense_gemm(p->g.p, I, p->wdown[l].p, g, cs))) return rc;
         }
         if (!e->is_self[l]) {

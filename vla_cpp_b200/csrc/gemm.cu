@@ -431,7 +431,7 @@ static bool choose_rows(const void *A, int lda, const void *W, const GemmParams 
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return false;
     const int nk = (p.K + G_BK - 1) / G_BK, tm = (p.M + G_BM - 1) / G_BM;
     if (p.epi == EPI_RESIDUAL && p.rows_in != 0) return false;
-    const bool can_split = p.epi == EPI_RESIDUAL;
+    const bool can_split = p.epi == EPI_RESIDUAL && p.M <= p.slice_rows;
     float best = 6.0f + 0.5f * (float)nk * tiling_cost(p.M, p.N, n_sm, nullptr);
     *bn_out = 0;
     for (int bn = 64; bn <= 128; bn *= 2)

@@ -25,6 +25,7 @@ struct GemmParams {
     // K slices on separate SMs followed by a fixed-order reduction (ksplit is chosen by dense_gemm)
     float *partial;
     int partial_slices, partial_rows, ksplit;
+    int slice_rows;  // RESIDUAL with at most this many rows: K may be cut over the CTAs of a cluster (other last bits than a whole K)
     int w_early;  // W was complete before any kernel that may still run in the stream: it may be read before the dependency wait
     int *status;
 };

@@ -357,7 +357,7 @@ int32_t vlab200_vision_run(vlab200_vision *v, const void *pixels, int32_t pixels
         vb::GemmParams g{};
         g.M = M; g.N = H; g.K = K; g.epi = vb::EPI_RESIDUAL; g.bias = bias;
         g.h = v->h.as<float>(); g.out_bf = v->hb.as<__nv_bfloat16>(); g.ld_out = H;
-        g.partial = v->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = v->split_rows; g.w_early = 1;
+        g.partial = v->splitk.as<float>(); g.partial_slices = vb::kSplitSlices; g.partial_rows = g.slice_rows = v->split_rows; g.w_early = 1;
         return vb::dense_gemm(A, K, W, g, cs);
     };
     auto layernorm = [&](const float *w, const float *b, __nv_bfloat16 *out, int shuffle) {
