@@ -168,6 +168,51 @@ __global__ void __launch_bounds__(256) adarms_norm_kernel(const float *__restric
     }
 }
 
+// The same with the row in registers (H % 4 == 0, H <= 128 NV): one pass, 16-byte loads all in flight, and the modulation, which is
+// computed when the engine is built, read before the dependency wait.
+template <int NV>
+__global__ void __launch_bounds__(128) adarms_norm_vec_kernel(const float *__restrict__ x, const float *__restrict__ mod,
+                                                              __nv_bfloat16 *__restrict__ y, int M, int H, float eps) {
+    const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, H4 = H >> 2;
+    float4 sc[NV], sh[NV], v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        sc[i] = sh[i] = v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane + 32 * i < H4) {
+            sc[i] = __ldg(reinterpret_cast<const float4 *>(mod) + lane + 32 * i);
+            sh[i] = __ldg(reinterpret_cast<const float4 *>(mod + H) + lane + 32 * i);
+        }
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    if (row >= M) return;
+    const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)row * H);
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+        if (lane + 32 * i < H4) v[i] = xr[lane + 32 * i];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    const float r = rsqrtf(ss / (float)H + eps);
+    uint2 *yr = reinterpret_cast<uint2 *>(y + (size_t)row * H);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        if (lane + 32 * i >= H4) break;
+        const float a = v[i].x * r, b = v[i].y * r, c = v[i].z * r, d = v[i].w * r;
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(a + a * sc[i].x + sh[i].x, b + b * sc[i].y + sh[i].y);
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(c + c * sc[i].z + sh[i].z, d + d * sc[i].w + sh[i].w);
+        yr[lane + 32 * i] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+    }
+}
+
+static int adarms_norm(const float *x, const float *mod, __nv_bfloat16 *y, int M, int H, float eps, cudaStream_t cs) {
+    if (H % 4 == 0 && H <= 1024) return launch_pdl(adarms_norm_vec_kernel<8>, dim3((M + 3) / 4), dim3(128), 0, cs, x, mod, y, M, H, eps);
+    if (H % 4 == 0 && H <= 1536) return launch_pdl(adarms_norm_vec_kernel<12>, dim3((M + 3) / 4), dim3(128), 0, cs, x, mod, y, M, H, eps);
+    return launch_pdl(adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, x, mod, y, M, H, eps);
+}
+
 // pi0: the state token (row 0 of each observation) of h / hb = W_sp state + b_sp.
 __global__ void __launch_bounds__(256) state_token_kernel(const float *__restrict__ state,
                                                           const __nv_bfloat16 *__restrict__ w_sp,
@@ -480,7 +525,7 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
     int rc;
     float *h = e->h.as<float>();
     __nv_bfloat16 *hb = e->hb.as<__nv_bfloat16>();
-    if ((rc = launch_pdl(adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, static_cast<const float *>(h), mod_in, hb, M, H, c.rms_eps)))
+    if ((rc = adarms_norm(h, mod_in, hb, M, H, c.rms_eps, cs)))
         return rc;
     GemmParams p{};
     if (rope_in_rows(M, hd)) {
@@ -496,7 +541,7 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
     p.M = M; p.N = H; p.K = e->qf; p.epi = EPI_RESIDUAL; p.colscale = mod_in + 2 * H;
     p.h = h; p.out_bf = hb; p.ld_out = H; p.slice_rows = kFewRows; p.w_early = 1;
     if ((rc = dense_gemm(e->att.p, e->qf, e->wo[l].p, p, cs))) return rc;
-    if ((rc = launch_pdl(adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, static_cast<const float *>(h), mod_post, hb, M, H, c.rms_eps)))
+    if ((rc = adarms_norm(h, mod_post, hb, M, H, c.rms_eps, cs)))
         return rc;
     p = GemmParams{};
     p.M = M; p.N = 2 * I; p.K = H; p.epi = EPI_GATED; p.act = ACT_GELU_TANH; p.out_bf = e->g.as<__nv_bfloat16>(); p.ld_out = I; p.w_early = 1;
@@ -678,8 +723,7 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
             for (int l = 0; l < c.n_layers; ++l)
                 if ((rc = vb::ada_layer(e, l, step, n_obs, rs, cs))) return rc;
             const float *mod_f = e->mods.as<float>() + (size_t)c.n_layers * 2 * c.steps * 3 * H + (size_t)step * 3 * H;
-            if ((rc = vb::launch_pdl(vb::adarms_norm_kernel, dim3((M + 7) / 8), dim3(256), 0, cs, static_cast<const float *>(e->h.as<float>()),
-                                     mod_f, e->hb.as<__nv_bfloat16>(), M, H, c.rms_eps)))
+            if ((rc = vb::adarms_norm(e->h.as<float>(), mod_f, e->hb.as<__nv_bfloat16>(), M, H, c.rms_eps, cs)))
                 return rc;
             vb::GemmParams p{};
             p.M = M; p.N = A; p.K = H; p.epi = vb::EPI_BIAS_ACT; p.act = vb::ACT_NONE;

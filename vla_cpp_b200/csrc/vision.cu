@@ -118,12 +118,20 @@ template <int NV>
 __global__ void __launch_bounds__(128) layernorm_vec_kernel(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
                                                             __nv_bfloat16 *__restrict__ out, int M, int H, float eps, int np, int grid,
                                                             int shuffle) {
-    pdl_launch_dependents();
     const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, H4 = H >> 2;
+    float4 v[NV], wv[NV], bv[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {  // the tower's own copies: complete before any kernel that may still run
+        wv[q] = bv[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane + 32 * q < H4) {
+            wv[q] = __ldg(reinterpret_cast<const float4 *>(w) + lane + 32 * q);
+            bv[q] = __ldg(reinterpret_cast<const float4 *>(b) + lane + 32 * q);
+        }
+    }
+    pdl_launch_dependents();
     pdl_wait();
     if (row >= M) return;
     const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)row * H);
-    float4 v[NV];
     float s = 0.0f;
 #pragma unroll
     for (int q = 0; q < NV; ++q) v[q] = lane + 32 * q < H4 ? xr[lane + 32 * q] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -154,9 +162,8 @@ __global__ void __launch_bounds__(128) layernorm_vec_kernel(const float *__restr
     for (int q = 0; q < NV; ++q) {
         const int i = lane + 32 * q;
         if (i >= H4) break;
-        const float4 wv = __ldg(reinterpret_cast<const float4 *>(w) + i), bv = __ldg(reinterpret_cast<const float4 *>(b) + i);
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(v[q].x * rstd * wv.x + bv.x, v[q].y * rstd * wv.y + bv.y);
-        const __nv_bfloat162 hi = __floats2bfloat162_rn(v[q].z * rstd * wv.z + bv.z, v[q].w * rstd * wv.w + bv.w);
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v[q].x * rstd * wv[q].x + bv[q].x, v[q].y * rstd * wv[q].y + bv[q].y);
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(v[q].z * rstd * wv[q].z + bv[q].z, v[q].w * rstd * wv[q].w + bv[q].w);
         reinterpret_cast<uint2 *>(orow)[i] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
     }
 }
