@@ -28,11 +28,13 @@ namespace vb {
 
 constexpr int R_BM = 128, R_BK = 64, R_THREADS = 320;
 
-template <int BN>
+// DEEP: a ring of most of an SM's shared memory for calls whose tiles leave no SM with two of them.  A K step of the shallow ring takes
+// 0.28 us there, a quarter (third) of a load's latency.
+template <int BN, bool DEEP>
 struct RowsCfg {
-    static constexpr int STAGES = BN == 64 ? 4 : 3;
+    static constexpr int STAGES = (BN == 64 ? 4 : 3) * (DEEP ? 2 : 1);
     static constexpr int A_BYTES = R_BM * 128, STAGE_BYTES = A_BYTES + BN * 128;
-    static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES, STATS_OFFSET = BAR_OFFSET + 128;
+    static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES, STATS_OFFSET = BAR_OFFSET + 256;
     static constexpr int SMEM = STATS_OFFSET + R_BM * 4 + 1024;  // + alignment slack
 };
 
@@ -48,11 +50,11 @@ __device__ __forceinline__ uint32_t rows_pack(float a, float b) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-template <int BN, int EPI>
-__global__ void __launch_bounds__(R_THREADS, 2)
+template <int BN, int EPI, bool DEEP>
+__global__ void __launch_bounds__(R_THREADS, DEEP ? 1 : 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ GemmParams p,
                  const __grid_constant__ RopeParams rp, int tiles_n, int slices) {
-    using Cfg = RowsCfg<BN>;
+    using Cfg = RowsCfg<BN, DEEP>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t rows_smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(rows_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -375,19 +377,28 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constan
 
 template <int BN>
 static int rows_clusters(int slices) {
-    if (ensure_dyn_smem(gemm_rows_kernel<BN, EPI_RESIDUAL>, RowsCfg<BN>::SMEM) != VLAB200_OK) return 0;
-    return max_active_clusters(reinterpret_cast<const void *>(gemm_rows_kernel<BN, EPI_RESIDUAL>), R_THREADS, RowsCfg<BN>::SMEM, slices);
+    // (of the deep form: one CTA an SM, which is also what the cost rule counts on)
+    if (ensure_dyn_smem(gemm_rows_kernel<BN, EPI_RESIDUAL, true>, RowsCfg<BN, true>::SMEM) != VLAB200_OK) return 0;
+    return max_active_clusters(reinterpret_cast<const void *>(gemm_rows_kernel<BN, EPI_RESIDUAL, true>), R_THREADS, RowsCfg<BN, true>::SMEM, slices);
 }
 int gemm_rows_clusters(int bn, int slices) { return bn == 64 ? rows_clusters<64>(slices) : rows_clusters<128>(slices); }
 
+template <int BN, int EPI, bool DEEP>
+static int launch_rows_as(const CUtensorMap &amap, const CUtensorMap &wmap, const GemmParams &p, const RopeParams &rp, int tiles, int tiles_n, int slices,
+                          cudaStream_t st) {
+    if (int rc = ensure_dyn_smem(gemm_rows_kernel<BN, EPI, DEEP>, RowsCfg<BN, DEEP>::SMEM)) return rc;
+    if (slices > 1)
+        return launch_pdl_cluster(gemm_rows_kernel<BN, EPI, DEEP>, dim3(tiles * slices), dim3(R_THREADS), RowsCfg<BN, DEEP>::SMEM, slices, st, amap, wmap, p, rp,
+                                  tiles_n, slices);
+    return launch_pdl(gemm_rows_kernel<BN, EPI, DEEP>, dim3(tiles), dim3(R_THREADS), RowsCfg<BN, DEEP>::SMEM, st, amap, wmap, p, rp, tiles_n, 1);
+}
+
 template <int BN, int EPI>
 static int launch_rows(const CUtensorMap &amap, const CUtensorMap &wmap, const GemmParams &p, const RopeParams &rp, int slices, cudaStream_t st) {
-    if (int rc = ensure_dyn_smem(gemm_rows_kernel<BN, EPI>, RowsCfg<BN>::SMEM)) return rc;
-    const int tiles_m = (p.M + R_BM - 1) / R_BM, tiles_n = (p.N + BN - 1) / BN;
-    if (slices > 1)
-        return launch_pdl_cluster(gemm_rows_kernel<BN, EPI>, dim3(tiles_m * tiles_n * slices), dim3(R_THREADS), RowsCfg<BN>::SMEM, slices, st, amap, wmap, p,
-                                  rp, tiles_n, slices);
-    return launch_pdl(gemm_rows_kernel<BN, EPI>, dim3(tiles_m * tiles_n), dim3(R_THREADS), RowsCfg<BN>::SMEM, st, amap, wmap, p, rp, tiles_n, 1);
+    const int tiles_n = (p.N + BN - 1) / BN, tiles = (p.M + R_BM - 1) / R_BM * tiles_n, nk = ((p.K + R_BK - 1) / R_BK + slices - 1) / slices;
+    const bool deep = tiles * slices <= sm_count() && nk > RowsCfg<BN, false>::STAGES;
+    if (deep) return launch_rows_as<BN, EPI, true>(amap, wmap, p, rp, tiles, tiles_n, slices, st);
+    return launch_rows_as<BN, EPI, false>(amap, wmap, p, rp, tiles, tiles_n, slices, st);
 }
 
 // Arguments were checked by the callers (dense_gemm and qkv_rope_rows): 16-byte aligned A and W, N % 8, K % 8, lda % 8 == 0.
