@@ -23,6 +23,7 @@
 // Sequences of equal length can be batched (n_seq); the reference runs one per call.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -134,14 +135,17 @@ __global__ void __launch_bounds__(256) norm_quant_kernel(__nv_bfloat16 *__restri
 // The same stage with 16-byte accesses and the row held in registers (packed bf16) between the passes: thread t
 // owns the 8-element groups t, t + 256, ... (at most NV of them), so K <= 2048 * NV and K % 8 == 0.  Per element the
 // arithmetic is the one of norm_quant_kernel; only the order of the float sum of squares differs.
+// What bounds a row is its chain (load, two block-wide reductions, store: some 3 us), so a CTA walks rows blockIdx.x, + gridDim.x, ... with the
+// next row's loads in flight and the norm's weights kept: 4,800 rows of 6,912 took 34.7 us with a CTA per row (4 resident per SM).
+constexpr int NQ_BLOCKS(int mode, int nv) { return nv == 2 ? 4 : (mode == NQ_PLAIN ? 3 : 2); }  // CTAs per SM
 template <int MODE, int NV>
-__global__ void __launch_bounds__(256) norm_quant_vec_kernel(__nv_bfloat16 *__restrict__ in,
-                                                             const __nv_bfloat16 *__restrict__ add,
-                                                             const __nv_bfloat16 *__restrict__ w, float eps, int K,
-                                                             int8_t *__restrict__ q_out, float *__restrict__ s_out,
-                                                             __nv_bfloat16 *__restrict__ out_bf, int w_early) {
+__global__ void __launch_bounds__(256, NQ_BLOCKS(MODE, NV)) norm_quant_vec_kernel(__nv_bfloat16 *__restrict__ in,
+                                                                            const __nv_bfloat16 *__restrict__ add,
+                                                                            const __nv_bfloat16 *__restrict__ w, float eps, int M, int K,
+                                                                            int8_t *__restrict__ q_out, float *__restrict__ s_out,
+                                                                            __nv_bfloat16 *__restrict__ out_bf, int w_early) {
     __shared__ float red[8];
-    const int m = blockIdx.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     const int K8 = K >> 3;
     // the norm's weights: ahead of the kernel in front where they cannot be its output (w_early)
     uint4 wv[NV];
@@ -152,76 +156,86 @@ __global__ void __launch_bounds__(256) norm_quant_vec_kernel(__nv_bfloat16 *__re
     pdl_launch_dependents();
     if (w_early) pdl_wait();
     const size_t ld = MODE == NQ_GATE_UP ? 2 * (size_t)K : (size_t)K;
-    uint4 *src = reinterpret_cast<uint4 *>(in + m * ld);
-    uint4 x[NV];
-    float ss = 0.f;
+    uint4 xn[NV], an[NV];  // the next row, and what is added to it or multiplied with it
+    auto load = [&](int m) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(in + m * ld);
+        const uint4 *src2 = MODE == NQ_GATE_UP ? src + K8 : reinterpret_cast<const uint4 *>(add + m * ld);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const int i = tid + v * 256;
-        if (i >= K8) break;
-        uint4 xv = src[i];
-        uint32_t *xw = reinterpret_cast<uint32_t *>(&xv);
-        if (MODE == NQ_ADD) {
-            const uint4 av = reinterpret_cast<const uint4 *>(add + m * ld)[i];
-            const uint32_t *aw = reinterpret_cast<const uint32_t *>(&av);
+        for (int v = 0; v < NV; ++v)
+            if (tid + v * 256 < K8) {
+                xn[v] = src[tid + v * 256];
+                if (MODE != NQ_PLAIN) an[v] = src2[tid + v * 256];
+            }
+    };
+    load(blockIdx.x);
+    for (int m = blockIdx.x; m < M; m += gridDim.x) {
+        uint4 *src = reinterpret_cast<uint4 *>(in + m * ld);
+        uint4 x[NV];
+        float ss = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int i = tid + v * 256;
+            if (i >= K8) break;
+            uint4 xv = xn[v];
+            uint32_t *xw = reinterpret_cast<uint32_t *>(&xv);
+            if (MODE == NQ_ADD) {
+                const uint32_t aw[4] = {an[v].x, an[v].y, an[v].z, an[v].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
+                    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&aw[e]));
+                    const __nv_bfloat162 r = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+                    xw[e] = *reinterpret_cast<const uint32_t *>(&r);
+                }
+                src[i] = xv;
+            } else if (MODE == NQ_GATE_UP) {
+                const uint32_t uw[4] = {an[v].x, an[v].y, an[v].z, an[v].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
+                    const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&uw[e]));
+                    const float g0 = fmaxf(g.x, 0.f), g1 = fmaxf(g.y, 0.f);
+                    const __nv_bfloat162 r = __floats2bfloat162_rn(g0 * g0 * u.x, g1 * g1 * u.y);
+                    xw[e] = *reinterpret_cast<const uint32_t *>(&r);
+                }
+            }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
-                const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&aw[e]));
-                const __nv_bfloat162 r = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
-                xw[e] = *reinterpret_cast<const uint32_t *>(&r);
+                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
+                ss += f.x * f.x + f.y * f.y;
             }
-            src[i] = xv;
-        } else if (MODE == NQ_GATE_UP) {
-            const uint4 uv = src[K8 + i];
-            const uint32_t *uw = reinterpret_cast<const uint32_t *>(&uv);
+            x[v] = xv;
+        }
+        if (m + (int)gridDim.x < M) load(m + (int)gridDim.x);
+        ss = block_sum_256(ss, red);
+        const float scale = rsqrtf(ss / (float)K + eps);
+        float amax = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int i = tid + v * 256;
+            if (i >= K8) break;
+            const uint32_t ww[4] = {wv[v].x, wv[v].y, wv[v].z, wv[v].w};
+            uint32_t *xw = reinterpret_cast<uint32_t *>(&x[v]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
-                const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&uw[e]));
-                const float g0 = fmaxf(g.x, 0.f), g1 = fmaxf(g.y, 0.f);
-                const __nv_bfloat162 r = __floats2bfloat162_rn(g0 * g0 * u.x, g1 * g1 * u.y);
-                xw[e] = *reinterpret_cast<const uint32_t *>(&r);
+                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
+                const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&ww[e]));
+                const __nv_bfloat162 y = __floats2bfloat162_rn(f.x * scale * g.x, f.y * scale * g.y);
+                xw[e] = *reinterpret_cast<const uint32_t *>(&y);
+                const float2 yf = __bfloat1622float2(y);
+                amax = fmaxf(amax, fmaxf(fabsf(yf.x), fabsf(yf.y)));
             }
+            if (out_bf) reinterpret_cast<uint4 *>(out_bf + (size_t)m * K)[i] = x[v];
         }
+        if (out_bf) continue;
+        amax = block_max_256(amax, red);
+        amax = amax < 1e-5f ? 1e-5f : amax;
+        const float qs = __fdiv_rn(127.0f, amax);
+        if (tid == 0) s_out[m] = qs;
+        uint2 *dst = reinterpret_cast<uint2 *>(q_out + (size_t)m * K);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
-            ss += f.x * f.x + f.y * f.y;
-        }
-        x[v] = xv;
-    }
-    ss = block_sum_256(ss, red);
-    const float scale = rsqrtf(ss / (float)K + eps);
-    float amax = 0.f;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const int i = tid + v * 256;
-        if (i >= K8) break;
-        const uint32_t ww[4] = {wv[v].x, wv[v].y, wv[v].z, wv[v].w};
-        uint32_t *xw = reinterpret_cast<uint32_t *>(&x[v]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&xw[e]));
-            const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&ww[e]));
-            const __nv_bfloat162 y = __floats2bfloat162_rn(f.x * scale * g.x, f.y * scale * g.y);
-            xw[e] = *reinterpret_cast<const uint32_t *>(&y);
-            const float2 yf = __bfloat1622float2(y);
-            amax = fmaxf(amax, fmaxf(fabsf(yf.x), fabsf(yf.y)));
-        }
-        if (out_bf) reinterpret_cast<uint4 *>(out_bf + (size_t)m * K)[i] = x[v];
-    }
-    if (out_bf) return;
-    amax = block_max_256(amax, red);
-    amax = amax < 1e-5f ? 1e-5f : amax;
-    const float qs = __fdiv_rn(127.0f, amax);
-    if (tid == 0) s_out[m] = qs;
-    uint2 *dst = reinterpret_cast<uint2 *>(q_out + (size_t)m * K);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const int i = tid + v * 256;
-        if (i >= K8) break;
-        dst[i] = quant8_bf16(x[v], qs);
+        for (int v = 0; v < NV; ++v)
+            if (tid + v * 256 < K8) dst[tid + v * 256] = quant8_bf16(x[v], qs);
     }
 }
 
@@ -461,8 +475,13 @@ static int launch_norm_quant(void *in, const void *add, const void *w, float eps
     const __nv_bfloat16 *add_b = static_cast<const __nv_bfloat16 *>(add), *w_b = static_cast<const __nv_bfloat16 *>(w);
     __nv_bfloat16 *out_b = static_cast<__nv_bfloat16 *>(out_bf);
     if (K % 8 == 0 && K <= 8192 && al16(in) && al16(add) && al16(w) && al16(out_bf) && (reinterpret_cast<uintptr_t>(q) & 7) == 0) {
-        if (K <= 4096) return launch_pdl(norm_quant_vec_kernel<MODE, 2>, dim3(M), dim3(256), 0, st, in_b, add_b, w_b, eps, K, q, s, out_b, w_early);
-        return launch_pdl(norm_quant_vec_kernel<MODE, 4>, dim3(M), dim3(256), 0, st, in_b, add_b, w_b, eps, K, q, s, out_b, w_early);
+        const int n_sm = sm_count();
+        if (n_sm <= 0) return cuda_fail(cudaGetLastError(), "sm_count");
+        if (K <= 4096)
+            return launch_pdl(norm_quant_vec_kernel<MODE, 2>, dim3(std::min(M, n_sm * NQ_BLOCKS(MODE, 2))), dim3(256), 0, st, in_b, add_b, w_b, eps, M, K, q, s,
+                              out_b, w_early);
+        return launch_pdl(norm_quant_vec_kernel<MODE, 4>, dim3(std::min(M, n_sm * NQ_BLOCKS(MODE, 4))), dim3(256), 0, st, in_b, add_b, w_b, eps, M, K, q, s, out_b,
+                          w_early);
     }
     const size_t smem = (size_t)K * 4;
     if (smem > 48 * 1024)
