@@ -268,10 +268,14 @@ __global__ void pages_to_f32_kernel(const __nv_bfloat16 *__restrict__ pages, flo
 }
 
 constexpr int kFewRows = 256;  // suffix rows (n_obs * S) up to which Wo and Wdown may run as K slices
-// Suffix rows up to which q | k | v runs as 64-column tiles (gemm_rows.cu): the fused kernel's 256-column tiles leave SMs idle or a last
-// wave nearly empty there (the same bits from both).
-constexpr int kRopeRows = 4096;
-static bool rope_in_rows(int M, int hd) { return hd % 64 == 0 && (M <= kFewRows || (M <= kRopeRows && dense_gemm_variant() == 0)); }
+// Whether q | k | v runs as 64-column tiles (gemm_rows.cu) instead of the fused kernel's 256-column ones (the same bits from both): while
+// two tiles an SM hold them, without row sums of squares four.  1,650 x 2560 x 1024 (520 tiles) without: 16.3 us against 30.3; with:
+// 3,200 x 960 x 720 (375 tiles) 19.3 against 17.3, 3,200 x 1600 x 720 (625) 28.3 against 22.9.
+static bool rope_in_rows(int M, int n_heads, int hd, bool rms) {
+    if (hd % 64) return false;
+    if (M <= kFewRows || dense_gemm_variant() != 0) return M <= kFewRows;
+    return (M + 127) / 128 * (n_heads * (hd / 64)) <= (rms ? 2 : 4) * sm_count();
+}
 // key-split attention: at most one (unit, slice) per SM, 128 rows of head_dim + 2 floats each
 static size_t kAttnWsBytes(int hd) { return (size_t)160 * 128 * (hd + 2) * sizeof(float); }
 }
@@ -469,7 +473,7 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
     switch (stage) {
     case 0: {
         const float *rope = self ? rs : rx;
-        if (rope_in_rows(M, hd)) {
+        if (rope_in_rows(M, c.n_q + (self ? 2 * c.n_kv : 0), hd, true)) {
             // Few rows: the fused kernel's 128 x 256 tiles leave most SMs idle
             return qkv_rope_rows(e->hb.p, e->wqkv[l].p, M, H, true, c.rms_eps, engine_rope(e, live, rope, self), cs);
         }
@@ -528,7 +532,7 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
     if ((rc = adarms_norm(h, mod_in, hb, M, H, c.rms_eps, cs)))
         return rc;
     GemmParams p{};
-    if (rope_in_rows(M, hd)) {
+    if (rope_in_rows(M, c.n_q + 2 * c.n_kv, hd, false)) {
         if ((rc = qkv_rope_rows(hb, e->wqkv[l].p, M, H, false, c.rms_eps, engine_rope(e, live, rope, true), cs))) return rc;
     } else if ((rc = vlab200_qkv_rope_append(&live, 0, hb, 0, nullptr, e->wqkv[l].p, rope, rope + (size_t)S * half, -1.0f, S, H, c.n_q,
                                              1, e->q.p, cs))) {  // the fused kernel without its RMS factor

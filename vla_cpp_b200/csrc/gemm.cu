@@ -423,23 +423,69 @@ static GemmParams with_al32(GemmParams p) {
     return p;
 }
 
-// Whether a problem goes to the kernel for few rows (gemm_rows.cu), and with which tile width and K slices.  us of a launch inside a
-// chain of launches: what it costs whatever its size, plus 64-wide K steps times what one costs an SM (operand bytes; two resident CTAs
-// share that), against the persistent kernels' tiles.
-static bool choose_rows(const void *A, int lda, const void *W, const GemmParams &p, int n_sm, int *bn_out, int *slices_out) {
+// K slices for which pair tiles are worth their float sums and second launch (0: none), and us of that.  Some hundred rows, long K (Wdown of
+// a backbone): one wave of narrow tiles streams all of K through each SM at about 0.35 us a 64-wide step, pair tiles would fill a
+// fraction of the machine at 0.42 us.  K slices of pair tiles do both; the float sums and the second launch cost about 8 us + 1 us per
+// 2.5 MB.  816 x 2048 x 16384: 97 us as 112 tiles of 128 x 128.
+static int pair_slices(const GemmParams &p, int n_sm, float *us) {
+    *us = 1e30f;
+    if (!(p.partial && p.epi == EPI_RESIDUAL && p.M > 2 * G_BM && p.M <= p.partial_rows && p.rows_in == 0 && p.scatter_hd == 0 && !p.use_rms && p.N % 4 == 0 &&
+          n_sm >= 2))
+        return 0;
+    const int pairs = n_sm / 2, ksteps = (p.K + G_BK - 1) / G_BK, units = ((p.M + 2 * G_BM - 1) / (2 * G_BM)) * ((p.N + 255) / 256);
+    auto waves = [](int tiles, int u) { return (tiles + u - 1) / u; };
+    const int tm = (p.M + G_BM - 1) / G_BM, w64 = waves(tm * ((p.N + 63) / 64), n_sm), w128 = waves(tm * ((p.N + 127) / 128), n_sm);
+    const float whole = (float)ksteps * std::min(0.35f * (float)std::min(w64, w128), 0.42f * (float)waves(units, pairs));
+    float best = 0.9f * whole;
+    int slices = 0;
+    for (int s = 2; s <= p.partial_slices && ksteps / s >= 8; ++s) {
+        const float c = 0.42f * (float)(waves(units * s, pairs) * waves(ksteps, s)) + 8.0f + (float)(s + 2) * (float)p.M * (float)p.N * 4.0f / 2.5e6f;
+        if (c < best) {
+            best = c;
+            slices = s;
+        }
+    }
+    if (slices) *us = best;
+    return slices;
+}
+
+// us of a launch of the persistent kernels inside a chain of launches, with the tiling they would take: what it costs whatever its size
+// (pair tiles: clusters start and a 256 x 256 tile drains last), plus 64-wide K steps a wave.  From kernel traces of the engines, the
+// towers and the backbones (39 to 512 tiles, 12 to 256 steps); within 15 %.
+static float persistent_us(int M, int N, int nk, int n_sm) {
+    int v = 0;
+    tiling_cost(M, N, n_sm, &v);
+    const int tm = (M + G_BM - 1) / G_BM;
+    auto per = [](int tiles, int units) { return std::max(1.0f, (float)tiles / (float)units); };
+    if (v == 3) return 12.0f + 0.31f * (float)nk * per((tm + 1) / 2 * ((N + 255) / 256), n_sm / 2);
+    if (v == 1) return 4.5f + 0.46f * (float)nk * per(tm * ((N + 255) / 256), n_sm);
+    if (v == 2) return 4.0f + 0.36f * (float)nk * per(tm * ((N + 127) / 128), n_sm);
+    return 4.0f + 0.26f * (float)nk * per(tm * ((N + 63) / 64), n_sm);
+}
+
+// Whether a problem goes to the kernel for few rows (gemm_rows.cu), and with which tile width and K slices: the same estimate of a launch
+// against `us`, the persistent kernels'.  Up to an SM per tile: 0.22 / 0.35 us a K step of 64 / 128 columns, 0.40 / 0.38 where the row
+// sums of squares are taken on the way; K slices add their exchange (0.4 + 0.5 s, 0.6 s).  Two tiles an SM: 0.5 to 0.8 us a step.  Beyond,
+// waves.  Measured in chains at 51 to 3,264 rows, e.g. 255 x 1024 x 2048: 64 columns in 1 / 2 / 4 slices + 3.9 / + 1.8 / 0 us, 128
+// columns + 8.6 / + 3.7 / + 2.2, persistent + 4.8; 768 x 1152 x 4304: 20.8 us persistent, 19.9 as 64 columns, 14.7 as 128 in two slices.
+static bool choose_rows(const void *A, int lda, const void *W, const GemmParams &p, int n_sm, float us, int *bn_out, int *slices_out) {
     if (p.N % 8 || (p.epi == EPI_GATED && p.N % 16) || p.K % 8 || lda % 8 || p.ld_out % 8 || p.M > kRowsMax) return false;
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return false;
-    const int nk = (p.K + G_BK - 1) / G_BK, tm = (p.M + G_BM - 1) / G_BM;
     if (p.epi == EPI_RESIDUAL && p.rows_in != 0) return false;
+    const int nk = (p.K + G_BK - 1) / G_BK, tm = (p.M + G_BM - 1) / G_BM;
     const bool can_split = p.epi == EPI_RESIDUAL && p.M <= p.slice_rows;
-    float best = 6.0f + 0.5f * (float)nk * tiling_cost(p.M, p.N, n_sm, nullptr);
+    float best = us;
     *bn_out = 0;
     for (int bn = 64; bn <= 128; bn *= 2)
         for (int s = 1; s <= (can_split ? 8 : 1); s *= 2) {
-            const int tiles = tm * ((p.N + bn - 1) / bn);
-            if (s > 1 && (nk < 2 * s || tiles * s > 2 * n_sm || tiles > gemm_rows_clusters(bn, s))) break;
-            const float waves = std::max(1.0f, (float)(tiles * s) / (float)n_sm);
-            const float c = 4.0f + (s > 1 ? 1.0f : 0.0f) + (bn == 64 ? 0.28f : 0.38f) * (float)((nk + s - 1) / s) * waves;
+            const int tiles = tm * ((p.N + bn - 1) / bn), n = tiles * s;
+            if (s > 1 && (nk < 2 * s || n > n_sm || tiles > gemm_rows_clusters(bn, s))) break;
+            float step = bn == 64 ? (p.use_rms ? 0.40f : 0.22f) : (p.use_rms ? 0.38f : 0.35f);
+            if (n > n_sm) {
+                const float over = std::min(1.0f, (float)(n - n_sm) / (float)n_sm);
+                step = ((bn == 64 ? 0.5f : 0.6f) + 0.2f * over) * (float)(n <= 2 * n_sm + n_sm / 10 ? 1 : (n + 2 * n_sm - 1) / (2 * n_sm));
+            }
+            const float c = 4.0f + (s > 1 ? (bn == 64 ? 0.4f + 0.5f * (float)s : 0.6f * (float)s) : 0.0f) + step * (float)((nk + s - 1) / s);
             if (c < best) {
                 best = c;
                 *bn_out = bn;
@@ -470,30 +516,13 @@ static int split_residual(const void *A, int lda, const void *W, const GemmParam
 int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t stream) {
     if (!A || !W || p.M <= 0 || p.N <= 0 || p.K <= 0) return VLAB200_ERR_ARG;
     const int n_sm = sm_count();
-    {
+    if (dense_gemm_variant() == 0 && n_sm > 0) {
+        float split_us = 0.0f;
+        const int split = pair_slices(p, n_sm, &split_us);
         int bn = 0, slices = 1;
-        if (dense_gemm_variant() == 0 && n_sm > 0 && choose_rows(A, lda, W, p, n_sm, &bn, &slices)) return dense_gemm_rows(A, lda, W, with_al32(p), bn, slices, stream);
-    }
-    // Some hundred rows, long K (Wdown of a backbone): one wave of narrow tiles streams all of K through each SM at about 0.35 us a 64-wide
-    // step, pair tiles would fill a fraction of the machine at 0.42 us.  K slices of pair tiles do both; the float sums and the second
-    // launch cost about 8 us + 1 us per 2.5 MB.  816 x 2048 x 16384: 97 us as 112 tiles of 128 x 128.  (fc2 of a vision tower, K up to 4304,
-    // stays whole.)
-    if (p.partial && p.epi == EPI_RESIDUAL && dense_gemm_variant() == 0 && p.M > 2 * G_BM && p.M <= p.partial_rows && p.rows_in == 0 &&
-        p.scatter_hd == 0 && !p.use_rms && p.N % 4 == 0 && n_sm >= 2) {
-        const int pairs = n_sm / 2, ksteps = (p.K + G_BK - 1) / G_BK, units = ((p.M + 2 * G_BM - 1) / (2 * G_BM)) * ((p.N + 255) / 256);
-        auto waves = [](int tiles, int u) { return (tiles + u - 1) / u; };
-        const int tm = (p.M + G_BM - 1) / G_BM, w64 = waves(tm * ((p.N + 63) / 64), n_sm), w128 = waves(tm * ((p.N + 127) / 128), n_sm);
-        const float whole = (float)ksteps * std::min(0.35f * (float)std::min(w64, w128), 0.42f * (float)waves(units, pairs));
-        float best = 0.9f * whole;
-        int slices = 0;
-        for (int s = 2; s <= p.partial_slices && ksteps / s >= 8; ++s) {
-            const float c = 0.42f * (float)(waves(units * s, pairs) * waves(ksteps, s)) + 8.0f + (float)(s + 2) * (float)p.M * (float)p.N * 4.0f / 2.5e6f;
-            if (c < best) {
-                best = c;
-                slices = s;
-            }
-        }
-        if (slices) return split_residual(A, lda, W, p, slices, n_sm, stream);
+        if (choose_rows(A, lda, W, p, n_sm, std::min(split_us, persistent_us(p.M, p.N, (p.K + G_BK - 1) / G_BK, n_sm)), &bn, &slices))
+            return dense_gemm_rows(A, lda, W, with_al32(p), bn, slices, stream);
+        if (split) return split_residual(A, lda, W, p, split, n_sm, stream);
     }
     static const bool split_off = std::getenv("VLAB200_NO_GEMM_SPLIT") != nullptr;  // measurement knob
     if (!split_off && dense_gemm_variant() == 0 && n_sm >= 2 && p.rows_in == 0 && p.scatter_hd == 0 && p.M > 2 * G_BM) {

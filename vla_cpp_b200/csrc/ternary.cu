@@ -984,8 +984,8 @@ static TernTiling choose_tiling(int M, int N, int K, bool gate_up, int n_sm) {
     if (N >= 256 && n_sm >= 2) consider(256, 1, 6400 + 360 * ks * waves(tp * ((N + 255) / 256), n_sm / 2));
     if (!gate_up)
         for (int sl = 2; sl <= 4 && ks >= 4 * sl; sl *= 2) {
-            if (t64 * sl <= n_sm && t64 <= tc_clusters<64>(sl)) consider(64, sl, 5000 + 370 * waves(ks, sl));
-            if (t128 * sl <= n_sm && t128 <= tc_clusters<128>(sl)) consider(128, sl, 5800 + 460 * waves(ks, sl));
+            if (t64 * sl <= n_sm && t64 <= tc_clusters<64>(sl)) consider(64, sl, 5400 + 370 * waves(ks, sl));
+            if (t128 * sl <= n_sm && t128 <= tc_clusters<128>(sl)) consider(128, sl, 6200 + 460 * waves(ks, sl));
         }
     return best;
 }
