@@ -10,8 +10,8 @@
 //   norm_quant_kernel   [residual add ->] RMSNorm (bf16 rounding as the reference) -> per-token
 //                       absmax int8; one pass over the row, nothing but int8 + scale written
 //   ternary GEMM        q, k, v as ONE matrix (rows concatenated at set_layer, one weight scale
-//                       per 'group' rows through ws_num)
-//   rope_split_kernel   NeoX RoPE on q and k, head split, K / V rows into the attention pages
+//                       per 'group' rows through ws_num); heads of 128 leave it rotated and split where a tile holds whole heads
+//   rope_split_kernel   otherwise: NeoX RoPE on q and k, head split, K / V rows into the attention pages
 //   attention           streaming tcgen05 kernel, no score matrix, no repeated K/V
 //   norm_quant_kernel   attn sub-norm -> int8
 //   ternary GEMM        o
@@ -595,14 +595,16 @@ extern "C" int32_t vlab200_bitvla_lm_forward(vlab200_bitvla_lm *ctx, const void 
     // runs the normalisations a second time without their fused quantisation.
     vb::L0Dump dump(n_seq == 1 ? std::getenv("VLA_BITVLA_DUMP_L0") : nullptr, st, (size_t)M * (size_t)(F > hq ? (F > H ? F : H) : (hq > H ? hq : H)));
     // the weights were complete before the copy above: the kernels below read them ahead of the kernel in front of them
-    auto linear = [&](const void *packed, void *out, const float *ws, int ws_num, int N, int K, int gate_up) {
+    auto linear = [&](const void *packed, void *out, const float *ws, int ws_num, int N, int K, int gate_up, bool rope = false) {
         vb::TernaryCall c{};
+        if (rope) c.rope = {ctx->cos_t.as<float>(), ctx->sin_t.as<float>(), ctx->q.p, ctx->k_pages.p, ctx->v_pages.p, seq, ctx->n_q, ctx->n_kv, ctx->max_seq};
         c.A = a8; c.W = static_cast<const uint8_t *>(packed); c.out = out; c.s = s; c.ws = ws; c.ws_num = ws_num; c.M = M; c.N = N; c.K = K;
         c.gate_up = gate_up; c.w_early = 1;
         return vb::ternary_linear(c, st);
     };
     // relu(gate)^2 * up in the product's epilogue (the GEMV of a few tokens has none): half of the gate_up traffic in both directions
     const int fused = M > 8 ? 1 : 0;
+    const bool can_rope = ctx->hd == 128 && ctx->qkv_group % 128 == 0 && vb::ternary_can_rope(M, hq + 2 * hkv, H);
     for (int L = 0; L < ctx->n_layers && !rc; ++L) {
         const vb::LmLayer &l = ctx->layers[L];
         auto sub_norm = [&](int8_t *q, float *sc, void *y) {
@@ -617,10 +619,13 @@ extern "C" int32_t vlab200_bitvla_lm_forward(vlab200_bitvla_lm *ctx, const void 
         if (L == 0) rc = vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->h.p, nullptr, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st, 1);
         else rc = vb::launch_norm_quant<vb::NQ_ADD>(ctx->h.p, ctx->proj.p, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st, 1);
         if (rc) break;
-        rc = linear(l.qkv_packed.p, ctx->qkv.p, l.qkv_ws.as<float>(), ctx->qkv_ws_num, hq + 2 * hkv, H, 0);
+        // the rotation in the product's epilogue where a tile holds whole heads (same bits); the stage dump wants the projection itself
+        const bool rope = can_rope && !dl;
+        rc = linear(l.qkv_packed.p, ctx->qkv.p, l.qkv_ws.as<float>(), ctx->qkv_ws_num, hq + 2 * hkv, H, 0, rope);
         if (rc) break;
         if (dl) dump.write_qkv("L0_02_qkv_proj", ctx->qkv.p, M, hq, hkv);
-        rc = vb::rope_split(ctx->qkv.p, ctx->cos_t.as<float>(), ctx->sin_t.as<float>(), ctx->q.p, ctx->k_pages.p,
+        if (!rope)
+            rc = vb::rope_split(ctx->qkv.p, ctx->cos_t.as<float>(), ctx->sin_t.as<float>(), ctx->q.p, ctx->k_pages.p,
                             ctx->v_pages.p, M, seq, ctx->n_q, ctx->n_kv, ctx->n_kv, ctx->hd, ctx->max_seq, 0, st);
         if (rc) break;
         rc = vlab200_attention(&store, 0, ctx->q.p, ctx->att.p, seq, ctx->n_q, seq, /*mask_mode=*/0, nullptr, st);

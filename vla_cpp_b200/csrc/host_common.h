@@ -113,6 +113,11 @@ struct DevBuf {
 };
 
 // The ternary linear as the kernels of this library call it (ternary.cu): vlab200_ternary_linear, and what its epilogue adds.
+struct TernaryRope {             // where a q | k | v projection of heads of 128 goes, rotated (rope_split's arguments)
+    const float *cos_t, *sin_t;  // [seq][64]; nullptr: the projection goes to `out`
+    void *q, *k_pages, *v_pages;
+    int seq, n_q, n_kv, cap;
+};
 struct TernaryCall {
     const int8_t *A;
     const uint8_t *W;  // ladder pack
@@ -123,9 +128,11 @@ struct TernaryCall {
     const void *bias;  // bf16 [N], added to the rounded result and rounded again (bitvla_add_bias_bf16), or nullptr
     int gelu;          // tanh-GELU behind the bias
     int gate_up;       // out [M][N / 2] = relu(column n)^2 * column N / 2 + n
+    TernaryRope rope;
     int w_early;       // the packed weights were complete before any kernel that may still run: they are read before the dependency wait
 };
 int ternary_linear(const TernaryCall &c, cudaStream_t st);
+bool ternary_can_rope(int M, int N, int K);  // the tiling that would be taken has whole heads of 128 columns in a tile
 
 // A checkpoint tensor ([d1][d0], d1 == 1 for vectors, d1 < 0: d0 elements of any shape; f32 / f16 / bf16 in the file) uploaded as bf16 or float32,
 // optionally with the Gemma-norm "+1" (gguf.cu).  VLAB200_OK or an error with the last-error text set.
