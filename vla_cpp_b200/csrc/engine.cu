@@ -45,9 +45,21 @@ __global__ void fold_rows_kernel(const __nv_bfloat16 *__restrict__ w, const floa
     }
 }
 
-__global__ void f32_to_bf16_kernel(const float *__restrict__ in, __nv_bfloat16 *__restrict__ out, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = __float2bfloat16(in[i]);
+// out0 = bf16(in0), out1 = bf16(in1), n elements each; blockIdx.y picks the pair.  Eight elements a thread where both ends are aligned.
+__global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float *__restrict__ in0, const float *__restrict__ in1, __nv_bfloat16 *__restrict__ out0,
+                                                          __nv_bfloat16 *__restrict__ out1, size_t n) {
+    const float *in = blockIdx.y ? in1 : in0;
+    __nv_bfloat16 *out = blockIdx.y ? out1 : out0;
+    const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    const size_t n8 = vec ? n / 8 : 0;
+    for (size_t i = first; i < n8; i += step) {
+        const float4 a = reinterpret_cast<const float4 *>(in)[2 * i], b = reinterpret_cast<const float4 *>(in)[2 * i + 1];
+        const __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y),
+                                     __floats2bfloat162_rn(b.z, b.w)};
+        reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(h);
+    }
+    for (size_t i = n8 * 8 + first; i < n; i += step) out[i] = __float2bfloat16(in[i]);
 }
 
 // tvec[s][o] = b_at1[o] + sum_k W_at1[o][H + k] * tau[s][k]   (one warp per output)
@@ -662,8 +674,8 @@ int32_t vlab200_engine_set_prefix(vlab200_engine *e, int32_t layer, int32_t obs0
     // (src/models/smolvla.cpp:853-860), written head-major into the pages of this layer
     const size_t n = (size_t)n_obs * e->P * e->kvf;
     __nv_bfloat16 *kb = e->tmp_bf.as<__nv_bfloat16>(), *vbuf = kb + (size_t)e->max_obs * e->P_max * e->kvf;
-    vb::f32_to_bf16_kernel<<<148 * 4, 256, 0, cs>>>(K, kb, n);
-    vb::f32_to_bf16_kernel<<<148 * 4, 256, 0, cs>>>(V, vbuf, n);
+    const size_t blocks = (n / 8 + 255) / 256 + 1;
+    vb::f32_to_bf16_kernel<<<dim3((unsigned)(blocks < 148 * 4 ? blocks : 148 * 4), 2), 256, 0, cs>>>(K, V, kb, vbuf, n);
     VB_CUDA(cudaGetLastError());
     const size_t page_off = ((size_t)layer * e->max_obs + obs0) * e->c.n_kv * e->cap * e->c.head_dim;
     for (int which = 0; which < 2; ++which) {
