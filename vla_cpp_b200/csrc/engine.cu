@@ -55,9 +55,14 @@ __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float *__restric
     const size_t n8 = vec ? n / 8 : 0;
     for (size_t i = first; i < n8; i += step) {
         const float4 a = reinterpret_cast<const float4 *>(in)[2 * i], b = reinterpret_cast<const float4 *>(in)[2 * i + 1];
-        const __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y),
-                                     __floats2bfloat162_rn(b.z, b.w)};
-        reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(h);
+        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+            w[e] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+        reinterpret_cast<uint4 *>(out)[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
     for (size_t i = n8 * 8 + first; i < n; i += step) out[i] = __float2bfloat16(in[i]);
 }
