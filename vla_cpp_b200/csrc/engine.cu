@@ -98,70 +98,82 @@ __device__ __forceinline__ float2 unpair2(uint64_t v) {
     return f;
 }
 
-// out[o] of EMB_ROWS input rows of A <= 64 floats: bias[o] + sum_k W[o][k] x[row][k], k in order.  One CTA takes EMB_ROWS rows, kept in shared
-// memory as [k][row], one thread one output column.  Bound by issue slots: a value of k costs a thread four 16-byte shared loads and
-// eight two-wide FMAs for sixteen rows (25,600 rows x 1024 columns: 140 us with a row at a time, scalar loads and the weights
-// unpacked for every row).
-constexpr int EMB_ROWS = 16;
+// Columns o, o + 1 of EMB_ROWS input rows of A <= 64 floats: bias[o] + sum_k W[o][k] x[row][k], k in order.  One CTA takes EMB_ROWS rows, kept in
+// shared memory as [k][row], one thread two output columns.  Bound by issue slots: a value of k costs a thread four 16-byte shared
+// loads and sixteen two-wide FMAs for 32 results (25,600 rows x 1024 columns: 140 us with a row at a time, scalar loads and the weights
+// unpacked for every row, 110 us with one column a thread).
+constexpr int EMB_ROWS = 16, EMB_THREADS = 128;
 __device__ __forceinline__ void embed_stage(float (*sx)[EMB_ROWS], const float *x, int row0, int rows, int A) {
     for (int i = threadIdx.x; i < EMB_ROWS * A; i += blockDim.x) sx[i % A][i / A] = i / A < rows ? x[(size_t)row0 * A + i] : 0.0f;
     __syncthreads();
 }
-__device__ __forceinline__ void embed_column(const float (*sx)[EMB_ROWS], const __nv_bfloat16 *wr, float bias, int A, uint64_t (&acc)[EMB_ROWS / 2]) {
+__device__ __forceinline__ void embed_weights(const __nv_bfloat16 *wr, int k8, int A, bool vec, float (&w)[8]) {
+    if (vec) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(wr + k8));
+        const __nv_bfloat162 *h2 = reinterpret_cast<const __nv_bfloat162 *>(&v);
 #pragma unroll
-    for (int r = 0; r < EMB_ROWS / 2; ++r) acc[r] = pair2(bias, bias);
-    const bool vec = A % 8 == 0 && (reinterpret_cast<uintptr_t>(wr) & 15) == 0;
-    for (int k8 = 0; k8 < A; k8 += 8) {
-        float w[8];
-        if (vec) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(wr + k8));
-            const __nv_bfloat162 *h2 = reinterpret_cast<const __nv_bfloat162 *>(&v);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = __bfloat1622float2(h2[e]);
-                w[2 * e] = f.x;
-                w[2 * e + 1] = f.y;
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) w[e] = k8 + e < A ? __bfloat162float(wr[k8 + e]) : 0.0f;
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(h2[e]);
+            w[2 * e] = f.x;
+            w[2 * e + 1] = f.y;
         }
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = k8 + e < A ? __bfloat162float(wr[k8 + e]) : 0.0f;
+    }
+}
+__device__ __forceinline__ void embed_columns(const float (*sx)[EMB_ROWS], const __nv_bfloat16 *W, const float *bias, int o, int A,
+                                              uint64_t (&acc)[2][EMB_ROWS / 2]) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const float b = bias ? bias[o + c] : 0.0f;
+#pragma unroll
+        for (int r = 0; r < EMB_ROWS / 2; ++r) acc[c][r] = pair2(b, b);
+    }
+    const __nv_bfloat16 *w0 = W + (size_t)o * A, *w1 = w0 + A;
+    const bool vec = A % 8 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+    for (int k8 = 0; k8 < A; k8 += 8) {
+        float a[8], b[8];
+        embed_weights(w0, k8, A, vec, a);
+        embed_weights(w1, k8, A, vec, b);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             if (k8 + e >= A) break;
-            const uint64_t ww = pair2(w[e], w[e]);
+            const uint64_t aa = pair2(a[e], a[e]), bb = pair2(b[e], b[e]);
             const ulonglong2 *xs = reinterpret_cast<const ulonglong2 *>(sx[k8 + e]);
 #pragma unroll
             for (int r = 0; r < EMB_ROWS / 4; ++r) {
                 const ulonglong2 v = xs[r];
-                acc[2 * r] = fma2(ww, v.x, acc[2 * r]);
-                acc[2 * r + 1] = fma2(ww, v.y, acc[2 * r + 1]);
+                acc[0][2 * r] = fma2(aa, v.x, acc[0][2 * r]);
+                acc[0][2 * r + 1] = fma2(aa, v.y, acc[0][2 * r + 1]);
+                acc[1][2 * r] = fma2(bb, v.x, acc[1][2 * r]);
+                acc[1][2 * r + 1] = fma2(bb, v.y, acc[1][2 * r + 1]);
             }
         }
     }
 }
 
-// a[row][o] = bf16(b_ain[o] + sum_k W_ain[o][k] x[row][k]) for the n_rows = n_obs*chunk action tokens
-__global__ void __launch_bounds__(256) action_in_kernel(const float *__restrict__ x,
-                                                        const __nv_bfloat16 *__restrict__ w_ain,
-                                                        const float *__restrict__ b_ain, __nv_bfloat16 *__restrict__ a,
-                                                        float *__restrict__ a_f32, int n_rows, int H, int A) {
+// a[row][o] = bf16(b_ain[o] + sum_k W_ain[o][k] x[row][k]) for the n_rows = n_obs*chunk action tokens (H is even)
+__global__ void __launch_bounds__(EMB_THREADS) action_in_kernel(const float *__restrict__ x,
+                                                                const __nv_bfloat16 *__restrict__ w_ain,
+                                                                const float *__restrict__ b_ain, __nv_bfloat16 *__restrict__ a,
+                                                                float *__restrict__ a_f32, int n_rows, int H, int A) {
     __shared__ __align__(16) float sx[64][EMB_ROWS];
     pdl_launch_dependents();
     pdl_wait();
     const int row0 = blockIdx.x * EMB_ROWS, rows = min(EMB_ROWS, n_rows - row0);
     embed_stage(sx, x, row0, rows, A);
-    const int o = blockIdx.y * blockDim.x + threadIdx.x;
+    const int o = 2 * (blockIdx.y * EMB_THREADS + threadIdx.x);
     if (o >= H) return;
-    uint64_t acc[EMB_ROWS / 2];
-    embed_column(sx, w_ain + (size_t)o * A, b_ain ? b_ain[o] : 0.0f, A, acc);
+    uint64_t acc[2][EMB_ROWS / 2];
+    embed_columns(sx, w_ain, b_ain, o, A, acc);
 #pragma unroll
     for (int r = 0; r < EMB_ROWS; ++r) {
-        const float2 f = unpair2(acc[r / 2]);
-        const float v = r & 1 ? f.y : f.x;
+        const float2 f = unpair2(acc[0][r / 2]), g = unpair2(acc[1][r / 2]);
+        const float v0 = r & 1 ? f.y : f.x, v1 = r & 1 ? g.y : g.x;
         if (r >= rows) break;
-        a[(size_t)(row0 + r) * H + o] = __float2bfloat16(v);
-        if (a_f32) a_f32[(size_t)(row0 + r) * H + o] = v;  // pi0.5: the embedding is the residual stream itself
+        *reinterpret_cast<__nv_bfloat162 *>(a + (size_t)(row0 + r) * H + o) = __floats2bfloat162_rn(v0, v1);
+        if (a_f32) *reinterpret_cast<float2 *>(a_f32 + (size_t)(row0 + r) * H + o) = make_float2(v0, v1);  // pi0.5: the embedding is the residual stream
     }
 }
 
@@ -231,26 +243,26 @@ static int adarms_norm(const float *x, const float *mod, __nv_bfloat16 *y, int M
 }
 
 // pi0: the state token (row 0 of each observation) of h / hb = W_sp state + b_sp.
-__global__ void __launch_bounds__(256) state_token_kernel(const float *__restrict__ state,
-                                                          const __nv_bfloat16 *__restrict__ w_sp,
-                                                          const float *__restrict__ b_sp, float *__restrict__ h,
-                                                          __nv_bfloat16 *__restrict__ hb, int n_obs, int H, int sd, int S) {
+__global__ void __launch_bounds__(EMB_THREADS) state_token_kernel(const float *__restrict__ state,
+                                                                  const __nv_bfloat16 *__restrict__ w_sp,
+                                                                  const float *__restrict__ b_sp, float *__restrict__ h,
+                                                                  __nv_bfloat16 *__restrict__ hb, int n_obs, int H, int sd, int S) {
     __shared__ __align__(16) float sx[64][EMB_ROWS];
     pdl_launch_dependents();
     pdl_wait();
     const int row0 = blockIdx.x * EMB_ROWS, rows = min(EMB_ROWS, n_obs - row0);
     embed_stage(sx, state, row0, rows, sd);
-    const int o = blockIdx.y * blockDim.x + threadIdx.x;
+    const int o = 2 * (blockIdx.y * EMB_THREADS + threadIdx.x);
     if (o >= H) return;
-    uint64_t acc[EMB_ROWS / 2];
-    embed_column(sx, w_sp + (size_t)o * sd, b_sp ? b_sp[o] : 0.0f, sd, acc);
+    uint64_t acc[2][EMB_ROWS / 2];
+    embed_columns(sx, w_sp, b_sp, o, sd, acc);
 #pragma unroll
     for (int r = 0; r < EMB_ROWS; ++r) {
-        const float2 f = unpair2(acc[r / 2]);
-        const float v = r & 1 ? f.y : f.x;
+        const float2 f = unpair2(acc[0][r / 2]), g = unpair2(acc[1][r / 2]);
+        const float v0 = r & 1 ? f.y : f.x, v1 = r & 1 ? g.y : g.x;
         if (r >= rows) break;
-        h[(size_t)(row0 + r) * S * H + o] = v;
-        hb[(size_t)(row0 + r) * S * H + o] = __float2bfloat16(v);
+        *reinterpret_cast<float2 *>(h + (size_t)(row0 + r) * S * H + o) = make_float2(v0, v1);
+        *reinterpret_cast<__nv_bfloat162 *>(hb + (size_t)(row0 + r) * S * H + o) = __floats2bfloat162_rn(v0, v1);
     }
 }
 
@@ -736,7 +748,7 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
     }
     const float dt = -1.0f / (float)c.steps;
     for (int step = 0; step < c.steps; ++step) {
-        if ((rc = vb::launch_pdl(vb::action_in_kernel, dim3((Mc + vb::EMB_ROWS - 1) / vb::EMB_ROWS, (H + 255) / 256), dim3(256), 0, cs,
+        if ((rc = vb::launch_pdl(vb::action_in_kernel, dim3((Mc + vb::EMB_ROWS - 1) / vb::EMB_ROWS, (H + 2 * vb::EMB_THREADS - 1) / (2 * vb::EMB_THREADS)), dim3(vb::EMB_THREADS), 0, cs,
                                  e->x.as<float>(), e->w_ain.as<__nv_bfloat16>(), e->b_ain.as<float>(), e->a.as<__nv_bfloat16>(),
                                  c.model == 2 ? e->h.as<float>() : static_cast<float *>(nullptr), Mc, H, A)))
             return rc;
@@ -756,7 +768,8 @@ int32_t vlab200_engine_denoise(vlab200_engine *e, int32_t n_obs, const float *st
             continue;
         }
         if (c.model == 0 &&
-            (rc = vb::launch_pdl(vb::state_token_kernel, dim3((n_obs + vb::EMB_ROWS - 1) / vb::EMB_ROWS, (H + 255) / 256), dim3(256), 0, cs, state,
+            (rc = vb::launch_pdl(vb::state_token_kernel, dim3((n_obs + vb::EMB_ROWS - 1) / vb::EMB_ROWS, (H + 2 * vb::EMB_THREADS - 1) / (2 * vb::EMB_THREADS)),
+                                 dim3(vb::EMB_THREADS), 0, cs, state,
                                  e->w_sp.as<__nv_bfloat16>(), e->b_sp.as<float>(), e->h.as<float>(), e->hb.as<__nv_bfloat16>(), n_obs, H,
                                  c.state_dim, S)))
             return rc;
