@@ -1,0 +1,14 @@
+"""Products of more tiles than CTAs (pairs): with row statistics in contiguous ranges of tiles, without in turn."""
+import pytest
+
+from tests.test_engine_gpu import run_case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_obs", [120, 187])  # 6,120 and 9,537 rows: 96 and 152 pair tiles, 192 and 300 of one CTA; the last one ragged
+@pytest.mark.parametrize("tiling", [0, 1, 3])  # the engine's choice, 256 columns of one CTA, CTA pairs
+def test_more_tiles_than_units_match_the_oracle(oracle, n_obs, tiling):
+    w, d = run_case(oracle, 55, n_obs=n_obs, P=20, tiling=tiling, check_obs=[0, n_obs // 2, n_obs - 1], model=0, L=1, H=1024, n_q=8, n_kv=1,
+                    hd=64, inter=1024, chunk=50, A=32, sd=32, T=1)
+    assert w < 1e-2 and d < 3e-2, (w, d)

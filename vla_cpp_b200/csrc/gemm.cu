@@ -60,8 +60,10 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
     constexpr int G_STAGES = Cfg::STAGES, G_STAGE_BYTES = Cfg::STAGE_BYTES;
     constexpr int TILE_M = PAIR ? 2 * G_BM : G_BM;  // rows of one work unit
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
-    // Every CTA (pair) walks a contiguous range of tiles; column tiles vary fastest, so consecutive tiles mostly
-    // share their rows of A and the row statistics are computed once per row tile instead of once per tile.
+    // Column tiles vary fastest.  With row statistics every CTA (pair) walks a contiguous range of tiles: consecutive ones mostly share
+    // their rows of A, whose statistics are computed once per row tile.  Without, the CTAs take the tiles in turn: those that run at the
+    // same time share few rows of A, which come from DRAM once.  (In contiguous ranges every pair holds rows of its own, read again for
+    // each column tile: at 26,112 x 1024 x 4096 74 x 2 MB, more than the L2 keeps.)
     const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int n_units = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     extern __shared__ uint8_t g_smem_raw[];
@@ -79,7 +81,8 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
     const int ksteps = (p.K + G_BK - 1) / G_BK;
     const int ks_n = SPLIT ? p.ksplit : 1;
     const int n_tiles = tiles_m * tiles_n * ks_n;
-    const int t_begin = (int)((long long)n_tiles * unit / n_units), t_end = (int)((long long)n_tiles * (unit + 1) / n_units);
+    const int t_begin = p.use_rms ? (int)((long long)n_tiles * unit / n_units) : unit;
+    const int t_end = p.use_rms ? (int)((long long)n_tiles * (unit + 1) / n_units) : n_tiles, t_step = p.use_rms ? 1 : n_units;
     const WaitCtx wc{abort_flag, p.status};
     const uint32_t empty_count = p.use_rms ? 5u : 1u;
 
@@ -126,7 +129,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
         if (lane == 0) {
             uint32_t st = 0, ph = 0;
             bool ok = true;
-            for (int tile = t_begin; ok && tile < t_end; ++tile) {
+            for (int tile = t_begin; ok && tile < t_end; tile += t_step) {
                 const int sp = SPLIT ? tile / ks_n : tile, ks = SPLIT ? tile % ks_n : 0;
                 const int kbeg = SPLIT ? ks * ksteps / ks_n : 0, kend = SPLIT ? (ks + 1) * ksteps / ks_n : ksteps;
                 const int m0 = (sp / tiles_n) * TILE_M + (int)rank * G_BM;
@@ -152,7 +155,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             const uint64_t b_desc0 = smem_desc_sw128(smem_u32(smem + G_A_BYTES), 16, 1024);
             uint32_t st = 0, ph = 0, j = 0;
             bool ok = true;
-            for (int tile = t_begin; ok && tile < t_end; ++tile, ++j) {
+            for (int tile = t_begin; ok && tile < t_end; tile += t_step, ++j) {
                 const uint32_t buf = j & 1u;
                 ok = warp_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
@@ -187,7 +190,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             // odd CTA of a pair: tell the even CTA when this CTA's stage has landed
             uint32_t st = 0, ph = 0;
             bool ok = true;
-            for (int tile = t_begin; ok && tile < t_end; ++tile) {
+            for (int tile = t_begin; ok && tile < t_end; tile += t_step) {
                 const int ks = SPLIT ? tile % ks_n : 0;
                 const int kbeg = SPLIT ? ks * ksteps / ks_n : 0, kend = SPLIT ? (ks + 1) * ksteps / ks_n : ksteps;
                 for (int kt = kbeg; kt < kend; ++kt) {
@@ -207,7 +210,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             bool ok = true;
             int prev_mt = -1;
             float row_sum = 0.0f;
-            for (int tile = t_begin; ok && tile < t_end; ++tile, ++j) {
+            for (int tile = t_begin; ok && tile < t_end; tile += t_step, ++j) {
                 const uint32_t buf = j & 1u;
                 const int mt = tile / tiles_n;
                 const bool fresh = mt != prev_mt;  // same rows of A as the previous tile: keep their sums
@@ -248,7 +251,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
         const int row = qtr * 32 + lane;
         uint32_t j = 0;
         bool ok = true;
-        for (int tile = t_begin; ok && tile < t_end; ++tile, ++j) {
+        for (int tile = t_begin; ok && tile < t_end; tile += t_step, ++j) {
             const uint32_t buf = j & 1u;
             const int sp = SPLIT ? tile / ks_n : tile;
             const int m0 = (sp / tiles_n) * TILE_M + (int)rank * G_BM, n0 = (sp % tiles_n) * G_BN;
@@ -631,8 +634,6 @@ static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, c
         return launch_pdl(dense_gemm_kernel<256>, dim3(nt < n_sm ? nt : n_sm), dim3(G_THREADS), GemmCfg<256, false>::SMEM, stream,
                           amap, wmap, p, tiles_m, tn256);
     }
-    VB_CUDA(cudaGetLastError());
-    return VLAB200_OK;
 }
 
 }  // namespace vb
