@@ -32,6 +32,7 @@ struct QkvParams {
     __nv_bfloat16 *k_pages; // layer base: [n_obs][n_kv][cap][hd]
     __nv_bfloat16 *v_pages;
     int M, H, S, hd, n_q, n_kv_proj, n_kv, cap, prefix_len;
+    int al32;               // q_out and both pages start on 32-byte boundaries: 256-bit stores
     float eps;
     int *status;
 };
@@ -253,10 +254,14 @@ qkv_rope_kernel(const __grid_constant__ CUtensorMap w_map, const QkvParams p) {
 //   warp 0      TMA loader (x tile 128 x 64, weight tile 256 x 64 per stage)
 //   warp 1      tcgen05.mma issuer
 //   warps 2-5, 10-13  epilogue (two warps per TMEM lane quarter, alternating heads):
-//               TMEM -> RMSNorm factor -> RoPE -> transpose in shared memory -> q buffer / KV pages
+//               TMEM -> RMSNorm factor -> RoPE -> q buffer / KV pages, a full 32-byte sector per thread and store
 //   warps 6-9   row statistics: read the x tile from shared memory, accumulate sum(x^2) per row
 constexpr int QKVF_THREADS = 448;
-constexpr int QKVF_STAGING = 8 * 4096;  // per epilogue warp: 2 pieces x 32 rows x 64 bytes
+// Shared memory is stages + barriers / statistics + the transposed RoPE table.  The products wait for their operands (a k step takes 0.75 us
+// with four stages of 32 KB in flight per SM, 0.52 with six), so every byte that is not the table is a stage: rows leave straight from
+// registers.  Through a 32 KB transposition buffer a table of 51 x 256 left four stages instead of five, one of 51 x 64 five instead of six.
+constexpr int QKVF_AUX = 256 + 1024, QKVF_SMEM = 227 * 1024;
+constexpr int QKVF_TABLE_RESERVE = 32 * 1024;  // tables within this of the largest that fits beside two stages are refused
 
 // PAIR: a cluster of two CTAs shares one 256 x 256 tile through tcgen05 cta_group::2; each CTA loads
 // its own 128 rows of x and only half of the weight tile (half the shared-memory bytes per flop).
@@ -281,8 +286,7 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(stats_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     float *stats = reinterpret_cast<float *>(aux + 256);   // [2][128]
-    uint8_t *staging = aux + 256 + 1024;                   // [4 warps][2][32][64 B]
-    float *rope_s = reinterpret_cast<float *>(staging + QKVF_STAGING);  // cos [half][S], sin [half][S]
+    float *rope_s = reinterpret_cast<float *>(aux + QKVF_AUX);  // cos [half][S], sin [half][S]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ksteps = (p.H + QKV_BK - 1) / QKV_BK;
@@ -452,8 +456,6 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
         const int row = qtr * 32 + lane;
         const int hd = p.hd;
         const int n_total = (p.n_q + 2 * p.n_kv_proj) * hd;
-        uint8_t *stg = staging + (grp * 4 + qtr) * 4096;
-        const uint32_t my_sw = (uint32_t)((lane >> 1) & 3);
         uint32_t j = 0;
         bool ok = true;
         for (int tile = t_begin; ok && tile < t_end; ++tile, ++j) {
@@ -461,16 +463,8 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
             const int m0 = (tile / tiles_n) * TILE_M + (int)rank * QKV_BM, n0 = (tile % tiles_n) * QKV_BN;
             const int m = m0 + row;
             const int tok = m % p.S;
-            // the four rows this lane writes out after the transpose through shared memory
-            int w_obs[4], w_tok[4];
-            bool w_ok[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int mr = m0 + qtr * 32 + (lane >> 2) + 8 * i;
-                w_ok[i] = mr < p.M;
-                w_obs[i] = mr / p.S;
-                w_tok[i] = mr % p.S;
-            }
+            const bool row_ok = m < p.M;
+            const size_t obs = (size_t)(m / p.S);
             ok = mbar_wait(&accum_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM);
             if (ok) ok = mbar_wait(&stats_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM);
             if (!ok) break;
@@ -499,10 +493,10 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
                     tok0 = (size_t)p.prefix_len;
                     rotate = !is_v;
                 }
+                __nv_bfloat16 *drow = base + obs * obs_stride + (tok0 + tok) * hd;
                 for (int c = (heads_in_tile > 1 ? 0 : grp * 32); c < half; c += (heads_in_tile > 1 ? 32 : 64)) {
                     // 16 columns of each half per round: lo / hi / packed output stay within 48 registers
                     // (the kernel is capped at 128 and spilled with 32-column rounds)
-                    uint8_t *mine = stg + lane * 64;
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {
                         uint32_t lo[16], hi[16];
@@ -528,30 +522,18 @@ __device__ __forceinline__ void qkv_rope_tma_body(const CUtensorMap &x_map, cons
                             olo[e >> 1] = *reinterpret_cast<const uint32_t *>(&l2);
                             ohi[e >> 1] = *reinterpret_cast<const uint32_t *>(&h2);
                         }
-                        // transpose through shared memory: thread-per-row -> 64 contiguous bytes per 4 lanes
+                        __nv_bfloat16 *d = drow + c + hh * 16;
+                        if (row_ok && p.al32) {
+                            st_global_v8(d, olo);
+                            st_global_v8(d + half, ohi);
+                        } else if (row_ok) {
 #pragma unroll
-                        for (int q2 = 0; q2 < 2; ++q2) {
-                            const uint32_t q4 = (uint32_t)(hh * 2 + q2);
-                            *reinterpret_cast<uint4 *>(mine + ((q4 ^ my_sw) << 4)) =
-                                make_uint4(olo[4 * q2], olo[4 * q2 + 1], olo[4 * q2 + 2], olo[4 * q2 + 3]);
-                            *reinterpret_cast<uint4 *>(mine + 2048 + ((q4 ^ my_sw) << 4)) =
-                                make_uint4(ohi[4 * q2], ohi[4 * q2 + 1], ohi[4 * q2 + 2], ohi[4 * q2 + 3]);
+                            for (int q2 = 0; q2 < 2; ++q2) {
+                                reinterpret_cast<uint4 *>(d)[q2] = make_uint4(olo[4 * q2], olo[4 * q2 + 1], olo[4 * q2 + 2], olo[4 * q2 + 3]);
+                                reinterpret_cast<uint4 *>(d + half)[q2] = make_uint4(ohi[4 * q2], ohi[4 * q2 + 1], ohi[4 * q2 + 2], ohi[4 * q2 + 3]);
+                            }
                         }
                     }
-                    __syncwarp();
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int rr = (lane >> 2) + 8 * i;
-                        const uint32_t off = (uint32_t)rr * 64 + ((((uint32_t)lane & 3u) ^ (uint32_t)((rr >> 1) & 3)) << 4);
-                        const uint4 vlo = *reinterpret_cast<const uint4 *>(stg + off);
-                        const uint4 vhi = *reinterpret_cast<const uint4 *>(stg + 2048 + off);
-                        if (w_ok[i]) {
-                            __nv_bfloat16 *d = base + (size_t)w_obs[i] * obs_stride + (tok0 + w_tok[i]) * hd + (lane & 3) * 8;
-                            *reinterpret_cast<uint4 *>(d + c) = vlo;
-                            *reinterpret_cast<uint4 *>(d + half + c) = vhi;
-                        }
-                    }
-                    __syncwarp();
                 }
             }
             tc_fence_before();
@@ -739,6 +721,7 @@ int32_t vlab200_qkv_rope_append(const vlab200_kv_store *st, int32_t layer, const
     p.v_pages = static_cast<__nv_bfloat16 *>(st->v_pages) + off;
     p.M = M; p.H = H; p.S = S; p.hd = hd; p.n_q = n_q; p.n_kv_proj = n_kv_proj; p.n_kv = st->n_kv;
     p.cap = st->cap; p.prefix_len = st->prefix_len; p.eps = eps; p.status = status;
+    p.al32 = ((reinterpret_cast<uintptr_t>(p.q_out) | reinterpret_cast<uintptr_t>(p.k_pages) | reinterpret_cast<uintptr_t>(p.v_pages)) & 31) == 0;
     const int ksteps = (H + vb::QKV_BK - 1) / vb::QKV_BK;
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     if (!ln_w) {
@@ -750,10 +733,9 @@ int32_t vlab200_qkv_rope_append(const vlab200_kv_store *st, int32_t layer, const
         rc = vb::make_tensor_map(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, xdims, xstrides, xbox,
                                  CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
-        // shared memory: stages + barriers/stats + store staging + transposed RoPE table
-        const int aux = 256 + 1024 + vb::QKVF_STAGING + 2 * (hd / 2) * S * 4;
-        if ((rc = vb::ensure_dyn_smem(vb::qkv_rope_tma_kernel, 227 * 1024))) return rc;
-        if ((rc = vb::ensure_dyn_smem(vb::qkv_rope_tma_pair_kernel, 227 * 1024))) return rc;
+        const int aux = vb::QKVF_AUX + 2 * (hd / 2) * S * 4;
+        if ((rc = vb::ensure_dyn_smem(vb::qkv_rope_tma_kernel, vb::QKVF_SMEM))) return rc;
+        if ((rc = vb::ensure_dyn_smem(vb::qkv_rope_tma_pair_kernel, vb::QKVF_SMEM))) return rc;
         const int n_sm = vb::sm_count();
         if (n_sm <= 0) return vb::cuda_fail(cudaGetLastError(), "sm_count");
         const int tiles_m = (M + vb::QKV_BM - 1) / vb::QKV_BM, tiles_n = (n_total + vb::QKV_BN - 1) / vb::QKV_BN;
@@ -771,24 +753,22 @@ int32_t vlab200_qkv_rope_append(const vlab200_kv_store *st, int32_t layer, const
                                      CU_TENSOR_MAP_SWIZZLE_128B);
             if (rc) return rc;
             const int stage = vb::QKV_A_BYTES + vb::QKV_B_BYTES / 2;
+            if (2 * stage + aux + vb::QKVF_TABLE_RESERVE + 1024 > vb::QKVF_SMEM) return VLAB200_ERR_UNSUPPORTED;
             int nst = 6;
-            while (nst > 2 && nst * stage + aux + 1024 > 227 * 1024) --nst;
+            while (nst * stage + aux + 1024 > vb::QKVF_SMEM) --nst;
             const int fsmem = nst * stage + aux + 1024;
-            if (fsmem > 227 * 1024) return VLAB200_ERR_UNSUPPORTED;
             const int nt = tiles_mp * tiles_n;
             return vb::launch_pdl(vb::qkv_rope_tma_pair_kernel, dim3(2 * (nt < pairs ? nt : pairs)), dim3(vb::QKVF_THREADS), fsmem, cs,
                                   xmap, wmap, p, tiles_mp, tiles_n, nst);
         } else {
+            if (2 * vb::QKV_STAGE_BYTES + aux + vb::QKVF_TABLE_RESERVE + 1024 > vb::QKVF_SMEM) return VLAB200_ERR_UNSUPPORTED;
             int nst = 4;
-            while (nst > 2 && nst * vb::QKV_STAGE_BYTES + aux + 1024 > 227 * 1024) --nst;
+            while (nst * vb::QKV_STAGE_BYTES + aux + 1024 > vb::QKVF_SMEM) --nst;
             const int fsmem = nst * vb::QKV_STAGE_BYTES + aux + 1024;
-            if (fsmem > 227 * 1024) return VLAB200_ERR_UNSUPPORTED;
             const int nt = tiles_m * tiles_n;
             return vb::launch_pdl(vb::qkv_rope_tma_kernel, dim3(nt < n_sm ? nt : n_sm), dim3(vb::QKVF_THREADS), fsmem, cs, xmap, wmap,
                                   p, tiles_m, tiles_n, nst);
         }
-        VB_CUDA(cudaGetLastError());
-        return VLAB200_OK;
     }
     const int smem = vb::QKV_STAGES * vb::QKV_STAGE_BYTES + 256 + ksteps * vb::QKV_BK * 4 + 1024;
     dim3 grid((M + vb::QKV_BM - 1) / vb::QKV_BM, (n_total + vb::QKV_BN - 1) / vb::QKV_BN);
