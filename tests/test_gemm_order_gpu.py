@@ -12,3 +12,10 @@ def test_more_tiles_than_units_match_the_oracle(oracle, n_obs, tiling):
     w, d = run_case(oracle, 55, n_obs=n_obs, P=20, tiling=tiling, check_obs=[0, n_obs // 2, n_obs - 1], model=0, L=1, H=1024, n_q=8, n_kv=1,
                     hd=64, inter=1024, chunk=50, A=32, sd=32, T=1)
     assert w < 1e-2 and d < 3e-2, (w, d)
+
+
+@pytest.mark.parametrize("H", [480, 720, 960])  # 3,264 rows: the widths 96, 160 and 192 are those whose tiles make one wave
+def test_tile_widths_that_fill_a_wave_match_the_oracle(oracle, H):
+    w, d = run_case(oracle, 56, n_obs=64, P=20, check_obs=[0, 31, 63], model=0, L=2, H=H, n_q=8, n_kv=1, hd=64, inter=H // 2, chunk=50, A=32,
+                    sd=32, T=1)
+    assert w < 1e-2 and d < 3e-2, (w, d)

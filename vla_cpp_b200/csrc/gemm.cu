@@ -35,15 +35,18 @@ namespace vb {
 
 constexpr int G_BM = 128, G_BK = 64, G_THREADS = 448;
 constexpr int G_A_BYTES = G_BM * 128;
-// BN = 256 minimises operand traffic per flop; BN = 128 doubles the number of tiles when the
-// problem has too few of them to occupy the SMs.
+// BN = 256 minimises operand traffic per flop; the narrower ones make more tiles where a problem has too few of them to
+// occupy the SMs: of all widths the one whose tiles fill the last wave (26 row tiles of 720 columns: 78 tiles of 256,
+// 156 of 128 in two waves, 130 of 160 in one).
 // PAIR: two CTAs (a cluster) share one 256 x 256 tile through tcgen05 cta_group::2 -- each loads its
 // own 128 activation rows and only HALF of the weight tile, which halves the shared-memory bytes
 // written and read per flop (a lone CTA moves 96 KB through shared memory per 512 tensor cycles,
 // more than the 128 B/clk the SM has).
 template <int BN, bool PAIR>
 struct GemmCfg {
-    static constexpr int STAGES = PAIR ? 6 : (BN == 256 ? 4 : (BN == 128 ? 6 : 8));
+    static constexpr int STAGES = PAIR ? 6 : (BN == 256 ? 4 : (BN == 192 ? 5 : (BN >= 128 ? 6 : 8)));
+    static constexpr int TMEM_BUF = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);  // columns of an accumulator; two of them
+    static constexpr int GRP0 = (BN / 32 + 1) / 2 * 32;                       // columns of epilogue group 0
     static constexpr int B_ROWS = PAIR ? BN / 2 : BN;  // weight rows this CTA stages
     static constexpr int B_BYTES = B_ROWS * 128;
     static constexpr int STAGE_BYTES = G_A_BYTES + B_BYTES;
@@ -106,10 +109,10 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
     }
     if (warp == 1) {
         if (PAIR) {
-            tmem_alloc_pair(tmem_slot, 2 * G_BN);
+            tmem_alloc_pair(tmem_slot, 2 * Cfg::TMEM_BUF);
             tmem_relinquish_pair();
         } else {
-            tmem_alloc(tmem_slot, 2 * G_BN);
+            tmem_alloc(tmem_slot, 2 * Cfg::TMEM_BUF);
             tmem_relinquish();
         }
     }
@@ -160,7 +163,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
                 ok = warp_wait(&accum_empty[buf], ((j >> 1) & 1u) ^ 1u, wc, DEV_TIMEOUT_EMPTY);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * G_BN;
+                const uint32_t d_tmem = tmem_base + buf * Cfg::TMEM_BUF;
                 const int ks = SPLIT ? tile % ks_n : 0;
                 const int kbeg = SPLIT ? ks * ksteps / ks_n : 0, kend = SPLIT ? (ks + 1) * ksteps / ks_n : ksteps;
                 for (int kt = kbeg; kt < kend; ++kt) {
@@ -245,7 +248,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             }
         }
     } else {
-        // ---- epilogue warps 2..5 (group 0: first half of the tile's columns) and 10..13 (group 1: second half) ----
+        // ---- epilogue warps 2..5 (group 0: the tile's first columns) and 10..13 (group 1: the others) ----
         const int qtr = warp & 3;
         const int grp = warp >= 10 ? 1 : 0;
         const int row = qtr * 32 + lane;
@@ -257,7 +260,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             const int m0 = (sp / tiles_n) * TILE_M + (int)rank * G_BM, n0 = (sp % tiles_n) * G_BN;
             const int m = m0 + row;
             const bool row_ok = m < p.M;
-            const int cbeg = grp * (G_BN / 2), cend = (grp + 1) * (G_BN / 2);
+            const int cbeg = grp * Cfg::GRP0, cend = grp ? G_BN : Cfg::GRP0;
             const bool residual = !SPLIT && p.epi == EPI_RESIDUAL;
             uint32_t hn[32];
             if (residual && row_ok) load_h32(p, mapped_row(p, m), n0 + cbeg, hn);
@@ -266,7 +269,7 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
             if (!ok) break;
             tc_fence_after();
             const float rms = p.use_rms ? rsqrtf(stats[buf * 128 + row] / (float)p.K + p.eps) : 1.0f;
-            const uint32_t lane_addr = tmem_base + buf * G_BN + ((uint32_t)(qtr * 32) << 16);
+            const uint32_t lane_addr = tmem_base + buf * Cfg::TMEM_BUF + ((uint32_t)(qtr * 32) << 16);
             const size_t mo = mapped_row(p, m);
             if (residual) {
                 for (int c = cbeg; c < cend; c += 32) {
@@ -331,8 +334,8 @@ __device__ __forceinline__ void dense_gemm_body(const CUtensorMap &a_map, const 
     if (PAIR) cluster_sync_all();  // neither CTA may exit while the other can still signal its barriers
     if (warp == 1) {
         tc_fence_after();
-        if (PAIR) tmem_dealloc_pair(tmem_base, 2 * G_BN);
-        else tmem_dealloc(tmem_base, 2 * G_BN);
+        if (PAIR) tmem_dealloc_pair(tmem_base, 2 * Cfg::TMEM_BUF);
+        else tmem_dealloc(tmem_base, 2 * Cfg::TMEM_BUF);
     }
 }
 
@@ -395,22 +398,42 @@ constexpr float kPairTileFactor = 0.95f;  // time of a pair's 256 x 256 tile rel
 void dense_gemm_set_variant(int v) { g_gemm_variant.store((v >= 0 && v <= 4) ? v : 0, std::memory_order_relaxed); }
 int dense_gemm_variant() { return g_gemm_variant.load(std::memory_order_relaxed); }
 
-// Four tilings: one CTA per 128 x 256 tile, per 128 x 128 or 128 x 64 tile (more CTAs streaming the weights when the
-// problem has few rows), a CTA pair per 256 x 256 tile (half the shared-memory traffic per flop).  Cost of the cheapest
-// one in units of one 128 x 256 tile on one SM; the per-tile factors are measured ratios.
+// One CTA per 128 x BN tile (variants 4, 5, 2, 7, 8, 1: more CTAs streaming the weights the narrower it is) or a CTA pair per 256 x 256 tile
+// (3: half the shared-memory traffic per flop; 6: K slices of those).
+static int tile_cols(int variant) {
+    switch (variant) {
+    case 4: return 64;
+    case 5: return 96;
+    case 2: return 128;
+    case 7: return 160;
+    case 8: return 192;
+    default: return 256;
+    }
+}
+
+// Cost of the cheapest tiling in units of one 128 x 256 tile on one SM; the per-tile factors of 64, 128 and 256 columns are measured ratios,
+// the others lie on the line through them.
 static float tiling_cost(int M, int N, int n_sm, int *variant_out) {
-    const int tiles_m = (M + G_BM - 1) / G_BM, tiles_mp = (M + 2 * G_BM - 1) / (2 * G_BM);
-    const int tn256 = (N + 255) / 256, tn128 = (N + 127) / 128, tn64 = (N + 63) / 64, pairs = n_sm / 2;
+    const int tiles_m = (M + G_BM - 1) / G_BM, tiles_mp = (M + 2 * G_BM - 1) / (2 * G_BM), pairs = n_sm / 2;
     auto waves = [](int tiles, int units) { return (tiles + units - 1) / units; };
-    const float cost256 = (float)waves(tiles_m * tn256, n_sm);
-    const float cost128 = N > 128 ? 0.60f * waves(tiles_m * tn128, n_sm) : 1e30f;
-    const float cost64 = N > 64 ? 0.33f * waves(tiles_m * tn64, n_sm) : 1e30f;  // few rows: as many CTAs as possible stream W
-    const float cost_pair = pairs > 0 ? kPairTileFactor * waves(tiles_mp * tn256, pairs) : 1e30f;
-    int variant = (cost_pair <= cost256 && cost_pair <= cost128) ? 3 : (cost128 < cost256 ? 2 : 1);
-    float best = variant == 3 ? cost_pair : (variant == 2 ? cost128 : cost256);
-    if (cost64 < best) {
-        variant = 4;
-        best = cost64;
+    int variant = 1;
+    float best = (float)waves(tiles_m * ((N + 255) / 256), n_sm);
+    if (pairs > 0) {
+        const float c = kPairTileFactor * (float)waves(tiles_mp * ((N + 255) / 256), pairs);
+        if (c <= best) {
+            best = c;
+            variant = 3;
+        }
+    }
+    static const struct { int variant; float factor; } narrow[] = {{8, 0.80f}, {7, 0.70f}, {2, 0.60f}, {5, 0.47f}, {4, 0.33f}};
+    for (const auto &t : narrow) {
+        const int bn = tile_cols(t.variant);
+        if (N <= bn) continue;
+        const float c = t.factor * (float)waves(tiles_m * ((N + bn - 1) / bn), n_sm);
+        if (c < best) {
+            best = c;
+            variant = t.variant;
+        }
     }
     if (variant_out) *variant_out = variant;
     return best;
@@ -461,9 +484,9 @@ static float persistent_us(int M, int N, int nk, int n_sm) {
     const int tm = (M + G_BM - 1) / G_BM;
     auto per = [](int tiles, int units) { return std::max(1.0f, (float)tiles / (float)units); };
     if (v == 3) return 12.0f + 0.31f * (float)nk * per((tm + 1) / 2 * ((N + 255) / 256), n_sm / 2);
-    if (v == 1) return 4.5f + 0.46f * (float)nk * per(tm * ((N + 255) / 256), n_sm);
-    if (v == 2) return 4.0f + 0.36f * (float)nk * per(tm * ((N + 127) / 128), n_sm);
-    return 4.0f + 0.26f * (float)nk * per(tm * ((N + 63) / 64), n_sm);
+    const int bn = tile_cols(v);
+    const float step = bn == 64 ? 0.26f : (bn == 96 ? 0.31f : (bn == 128 ? 0.36f : (bn == 160 ? 0.39f : (bn == 192 ? 0.42f : 0.46f))));
+    return (bn == 256 ? 4.5f : 4.0f) + step * (float)nk * per(tm * ((N + bn - 1) / bn), n_sm);
 }
 
 // Whether a problem goes to the kernel for few rows (gemm_rows.cu), and with which tile width and K slices: the same estimate of a launch
@@ -561,6 +584,14 @@ int dense_gemm(const void *A, int lda, const void *W, GemmParams p, cudaStream_t
     return dense_gemm_one(A, lda, W, p, stream, 0);
 }
 
+template <int BN>
+static int launch_single(const CUtensorMap &amap, const CUtensorMap &wmap, const GemmParams &p, int tiles_m, int n_sm, cudaStream_t stream) {
+    if (int rc = ensure_dyn_smem(dense_gemm_kernel<BN>, GemmCfg<BN, false>::SMEM)) return rc;
+    const int tiles_n = (p.N + BN - 1) / BN, nt = tiles_m * tiles_n;
+    return launch_pdl(dense_gemm_kernel<BN>, dim3(nt < n_sm ? nt : n_sm), dim3(G_THREADS), GemmCfg<BN, false>::SMEM, stream, amap, wmap, p,
+                      tiles_m, tiles_n);
+}
+
 static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, cudaStream_t stream, int forced_variant) {
     if (!A || !W || p.M <= 0 || p.N <= 0 || p.K <= 0) return VLAB200_ERR_ARG;
     if (p.N % 8 || (p.epi == EPI_GATED && p.N % 16) || p.K % 8 || lda % 8 || p.ld_out % 8) return VLAB200_ERR_UNSUPPORTED;
@@ -577,62 +608,41 @@ static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, c
                                  CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }
-    {
-        const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.N};
-        const uint64_t strides[1] = {(uint64_t)p.K * 2};
-        const uint32_t box[2] = {G_BK, 256};
-        int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, dims, strides, box,
-                                 CU_TENSOR_MAP_SWIZZLE_128B);
-        if (rc) return rc;
-    }
     const int n_sm = sm_count();
     if (n_sm <= 0) return cuda_fail(cudaGetLastError(), "sm_count");
     int variant = forced_variant > 0 ? forced_variant : dense_gemm_variant();
     if (variant == 0) tiling_cost(p.M, p.N, n_sm, &variant);
     const int tiles_m = (p.M + G_BM - 1) / G_BM, tiles_mp = (p.M + 2 * G_BM - 1) / (2 * G_BM);
-    const int tn256 = (p.N + 255) / 256, tn128 = (p.N + 127) / 128, tn64 = (p.N + 63) / 64, pairs = n_sm / 2;
-    if (variant == 2 && p.N <= 128) variant = 1;
-    if (variant == 4 && p.N <= 64) variant = 1;
-    const uint64_t wdims[2] = {(uint64_t)p.K, (uint64_t)p.N};
-    const uint64_t wstrides[1] = {(uint64_t)p.K * 2};
-    if (variant == 3 || variant == 6) {
-        const uint32_t box[2] = {G_BK, 128};  // each CTA of a pair stages half of the 256 weight rows
-        int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, wdims, wstrides, box,
+    const int tn256 = (p.N + 255) / 256, pairs = n_sm / 2;
+    const bool pair = variant == 3 || variant == 6;
+    if (!pair && p.N <= tile_cols(variant)) variant = 1;
+    {
+        const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.N};
+        const uint64_t strides[1] = {(uint64_t)p.K * 2};
+        const uint32_t box[2] = {G_BK, (uint32_t)(pair ? 128 : tile_cols(variant))};  // each CTA of a pair stages half of the 256 weight rows
+        int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, dims, strides, box,
                                  CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
-        if (variant == 6) {
-            if (int rc = ensure_dyn_smem(dense_gemm_pair_splitk_kernel, GemmCfg<256, true>::SMEM)) return rc;
-            const int nt = tiles_mp * tn256 * p.ksplit;
-            return launch_pdl(dense_gemm_pair_splitk_kernel, dim3(2 * (nt < pairs ? nt : pairs)), dim3(G_THREADS), GemmCfg<256, true>::SMEM,
-                              stream, amap, wmap, p, tiles_mp, tn256);
-        }
+    }
+    switch (variant) {
+    case 6: {
+        if (int rc = ensure_dyn_smem(dense_gemm_pair_splitk_kernel, GemmCfg<256, true>::SMEM)) return rc;
+        const int nt = tiles_mp * tn256 * p.ksplit;
+        return launch_pdl(dense_gemm_pair_splitk_kernel, dim3(2 * (nt < pairs ? nt : pairs)), dim3(G_THREADS), GemmCfg<256, true>::SMEM,
+                          stream, amap, wmap, p, tiles_mp, tn256);
+    }
+    case 3: {
         if (int rc = ensure_dyn_smem(dense_gemm_pair_kernel, GemmCfg<256, true>::SMEM)) return rc;
         const int nt = tiles_mp * tn256;
         return launch_pdl(dense_gemm_pair_kernel, dim3(2 * (nt < pairs ? nt : pairs)), dim3(G_THREADS), GemmCfg<256, true>::SMEM,
                           stream, amap, wmap, p, tiles_mp, tn256);
-    } else if (variant == 4) {
-        const uint32_t box[2] = {G_BK, 64};
-        int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, wdims, wstrides, box,
-                                 CU_TENSOR_MAP_SWIZZLE_128B);
-        if (rc) return rc;
-        if (int rc = ensure_dyn_smem(dense_gemm_kernel<64>, GemmCfg<64, false>::SMEM)) return rc;
-        const int nt = tiles_m * tn64;
-        return launch_pdl(dense_gemm_kernel<64>, dim3(nt < n_sm ? nt : n_sm), dim3(G_THREADS), GemmCfg<64, false>::SMEM, stream,
-                          amap, wmap, p, tiles_m, tn64);
-    } else if (variant == 2) {
-        const uint32_t box[2] = {G_BK, 128};
-        int rc = make_tensor_map(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, wdims, wstrides, box,
-                                 CU_TENSOR_MAP_SWIZZLE_128B);
-        if (rc) return rc;
-        if (int rc = ensure_dyn_smem(dense_gemm_kernel<128>, GemmCfg<128, false>::SMEM)) return rc;
-        const int nt = tiles_m * tn128;
-        return launch_pdl(dense_gemm_kernel<128>, dim3(nt < n_sm ? nt : n_sm), dim3(G_THREADS), GemmCfg<128, false>::SMEM, stream,
-                          amap, wmap, p, tiles_m, tn128);
-    } else {
-        if (int rc = ensure_dyn_smem(dense_gemm_kernel<256>, GemmCfg<256, false>::SMEM)) return rc;
-        const int nt = tiles_m * tn256;
-        return launch_pdl(dense_gemm_kernel<256>, dim3(nt < n_sm ? nt : n_sm), dim3(G_THREADS), GemmCfg<256, false>::SMEM, stream,
-                          amap, wmap, p, tiles_m, tn256);
+    }
+    case 4: return launch_single<64>(amap, wmap, p, tiles_m, n_sm, stream);
+    case 5: return launch_single<96>(amap, wmap, p, tiles_m, n_sm, stream);
+    case 2: return launch_single<128>(amap, wmap, p, tiles_m, n_sm, stream);
+    case 7: return launch_single<160>(amap, wmap, p, tiles_m, n_sm, stream);
+    case 8: return launch_single<192>(amap, wmap, p, tiles_m, n_sm, stream);
+    default: return launch_single<256>(amap, wmap, p, tiles_m, n_sm, stream);
     }
 }
 
