@@ -17,8 +17,6 @@
 // matrix and two permuted copies of K/V in HBM every layer-step), mask src/models/pi0.cpp:640-651.
 #include <cuda_bf16.h>
 
-#include <algorithm>
-
 #include "gemm.h"
 #include "host_common.h"
 #include "tc5.cuh"
@@ -37,9 +35,11 @@ struct FlashParams {
     int out_hd;    // columns of a head in the output: HD, or the width of the heads that were zero-padded to HD (a multiple of 8)
     int row_major; // the maps' dimensions are (column, head, row) instead of (column, row, item)
     int *status;
-    // key-split mode (few work units): a unit's key blocks are cut over the n_split CTAs of a cluster, which merge their un-normalised O
-    // rows, running maxima and row sums through distributed shared memory
+    // key-split mode (few work units): a unit's key blocks are cut into n_split slices that run as separate work items;
+    // a slice leaves its un-normalised O rows, running maximum and row sum in the workspace for attn_split_combine_kernel
     int n_split;
+    float *ws_o;   // [n_units * n_split][128][HD]
+    float *ws_ml;  // [n_units * n_split][128][2]: maximum (log2 units), row sum
 };
 
 __device__ __forceinline__ float fa_ex2(float x) {
@@ -92,8 +92,6 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     const int nb = p.n_blocks;
     const int ns = SPLIT ? p.n_split : 1;  // key slices per unit
     const int n_work = p.n_units * ns;
-    float m_slice = -INFINITY, l_slice = 0.0f;  // SPLIT: this row's maximum (log2 units) and sum over the slice's keys
-    bool slice_ok = false;
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -118,7 +116,6 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     }
     tc_fence_before();
     __syncthreads();
-    if (SPLIT) cluster_sync_all();  // every CTA of the cluster runs before another one writes to its shared memory
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     if (threadIdx.x == 0) {  // kernel parameters: independent of the previous kernel
@@ -344,12 +341,26 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             // ---- epilogue: O / l -> bf16 -> out ----
             ok = mbar_wait(o_done, ui & 1u, wc, DEV_TIMEOUT_ACCUM);
             if (!ok) break;
-            slice_ok = true;
             tc_fence_after();
-            if constexpr (SPLIT) {  // one work item per CTA: its rows are merged with the other slices' below
-                m_slice = m_used;
-                l_slice = l_sum;
-                break;
+            if constexpr (SPLIT) {
+                // this slice's un-normalised rows and their (maximum, sum): attn_split_combine_kernel merges the slices
+                const size_t wrow = (size_t)wu * 128 + qtr * 32 + lane;
+                float4 *wo = reinterpret_cast<float4 *>(p.ws_o + wrow * HD);
+                for (int c = 0; c < HD; c += 32) {
+                    uint32_t ov[32];
+                    tmem_ld32(tmem_base + lane_sel + (uint32_t)c, ov);
+                    tmem_ld_wait();
+                    if (row_ok) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            wo[(c >> 2) + e] = make_float4(__uint_as_float(ov[4 * e]), __uint_as_float(ov[4 * e + 1]),
+                                                           __uint_as_float(ov[4 * e + 2]), __uint_as_float(ov[4 * e + 3]));
+                    }
+                }
+                if (row_ok) *reinterpret_cast<float2 *>(p.ws_ml + wrow * 2) = make_float2(m_used, l_sum);
+                tc_fence_before();
+                mbar_arrive(o_free);
+                continue;
             }
             const float inv = 1.0f / l_sum;
             __nv_bfloat16 *dst = p.out + (((size_t)obs * p.S + tok) * p.n_q + kvh * p.g + head_l) * p.out_hd;
@@ -380,71 +391,6 @@ attn_flash_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             }
             tc_fence_before();
             mbar_arrive(o_free);
-        }
-    }
-    if constexpr (SPLIT) {
-        // CTA r of the cluster merges rows [128 r / ns, 128 (r + 1) / ns) of the unit: every CTA sends it those rows of its O, [slice][row][HD]
-        // with a row's 16-byte pieces rotated by the row (lanes hold rows), over the drained Q, K and V tiles.
-        constexpr int PIECES = HD / 4;
-        static_assert((128 + 7) * (HD + 2) * 4 <= L::BAR_OFF, "up to 8 slices of 128 / slices rows, rounded up, with maximum and sum");
-        const int rank = (int)cluster_ctarank();
-        const int rows_max = (128 + ns - 1) / ns, o_bytes = ns * rows_max * HD * 4;
-        __syncwarp();
-        cluster_sync_all();  // every slice's products are done: nothing reads the tiles any more
-        if (warp < 4 && __all_sync(0xffffffffu, slice_ok)) {
-            const int r = warp * 32 + lane;
-            int owner = r * ns / 128;
-            while (128 * (owner + 1) / ns <= r) ++owner;
-            const int local = r - 128 * owner / ns;
-            const uint32_t base = cluster_addr(smem_u32(smem), (uint32_t)owner);
-            const uint32_t dst = base + (uint32_t)((rank * rows_max + local) * HD * 4);
-            for (int c = 0; c < HD; c += 32) {
-                uint32_t ov[32];
-                tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, ov);
-                tmem_ld_wait();
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    st_cluster_v4(dst + (uint32_t)((((c >> 2) + e) ^ (r & (PIECES - 1) & 31)) * 16), ov[4 * e], ov[4 * e + 1], ov[4 * e + 2], ov[4 * e + 3]);
-            }
-            st_cluster_v2(base + (uint32_t)(o_bytes + (rank * rows_max + local) * 8), __float_as_uint(m_slice), __float_as_uint(l_slice));
-        }
-        __syncwarp();
-        cluster_sync_all();
-        const int row_lo = 128 * rank / ns, n_rows = 128 * (rank + 1) / ns - row_lo;
-        const int unit = (int)blockIdx.x / ns, item = unit / p.n_mt, mt = unit % p.n_mt, obs = item / p.n_kv, kvh = item % p.n_kv;
-        const float2 *mls = reinterpret_cast<const float2 *>(smem + o_bytes);
-        for (int lr = warp; lr < n_rows && !*abort_flag; lr += FA_THREADS / 32) {  // a warp per row: M = max m_s; O = sum O_s 2^(m_s - M); l alike
-            const int r = row_lo + lr, row = mt * 128 + r;
-            if (row >= p.R) break;
-            float M = -INFINITY, l = 0.0f;
-            for (int t = 0; t < ns; ++t) M = fmaxf(M, mls[t * rows_max + lr].x);
-            float4 acc[(PIECES + 31) / 32];
-#pragma unroll
-            for (int i = 0; i < (PIECES + 31) / 32; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int t = 0; t < ns; ++t) {
-                const float2 ml = mls[t * rows_max + lr];
-                const float w = ml.x == -INFINITY ? 0.0f : fa_ex2(ml.x - M);
-                l = fmaf(ml.y, w, l);
-                const float4 *src = reinterpret_cast<const float4 *>(smem) + (size_t)(t * rows_max + lr) * PIECES;
-#pragma unroll
-                for (int i = 0; i < (PIECES + 31) / 32; ++i) {
-                    const int piece = lane + 32 * i;
-                    if (piece < PIECES) {
-                        const float4 v = src[piece ^ (r & (PIECES - 1) & 31)];
-                        acc[i].x = fmaf(v.x, w, acc[i].x); acc[i].y = fmaf(v.y, w, acc[i].y);
-                        acc[i].z = fmaf(v.z, w, acc[i].z); acc[i].w = fmaf(v.w, w, acc[i].w);
-                    }
-                }
-            }
-            const float inv = 1.0f / l;
-            const int head_l = row / p.S, tok = row % p.S;
-            uint2 *dst = reinterpret_cast<uint2 *>(p.out + (((size_t)obs * p.S + tok) * p.n_q + kvh * p.g + head_l) * HD);
-#pragma unroll
-            for (int i = 0; i < (PIECES + 31) / 32; ++i) {
-                if (lane + 32 * i >= PIECES) break;
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[i].x * inv, acc[i].y * inv), hi = __floats2bfloat162_rn(acc[i].z * inv, acc[i].w * inv);
-                dst[lane + 32 * i] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-            }
         }
     }
     tc_fence_before();
@@ -915,10 +861,62 @@ attn_flash_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     }
 }
 
+// Merges the key slices of every (unit, row): M = max_s m_s; O = sum_s O_s 2^(m_s - M); l = sum_s l_s 2^(m_s - M);
+// out = bf16(O / l), slices in order.  One warp per row, 2 x HD / 64 columns per lane; the slices' rows are requested
+// four at a time (one after the other, each a round trip to L2, the merge took 8 us of an attention's 20 at five observations).
+template <int HD>
+__global__ void __launch_bounds__(256) attn_split_combine_kernel(const FlashParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp_g = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (warp_g >= p.n_units * 128) return;
+    const int unit = warp_g >> 7, r = warp_g & 127;
+    const int item = unit / p.n_mt, mt = unit % p.n_mt;
+    const int obs = item / p.n_kv, kvh = item % p.n_kv;
+    const int row = mt * 128 + r;
+    if (row >= p.R) return;
+    const int head_l = row / p.S, tok = row % p.S, ns = p.n_split;
+    constexpr int NV = HD / 64;  // float2 pieces per lane
+    const float2 *src = reinterpret_cast<const float2 *>(p.ws_o) + ((size_t)unit * ns * 128 + r) * (HD / 2) + lane;
+    const float *mls = p.ws_ml + ((size_t)unit * ns * 128 + r) * 2;
+    float2 acc[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) acc[i] = make_float2(0.0f, 0.0f);
+    float l = 0.0f, M = -INFINITY;
+    for (int s = lane; s < ns; s += 32) M = fmaxf(M, mls[(size_t)s * 256]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+    for (int s0 = 0; s0 < ns; s0 += 4) {
+        float2 v[4][NV], ml[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int s = min(s0 + t, ns - 1);
+            ml[t] = *reinterpret_cast<const float2 *>(mls + (size_t)s * 256);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[t][i] = src[(size_t)s * 128 * (HD / 2) + i * 32];
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (s0 + t >= ns) break;
+            const float w = ml[t].x == -INFINITY ? 0.0f : fa_ex2(ml[t].x - M);
+            l = fmaf(ml[t].y, w, l);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                acc[i].x = fmaf(v[t][i].x, w, acc[i].x);
+                acc[i].y = fmaf(v[t][i].y, w, acc[i].y);
+            }
+        }
+    }
+    const float inv = 1.0f / l;
+    __nv_bfloat16 *dst = p.out + ((size_t)obs * p.S + tok) * ((size_t)p.n_q * HD) + (size_t)(kvh * p.g + head_l) * HD;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) reinterpret_cast<__nv_bfloat162 *>(dst)[i * 32 + lane] = __floats2bfloat162_rn(acc[i].x * inv, acc[i].y * inv);
+}
+
 template <int HD>
 static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len,
-                        int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, bool key_slices,
-                        int row_major_hd) {
+                        int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws,
+                        size_t ws_bytes, int row_major_hd) {
     using L = FlashSmem<HD>;
     int *status = device_status_ptr();
     if (!status) return cuda_fail(cudaGetLastError(), "device_status_ptr");
@@ -976,7 +974,7 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
         // 19.97 -> 19.25 ms; with one to three blocks of 64 keys it loses: 64 tokens 1.82 -> 1.88 ms); or when forced for tests
         const int n_pair_units = st->n_obs * st->n_kv * ((p.n_mt + 1) / 2), pairs = n_sm / 2;
         const int forced = dense_gemm_variant();
-        const bool one_wave = p.n_units <= n_sm && p.n_blocks >= 4 && !(key_slices && !row_major_hd && p.n_units * 2 <= n_sm);
+        const bool one_wave = p.n_units <= n_sm && p.n_blocks >= 4 && !(ws && !row_major_hd && p.n_units * 2 <= n_sm);
         if (p.n_mt >= 2 && forced != 1 && (forced == 3 || n_pair_units >= pairs || one_wave)) {
             using LP = FlashPairSmem<HD>;
             // each CTA stages 64 of a block's 128 keys (the one-CTA kernel's K map has that box) and, for V, all
@@ -994,16 +992,21 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
         }
     }
     p.n_split = 1;
-    if (key_slices && !p.row_major && p.n_units * 2 <= n_sm && p.n_blocks >= 4) {
-        // few units (a handful of observations): every unit's keys are cut over the CTAs of a cluster, at least two 64-key blocks each
-        // (flash-decoding).  With the slices' rows merged by a second kernel through global memory, that kernel took 7 to 8 us of 20 at
-        // five observations of 8 heads on one, 867 keys.
-        if (int rc = ensure_dyn_smem(attn_flash_kernel<HD, true>, L::TOTAL)) return rc;
-        for (int n = std::min(8, p.n_blocks / 2); n >= 2; --n) {
-            if (p.n_units * n > n_sm || p.n_units > max_active_clusters(reinterpret_cast<const void *>(attn_flash_kernel<HD, true>), FA_THREADS, L::TOTAL, n))
-                continue;
-            p.n_split = n;
-            return launch_pdl_cluster(attn_flash_kernel<HD, true>, dim3(p.n_units * n), dim3(FA_THREADS), L::TOTAL, n, stream, qmap, kmap, vmap, p);
+    if (ws && !p.row_major && p.n_units * 2 <= n_sm && p.n_blocks >= 4) {
+        // few units (one observation): cut every unit's keys into slices of at least two 64-key blocks so that the slices fill
+        // the machine, then merge them (flash-decoding)
+        int n_split = n_sm / p.n_units;
+        if (n_split > p.n_blocks / 2) n_split = p.n_blocks / 2;  // two to four blocks per slice measured alike, one slower
+        const size_t need = (size_t)p.n_units * n_split * 128 * (HD + 2) * sizeof(float);
+        if (n_split >= 2 && need <= ws_bytes) {
+            p.n_split = n_split;
+            p.ws_o = ws;
+            p.ws_ml = ws + (size_t)p.n_units * n_split * 128 * HD;
+            if (int rc = ensure_dyn_smem(attn_flash_kernel<HD, true>, L::TOTAL)) return rc;
+            if (int rc = launch_pdl(attn_flash_kernel<HD, true>, dim3(p.n_units * n_split), dim3(FA_THREADS), L::TOTAL, stream, qmap, kmap,
+                                    vmap, p))
+                return rc;
+            return launch_pdl(attn_split_combine_kernel<HD>, dim3((p.n_units * 128 + 7) / 8), dim3(256), 0, stream, p);
         }
     }
     if (int rc = ensure_dyn_smem(attn_flash_kernel<HD>, L::TOTAL)) return rc;
@@ -1013,17 +1016,17 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
 }
 
 int attention_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len,
-                    int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, bool key_slices,
-                    int row_major_hd) {
+                    int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws,
+                    size_t ws_bytes, int row_major_hd) {
     // a key block may reach into the next observation's rows (hidden, but multiplied by 0): several need whole blocks
     if (row_major_hd && (row_major_hd % 8 || row_major_hd > st->head_dim || n_q != st->n_kv || kv_len != S || (st->n_obs > 1 && S % FP_BKV)))
         return VLAB200_ERR_UNSUPPORTED;
     if (st->head_dim == 256)
-        return launch_flash<256>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, key_slices, row_major_hd);
+        return launch_flash<256>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes, row_major_hd);
     if (st->head_dim == 128)
-        return launch_flash<128>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, key_slices, row_major_hd);
+        return launch_flash<128>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes, row_major_hd);
     if (st->head_dim == 64)
-        return launch_flash<64>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, key_slices, row_major_hd);
+        return launch_flash<64>(st, layer, q, out, S, n_q, kv_len, mask_mode, pad_ranges, stream, softmax_scale, ws, ws_bytes, row_major_hd);
     return VLAB200_ERR_UNSUPPORTED;
 }
 

@@ -37,7 +37,7 @@
 namespace vb {
 
 int attention_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len,
-                    int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, bool key_slices,
+                    int mask_mode, const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws, size_t ws_bytes,
                     int row_major_hd);
 
 __device__ __forceinline__ float vit_block_sum(float v, float *red) {
@@ -569,7 +569,7 @@ int bitvla_vit_cuda_forward(bitvla_vit_cuda_ctx *ctx, const void *d_patches, voi
         // the attention reads q, k and v as column ranges of the projection and leaves packed heads: no head split, no merge
         __nv_bfloat16 *qkv = ctx->qkv.as<__nv_bfloat16>();
         vlab200_kv_store view{qkv + H, qkv + 2 * H, 1, 1, heads, hp, S, 0};
-        if ((rc = vb::attention_flash(&view, 0, qkv, ctx->att.p, S, heads, S, 0, nullptr, cs, scale, false, hd))) return fail("attention", rc);
+        if ((rc = vb::attention_flash(&view, 0, qkv, ctx->att.p, S, heads, S, 0, nullptr, cs, scale, nullptr, 0, hd))) return fail("attention", rc);
         if ((rc = vb::launch_pdl(vb::vit_quant_rows_kernel<vb::VIT_Q_WARPS, 1>, dim3(S), dim3(32 * vb::VIT_Q_WARPS), 0, cs, ctx->att.as<__nv_bfloat16>(),
                                  H, H, a8, s)))
             return fail("attention quantisation", rc);
@@ -595,7 +595,7 @@ int bitvla_vit_cuda_forward(bitvla_vit_cuda_ctx *ctx, const void *d_patches, voi
                                  bf(w.v_b), ctx->q.as<__nv_bfloat16>(), ctx->kp.as<__nv_bfloat16>(), ctx->vp.as<__nv_bfloat16>(), S, heads, hd, hp)))
             return fail("head split", rc);
         vlab200_kv_store view{ctx->kp.p, ctx->vp.p, 1, 1, heads, hp, S, 0};
-        if ((rc = vb::attention_flash(&view, 0, ctx->q.p, ctx->att.p, S, heads, S, 0, nullptr, cs, scale, false, 0))) return fail("attention", rc);
+        if ((rc = vb::attention_flash(&view, 0, ctx->q.p, ctx->att.p, S, heads, S, 0, nullptr, cs, scale, nullptr, 0, 0))) return fail("attention", rc);
         if ((rc = vb::launch_pdl(vb::vit_merge_quant_kernel, dim3(S), dim3(256), (size_t)H * 4, cs, ctx->att.as<__nv_bfloat16>(), heads, hd,
                                  hp, a8, s)))
             return fail("merge", rc);

@@ -305,6 +305,8 @@ static bool rope_in_rows(int M, int n_heads, int hd, bool rms) {
     if (M <= kFewRows || dense_gemm_variant() != 0) return M <= kFewRows;
     return (M + 127) / 128 * (n_heads * (hd / 64)) <= (rms ? 2 : 4) * sm_count();
 }
+// key-split attention: at most one (unit, slice) per SM, 128 rows of head_dim + 2 floats each
+static size_t kAttnWsBytes(int hd) { return (size_t)160 * 128 * (hd + 2) * sizeof(float); }
 }
 
 // ------------------------------------------------------------------------ engine --
@@ -316,6 +318,7 @@ struct vlab200_engine {
     // prepared weights
     std::vector<vb::DevBuf> wqkv, wo, wgu, wdown, wkx, wvx;
     vb::DevBuf w_ain, b_ain, w_sp, b_sp, w_at1l, tvec, w_at2, b_at2, out_norm, w_aout, b_aout;
+    vb::DevBuf attn_ws;  // float32 workspace of the key-split attention path (calls with one or two observations)
     vb::DevBuf mods;  // pi0.5: float32 [n_layers][2][steps][3H] (scale | shift | gate of the two norms), then [steps][3H] final
     // workspace
     vb::DevBuf k_pages, v_pages, h, hb, q, att, g, a, m1, x, rope_self, rope_cross, tmp_bf, x_stage, state_stage, pad_stage, vbuf;
@@ -445,7 +448,8 @@ static int engine_build(vlab200_engine *e, const vlab200_policy_weights *w) {
         (rc = e->rope_cross.alloc((size_t)2 * e->S * (hd / 2) * 4)) ||
         (rc = e->tmp_bf.alloc((size_t)2 * B * e->P * kvf * 2)) || (rc = e->x_stage.alloc(Mc * A * 4)) ||
         (rc = e->state_stage.alloc(B * (size_t)(c.state_dim > 0 ? c.state_dim : 1) * 4)) ||
-        (rc = e->pad_stage.alloc(B * 2 * 4)) || (rc = e->vbuf.alloc(M * A * 4)))
+        (rc = e->pad_stage.alloc(B * 2 * 4)) || (rc = e->vbuf.alloc(M * A * 4)) ||
+        (rc = e->attn_ws.alloc(kAttnWsBytes(hd))))
         return rc;
     VB_CUDA(cudaMemset(e->h.p, 0, M * H * 4));
     VB_CUDA(cudaMemset(e->hb.p, 0, M * H * 2));
@@ -508,7 +512,8 @@ static int layer_stage(vlab200_engine *e, int l, int stage, int n_obs, const flo
     case 1: {
         const int kv_len = self ? e->P + S : e->P;
         const int mode = self ? (c.model == 0 ? 1 : 2) : 0;
-        return attention_sliced(&live, 0, e->q.p, e->att.p, S, c.n_q, kv_len, mode, pad_ranges, cs, true);
+        return attention_ws(&live, 0, e->q.p, e->att.p, S, c.n_q, kv_len, mode, pad_ranges, cs, e->attn_ws.as<float>(),
+                            kAttnWsBytes(hd));
     }
     case 2: {
         GemmParams p{};
@@ -563,7 +568,7 @@ static int ada_layer(vlab200_engine *e, int l, int step, int n_obs, const float 
         return rc;
     }
     // no mask: every action token sees the prefix and every action token (soft_max_ext without a mask, pi05.cpp:264)
-    if ((rc = attention_sliced(&live, 0, e->q.p, e->att.p, S, c.n_q, e->P + S, 0, nullptr, cs, true)))
+    if ((rc = attention_ws(&live, 0, e->q.p, e->att.p, S, c.n_q, e->P + S, 0, nullptr, cs, e->attn_ws.as<float>(), kAttnWsBytes(hd))))
         return rc;
     p = GemmParams{};
     p.M = M; p.N = H; p.K = e->qf; p.epi = EPI_RESIDUAL; p.colscale = mod_in + 2 * H;

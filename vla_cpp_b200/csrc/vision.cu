@@ -27,7 +27,7 @@
 
 namespace vb {
 int attention_flash(const vlab200_kv_store *st, int layer, const void *q, void *out, int S, int n_q, int kv_len, int mask_mode,
-                    const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, bool key_slices, int row_major_hd);
+                    const int32_t *pad_ranges, cudaStream_t stream, float softmax_scale, float *ws, size_t ws_bytes, int row_major_hd);
 }
 
 struct vlab200_vision {
@@ -388,7 +388,7 @@ int32_t vlab200_vision_run(vlab200_vision *v, const void *pixels, int32_t pixels
         if (v->packed) {
             __nv_bfloat16 *qkv = v->qkv.as<__nv_bfloat16>();
             vlab200_kv_store view{qkv + qf, qkv + 2 * qf, 1, n_views, c.n_heads, v->att_hd, np, 0};
-            if ((rc = vb::attention_flash(&view, 0, qkv, v->att.p, np, c.n_heads, np, 0, nullptr, cs, 1.0f / std::sqrt((float)v->hd), false, v->hd)))
+            if ((rc = vb::attention_flash(&view, 0, qkv, v->att.p, np, c.n_heads, np, 0, nullptr, cs, 1.0f / std::sqrt((float)v->hd), nullptr, 0, v->hd)))
                 return rc;
         } else {
             if ((rc = vb::rope_split(v->qkv.p, cos_t, sin_t, v->q.p, v->kpg.p, v->vpg.p, M, np, c.n_heads, c.n_heads, c.n_heads, v->hd_pad,
