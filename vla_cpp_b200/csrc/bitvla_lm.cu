@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(256) norm_quant_kernel(__nv_bfloat16 *__restri
 // next row's loads in flight and the norm's weights kept: 4,800 rows of 6,912 took 34.7 us with a CTA per row (4 resident per SM).
 constexpr int NQ_BLOCKS(int mode, int nv) { return nv == 2 ? 4 : (mode == NQ_PLAIN ? 3 : 2); }  // CTAs per SM
 template <int MODE, int NV>
-__global__ void __launch_bounds__(256, NQ_BLOCKS(MODE, NV)) norm_quant_vec_kernel(__nv_bfloat16 *__restrict__ in,
-                                                                            const __nv_bfloat16 *__restrict__ add,
+__global__ void __launch_bounds__(256, NQ_BLOCKS(MODE, NV)) norm_quant_vec_kernel(__nv_bfloat16 *in,
+                                                                            const __nv_bfloat16 *add,
                                                                             const __nv_bfloat16 *__restrict__ w, float eps, int M, int K,
                                                                             int8_t *__restrict__ q_out, float *__restrict__ s_out,
                                                                             __nv_bfloat16 *__restrict__ out_bf, int w_early) {

@@ -259,7 +259,7 @@ __device__ __forceinline__ float vit_row_sum(const float (&x)[8], int n_warps, f
 // read before the dependency wait (nothing that may still run writes them).  With a whole row in one warp the 1,200 instructions of a
 // lane took longer than the block barriers it saved (5.5 us inside the tower, the scalar kernel 5.0).
 constexpr int VIT_LN_WARPS = 8;
-__global__ void __launch_bounds__(32 * VIT_LN_WARPS) vit_ln_quant_rows_kernel(__nv_bfloat16 *__restrict__ h, const __nv_bfloat16 *__restrict__ add,
+__global__ void __launch_bounds__(32 * VIT_LN_WARPS) vit_ln_quant_rows_kernel(__nv_bfloat16 *h, const __nv_bfloat16 *add,
                                                                               const __nv_bfloat16 *__restrict__ add_bias,
                                                                               const __nv_bfloat16 *__restrict__ ln_w,
                                                                               const __nv_bfloat16 *__restrict__ ln_b, float eps, int K,

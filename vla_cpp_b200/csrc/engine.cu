@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) adarms_norm_kernel(const float *__restric
 // The same with the row in registers (H % 4 == 0, H <= 128 NV): one pass, 16-byte loads all in flight, and the modulation, which is
 // computed when the engine is built, read before the dependency wait.
 template <int NV>
-__global__ void __launch_bounds__(128) adarms_norm_vec_kernel(const float *__restrict__ x, const float *__restrict__ mod,
+__global__ void __launch_bounds__(128) adarms_norm_vec_kernel(const float *x, const float *__restrict__ mod,
                                                               __nv_bfloat16 *__restrict__ y, int M, int H, float eps) {
     const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, H4 = H >> 2;
     float4 sc[NV], sh[NV], v[NV];

@@ -32,6 +32,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 // visible, so everything before it (barrier set-up, TMEM allocation, descriptor prefetch) overlaps the
 // predecessor's tail.  pdl_launch_dependents() lets the successor start launching; it never relaxes what
 // the successor's own pdl_wait() waits for.  Both are no-ops for a kernel launched the ordinary way.
+// A kernel that reads weights ahead of the wait takes what the predecessor writes through pointers without __restrict__: loads through
+// const __restrict__ ones count as invariant, and the compiler may move those across the wait too.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -115,7 +115,7 @@ __global__ void layernorm_kernel(const float *__restrict__ x, const float *__res
 // are in flight together: H % 4 == 0, H <= 128 * NV.  What bounds it is one round trip to L2 and the hand-over between kernels, which
 // is why it takes part in programmatic dependent launch: 768 x 1152 took 9.2 us with three dependent passes over the row.
 template <int NV>
-__global__ void __launch_bounds__(128) layernorm_vec_kernel(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ b,
+__global__ void __launch_bounds__(128) layernorm_vec_kernel(const float *x, const float *__restrict__ w, const float *__restrict__ b,
                                                             __nv_bfloat16 *__restrict__ out, int M, int H, float eps, int np, int grid,
                                                             int shuffle) {
     const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, H4 = H >> 2;
