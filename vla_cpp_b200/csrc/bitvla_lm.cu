@@ -10,7 +10,7 @@
 //   norm_quant_kernel   [residual add ->] RMSNorm (bf16 rounding as the reference) -> per-token
 //                       absmax int8; one pass over the row, nothing but int8 + scale written
 //   ternary GEMM        q, k, v as ONE matrix (rows concatenated at set_layer, one weight scale
-//                       per 'group' rows through ws_num); heads of 128 leave it rotated and split where a tile holds whole heads
+//                       per 'group' rows through ws_num); heads of 128 leave it rotated and split where a tile holds one head
 //   rope_split_kernel   otherwise: NeoX RoPE on q and k, head split, K / V rows into the attention pages
 //   attention           streaming tcgen05 kernel, no score matrix, no repeated K/V
 //   norm_quant_kernel   attn sub-norm -> int8
@@ -619,7 +619,7 @@ extern "C" int32_t vlab200_bitvla_lm_forward(vlab200_bitvla_lm *ctx, const void 
         if (L == 0) rc = vb::launch_norm_quant<vb::NQ_PLAIN>(ctx->h.p, nullptr, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st, 1);
         else rc = vb::launch_norm_quant<vb::NQ_ADD>(ctx->h.p, ctx->proj.p, l.w.attn_norm_w, ctx->eps, M, H, a8, s, nullptr, st, 1);
         if (rc) break;
-        // the rotation in the product's epilogue where a tile holds whole heads (same bits); the stage dump wants the projection itself
+        // the rotation in the product's epilogue where a tile holds one head (same bits); the stage dump wants the projection itself
         const bool rope = can_rope && !dl;
         rc = linear(l.qkv_packed.p, ctx->qkv.p, l.qkv_ws.as<float>(), ctx->qkv_ws_num, hq + 2 * hkv, H, 0, rope);
         if (rc) break;

@@ -132,7 +132,7 @@ struct TernaryCall {
     int w_early;       // the packed weights were complete before any kernel that may still run: they are read before the dependency wait
 };
 int ternary_linear(const TernaryCall &c, cudaStream_t st);
-bool ternary_can_rope(int M, int N, int K);  // the tiling that would be taken has whole heads of 128 columns in a tile
+bool ternary_can_rope(int M, int N, int K);  // the tiling that would be taken has a head of 128 columns per tile
 
 // A checkpoint tensor ([d1][d0], d1 == 1 for vectors, d1 < 0: d0 elements of any shape; f32 / f16 / bf16 in the file) uploaded as bf16 or float32,
 // optionally with the Gemma-norm "+1" (gguf.cu).  VLAB200_OK or an error with the last-error text set.

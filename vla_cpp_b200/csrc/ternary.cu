@@ -329,64 +329,61 @@ __device__ __forceinline__ void tern_epilogue_tile(uint32_t lane_addr, uint8_t *
     uint8_t *mine = stg + lane * 128;
     const uint32_t sw = (uint32_t)(lane & 7);
     const int m = m_first + lane;
-    if constexpr (BN >= 128) {
+    if constexpr (BN == 128) {
         if (e.rope.cos_t) {
             // Heads of 128: 32 columns of a head's first half and the 32 they are rotated with make a row's 128-byte line of the staging area.
-            // The rotation works on the rounded projection and rounds again, as rope_split does.
+            // The rotation works on the rounded projection and rounds again, as rope_split does.  Not for the pair kernel, whose epilogue of a
+            // thousand rows hides behind the next tile's products only as long as it is short.
             const TernaryRope &rp = e.rope;
             const float *cs_row = rp.cos_t + (size_t)(min(m, M - 1) % rp.seq) * 64, *sn_row = rp.sin_t + (size_t)(min(m, M - 1) % rp.seq) * 64;
+            const int head = n0 / 128;
+            const bool rot = head < rp.n_q + rp.n_kv;
+            const float cs = __fdiv_rn(ws[n0 / group], sm);
 #pragma unroll 1
-            for (int c = 0; c < BN; c += 128) {
-                const int n = n0 + c, head = n / 128;
-                if (n >= N) break;
-                const bool rot = head < rp.n_q + rp.n_kv;
-                const float cs = __fdiv_rn(ws[n / group], sm);
+            for (int k0 = 0; k0 < 64; k0 += 32) {
 #pragma unroll 1
-                for (int k0 = 0; k0 < 64; k0 += 32) {
-#pragma unroll 1
-                    for (int k = 0; k < 32; k += 16) {
-                        uint32_t lo[16], hi[16], wl[8], wh[8];
-                        tmem_ld16(lane_addr + (uint32_t)(c + k0 + k), lo);
-                        tmem_ld16(lane_addr + (uint32_t)(c + 64 + k0 + k), hi);
-                        tmem_ld_wait();
-                        tern_finish<16>(lo, cs, nullptr, 0, wl);
-                        tern_finish<16>(hi, cs, nullptr, 0, wh);
-                        if (rot) {
+                for (int k = 0; k < 32; k += 16) {
+                    uint32_t lo[16], hi[16], wl[8], wh[8];
+                    tmem_ld16(lane_addr + (uint32_t)(k0 + k), lo);
+                    tmem_ld16(lane_addr + (uint32_t)(64 + k0 + k), hi);
+                    tmem_ld_wait();
+                    tern_finish<16>(lo, cs, nullptr, 0, wl);
+                    tern_finish<16>(hi, cs, nullptr, 0, wh);
+                    if (rot) {
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float4 co = __ldg(reinterpret_cast<const float4 *>(cs_row + k0 + k) + i), si = __ldg(reinterpret_cast<const float4 *>(sn_row + k0 + k) + i);
-                                const float cv[4] = {co.x, co.y, co.z, co.w}, sv[4] = {si.x, si.y, si.z, si.w};
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 co = __ldg(reinterpret_cast<const float4 *>(cs_row + k0 + k) + i), si = __ldg(reinterpret_cast<const float4 *>(sn_row + k0 + k) + i);
+                            const float cv[4] = {co.x, co.y, co.z, co.w}, sv[4] = {si.x, si.y, si.z, si.w};
 #pragma unroll
-                                for (int j = 0; j < 2; ++j) {
-                                    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&wl[2 * i + j]));
-                                    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&wh[2 * i + j]));
-                                    wl[2 * i + j] = pack_bf16(a.x * cv[2 * j] - b.x * sv[2 * j], a.y * cv[2 * j + 1] - b.y * sv[2 * j + 1]);
-                                    wh[2 * i + j] = pack_bf16(b.x * cv[2 * j] + a.x * sv[2 * j], b.y * cv[2 * j + 1] + a.y * sv[2 * j + 1]);
-                                }
+                            for (int j = 0; j < 2; ++j) {
+                                const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&wl[2 * i + j]));
+                                const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&wh[2 * i + j]));
+                                wl[2 * i + j] = pack_bf16(a.x * cv[2 * j] - b.x * sv[2 * j], a.y * cv[2 * j + 1] - b.y * sv[2 * j + 1]);
+                                wh[2 * i + j] = pack_bf16(b.x * cv[2 * j] + a.x * sv[2 * j], b.y * cv[2 * j + 1] + a.y * sv[2 * j + 1]);
                             }
                         }
-                        const uint32_t p0 = (uint32_t)(k >> 3);
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            *reinterpret_cast<uint4 *>(mine + (((p0 + i) ^ sw) << 4)) = make_uint4(wl[4 * i], wl[4 * i + 1], wl[4 * i + 2], wl[4 * i + 3]);
-                            *reinterpret_cast<uint4 *>(mine + (((4 + p0 + i) ^ sw) << 4)) = make_uint4(wh[4 * i], wh[4 * i + 1], wh[4 * i + 2], wh[4 * i + 3]);
-                        }
                     }
-                    __syncwarp();
+                    const uint32_t p0 = (uint32_t)(k >> 3);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int rr = (lane >> 3) + 4 * i, ch = lane & 7, mr = m_first + rr;
-                        const uint4 v = *reinterpret_cast<const uint4 *>(stg + rr * 128 + (((uint32_t)ch ^ (uint32_t)(rr & 7)) << 4));
-                        if (mr >= M) continue;
-                        const size_t sq = mr / rp.seq, tok = mr % rp.seq;
-                        __nv_bfloat16 *dst;
-                        if (head < rp.n_q) dst = static_cast<__nv_bfloat16 *>(rp.q) + ((sq * rp.n_q + head) * rp.seq + tok) * 128;
-                        else if (rot) dst = static_cast<__nv_bfloat16 *>(rp.k_pages) + ((sq * rp.n_kv + head - rp.n_q) * rp.cap + tok) * 128;
-                        else dst = static_cast<__nv_bfloat16 *>(rp.v_pages) + ((sq * rp.n_kv + head - rp.n_q - rp.n_kv) * rp.cap + tok) * 128;
-                        *reinterpret_cast<uint4 *>(dst + k0 + (ch & 3) * 8 + (ch >> 2) * 64) = v;
+                    for (int i = 0; i < 2; ++i) {
+                        *reinterpret_cast<uint4 *>(mine + (((p0 + i) ^ sw) << 4)) = make_uint4(wl[4 * i], wl[4 * i + 1], wl[4 * i + 2], wl[4 * i + 3]);
+                        *reinterpret_cast<uint4 *>(mine + (((4 + p0 + i) ^ sw) << 4)) = make_uint4(wh[4 * i], wh[4 * i + 1], wh[4 * i + 2], wh[4 * i + 3]);
                     }
-                    __syncwarp();
                 }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int rr = (lane >> 3) + 4 * i, ch = lane & 7, mr = m_first + rr;
+                    const uint4 v = *reinterpret_cast<const uint4 *>(stg + rr * 128 + (((uint32_t)ch ^ (uint32_t)(rr & 7)) << 4));
+                    if (mr >= M) continue;
+                    const size_t sq = mr / rp.seq, tok = mr % rp.seq;
+                    __nv_bfloat16 *dst;
+                    if (head < rp.n_q) dst = static_cast<__nv_bfloat16 *>(rp.q) + ((sq * rp.n_q + head) * rp.seq + tok) * 128;
+                    else if (rot) dst = static_cast<__nv_bfloat16 *>(rp.k_pages) + ((sq * rp.n_kv + head - rp.n_q) * rp.cap + tok) * 128;
+                    else dst = static_cast<__nv_bfloat16 *>(rp.v_pages) + ((sq * rp.n_kv + head - rp.n_q - rp.n_kv) * rp.cap + tok) * 128;
+                    *reinterpret_cast<uint4 *>(dst + k0 + (ch & 3) * 8 + (ch >> 2) * 64) = v;
+                }
+                __syncwarp();
             }
             return;
         }
@@ -1089,7 +1086,7 @@ int ternary_linear(const TernaryCall &c, cudaStream_t st) {
     else if (path == 3) t = {256, 1};
     else if ((path & 0xff) == 64 || (path & 0xff) == 128) t = {path & 0xff, (path >> 8) > 1 ? path >> 8 : 1};
     if (t.slices != 1 && ((t.slices != 2 && t.slices != 4) || K / GEMM_BK < t.slices || e.gate_up)) return VLAB200_ERR_UNSUPPORTED;
-    if (e.rope.cos_t && (t.bn < 128 || t.slices != 1 || N % 128 || c.acc || e.bias || e.gate_up || (N / ws_num) % 128)) return VLAB200_ERR_UNSUPPORTED;
+    if (e.rope.cos_t && (t.bn != 128 || t.slices != 1 || N % 128 || c.acc || e.bias || e.gate_up || (N / ws_num) % 128)) return VLAB200_ERR_UNSUPPORTED;
     if (t.bn == 256) return launch_gemm_pair(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, e, st);
     if (t.bn == 64) return launch_gemm_tc<64>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, e, t.slices, st);
     return launch_gemm_tc<128>(A, W, out, c.acc, c.s, c.ws, ws_num, M, N, K, e, t.slices, st);
@@ -1099,7 +1096,7 @@ bool ternary_can_rope(int M, int N, int K) {
     const int n_sm = sm_count();
     if (M <= 8 || n_sm <= 0 || N % 128) return false;
     const TernTiling t = choose_tiling(M, N, K, false, n_sm);
-    return t.bn >= 128 && t.slices == 1;
+    return t.bn == 128 && t.slices == 1;
 }
 
 static int ternary_linear(const int8_t *A, const uint8_t *W, void *out, int32_t *acc, const float *s, const float *ws, int ws_num, int M, int N,
