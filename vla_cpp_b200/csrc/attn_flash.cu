@@ -971,10 +971,11 @@ static int launch_flash(const vlab200_kv_store *st, int layer, const void *q, vo
     if constexpr (HD >= 128) {
         // CTA pairs once an item has two row tiles and the pairs fill the machine, or where every unit has an SM of its own anyway and its
         // chain of key blocks is what takes the time (a pair walks half as many, with twice the softmax warps: pi0.5 at 33 observations
-        // 19.97 -> 19.25 ms; with one to three blocks of 64 keys it loses: 64 tokens 1.82 -> 1.88 ms); or when forced for tests
+        // 19.97 -> 19.25 ms; with one to three blocks of 64 keys it loses: 64 tokens 1.82 -> 1.88 ms; heads of 128
+        // gain nothing: 300 tokens of 20 on 5 heads 10.4 us either way); or when forced for tests
         const int n_pair_units = st->n_obs * st->n_kv * ((p.n_mt + 1) / 2), pairs = n_sm / 2;
         const int forced = dense_gemm_variant();
-        const bool one_wave = p.n_units <= n_sm && p.n_blocks >= 4 && !(ws && !row_major_hd && p.n_units * 2 <= n_sm);
+        const bool one_wave = HD == 256 && p.n_units <= n_sm && p.n_blocks >= 4 && !(ws && !row_major_hd && p.n_units * 2 <= n_sm);
         if (p.n_mt >= 2 && forced != 1 && (forced == 3 || n_pair_units >= pairs || one_wave)) {
             using LP = FlashPairSmem<HD>;
             // each CTA stages 64 of a block's 128 keys (the one-CTA kernel's K map has that box) and, for V, all
