@@ -259,7 +259,8 @@ qkv_rope_kernel(const __grid_constant__ CUtensorMap w_map, const QkvParams p) {
 constexpr int QKVF_THREADS = 448;
 // Shared memory is stages + barriers / statistics + the transposed RoPE table.  The products wait for their operands (a k step takes 0.75 us
 // with four stages of 32 KB in flight per SM, 0.52 with six), so every byte that is not the table is a stage: rows leave straight from
-// registers.  Through a 32 KB transposition buffer a table of 51 x 256 left four stages instead of five, one of 51 x 64 five instead of six.
+// registers.  Through a 32 KB transposition buffer a table of 51 x 256 left four stages instead of five, one of 51 x 64 five instead of six:
+// 26,112 x 2560 x 1024 165 -> 146 us, 13,056 x 1600 x 720 43 -> 42.
 constexpr int QKVF_AUX = 256 + 1024, QKVF_SMEM = 227 * 1024;
 constexpr int QKVF_TABLE_RESERVE = 32 * 1024;  // tables within this of the largest that fits beside two stages are refused
 
