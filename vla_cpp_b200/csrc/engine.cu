@@ -101,7 +101,7 @@ __device__ __forceinline__ float2 unpair2(uint64_t v) {
 // Columns o, o + 1 of EMB_ROWS input rows of A <= 64 floats: bias[o] + sum_k W[o][k] x[row][k], k in order.  One CTA takes EMB_ROWS rows, kept in
 // shared memory as [k][row], one thread two output columns.  Bound by issue slots: a value of k costs a thread four 16-byte shared
 // loads and sixteen two-wide FMAs for 32 results (25,600 rows x 1024 columns: 140 us with a row at a time, scalar loads and the weights
-// unpacked for every row, 110 us with one column a thread).
+// unpacked for every row, 110 us with one column a thread, 91 with two).
 constexpr int EMB_ROWS = 16, EMB_THREADS = 128;
 __device__ __forceinline__ void embed_stage(float (*sx)[EMB_ROWS], const float *x, int row0, int rows, int A) {
     for (int i = threadIdx.x; i < EMB_ROWS * A; i += blockDim.x) sx[i % A][i / A] = i / A < rows ? x[(size_t)row0 * A + i] : 0.0f;
