@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) norm_quant_kernel(__nv_bfloat16 *__restri
 // owns the 8-element groups t, t + 256, ... (at most NV of them), so K <= 2048 * NV and K % 8 == 0.  Per element the
 // arithmetic is the one of norm_quant_kernel; only the order of the float sum of squares differs.
 // What bounds a row is its chain (load, two block-wide reductions, store: some 3 us), so a CTA walks rows blockIdx.x, + gridDim.x, ... with the
-// next row's loads in flight and the norm's weights kept: 4,800 rows of 6,912 took 34.7 us with a CTA per row (4 resident per SM).
+// next row's loads in flight and the norm's weights kept: 4,800 rows of 6,912 took 34.7 us with a CTA per row (4 resident per SM), 32.1 so.
 constexpr int NQ_BLOCKS(int mode, int nv) { return nv == 2 ? 4 : (mode == NQ_PLAIN ? 3 : 2); }  // CTAs per SM
 template <int MODE, int NV>
 __global__ void __launch_bounds__(256, NQ_BLOCKS(MODE, NV)) norm_quant_vec_kernel(__nv_bfloat16 *in,

@@ -333,7 +333,8 @@ __device__ __forceinline__ void tern_epilogue_tile(uint32_t lane_addr, uint8_t *
         if (e.rope.cos_t) {
             // Heads of 128: 32 columns of a head's first half and the 32 they are rotated with make a row's 128-byte line of the staging area.
             // The rotation works on the rounded projection and rounds again, as rope_split does.  Not for the pair kernel, whose epilogue of a
-            // thousand rows hides behind the next tile's products only as long as it is short.
+            // thousand rows hides behind the next tile's products only as long as it is short: 4,800 x 3840 x 2560 71 us with the rotation
+            // in it, 33 without and 12 for rope_split.
             const TernaryRope &rp = e.rope;
             const float *cs_row = rp.cos_t + (size_t)(min(m, M - 1) % rp.seq) * 64, *sn_row = rp.sin_t + (size_t)(min(m, M - 1) % rp.seq) * 64;
             const int head = n0 / 128;
