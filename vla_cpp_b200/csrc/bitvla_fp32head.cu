@@ -32,7 +32,7 @@ enum { SK_ACT_NONE = 0, SK_ACT_RELU = 1, SK_ACT_GELU_ERF = 2, SK_ACT_SILU = 3 };
 
 // out[m][n] = (residual ? residual[m][n] : 0) + act(bias[n] + sum_k x[m][k] W[n][k]),  m in [m0, m0 + rows)
 __global__ void __launch_bounds__(256) f32_skinny_linear_kernel(const float *__restrict__ W, const float *__restrict__ bias,
-                                                                const float *__restrict__ x, const float *residual, float *out,
+                                                                const float *x, const float *residual, float *out,
                                                                 int m0, int rows, int N, int K, int act) {
     __shared__ __align__(16) float xs[SK_ROWS][SK_KT];
     pdl_launch_dependents();
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256) f32_skinny_linear_kernel(const float *__r
 
 // (x - mean) * rsqrt(var + eps) * w + b over rows of K floats: the mean, then the variance of the centred values
 // (layernorm_fp32_kernel, bitvla_fp32head_cuda.cu:71-117)
-__global__ void __launch_bounds__(256) f32_layernorm_kernel(const float *__restrict__ x, const float *__restrict__ w,
+__global__ void __launch_bounds__(256) f32_layernorm_kernel(const float *x, const float *__restrict__ w,
                                                             const float *__restrict__ b, float *__restrict__ out, float eps, int K) {
     __shared__ float red[8];
     pdl_launch_dependents();

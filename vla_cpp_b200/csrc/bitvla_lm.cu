@@ -76,8 +76,8 @@ __device__ __forceinline__ float block_max_256(float v, float *red) {
 // q = clamp(rne(y * s), -128, 127) (act_quant_kernel, src/kernels/bitvla/bitnet_kernels.h:465-521).
 // The row lives in shared memory as float between the passes (K * 4 bytes).
 template <int MODE>
-__global__ void __launch_bounds__(256) norm_quant_kernel(__nv_bfloat16 *__restrict__ in,
-                                                         const __nv_bfloat16 *__restrict__ add,
+__global__ void __launch_bounds__(256) norm_quant_kernel(__nv_bfloat16 *in,
+                                                         const __nv_bfloat16 *add,
                                                          const __nv_bfloat16 *__restrict__ w, float eps, int K,
                                                          int8_t *__restrict__ q_out, float *__restrict__ s_out,
                                                          __nv_bfloat16 *__restrict__ out_bf) {
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(256, NQ_BLOCKS(MODE, NV)) norm_quant_vec_kerne
 // sequence goes to page row row0 + s.  n_kv_proj == 0: only q heads are present (cross-attention).
 // The rotation is computed in float on bf16 inputs and rounded once, as rope_neox_bf16_kernel
 // (bitvla_lm_cuda.cu:77-99) does after the head split (bitvla_lm_cuda.cu:441-446).
-__global__ void __launch_bounds__(128) rope_split_kernel(const __nv_bfloat16 *__restrict__ qkv,
+__global__ void __launch_bounds__(128) rope_split_kernel(const __nv_bfloat16 *qkv,
                                                          const float *__restrict__ cos_t,
                                                          const float *__restrict__ sin_t,
                                                          __nv_bfloat16 *__restrict__ q_out,
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(128) rope_split_kernel(const __nv_bfloat16 *__
 
 // The same with 16-byte accesses: one work item = 8 consecutive elements of a head's first half and the matching
 // 8 of its second half (hd % 16 == 0, 16-byte aligned buffers).
-__global__ void __launch_bounds__(128) rope_split_vec_kernel(const __nv_bfloat16 *__restrict__ qkv,
+__global__ void __launch_bounds__(128) rope_split_vec_kernel(const __nv_bfloat16 *qkv,
                                                              const float *__restrict__ cos_t,
                                                              const float *__restrict__ sin_t,
                                                              __nv_bfloat16 *__restrict__ q_out,

@@ -79,7 +79,7 @@ __device__ __forceinline__ void vit_quant_row(const float *row, float amax, int 
 // bitvla_add_bf16, bitvla_vit_cuda.cu:226-227,246-247).  ln_w == nullptr: only that update.  Otherwise
 // y = bf16((h - mean) * rsqrt(var + eps) * w + b) with the mean and the centred variance of the bf16 row in float
 // (layernorm_bias_bf16_kernel, bitvla_lm_cuda.cu:552-607), then the act-quant of y.
-__global__ void __launch_bounds__(256) vit_ln_quant_kernel(__nv_bfloat16 *__restrict__ h, const __nv_bfloat16 *__restrict__ add,
+__global__ void __launch_bounds__(256) vit_ln_quant_kernel(__nv_bfloat16 *h, const __nv_bfloat16 *add,
                                                            const __nv_bfloat16 *__restrict__ add_bias,
                                                            const __nv_bfloat16 *__restrict__ ln_w,
                                                            const __nv_bfloat16 *__restrict__ ln_b, float eps, int K,
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) vit_ln_quant_kernel(__nv_bfloat16 *__rest
 // qkv [seq][3 H] (q | k | v) + bias -> q [heads][seq][hd_pad], K / V pages [heads][seq][hd_pad], zero past hd.
 // (bitvla_add_bias_bf16 + bitvla_transpose_sNhd_to_NshHd_bf16, bitvla_vit_cuda.cu:185-195)
 // One CTA per token; a thread moves 8 consecutive head-dim elements (16 bytes) at a time when hd % 8 == 0.
-__global__ void __launch_bounds__(256) vit_split_heads_kernel(const __nv_bfloat16 *__restrict__ qkv, const __nv_bfloat16 *__restrict__ bq,
+__global__ void __launch_bounds__(256) vit_split_heads_kernel(const __nv_bfloat16 *qkv, const __nv_bfloat16 *__restrict__ bq,
                                                               const __nv_bfloat16 *__restrict__ bk, const __nv_bfloat16 *__restrict__ bv,
                                                               __nv_bfloat16 *__restrict__ q, __nv_bfloat16 *__restrict__ kp,
                                                               __nv_bfloat16 *__restrict__ vp, int seq, int heads, int hd, int hd_pad) {
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256) vit_split_heads_kernel(const __nv_bfloat1
 
 // attention output [seq][heads * hd_pad] -> the real head_dim columns [seq][H] -> act-quant
 // (bitvla_transpose_NshHd_to_sNhd_bf16 + bitvla_act_quant_cuda, bitvla_vit_cuda.cu:222-223)
-__global__ void __launch_bounds__(256) vit_merge_quant_kernel(const __nv_bfloat16 *__restrict__ att, int heads, int hd, int hd_pad,
+__global__ void __launch_bounds__(256) vit_merge_quant_kernel(const __nv_bfloat16 *att, int heads, int hd, int hd_pad,
                                                               int8_t *__restrict__ q_out, float *__restrict__ s_out) {
     extern __shared__ float row[];
     __shared__ float red[8];
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) vit_merge_quant_kernel(const __nv_bfloat1
 
 // y = bf16(gelu_tanh(bf16(x + bias))) over the real F columns, zero up to F_pad, then act-quant over F_pad
 // (bitvla_add_bias_bf16, gelu_tanh_bf16_kernel bitvla_lm_cuda.cu:610-621, padded copy, bitvla_vit_cuda.cu:233-243)
-__global__ void __launch_bounds__(256) vit_gelu_quant_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ bias,
+__global__ void __launch_bounds__(256) vit_gelu_quant_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *__restrict__ bias,
                                                              int F, int F_pad, int8_t *__restrict__ q_out, float *__restrict__ s_out) {
     extern __shared__ float row[];
     __shared__ float red[8];
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(32 * VIT_LN_WARPS) vit_ln_quant_rows_kernel(__
 
 // Act-quant of a row of K columns into K_pad int8 (zero past K), WARPS warps per row and NV x 8 columns per lane.
 template <int WARPS, int NV>
-__global__ void __launch_bounds__(32 * WARPS) vit_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int K, int K_pad,
+__global__ void __launch_bounds__(32 * WARPS) vit_quant_rows_kernel(const __nv_bfloat16 *x, int K, int K_pad,
                                                                     int8_t *__restrict__ q_out, float *__restrict__ s_out) {
     __shared__ float red[WARPS];
     constexpr int T = 32 * WARPS;

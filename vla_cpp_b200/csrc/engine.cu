@@ -154,7 +154,7 @@ __device__ __forceinline__ void embed_columns(const float (*sx)[EMB_ROWS], const
 }
 
 // a[row][o] = bf16(b_ain[o] + sum_k W_ain[o][k] x[row][k]) for the n_rows = n_obs*chunk action tokens (H is even)
-__global__ void __launch_bounds__(EMB_THREADS) action_in_kernel(const float *__restrict__ x,
+__global__ void __launch_bounds__(EMB_THREADS) action_in_kernel(const float *x,
                                                                 const __nv_bfloat16 *__restrict__ w_ain,
                                                                 const float *__restrict__ b_ain, __nv_bfloat16 *__restrict__ a,
                                                                 float *__restrict__ a_f32, int n_rows, int H, int A) {
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(EMB_THREADS) action_in_kernel(const float *__r
 
 // Adaptive RMSNorm (build_adarms, src/models/pi05.cpp:208-224): n = x * rsqrt(mean x^2 + eps);
 // y = bf16(n + n * scale[k] + shift[k]); mod = scale | shift | gate, H floats each.  One warp per row.
-__global__ void __launch_bounds__(256) adarms_norm_kernel(const float *__restrict__ x, const float *__restrict__ mod,
+__global__ void __launch_bounds__(256) adarms_norm_kernel(const float *x, const float *__restrict__ mod,
                                                           __nv_bfloat16 *__restrict__ y, int M, int H, float eps) {
     pdl_launch_dependents();
     pdl_wait();
@@ -243,7 +243,7 @@ static int adarms_norm(const float *x, const float *mod, __nv_bfloat16 *y, int M
 }
 
 // pi0: the state token (row 0 of each observation) of h / hb = W_sp state + b_sp.
-__global__ void __launch_bounds__(EMB_THREADS) state_token_kernel(const float *__restrict__ state,
+__global__ void __launch_bounds__(EMB_THREADS) state_token_kernel(const float *state,
                                                                   const __nv_bfloat16 *__restrict__ w_sp,
                                                                   const float *__restrict__ b_sp, float *__restrict__ h,
                                                                   __nv_bfloat16 *__restrict__ hb, int n_obs, int H, int sd, int S) {
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(EMB_THREADS) state_token_kernel(const float *_
 }
 
 // x[obs][t][a] += dt * v[obs*S + (S - chunk) + t][a]   (v from the head GEMM, row stride A)
-__global__ void euler_kernel(float *__restrict__ x, const float *__restrict__ v, int n, int A, int chunk, int S,
+__global__ void euler_kernel(float *x, const float *v, int n, int A, int chunk, int S,
                              float dt) {
     pdl_launch_dependents();
     pdl_wait();

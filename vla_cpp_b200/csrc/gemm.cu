@@ -360,9 +360,9 @@ dense_gemm_pair_splitk_kernel(const __grid_constant__ CUtensorMap a_map, const _
 }
 
 // h[m][n] += (sum over the K slices, in slice order) (* colscale[n]) (+ bias[n]); hb = bf16(h).  Four columns per thread.
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ partial, int ksplit, int M, int N,
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *partial, int ksplit, int M, int N,
                                                             const float *__restrict__ colscale, const float *__restrict__ bias,
-                                                            float *__restrict__ h, __nv_bfloat16 *__restrict__ hb, int ld) {
+                                                            float *h, __nv_bfloat16 *__restrict__ hb, int ld) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t total4 = (size_t)M * N / 4;

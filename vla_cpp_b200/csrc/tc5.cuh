@@ -32,8 +32,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 // visible, so everything before it (barrier set-up, TMEM allocation, descriptor prefetch) overlaps the
 // predecessor's tail.  pdl_launch_dependents() lets the successor start launching; it never relaxes what
 // the successor's own pdl_wait() waits for.  Both are no-ops for a kernel launched the ordinary way.
-// A kernel that reads weights ahead of the wait takes what the predecessor writes through pointers without __restrict__: loads through
-// const __restrict__ ones count as invariant, and the compiler may move those across the wait too.
+// What the predecessor writes is taken through pointers without __restrict__ and without __ldg, in every kernel that waits: loads through
+// __restrict__ pointers that the kernel does not write count as invariant, and the compiler may move them ahead of the wait.
+// Only weights and tables, complete before the chain began, keep it (tests/test_dependent_launch_sources.py).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

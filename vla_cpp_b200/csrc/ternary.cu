@@ -125,11 +125,11 @@ __device__ __forceinline__ float ternary_scale_out(int acc, float s, float ws) {
 // SM, not the bandwidth, set the time.
 constexpr int GEMV_WARPS = 8, GEMV_THREADS = GEMV_WARPS * 32;
 template <int MT>
-__global__ void __launch_bounds__(GEMV_THREADS) ternary_gemv_kernel(const int8_t *__restrict__ A,
+__global__ void __launch_bounds__(GEMV_THREADS) ternary_gemv_kernel(const int8_t *A,
                                                            const uint8_t *__restrict__ Wp,
                                                            __nv_bfloat16 *__restrict__ out,
                                                            int32_t *__restrict__ acc_out,
-                                                           const float *__restrict__ s,
+                                                           const float *s,
                                                            const float *__restrict__ ws, int ws_num, int M, int N,
                                                            int K, int m0) {
     extern __shared__ __align__(16) uint8_t gemv_smem[];
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) ternary_gemv_kernel(const int8_t
     for (int i = tid; i < MT * (K >> 4); i += GEMV_THREADS) {
         const int mm = i / (K >> 4), kk = i % (K >> 4);
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (mm < rows_here) v = __ldg(reinterpret_cast<const uint4 *>(A + (size_t)(m0 + mm) * K) + kk);
+        if (mm < rows_here) v = reinterpret_cast<const uint4 *>(A + (size_t)(m0 + mm) * K)[kk];
         reinterpret_cast<uint4 *>(As + (size_t)mm * K)[kk] = v;
     }
     __syncthreads();
@@ -455,7 +455,7 @@ template <int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t *__restrict__ Wp,
                        __nv_bfloat16 *__restrict__ out, int32_t *__restrict__ acc_out,
-                       const float *__restrict__ s, const float *__restrict__ ws, int ws_num, int M, int N, int K,
+                       const float *s, const float *__restrict__ ws, int ws_num, int M, int N, int K,
                        int tiles_m, int tiles_n, int slices, const TernEpi e, int *status) {
     using L = GemmSmem<BN>;
     extern __shared__ uint8_t gemm_smem_raw[];
@@ -743,7 +743,7 @@ struct PairSmem {
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t *__restrict__ Wp,
                          __nv_bfloat16 *__restrict__ out, int32_t *__restrict__ acc_out,
-                         const float *__restrict__ s, const float *__restrict__ ws, int ws_num, int M, int N, int K,
+                         const float *s, const float *__restrict__ ws, int ws_num, int M, int N, int K,
                          int tiles_mp, int tiles_n, const TernEpi e, int *status) {
     using L = PairSmem;
     constexpr int BN = 256;
