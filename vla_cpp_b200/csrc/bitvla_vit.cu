@@ -386,7 +386,7 @@ __global__ void vit_bf16_to_f32_kernel(const __nv_bfloat16 *__restrict__ src, fl
 
 struct VitLayer {
     bitvla_vit_layer_cuda w{};
-    DevBuf qkv_packed, qkv_ws, qkv_b;
+    DevBuf qkv_packed, qkv_ws;
     bool set = false;
 };
 
@@ -446,7 +446,6 @@ bitvla_vit_cuda_ctx *bitvla_vit_cuda_init(int n_layers, int hidden, int n_heads,
     for (int l = 0; l < n_layers && !rc; ++l) {
         rc = c->layers[(size_t)l].qkv_packed.alloc(3 * H * H / 4);
         if (!rc) rc = c->layers[(size_t)l].qkv_ws.alloc(3 * sizeof(float));
-        if (!rc) rc = c->layers[(size_t)l].qkv_b.alloc(3 * H * 2);
     }
     if (rc) {
         delete c;
@@ -469,13 +468,10 @@ void bitvla_vit_cuda_set_layer(bitvla_vit_cuda_ctx *ctx, int L, const bitvla_vit
     const size_t bytes = (size_t)ctx->hidden * ctx->hidden / 4;
     const int8_t *packs[3] = {layer->q_packed, layer->k_packed, layer->v_packed};
     const float *wss[3] = {layer->q_ws, layer->k_ws, layer->v_ws};
-    const void *bias[3] = {layer->q_b, layer->k_b, layer->v_b};
-    const size_t bias_bytes = (size_t)ctx->hidden * 2;
     bool ok = true;
     for (int j = 0; j < 3; ++j) {
         ok = ok && cudaMemcpy(static_cast<char *>(dst.qkv_packed.p) + j * bytes, packs[j], bytes, cudaMemcpyDeviceToDevice) == cudaSuccess;
         ok = ok && cudaMemcpy(dst.qkv_ws.as<float>() + j, wss[j], sizeof(float), cudaMemcpyDeviceToDevice) == cudaSuccess;
-        ok = ok && cudaMemcpy(static_cast<char *>(dst.qkv_b.p) + j * bias_bytes, bias[j], bias_bytes, cudaMemcpyDeviceToDevice) == cudaSuccess;
     }
     if (!ok) {
         vb::cuda_fail(cudaGetLastError(), "bitvla_vit_cuda_set_layer");
@@ -551,10 +547,11 @@ int bitvla_vit_cuda_forward(bitvla_vit_cuda_ctx *ctx, const void *d_patches, voi
     for (const vb::VitLayer &l : ctx->layers)
         for (const void *p : {l.w.ln1_w, l.w.ln1_b, l.w.ln2_w, l.w.ln2_b, l.w.o_b, l.w.fc2_b}) fast = fast && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
     // weights were complete before the embedding kernels above started: the layers' kernels read them ahead of the kernel in front
-    auto ternary = [&](const int8_t *a, const void *wp, const float *ws, int ws_num, void *out, int N, int K, const void *bias, int gelu) {
+    auto ternary = [&](const int8_t *a, const void *wp, const float *ws, int ws_num, void *out, int N, int K, const void *bias, int gelu,
+                       const void *bias_2 = nullptr, const void *bias_3 = nullptr) {
         vb::TernaryCall c{};
         c.A = a; c.W = static_cast<const uint8_t *>(wp); c.out = out; c.s = s; c.ws = ws; c.ws_num = ws_num; c.M = S; c.N = N; c.K = K;
-        c.bias = bias; c.gelu = gelu; c.w_early = 1;
+        c.bias = bias; c.bias_2 = bias_2; c.bias_3 = bias_3; c.gelu = gelu; c.w_early = 1;
         return vb::ternary_linear(c, cs);
     };
     for (int L = 0; fast && L < ctx->n_layers; ++L) {
@@ -565,7 +562,8 @@ int bitvla_vit_cuda_forward(bitvla_vit_cuda_ctx *ctx, const void *d_patches, voi
                                   ctx->ln_eps, H, a8, s);
         };
         if ((rc = ln(pend, pend_bias, w.ln1_w, w.ln1_b))) return fail("ln1", rc);
-        if ((rc = ternary(a8, lr.qkv_packed.p, lr.qkv_ws.as<float>(), 3, ctx->qkv.p, 3 * H, H, lr.qkv_b.p, 0))) return fail("qkv projection", rc);
+        if ((rc = ternary(a8, lr.qkv_packed.p, lr.qkv_ws.as<float>(), 3, ctx->qkv.p, 3 * H, H, w.q_b, 0, w.k_b, w.v_b)))
+            return fail("qkv projection", rc);
         // the attention reads q, k and v as column ranges of the projection and leaves packed heads: no head split, no merge
         __nv_bfloat16 *qkv = ctx->qkv.as<__nv_bfloat16>();
         vlab200_kv_store view{qkv + H, qkv + 2 * H, 1, 1, heads, hp, S, 0};

@@ -126,6 +126,7 @@ struct TernaryCall {
     const float *s, *ws;
     int ws_num, M, N, K, path;
     const void *bias;  // bf16 [N], added to the rounded result and rounded again (bitvla_add_bias_bf16), or nullptr
+    const void *bias_2, *bias_3;  // q | k | v: bf16 [N / 3] each of `bias` and these for a third of the columns; nullptr otherwise
     int gelu;          // tanh-GELU behind the bias
     int gate_up;       // out [M][N / 2] = relu(column n)^2 * column N / 2 + n
     TernaryRope rope;

@@ -251,10 +251,15 @@ constexpr int GEMM_THREADS = 448;
 // What the epilogue does behind bf16(acc * ws / s): nothing, [+ bias, rounded] [tanh-GELU, rounded], or with gate_up
 // relu(gate)^2 * up of columns n and N / 2 + n (the output then has N / 2 columns).
 struct TernEpi {
-    const __nv_bfloat16 *bias;
-    int gelu, gate_up, w_early;
+    const __nv_bfloat16 *bias, *bias_2, *bias_3;  // of columns [0, split), [split, 2 split) and the rest, each indexed by the column
+    int split, gelu, gate_up, w_early;
     TernaryRope rope;
 };
+
+__device__ __forceinline__ float tern_bias(const TernEpi &e, int n, int N) {
+    const __nv_bfloat16 *b = n < e.split ? e.bias : (n < 2 * e.split ? e.bias_2 : e.bias_3);
+    return n < N ? __bfloat162float(b[n]) : 0.0f;
+}
 
 // tanh.approx: what the reference's tanhf becomes under its --use_fast_math build
 __device__ __forceinline__ float gelu_tanh_fast(float v) {
@@ -634,7 +639,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
             const int m_first = (tile % tiles_m) * GEMM_BM + q * 32, n0 = (tile / tiles_m) * cols_tile;
             const float sm = (m_first + lane < M) ? s[m_first + lane] : 1.0f;
             if (bias) {
-                for (int c = lane; c < BN; c += 32) bias[c] = n0 + c < N ? __bfloat162float(e.bias[n0 + c]) : 0.0f;
+                for (int c = lane; c < BN; c += 32) bias[c] = tern_bias(e, n0 + c, N);
                 __syncwarp();
             }
             ok = mbar_wait(&accum_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM);
@@ -662,7 +667,7 @@ ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_t 
         if (epi) {
             if (m < M) sm = s[m];
             if (bias) {
-                for (int c = lane; c < width; c += 32) bias[c] = n0 + c < N ? __bfloat162float(e.bias[n0 + c]) : 0.0f;
+                for (int c = lane; c < width; c += 32) bias[c] = tern_bias(e, n0 + c, N);
                 __syncwarp();
             }
             ok = mbar_wait(&accum_full[0], 0u, wc, DEV_TIMEOUT_ACCUM);
@@ -925,7 +930,7 @@ ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap a_map, const uint8_
             const int m0 = (tile % tiles_mp) * 256 + (int)rank * 128, m_first = m0 + q * 32, n0 = (tile / tiles_mp) * (e.gate_up ? BN / 2 : BN);
             const float sm = (m_first + lane < M) ? s[m_first + lane] : 1.0f;
             if (bias) {
-                for (int c = lane; c < BN; c += 32) bias[c] = n0 + c < N ? __bfloat162float(e.bias[n0 + c]) : 0.0f;
+                for (int c = lane; c < BN; c += 32) bias[c] = tern_bias(e, n0 + c, N);
                 __syncwarp();
             }
             ok = mbar_wait_backoff(&accum_full[buf], (j >> 1) & 1u, wc, DEV_TIMEOUT_ACCUM, 256);
@@ -1060,7 +1065,14 @@ int ternary_linear(const TernaryCall &c, cudaStream_t st) {
     if (rc) return rc;
     if (M == 0) return VLAB200_OK;
     const bool gemv = path == 1 || (path == 0 && M <= 8);
-    const TernEpi e{static_cast<const __nv_bfloat16 *>(c.bias), c.gelu, c.gate_up, c.w_early, c.rope};
+    TernEpi e{};
+    e.bias = e.bias_2 = e.bias_3 = static_cast<const __nv_bfloat16 *>(c.bias);
+    e.split = N; e.gelu = c.gelu; e.gate_up = c.gate_up; e.w_early = c.w_early; e.rope = c.rope;
+    if (c.bias_2) {
+        e.split = N / 3;
+        e.bias_2 = static_cast<const __nv_bfloat16 *>(c.bias_2) - e.split;
+        e.bias_3 = static_cast<const __nv_bfloat16 *>(c.bias_3) - 2 * e.split;
+    }
     if (gemv) {
         if (e.bias || e.gelu || e.gate_up || e.rope.cos_t) return VLAB200_ERR_UNSUPPORTED;
         if ((size_t)8 * K + 4 * 8 * 16 * sizeof(int) > 200 * 1024) return VLAB200_ERR_UNSUPPORTED;
