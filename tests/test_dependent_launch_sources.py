@@ -14,6 +14,7 @@ INVARIANT = {  # kernel -> weights, biases, modulations, rotation tables
     "adarms_norm_kernel": {"mod"}, "adarms_norm_vec_kernel": {"mod"}, "action_in_kernel": {"w_ain", "b_ain"}, "state_token_kernel": {"w_sp", "b_sp"},
     "euler_kernel": set(), "splitk_reduce_kernel": {"colscale", "bias"}, "f32_skinny_linear_kernel": {"W", "bias"}, "f32_layernorm_kernel": {"w", "b"},
     "norm_quant_kernel": {"w"}, "norm_quant_vec_kernel": {"w"}, "rope_split_kernel": {"cos_t", "sin_t"}, "rope_split_vec_kernel": {"cos_t", "sin_t"},
+    "rope_split_f32_kernel": {"cos_t", "sin_t"},
     "vit_ln_quant_kernel": {"add_bias", "ln_w", "ln_b"}, "vit_ln_quant_rows_kernel": {"add_bias", "ln_w", "ln_b"},
     "vit_split_heads_kernel": {"bq", "bk", "bv"}, "vit_merge_quant_kernel": set(), "vit_gelu_quant_kernel": {"bias"}, "vit_quant_rows_kernel": set(),
     "ternary_gemv_kernel": {"Wp", "ws"}, "ternary_gemm_tc_kernel": {"Wp", "ws"}, "ternary_gemm_pair_kernel": {"Wp", "ws"},

@@ -134,3 +134,39 @@ def test_prefill_long_k_in_slices_of_pair_tiles(oracle):
                             vlm_dims=(2, 1064, 4, 1, 64, 12288),
                             expert_kw=dict(H=128, inter=256, chunk=10, A=32, sd=32, T=1), act=2, check_denoise=False)
     print(f"long-K prefill: worst K/V rel_l2 {w:.3e}")
+
+
+def test_more_rows_than_one_kernel_takes(oracle):
+    """6 prompts of 200 rows: the projection and its rotation in two kernels."""
+    w, o = run_prefill_case(oracle, 6, model=0, n_obs=6, P=200, pos=None, mask_mode=0, pad=None, vlm_dims=(3, 256, 4, 2, 64, 512),
+                            expert_kw=dict(H=128, inter=256, chunk=10, A=32, sd=32, T=2), act=2)
+    print(f"1,200-row prefill: worst K/V rel_l2 {w:.3e}, chunk rel_l2 {o:.3e}")
+
+
+@pytest.mark.parametrize("n_kv,hd", [(2, 64), (1, 128), (1, 256)])
+def test_a_prompt_alone_and_among_others(oracle, n_kv, hd):
+    """The first layer's K and V (products and row sums in one order whatever the tiling, one rounding behind the rotation) are the same bits
+    in a call of one prompt and in one of more than 1,024 rows."""
+    torch = require_cuda()
+    import vla_cpp_b200 as vb
+
+    n_obs, P, hidden, n_q = 6, 200, 264, 4
+    rng = np.random.default_rng(hd)
+    cfg, per, glob, _ = make_policy(oracle, rng, P=P, model=0, L=2, H=128, n_q=n_q, n_kv=n_kv, hd=hd, inter=256, chunk=10, A=32, sd=32, T=1)
+    bf = lambda a: bits_to_bf16_tensor(oracle.f32_to_bf16_bits(a))
+    weights = {k: [bf(a) if k.startswith("w") else to_dev(a) for a in v] for k, v in per.items()}
+    weights.update({k: (bf(a) if k.startswith("w_") else to_dev(a)) for k, v in glob.items() for a in [v]})
+    eng = vb.PolicyEngine(cfg, weights, max_obs=n_obs, prefix_len=P)
+    layers = make_vlm(oracle, rng, 2, hidden, n_q, n_kv, hd, 512)
+    pw = {k: [bf(lw[k]) if k.startswith("w") else to_dev(lw[k]) for lw in layers]
+          for k in ("wq", "wk", "wv", "wo", "wgate", "wup", "wdown", "ln_in", "ln_post")}
+    pre = vb.Prefill(dict(n_layers=2, hidden=hidden, n_q=n_q, n_kv=n_kv, head_dim=hd, inter=512, act=2, rms_eps=1e-6, rope_base=10000.0), pw,
+                     max_obs=n_obs, max_prefix=P)
+    x = torch.randn((n_obs, P, hidden), device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    pre.run(eng, x)
+    k_all, v_all = (t.clone() for t in eng.get_prefix(0, n_kv, hd, n_obs=n_obs))
+    for b in (0, 3, 5):
+        pre.run(eng, x[b:b + 1].contiguous())
+        k, v = eng.get_prefix(0, n_kv, hd, n_obs=1)
+        assert torch.equal(v[0], v_all[b]) and torch.equal(k[0], k_all[b]), b
+    assert vb.device_status() == 0

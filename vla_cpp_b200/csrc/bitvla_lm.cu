@@ -341,6 +341,62 @@ int rope_split(const void *qkv, const float *cos_t, const float *sin_t, void *q_
                       static_cast<__nv_bfloat16 *>(v_pages), seq, n_q, n_kv_proj, n_kv_store, hd, cap, row0);
 }
 
+// The same of a projection kept in float32, rounded once behind the rotation.  Written out as fmaf in the form that the compiler gives the
+// epilogue of gemm_rows_kernel, so that a row has the same bits from either (it may round either product of a sum first).
+__global__ void __launch_bounds__(128) rope_split_f32_kernel(const float *qkv, const float *__restrict__ cos_t, const float *__restrict__ sin_t,
+                                                             __nv_bfloat16 *__restrict__ q_out, __nv_bfloat16 *__restrict__ k_pages,
+                                                             __nv_bfloat16 *__restrict__ v_pages, int seq, int n_q, int n_kv, int hd, int cap) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int sq = blockIdx.x / seq, s = blockIdx.x % seq, half = hd >> 1, h8 = half >> 3, n_heads = n_q + 2 * n_kv;
+    const float *src = qkv + (size_t)blockIdx.x * n_heads * hd;
+    for (int i = threadIdx.x; i < n_heads * h8; i += blockDim.x) {
+        const int head = i / h8, k = (i % h8) * 8;
+        const bool rot = head < n_q + n_kv;
+        const float4 *lp = reinterpret_cast<const float4 *>(src + (size_t)head * hd + k), *hp = reinterpret_cast<const float4 *>(src + (size_t)head * hd + half + k);
+        const float4 *cp = reinterpret_cast<const float4 *>(cos_t + (size_t)s * half + k), *sp = reinterpret_cast<const float4 *>(sin_t + (size_t)s * half + k);
+        float4 lo[2], hi[2], c[2], sn[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            lo[e] = lp[e];
+            hi[e] = hp[e];
+            c[e] = __ldg(cp + e);
+            sn[e] = __ldg(sp + e);
+        }
+        uint32_t wl[4], wh[4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float x[4] = {lo[e].x, lo[e].y, lo[e].z, lo[e].w}, y[4] = {hi[e].x, hi[e].y, hi[e].z, hi[e].w};
+            const float cv[4] = {c[e].x, c[e].y, c[e].z, c[e].w}, sv[4] = {sn[e].x, sn[e].y, sn[e].z, sn[e].w};
+            float l[4], h[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                l[t] = rot ? fmaf(x[t], cv[t], -__fmul_rn(y[t], sv[t])) : x[t];
+                h[t] = rot ? fmaf(y[t], cv[t], __fmul_rn(x[t], sv[t])) : y[t];
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const __nv_bfloat162 l2 = __floats2bfloat162_rn(l[2 * t], l[2 * t + 1]), h2 = __floats2bfloat162_rn(h[2 * t], h[2 * t + 1]);
+                wl[2 * e + t] = *reinterpret_cast<const uint32_t *>(&l2);
+                wh[2 * e + t] = *reinterpret_cast<const uint32_t *>(&h2);
+            }
+        }
+        __nv_bfloat16 *dst = head < n_q ? q_out + (((size_t)sq * n_q + head) * seq + s) * hd
+                                        : (rot ? k_pages + (((size_t)sq * n_kv + (head - n_q)) * cap + s) * hd
+                                               : v_pages + (((size_t)sq * n_kv + (head - n_q - n_kv)) * cap + s) * hd);
+        *reinterpret_cast<uint4 *>(dst + k) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+        *reinterpret_cast<uint4 *>(dst + half + k) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+    }
+}
+
+int rope_split_f32(const float *qkv, const RopeParams &r, int M, cudaStream_t st) {
+    for (const void *p : {static_cast<const void *>(qkv), static_cast<const void *>(r.cos_t), static_cast<const void *>(r.sin_t), static_cast<const void *>(r.q_out),
+                          static_cast<const void *>(r.k_pages), static_cast<const void *>(r.v_pages)})
+        if (r.hd % 16 || (reinterpret_cast<uintptr_t>(p) & 15)) return VLAB200_ERR_UNSUPPORTED;
+    return launch_pdl(rope_split_f32_kernel, dim3(M), dim3(128), 0, st, qkv, r.cos_t, r.sin_t, r.q_out, r.k_pages, r.v_pages, r.seq, r.n_q, r.n_kv_proj, r.hd,
+                      r.cap);
+}
+
 static int gcd_int(int a, int b) {
     while (b) {
         const int t = a % b;

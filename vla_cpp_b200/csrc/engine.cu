@@ -1021,7 +1021,7 @@ vlab200_prefill *vlab200_prefill_create(const vlab200_prefill_config *cfg, const
     const size_t M = (size_t)max_obs * max_prefix;
     if (!rc) rc = p->h.alloc(M * H * 4);
     if (!rc) rc = p->hb.alloc(M * H * 2);
-    if (!rc) rc = p->qkv.alloc(M * (size_t)(qf + 2 * kvf) * 2);
+    if (!rc && M > (size_t)vb::kSplitRows) rc = p->qkv.alloc(M * (size_t)(qf + 2 * kvf) * 4);
     if (!rc) rc = p->q.alloc(M * qf * 2);
     if (!rc) rc = p->att.alloc(M * qf * 2);
     if (!rc) rc = p->g.alloc(M * I * 2);
@@ -1069,18 +1069,21 @@ int32_t vlab200_prefill_run(vlab200_prefill *p, vlab200_engine *e, int32_t obs0,
     for (int l = 0; l < c.n_layers; ++l) {
         const size_t page_off = ((size_t)l * e->max_obs + obs0) * c.n_kv * e->cap * hd;
         __nv_bfloat16 *kp = e->k_pages.as<__nv_bfloat16>() + page_off, *vp = e->v_pages.as<__nv_bfloat16>() + page_off;
-        {   // RMSNorm (factor in the epilogue, weight folded) + q | k | v, then rotation and the page write
+        // RMSNorm (factor in the epilogue, weight folded) + q | k | v, rotation and the page write: in one kernel of 64-column tiles for some
+        // hundred rows.  Beyond, wider tiles and the rotation in a kernel of its own, from a float32 projection, so that a prompt's q and k
+        // are rounded once whatever the number of prompts in a call (from a bf16 one, which rounds them twice, 8 and 32 prompts of SmolVLA
+        // take 1,183 and 2,521 us, so 1,199 and 2,505; 8 of pi0 23.4 and 23.7 ms).
+        vb::RopeParams r{};
+        r.cos_t = cos_t; r.sin_t = sin_t; r.q_out = p->q.as<__nv_bfloat16>(); r.k_pages = kp; r.v_pages = vp; r.seq = P;
+        r.n_q = c.n_q; r.n_kv_proj = r.n_kv_store = c.n_kv; r.hd = hd; r.cap = e->cap; r.row0 = 0;
+        if (M <= vb::kSplitRows) {
+            if ((rc = vb::qkv_rope_rows(p->hb.p, p->wqkv[l].p, M, H, true, c.rms_eps, r, cs))) return rc;
+        } else {
             vb::GemmParams g{};
             g.M = M; g.N = qkv_n; g.K = H; g.epi = vb::EPI_BIAS_ACT; g.act = vb::ACT_NONE; g.use_rms = 1; g.eps = c.rms_eps;
-            g.out_bf = p->qkv.as<__nv_bfloat16>(); g.ld_out = qkv_n; g.w_early = 1;
-            vb::RopeParams r{};
-            r.cos_t = cos_t; r.sin_t = sin_t; r.q_out = p->q.as<__nv_bfloat16>(); r.k_pages = kp; r.v_pages = vp; r.seq = P;
-            r.n_q = c.n_q; r.n_kv_proj = r.n_kv_store = c.n_kv; r.hd = hd; r.cap = e->cap; r.row0 = 0;
-            const bool rows = M <= vb::kSplitRows && (reinterpret_cast<uintptr_t>(sin_t) & 31) == 0;
-            if (rows && (rc = vb::qkv_rope_rows(p->hb.p, p->wqkv[l].p, M, H, true, c.rms_eps, r, cs))) return rc;
-            if (!rows && (rc = vb::dense_gemm(p->hb.p, H, p->wqkv[l].p, g, cs))) return rc;
-            if (!rows && (rc = vb::rope_split(p->qkv.p, cos_t, sin_t, p->q.p, kp, vp, M, P, c.n_q, c.n_kv, c.n_kv, hd, e->cap, 0, cs)))
-                return rc;
+            g.out_f32 = p->qkv.as<float>(); g.ld_out = qkv_n; g.w_early = 1;
+            if ((rc = vb::dense_gemm(p->hb.p, H, p->wqkv[l].p, g, cs))) return rc;
+            if ((rc = vb::rope_split_f32(p->qkv.as<float>(), r, M, cs))) return rc;
         }
         if (l + 1 < c.n_layers) {
             vlab200_kv_store view{kp, vp, 1, n_obs, c.n_kv, hd, e->cap, 0};

@@ -444,7 +444,7 @@ static int dense_gemm_one(const void *A, int lda, const void *W, GemmParams p, c
 
 // 256-bit epilogue accesses need every touched row segment on a 32-byte boundary
 static GemmParams with_al32(GemmParams p) {
-    const bool f32_ok = !p.h || ((reinterpret_cast<uintptr_t>(p.h) & 31) == 0 && p.ld_out % 8 == 0);
+    const bool f32_ok = ((reinterpret_cast<uintptr_t>(p.h) | reinterpret_cast<uintptr_t>(p.out_f32)) & 31) == 0 && ((!p.h && !p.out_f32) || p.ld_out % 8 == 0);
     const bool bf_ok = !p.out_bf || ((reinterpret_cast<uintptr_t>(p.out_bf) & 31) == 0 && p.ld_out % 16 == 0);
     p.al32 = (p.rows_in == 0 && f32_ok && bf_ok) ? 1 : 0;
     return p;

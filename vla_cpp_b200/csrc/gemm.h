@@ -47,6 +47,9 @@ int gemm_rows_clusters(int bn, int slices);  // clusters of that many CTAs the d
 // q | k | v of few rows: A [M][K] times W [(n_q + 2 n_kv_proj) hd][K], RMS factor, rotation, head split and page write in one kernel.
 int qkv_rope_rows(const void *A, const void *W, int M, int K, bool use_rms, float eps, const RopeParams &rp, cudaStream_t stream);
 
+// The same of a projection kept in float32 (n_kv_proj == n_kv_store, row0 == 0, hd % 16 == 0, 16-byte aligned buffers); bitvla_lm.cu.
+int rope_split_f32(const float *qkv, const RopeParams &r, int M, cudaStream_t stream);
+
 // NeoX rotation + head split of a fused [M][(n_q + 2 n_kv_proj) hd] bf16 projection into the q buffer
 // [M / seq][n_q][seq][hd] and K / V page rows row0 + s (pages [.][n_kv_store][cap][hd]); bitvla_lm.cu.
 int rope_split(const void *qkv, const float *cos_t, const float *sin_t, void *q_out, void *k_pages, void *v_pages,
