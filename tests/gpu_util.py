@@ -50,3 +50,19 @@ def reference_bitnet_lib():
     if not os.path.exists(p):
         return None
     return C.CDLL(p)
+
+
+def kernels_of(call):
+    """Names of the kernels that call() launches, in order, from the torch profiler's trace; skips the test where there is none."""
+    import torch
+
+    call()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA, torch.profiler.ProfilerActivity.CPU]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in sorted(prof.events(), key=lambda e: e.time_range.start)
+             if e.device_type == torch.autograd.DeviceType.CUDA and not e.name.startswith(("Memcpy", "Memset"))]
+    if not names:
+        pytest.skip("no kernel trace on this device")
+    return names

@@ -1,22 +1,26 @@
-"""The language model's q | k | v product with the rotation in its epilogue (one-CTA tiles of 128 columns at some hundred rows, CTA pairs at more)
-against the separate rotation that few rows take: integer sums and the same roundings, so a sequence gives the same bits alone and in
-a batch.  Sequence lengths that are no multiple of the tile's rows."""
+"""The language model's q | k | v product with the rotation in its epilogue (one-CTA tiles of 128 columns, at some hundred rows) against the
+separate rotation of the other tilings (few rows, CTA pairs): integer sums and the same roundings, so a sequence gives the same bits alone
+and in a batch.  Sequence lengths that are no multiple of the tile's rows.  The kernel trace tells which of the two a call took."""
 import pytest
 
-from tests.gpu_util import require_cuda
+from tests.gpu_util import kernels_of, require_cuda
 
 pytestmark = pytest.mark.gpu
 
-HID, NQ, NKV, HD, FFN = 2560, 20, 5, 128, 6912
+NQ, NKV, HD = 20, 5, 128
 
 
-@pytest.mark.parametrize("n_seq,seq", [(5, 61), (3, 97), (14, 61)])
-def test_a_sequence_alone_and_in_a_batch(n_seq, seq):
+# rotated in the epilogue: at a width of 2560 the pair tiling is estimated alike, at 1280 a tenth above; 854 rows run as pairs
+@pytest.mark.parametrize("n_seq,seq,hidden,ffn,fused", [(5, 61, 2560, 6912, True), (3, 97, 2560, 6912, True), (14, 61, 2560, 6912, False),
+                                                        (5, 61, 1280, 1024, True), (3, 128, 1280, 1024, True)])
+def test_a_sequence_alone_and_in_a_batch(n_seq, seq, hidden, ffn, fused):
     torch = require_cuda()
     import vla_cpp_b200 as vb
 
     g = torch.Generator(device="cuda")
     g.manual_seed(n_seq)
+
+    HID, FFN = hidden, ffn
 
     def tern(n, k):
         c = torch.randint(1, 4, (n * k // 4, 4), device="cuda", generator=g, dtype=torch.uint8)
@@ -38,3 +42,5 @@ def test_a_sequence_alone_and_in_a_batch(n_seq, seq):
     for i in range(n_seq):
         assert torch.equal(lm.forward(x[i:i + 1].contiguous())[0], together[i]), i
     assert vb.device_status() == 0
+    split = [any("rope_split" in k for k in kernels_of(lambda: lm.forward(y))) for y in (x[:1].contiguous(), x)]
+    assert split == [True, not fused], split

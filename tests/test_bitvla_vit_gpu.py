@@ -20,6 +20,7 @@ pytestmark = pytest.mark.gpu
     (384, 32, 256, 40, 1),   # head_dim 12: general kernels
     (1408, 16, 512, 33, 1),  # rows longer than the register kernels hold: general kernels
     (256, 4, 272, 5, 1),     # the GEMV's rows: general kernels
+    (1152, 8, 512, 200, 1), (512, 2, 256, 257, 1),  # head_dim 144 and 256 from 193 patches on: attention on CTA pairs
 ])
 def test_tower_matches_oracle(oracle, hidden, heads, ffn, n_patches, n_layers):
     require_cuda()

@@ -31,6 +31,12 @@ def test_same_bits_as_the_persistent_tilings(m, n, k):
     assert ((got.float() - ref).norm() / ref.norm()).item() < 4e-3  # bf16 rounding of the result: 2^-9 / sqrt(3) is 1.1e-3
 
 
+def test_projection_of_two_tiles_an_sm_matches_oracle(oracle):
+    """16 observations: 280 tiles of 64 columns with row sums of squares, two CTAs an SM; the last row tile of 48 rows."""
+    w, d = run_case(oracle, 90, n_obs=16, P=30, check_obs=[0, 7, 15], model=0, L=1, H=136, n_q=8, n_kv=1, hd=256, inter=512, chunk=50, A=32, sd=32, T=1)
+    assert w < 1e-2 and d < 3e-2, (w, d)
+
+
 @pytest.mark.parametrize("hd,n_obs", [(64, 1), (64, 5), (128, 2), (256, 5)])
 @pytest.mark.parametrize("model", [0, 1])
 def test_few_observations_match_oracle(oracle, monkeypatch, hd, n_obs, model):

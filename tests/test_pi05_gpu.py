@@ -74,6 +74,12 @@ def test_pi05_loop_small(oracle, n_obs, P, kw):
     assert err <= 1e-2, err
 
 
+@pytest.mark.parametrize("n_obs", [17, 33])  # 280 and 520 tiles of 64 columns: two CTAs an SM, and more than those
+def test_pi05_projection_of_more_tiles_than_sms(oracle, n_obs):
+    err = run_pi05(oracle, 60 + n_obs, n_obs, 30, check_obs=[0, n_obs // 2, n_obs - 1], L=1, H=136, n_q=8, n_kv=1, hd=256, inter=2560, chunk=50, A=32, T=1)
+    assert err <= 1e-2, err
+
+
 @pytest.mark.parametrize("n_obs,sigma", [(1, None), (6, 0.02)])
 def test_pi05_loop_full_size(oracle, n_obs, sigma):
     """The expert at its real size, every layer and every Euler step; unit-scale weights and the N(0, 0.02) of the

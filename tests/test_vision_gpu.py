@@ -8,7 +8,7 @@ depth.  The same bar as the prefix K/V."""
 import numpy as np
 import pytest
 
-from tests.gpu_util import bits_to_bf16_tensor, rel_l2, require_cuda, to_dev
+from tests.gpu_util import bits_to_bf16_tensor, kernels_of, rel_l2, require_cuda, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -83,6 +83,31 @@ def test_tower_matches_the_oracle(oracle, name, cfg, n_views, bias):
     assert np.array_equal(got, got_f)
     print(f"vision tower {name}: worst rel_l2 {worst:.3e} over {n_views} views")
     assert worst <= 2e-2, worst
+
+
+@pytest.mark.parametrize("n_views,tiling", [(1, 3), (2, 3), (5, 0)])
+def test_attention_pairs_on_column_ranges(oracle, n_views, tiling):
+    """Heads of 72 read from the q | k | v matrix by the CTA-pair attention kernel: forced, and its own choice from 5 views of 16 heads on."""
+    torch = require_cuda()
+    import vla_cpp_b200 as vb
+
+    cfg = dict(PI0, n_layers=2, inter=536, out_dim=256)
+    rng = np.random.default_rng(n_views)
+    w = make_tower(oracle, rng, cfg)
+    tower = vb.VisionTower(cfg, tower_to_dev(oracle, w), max_views=n_views)
+    u8 = rng.integers(0, 256, (n_views, 224, 224, 3), dtype=np.uint8)
+    px = torch.from_numpy(u8).cuda()
+    vb.set_gemm_tiling(tiling)
+    try:
+        got = tower.run(px).cpu().numpy().reshape(n_views, -1)
+        names = kernels_of(lambda: tower.run(px))
+    finally:
+        vb.set_gemm_tiling(0)
+    assert vb.device_status() == 0
+    for v in range(n_views):
+        err = rel_l2(got[v], oracle.siglip_tower(u8[v], w, cfg).reshape(-1))
+        assert err <= 2e-2, (v, err)
+    assert sum("attn_flash_pair_kernel<128>" in k for k in names) == cfg["n_layers"]
 
 
 def test_tower_rejects_bad_arguments(oracle):
