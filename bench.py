@@ -544,11 +544,12 @@ def measure_bitvla_lm(torch, vb, dev, steps, warmup, n_layers=30):
         ms = e0.elapsed_time(e1) / steps
         if not torch.isfinite(out.float()).all():
             raise SystemExit("non-finite output")
+        # one sequence: q and k are rotated in the product's epilogue; many (CTA pairs) and one token: in a kernel of their own
         rows.append({"n_seq": n_seq, "seq": seq, "ms": ms, "tokens_per_s": n_seq * seq / ms * 1e3,
                      "ternary_tops": 2.0 * macs_per_token * n_seq * seq / ms / 1e9,
-                     "launches": 1 + 9 * n_layers + 1})
+                     "launches": (9 if n_seq == 1 else 10) * n_layers + 1})
     # one token through the 30 layers: every ternary linear takes the packed-weight GEMV path, so the floor is the
-    # 521 MB of packed weights crossing HBM once (launch- and latency-bound in practice: 9 small kernels per layer)
+    # 521 MB of packed weights crossing HBM once (launch- and latency-bound in practice: 10 small kernels per layer)
     x1 = torch.randn((1, 1, hidden), device=dev, generator=g).bfloat16()
     o1 = torch.empty_like(x1)
     for _ in range(warmup):
@@ -571,7 +572,7 @@ def measure_bitvla_lm(torch, vb, dev, steps, warmup, n_layers=30):
                  "frac_of_hbm": packed_bytes / ms1 / 1e6 / hbm_peak, "peak_kind": f"of {hbm_kind}",
                  "ms_cuda_graph": ms1_graph,
                  "frac_of_hbm_cuda_graph": packed_bytes / ms1_graph / 1e6 / hbm_peak if ms1_graph else None,
-                 "launches": 1 + 9 * n_layers + 1}
+                 "launches": 10 * n_layers + 1}
     if vb.device_status() != 0:
         raise SystemExit("device status word reports a kernel failure")
     reference_cuda = time_reference_lm(torch, dev, layers, norm(hidden), hidden, n_q, n_kv, hd, ffn, seq, rows[0]["ms"])
@@ -698,7 +699,7 @@ def measure_bitvla_vit(torch, vb, dev, n_layers=26):
     ours = timed(vb.lib())
     assert vb.device_status() == 0 and bool(torch.isfinite(out.float()).all())
     rec = {"config": f"BitVLA vision tower: {n_layers} ternary ViT layers, hidden {H}, {heads} heads of {H // heads}, MLP {F}, "
-                     f"{S} patches, projector to {M}; one image per call", "ms": ours, "launches": 3 + 10 * n_layers + 3}
+                     f"{S} patches, projector to {M}; one image per call", "ms": ours, "launches": 3 + 9 * n_layers + 3}
     ref = reference_lib("libbitvla_vit_ref.so")
     ref_ms = timed(ref) if ref is not None else None
     if ref_ms:
@@ -1239,17 +1240,19 @@ def oracle_predict_seconds(orc, d, arch, n_views):
 
 
 def predict_launches(d, arch):
-    """Kernels of one request, counted from the host code: tower (patchify, stream init, patch GEMM; 8 per layer;
-    post-LayerNorm, connector, pi0's scale), prefix embeddings, prefill (tables, 2 per layer for q|k|v + rotation, 4 more
-    on every layer but the last, 4 for the K/V projection of a cross-attention layer), denoise loop (one persistent kernel;
-    VLAB200_CHUNK_LOOP=0: the few-row path, a launch per operator)."""
+    """Kernels of one request, counted from the host code: tower (patchify, stream init, patch GEMM; 7 per layer;
+    post-LayerNorm, connector, pi0's scale), prefix embeddings, prefill (tables, 1 per layer for q|k|v + rotation, 4 more
+    on every layer but the last, there one for the sum of Wdown's K slices at pi0's width, 4 for the K/V projection of a
+    cross-attention layer), denoise loop (one persistent kernel; VLAB200_CHUNK_LOOP=0: a launch per operator)."""
     L = d["n_layers"]
     every = d.get("self_attn_every_n_layers", 0) if arch == "smolvla" else 0
     cross = sum(1 for i in range(L) if every > 1 and i % every != 0)
-    tower = 3 + 8 * d["vit_layers"] + 2 + (0 if arch == "smolvla" else 1)
+    tower = 3 + 7 * d["vit_layers"] + 2 + (0 if arch == "smolvla" else 1)
     embed = 3 if arch == "smolvla" else 2
-    prefill = 2 + 2 * L + 4 * (L - 1) + 4 * cross
-    denoise = d["num_steps"] * ((3 if arch == "smolvla" else 4) + L * 6 + 2) + 2  # pi0: + the state-token kernel; 2 RoPE tables
+    prefill = 2 + L + (4 if arch == "smolvla" else 5) * (L - 1) + 4 * cross
+    # pi0: + the state-token kernel; attention in key slices + their merge where it sees more than 192 keys; 2 RoPE tables
+    per_step = {"smolvla": 3 + L * 6 - cross + 2, "pi0": 4 + L * 6 + 2, "pi05": 1 + L * 8 + 3}[arch]
+    denoise = d["num_steps"] * per_step + 2
     if os.environ.get("VLAB200_CHUNK_LOOP") != "0":
         denoise = 3  # one observation: two rotation tables + the persistent loop kernel
     return tower + embed + prefill + denoise

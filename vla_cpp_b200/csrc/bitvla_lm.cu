@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(128) rope_split_vec_kernel(const __nv_bfloat16
     }
 }
 
-// Host entry for other translation units (the engine's few-row path).
+// Host entry: this stack's pair products, and vision towers whose heads are padded (vision.cu).
 int rope_split(const void *qkv, const float *cos_t, const float *sin_t, void *q_out, void *k_pages, void *v_pages,
                int M, int seq, int n_q, int n_kv_proj, int n_kv_store, int hd, int cap, int row0, cudaStream_t st) {
     auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };

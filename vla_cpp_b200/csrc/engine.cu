@@ -298,8 +298,9 @@ __global__ void pages_to_f32_kernel(const __nv_bfloat16 *__restrict__ pages, flo
 
 constexpr int kFewRows = 256;  // suffix rows (n_obs * S) up to which Wo and Wdown may run as K slices
 // Whether q | k | v runs as 64-column tiles (gemm_rows.cu) instead of the fused kernel's 256-column ones (the same bits from both): while
-// two tiles an SM hold them, without row sums of squares four.  1,650 x 2560 x 1024 (520 tiles) without: 16.3 us against 30.3; with:
-// 3,200 x 960 x 720 (375 tiles) 19.3 against 17.3, 3,200 x 1600 x 720 (625) 28.3 against 22.9.
+// two tiles an SM hold them, without row sums of squares four.  Both lines lie short of the crossings.  The fused kernel's time less this
+// one's, us a layer inside the loop, by tiles an SM: with sums pi0 (K = 1024) 11.6 at 1.9, 5.4 at 2.2, 3.1 at 3.5, 1.1 at 4.1, -0.9 at 4.3,
+// -6 at 5.4; SmolVLA (K = 720) 5.3 at 1.4, 1.1 at 2.2 to 2.7, -0.2 at 3.2; without sums pi0.5 12 at 2.2, 10 at 3.5 to 4.3, 8.6 at 5.1, -1.2 at 6.8.
 static bool rope_in_rows(int M, int n_heads, int hd, bool rms) {
     if (hd % 64) return false;
     if (M <= kFewRows || dense_gemm_variant() != 0) return M <= kFewRows;
@@ -647,6 +648,7 @@ vlab200_engine *vlab200_engine_create(const vlab200_policy_config *cfg, const vl
         vb::set_last_error("vlab200_engine_create: hidden size %d is not a multiple of 8", c.H);
         return nullptr;
     }
+    // (a width within the MLP's: q | k | v needs no room there, but what an engine accepts has not been widened or tested beyond it)
     if (c.model == 2 && (!w->ada_in_w || !w->ada_in_b || !w->ada_post_w || !w->ada_post_b || !w->ada_final_w || !w->ada_final_b ||
                          !w->w_tin || !w->b_tin || !w->w_tout || !w->b_tout || (c.n_q + 2 * c.n_kv) * c.head_dim > c.inter)) {
         vb::set_last_error("vlab200_engine_create: pi0.5 needs the adaptive-norm and time-MLP weights and (n_q + 2 n_kv) head_dim <= inter");

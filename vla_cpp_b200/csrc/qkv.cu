@@ -262,7 +262,9 @@ constexpr int QKVF_THREADS = 448;
 // registers.  Through a 32 KB transposition buffer a table of 51 x 256 left four stages instead of five, one of 51 x 64 five instead of six:
 // 26,112 x 2560 x 1024 165 -> 146 us, 13,056 x 1600 x 720 43 -> 42.
 constexpr int QKVF_AUX = 256 + 1024, QKVF_SMEM = 227 * 1024;
-constexpr int QKVF_TABLE_RESERVE = 32 * 1024;  // tables within this of the largest that fits beside two stages are refused
+// Tables within this of the largest that fits beside two stages are refused: the range of sizes that the callers know, kept as it was when a
+// transposition buffer of that size lay between (larger ones would fit now and are not tested).
+constexpr int QKVF_TABLE_RESERVE = 32 * 1024;
 
 // PAIR: a cluster of two CTAs shares one 256 x 256 tile through tcgen05 cta_group::2; each CTA loads
 // its own 128 rows of x and only half of the weight tile (half the shared-memory bytes per flop).
