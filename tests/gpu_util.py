@@ -53,16 +53,25 @@ def reference_bitnet_lib():
 
 
 def kernels_of(call):
-    """Names of the kernels that call() launches, in order, from the torch profiler's trace; skips the test where there is none."""
+    """Mangled names of the kernels that call() launches, from its capture into a CUDA graph."""
     import torch
+    from cuda.bindings import driver
+
+    def ok(r):
+        assert r[0] == driver.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) == 2 else r[1:]
 
     call()
     torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA, torch.profiler.ProfilerActivity.CPU]) as prof:
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
         call()
-        torch.cuda.synchronize()
-    names = [e.name for e in sorted(prof.events(), key=lambda e: e.time_range.start)
-             if e.device_type == torch.autograd.DeviceType.CUDA and not e.name.startswith(("Memcpy", "Memset"))]
-    if not names:
-        pytest.skip("no kernel trace on this device")
+    graph = driver.CUgraph(g.raw_cuda_graph())
+    nodes, _ = ok(driver.cuGraphGetNodes(graph, ok(driver.cuGraphGetNodes(graph, 0))[1]))
+    names = []
+    for node in nodes:
+        if ok(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            p = ok(driver.cuGraphKernelNodeGetParams(node))
+            names.append(ok(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern)).decode())
+    assert names
     return names

@@ -1,6 +1,6 @@
 """The language model's q | k | v product with the rotation in its epilogue (one-CTA tiles of 128 columns, at some hundred rows) against the
 separate rotation of the other tilings (few rows, CTA pairs): integer sums and the same roundings, so a sequence gives the same bits alone
-and in a batch.  Sequence lengths that are no multiple of the tile's rows.  The kernel trace tells which of the two a call took."""
+and in a batch.  Sequence lengths that are no multiple of the tile's rows.  The captured launches tell which of the two a call took."""
 import pytest
 
 from tests.gpu_util import kernels_of, require_cuda

@@ -39,4 +39,4 @@ def test_those_widths_are_taken(H, width):
     vb.set_gemm_tiling(0)
     assert torch.equal(got, want) and vb.device_status() == 0
     names = kernels_of(lambda: vb.node_mul_mat(w, x))
-    assert any(f"dense_gemm_kernel<{width}>" in k for k in names), names
+    assert any(f"dense_gemm_kernelILi{width}E" in k for k in names), names
